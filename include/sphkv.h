@@ -71,6 +71,38 @@ typedef struct sphkv_tiers {
 int sphkv_rope_table_build(float* table, int32_t max_pos, int32_t dh, const float* inv_freq,
                            void* stream);
 
+/* ---- Page lists -------------------------------------------------------------------
+ * Groups retained tokens into pages on the device: the grouping and sort of
+ * _build_per_head_pages (spherical_kv_pipeline.py:1146-1228) and the pointer table of
+ * pointer_table.py:4-21 for all units at once.  Two calls, because the sizes of the tables
+ * follow from the tiers: sphkv_page_lists_count returns them (it synchronises the stream),
+ * sphkv_page_lists_fill writes every table.  Both take the same struct and scratch. */
+typedef struct sphkv_page_lists_params {
+  const void* tier_assign;  /* [units][T] tier id per token, contiguous; ids that no slot has:
+                               dropped.  elem_size 1 = u8, 4 = i32, 8 = i64             */
+  void* scratch;            /* sphkv_page_lists_scratch_bytes() bytes, 16-aligned; what
+                               _count leaves in it is read by _fill                    */
+  int64_t scratch_bytes;
+  int64_t T;
+  int32_t elem_size, units, Hkv, n_slots;
+  int32_t page_size, radius_fmt, page_align; /* page_align: pages start at its multiples   */
+  int32_t tier_id[SPHKV_MAX_TIER_SLOTS], G[SPHKV_MAX_TIER_SLOTS], bits[SPHKV_MAX_TIER_SLOTS];
+  /* outputs of _fill, all i32; P = n_pages                                             */
+  int32_t n_pages, max_blocks;
+  const int64_t* perm;      /* physical page of each logical page, i64 [P]; NULL = the same */
+  int32_t *positions, *src_index;               /* [P][page_size], -1 = empty           */
+  int32_t *page_head, *page_slot, *page_count;  /* [P]                                  */
+  int32_t* ptable;                              /* [P][3]                               */
+  int32_t *block_table, *bits_table;            /* [units][max_blocks], -1 / 0 past the end */
+  int32_t* num_blocks;                          /* [units]                              */
+  int32_t* bundles;                             /* [n_bundles][8]                       */
+} sphkv_page_lists_params;
+
+int64_t sphkv_page_lists_scratch_bytes(int32_t units, int64_t T, int32_t n_slots);
+/* totals (host, i64 [4]): pages, most blocks of one unit, bundles, bytes of the K pool. */
+int sphkv_page_lists_count(const sphkv_page_lists_params* p, int64_t* totals, void* stream);
+int sphkv_page_lists_fill(const sphkv_page_lists_params* p, void* stream);
+
 /* ---- Encode ----------------------------------------------------------------------
  * Bulk spherical encode + page build.  Replaces _encode_keys_with_codebooks
  * (spherical_kv_pipeline.py:1130-1144) + build_page (pagebuilder.py:8-33) +
@@ -364,8 +396,9 @@ int sphkv_omega_ema(const float* ml, float* omega, int32_t n_units, int32_t kv_g
 /* ---- Library ---------------------------------------------------------------------*/
 int sphkv_abi_version(void);
 const char* sphkv_last_error(void);
-/* sizeof() of sphkv_tiers (0), sphkv_encode_params (1), sphkv_decode_params (2) as this
- * library was compiled; foreign-language bindings compare it with their own layout. */
+/* sizeof() of sphkv_tiers (0), sphkv_encode_params (1), sphkv_decode_params (2),
+ * sphkv_page_lists_params (4) as this library was compiled (-1 for other values); foreign-language
+ * bindings compare it with their own layout. */
 int sphkv_struct_size(int which);
 /* Number of SMs of the current device (grid sizing), or a negative error. */
 int sphkv_sm_count(void);

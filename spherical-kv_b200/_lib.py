@@ -61,6 +61,18 @@ class DecodeParams(C.Structure):
     ]
 
 
+class PageListsParams(C.Structure):
+    _fields_ = [
+        ("tier_assign", C.c_void_p), ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64), ("T", C.c_int64),
+        ("elem_size", C.c_int32), ("units", C.c_int32), ("Hkv", C.c_int32), ("n_slots", C.c_int32),
+        ("page_size", C.c_int32), ("radius_fmt", C.c_int32), ("page_align", C.c_int32),
+        ("tier_id", _I4), ("G", _I4), ("bits", _I4), ("n_pages", C.c_int32), ("max_blocks", C.c_int32),
+        ("perm", C.c_void_p), ("positions", C.c_void_p), ("src_index", C.c_void_p), ("page_head", C.c_void_p),
+        ("page_slot", C.c_void_p), ("page_count", C.c_void_p), ("ptable", C.c_void_p), ("block_table", C.c_void_p),
+        ("bits_table", C.c_void_p), ("num_blocks", C.c_void_p), ("bundles", C.c_void_p),
+    ]
+
+
 # name -> (restype, argtypes); every symbol include/sphkv.h declares
 SIGNATURES = {
     "sphkv_abi_version": (C.c_int, []),
@@ -68,6 +80,9 @@ SIGNATURES = {
     "sphkv_sm_count": (C.c_int, []),
     "sphkv_struct_size": (C.c_int, [C.c_int]),
     "sphkv_rope_table_build": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
+    "sphkv_page_lists_scratch_bytes": (C.c_int64, [C.c_int32, C.c_int64, C.c_int32]),
+    "sphkv_page_lists_count": (C.c_int, [C.POINTER(PageListsParams), C.POINTER(C.c_int64), C.c_void_p]),
+    "sphkv_page_lists_fill": (C.c_int, [C.POINTER(PageListsParams), C.c_void_p]),
     "sphkv_encode_pages": (C.c_int, [C.POINTER(EncodeParams), C.c_void_p]),
     "sphkv_pages_from_codes": (C.c_int, [C.POINTER(EncodeParams), C.c_void_p]),
     "sphkv_encode_codes": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_int32, C.c_int32,
@@ -121,7 +136,7 @@ def load() -> C.CDLL:
     ver = lib.sphkv_abi_version()
     if ver != 4:
         raise SphKVError(f"libsphkv_b200.so ABI version {ver}, expected 4")
-    for which, st in enumerate((Tiers, EncodeParams, DecodeParams)):
+    for which, st in ((0, Tiers), (1, EncodeParams), (2, DecodeParams), (4, PageListsParams)):
         if lib.sphkv_struct_size(which) != C.sizeof(st):
             raise SphKVError(f"struct layout mismatch for {st.__name__}: library "
                              f"{lib.sphkv_struct_size(which)} B, binding {C.sizeof(st)} B")

@@ -65,6 +65,7 @@ extern "C" int sphkv_struct_size(int which) {
     case 0: return (int)sizeof(sphkv_tiers);
     case 1: return (int)sizeof(sphkv_encode_params);
     case 2: return (int)sizeof(sphkv_decode_params);
+    case 4: return (int)sizeof(sphkv_page_lists_params);
     default: return -1;
   }
 }

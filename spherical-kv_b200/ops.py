@@ -49,6 +49,15 @@ def rope_table(max_pos: int, dh: int, base: float = 500000.0, device="cuda",
     return table
 
 
+def _new_cache(lists: PageLists, tiers: TierSet, codebooks: torch.Tensor, dh: int, has_v: bool, v_dtype: torch.dtype,
+               radius_fmt: int, dev) -> PagedCache:
+    """Pools for `lists`: zeroed, except a V pool of which the kernels write every slot (zeros included)."""
+    make = torch.empty if has_v and lists.covers_pool else torch.zeros
+    return PagedCache(tiers=tiers, lists=lists, codebooks=codebooks,
+                      k_pages=torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev),
+                      v_pool=make(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev), radius_fmt=radius_fmt)
+
+
 def encode_pages(k_src: torch.Tensor, v_src: Optional[torch.Tensor], lists: PageLists,
                  codebooks: torch.Tensor, tiers: TierSet, radius_fmt: int = _lib.RADIUS_I8,
                  v_dtype: torch.dtype = torch.float16,
@@ -65,10 +74,7 @@ def encode_pages(k_src: torch.Tensor, v_src: Optional[torch.Tensor], lists: Page
     assert dh == tiers.dh and hkv == lists.Hkv
     dev = k_src.device
     if out is None:
-        k_pages = torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev)
-        v_pool = torch.zeros(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev)
-        out = PagedCache(tiers=tiers, lists=lists, codebooks=codebooks, k_pages=k_pages,
-                         v_pool=v_pool, radius_fmt=radius_fmt)
+        out = _new_cache(lists, tiers, codebooks, dh, v_src is not None, v_dtype, radius_fmt, dev)
     p = _lib.EncodeParams()
     p.k_src, p.v_src = k_src.data_ptr(), _ptr(v_src)
     p.src_index, p.bundles = lists.src_index.data_ptr(), lists.bundles.data_ptr()
@@ -135,10 +141,7 @@ def pages_from_codes(codes: CodeCache, v_src: Optional[torch.Tensor], lists: Pag
     hkv, dh = lists.Hkv, tiers.dh
     dev = codes.r[0].device
     if out is None:
-        k_pages = torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev)
-        v_pool = torch.zeros(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev)
-        out = PagedCache(tiers=tiers, lists=lists, codebooks=codebooks, k_pages=k_pages,
-                         v_pool=v_pool, radius_fmt=radius_fmt)
+        out = _new_cache(lists, tiers, codebooks, dh, v_src is not None, v_dtype, radius_fmt, dev)
     p = _lib.EncodeParams()
     p.v_src = _ptr(v_src)
     p.src_index, p.bundles = lists.src_index.data_ptr(), lists.bundles.data_ptr()

@@ -15,6 +15,7 @@ decode arithmetic lives in the CUDA library.
 """
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
@@ -120,6 +121,52 @@ class PageLists:
     B: int
     Hkv: int
     max_blocks: int
+    covers_pool: bool = False    # every page is in `bundles`: an encode writes every V slot
+
+
+_NATIVE_IDS = (torch.uint8, torch.int32, torch.int64)
+
+
+def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fmt: int, page_align: int,
+                     shuffle_seed: Optional[int], extra_blocks: int) -> PageLists:
+    """build_page_lists in the library: two launches, one read of the four table sizes, one launch (two
+    with a page permutation).  32768 tokens x 8 heads: 1.8 ms as array operations."""
+    B, Hkv, T = ta.shape
+    U, N, S, dev = B * Hkv, page_size, len(tiers), ta.device
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    ta = ta.contiguous()
+    p = _lib.PageListsParams()
+    need = lib.sphkv_page_lists_scratch_bytes(U, T, S)
+    scratch = torch.empty(need, dtype=torch.uint8, device=dev)
+    p.tier_assign, p.scratch, p.scratch_bytes, p.T = ta.data_ptr(), scratch.data_ptr(), need, T
+    p.elem_size, p.units, p.Hkv, p.n_slots = ta.element_size(), U, Hkv, S
+    p.page_size, p.radius_fmt, p.page_align = N, radius_fmt, page_align
+    for s, t in enumerate(tiers.tiers):
+        p.tier_id[s], p.G[s], p.bits[s] = t.tier_id, tiers.dh // t.g, t.b_theta
+    totals = (C.c_int64 * 4)()
+    _lib.check(lib.sphkv_page_lists_count(C.byref(p), totals, st), "sphkv_page_lists_count")
+    P, most, n_bundles, pool_bytes = totals
+    if P == 0:
+        raise ValueError("no retained tokens")
+    if pool_bytes >= 2 ** 31:
+        raise ValueError("byte pool exceeds int32 pointer-table offsets")
+    max_blocks = most + extra_blocks
+    perm = None
+    if shuffle_seed is not None:
+        perm = torch.randperm(P, generator=torch.Generator().manual_seed(shuffle_seed)).to(dev)
+    new = lambda *shape: torch.empty(shape, dtype=torch.int32, device=dev)  # noqa: E731
+    L = PageLists(page_size=N, n_pages=P, positions=new(P, N), src_index=new(P, N), page_head=new(P), page_slot=new(P),
+                  page_count=new(P), ptable=new(P, 3), block_table=new(U, max_blocks), bits_table=new(U, max_blocks),
+                  num_blocks=new(U), bundles=new(n_bundles, 8), pool_bytes=pool_bytes, B=B, Hkv=Hkv,
+                  max_blocks=max_blocks, covers_pool=True)
+    p.n_pages, p.max_blocks = P, max_blocks
+    p.perm = None if perm is None else perm.data_ptr()
+    p.positions, p.src_index = L.positions.data_ptr(), L.src_index.data_ptr()
+    p.page_head, p.page_slot, p.page_count = L.page_head.data_ptr(), L.page_slot.data_ptr(), L.page_count.data_ptr()
+    p.ptable, p.block_table, p.bits_table = L.ptable.data_ptr(), L.block_table.data_ptr(), L.bits_table.data_ptr()
+    p.num_blocks, p.bundles = L.num_blocks.data_ptr(), L.bundles.data_ptr()
+    _lib.check(lib.sphkv_page_lists_fill(C.byref(p), st), "sphkv_page_lists_fill")
+    return L
 
 
 def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
@@ -139,6 +186,12 @@ def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
     dev = tier_assign.device
     B, Hkv, T = tier_assign.shape
     N = page_size
+    # On a GPU the library builds the lists; the array operations below serve host tensors, and the page
+    # sizes and id types that the kernels do not take.
+    if (dev.type == "cuda" and N in (16, 32, 64, 128) and tier_assign.dtype in _NATIVE_IDS and T > 0
+            and 0 < B * Hkv <= 65535 and extra_blocks >= 0):
+        with torch.cuda.device(dev):
+            return _build_on_device(tier_assign, tiers, N, radius_fmt, page_align, shuffle_seed, extra_blocks)
     U = B * Hkv
     rb = 2 if radius_fmt == _lib.RADIUS_F16 else 1
     ppb = 128 // N
@@ -232,7 +285,7 @@ def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
                      page_head=page_head, page_slot=page_slot, page_count=page_count,
                      ptable=ptable.contiguous(), block_table=block_table, bits_table=bits_table,
                      num_blocks=blocks_per_unit.to(torch.int32), bundles=torch.cat(bundle_rows, 0),
-                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks)
+                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks, covers_pool=True)
 
 
 @dataclass
