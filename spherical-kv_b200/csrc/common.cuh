@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "sphkv.h"
 
 // unroll factor of the centroid loops of the similarity searches (independent fma chains in flight)
@@ -59,6 +61,25 @@ inline int check_launch(const char* what) {
     return (int)e;
   }
   return 0;
+}
+
+// Launch with programmatic stream serialization: the grid may become resident while the kernel
+// before it in the stream is still running.  Only for kernels that call griddep_wait() before
+// their first global-memory access.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_overlapped(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t st,
+                                     Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
 }
 
 // ---- tensor-core / async-copy wrappers (inline PTX) ------------------------------
@@ -176,17 +197,56 @@ __device__ __forceinline__ void pool_append_token(
   if (warp >= G) return;
   const int grp = warp;
   const float* k_g = k_post + (int64_t)h * dh + grp * g;
-  float norm_sq = 0.f;
-  for (int d = 0; d < g; ++d) norm_sq += k_g[d] * k_g[d];
-  const float norm = sqrtf(norm_sq + 1e-16f);
-  const float inv_norm = 1.0f / (norm + 1e-8f);
   const float* cb = decode_cb + ((int64_t)h * G * C + (int64_t)grp * C) * g;
-  float best_sim = -1e30f;
+  // issued before the search: the page's running scale is one more memory latency otherwise
+  const float prev_scale = is_new_page ? 0.f : r_scales[pid * G_max + grp];
+  float norm, best_sim = -1e30f;
   int best_code = 0;
-  for (int c = lane; c < C; c += 32) {  // ascending per lane: strict > keeps the lowest index
-    float sim = 0.f;
-    for (int d = 0; d < g; ++d) sim += k_g[d] * inv_norm * cb[(int64_t)c * g + d];
-    if (sim > best_sim) { best_sim = sim; best_code = c; }
+  // The group vector and a lane's centroid rows as 16-byte loads, all in flight at once; element by
+  // element (other group sizes, unaligned rows) each of the g steps waits for its own load.
+  auto search_rows = [&](auto gs) {
+    constexpr int GS = decltype(gs)::value;
+    float k[GS];
+#pragma unroll
+    for (int q = 0; q < GS / 4; ++q) {
+      const float4 v = *reinterpret_cast<const float4*>(k_g + 4 * q);
+      k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+    }
+    float norm_sq = 0.f;
+#pragma unroll
+    for (int d = 0; d < GS; ++d) norm_sq += k[d] * k[d];
+    norm = sqrtf(norm_sq + 1e-16f);
+    const float inv_norm = 1.0f / (norm + 1e-8f);
+#pragma unroll 2
+    for (int c = lane; c < C; c += 32) {  // ascending per lane: strict > keeps the lowest index
+      const float4* row = reinterpret_cast<const float4*>(cb + (int64_t)c * GS);
+      float sim = 0.f;
+#pragma unroll
+      for (int q = 0; q < GS / 4; ++q) {
+        const float4 v = __ldg(row + q);
+        sim += k[4 * q] * inv_norm * v.x;
+        sim += k[4 * q + 1] * inv_norm * v.y;
+        sim += k[4 * q + 2] * inv_norm * v.z;
+        sim += k[4 * q + 3] * inv_norm * v.w;
+      }
+      if (sim > best_sim) { best_sim = sim; best_code = c; }
+    }
+  };
+  if ((g == 16 || g == 32) && ((reinterpret_cast<uintptr_t>(k_g) | reinterpret_cast<uintptr_t>(cb)) & 15) == 0) {
+    if (g == 16)
+      search_rows(std::integral_constant<int, 16>());
+    else
+      search_rows(std::integral_constant<int, 32>());
+  } else {
+    float norm_sq = 0.f;
+    for (int d = 0; d < g; ++d) norm_sq += k_g[d] * k_g[d];
+    norm = sqrtf(norm_sq + 1e-16f);
+    const float inv_norm = 1.0f / (norm + 1e-8f);
+    for (int c = lane; c < C; c += 32) {
+      float sim = 0.f;
+      for (int d = 0; d < g; ++d) sim += k_g[d] * inv_norm * cb[(int64_t)c * g + d];
+      if (sim > best_sim) { best_sim = sim; best_code = c; }
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -195,7 +255,6 @@ __device__ __forceinline__ void pool_append_token(
     if (os > best_sim || (os == best_sim && oc < best_code)) { best_sim = os; best_code = oc; }
   }
   float r_scale;
-  const float prev_scale = is_new_page ? 0.f : r_scales[pid * G_max + grp];
   if (is_new_page || norm > prev_scale) {
     if (!is_new_page) {
       const float ratio = prev_scale / (norm + 1e-8f);

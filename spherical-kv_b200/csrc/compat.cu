@@ -19,12 +19,16 @@ namespace sphkv {
 constexpr int kPoolThreads = 256;
 
 // ---- pool decode: per (KV head, logical page) partial (m, l, acc) for each query head ----
-// The q.centroid table depends only on (query head, tier), not on the page: a CTA builds the
-// tables of ALL tiers of its KV head once, then each of its warps walks pages on its own (no
-// CTA barrier per page): logits through the table, softmax statistics by shuffles, and one
-// pass over the page's V rows that feeds the accumulators of four query heads at a time.
+// The q.centroid table depends only on (query head, tier), not on the page: a CTA builds the tables
+// of the tiers its pages use, then `wpp` warps share a page: each takes page_size / wpp tokens --
+// logits through the table, softmax statistics by shuffles, one pass over its V rows that feeds the
+// accumulators of four query heads at a time -- and the wpp (m, l, acc) triples of the page are
+// folded through shared memory.  wpp is the largest split that leaves a warp 16 tokens, so 128-token
+// pages (33 of them per head at 4K) fill the GPU as 16-token pages do.  Bound: latency of the table
+// build and of the V rows (a 4000-token, 8-head step reads 8 MB).  That step, page kernel: 50 us with a
+// warp walking a whole page, POOL_US us so.
 constexpr int kPoolWarps = kPoolThreads / 32;
-constexpr int kMaxPagesPerWarp = 4;  // fewer when the grid would not fill the GPU
+constexpr int kMaxPageRounds = 4;  // rounds of pages per CTA: amortise the tables once the GPU is full
 
 __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
     const float* __restrict__ q_all, const float* __restrict__ cb_flat,
@@ -33,152 +37,237 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
     const float* __restrict__ r_scales, const __half* __restrict__ v_pool,
     const int* __restrict__ block_table, const int* __restrict__ bits_table,
     float* __restrict__ partial_out, int num_q_heads, int kv_groups, int num_tiers, int max_blocks,
-    int page_size, int dh, int G_max, int cb_max, int g_max, float sm_scale, int pages_per_warp) {
+    int page_size, int dh, int G_max, int cb_max, int g_max, float sm_scale, int wpp, int rounds,
+    int stage_bytes) {
   const int hkv = blockIdx.x, tid = threadIdx.x;
   const int hq0 = hkv * kv_groups;
   const int warp = tid >> 5, lane = tid & 31;
+  const int seg = page_size / wpp;             // tokens of a warp
+  const int at_once = kPoolWarps / wpp;        // pages the CTA works on at a time
+  const int sub = warp % wpp, group = warp / wpp;
 
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* sq = reinterpret_cast<float*>(smem_raw);                 // [kv_groups][dh]
   float* lut = sq + kv_groups * dh;                                // [num_tiers][kv_groups][G_max][cb_max]
-  float* slog_all = lut + num_tiers * kv_groups * G_max * cb_max;  // [warps][kv_groups][page_size]
-  float* srs_all = slog_all + kPoolWarps * kv_groups * page_size;  // [warps][G_max]
-  float* slog = slog_all + warp * kv_groups * page_size;
+  float* slog_all = lut + num_tiers * kv_groups * G_max * cb_max;  // [warps][kv_groups][seg]
+  float* srs_all = slog_all + kPoolWarps * kv_groups * seg;        // [warps][G_max]
+  float* fold_all = srs_all + kPoolWarps * G_max;                  // wpp > 1: [warps][kv_groups][dh + 2]
+  float* slog = slog_all + warp * kv_groups * seg;
   float* srs = srs_all + warp * G_max;
+  // stage_bytes > 0: this warp's tokens of a page -- V rows, centroid indices, radii -- travel to shared
+  // memory asynchronously, the first page's while the tables are built
+  uint8_t* stage = smem_raw + (((fold_all + (wpp > 1 ? kPoolWarps * kv_groups * (dh + 2) : 0)) - sq) * 4 + 15) / 16 * 16 +
+                   warp * stage_bytes;
+  const int v_bytes = seg * dh * 2, c_bytes = seg * G_max;
+  float* fold = fold_all + warp * kv_groups * (dh + 2);
+  __shared__ unsigned s_tiers;
 
+  if (tid == 0) s_tiers = 0;
+  griddep_wait();
+  griddep_launch();
+  const int pg0 = blockIdx.y * at_once * rounds;
+  const int pg_end = min(max_blocks, pg0 + at_once * rounds);
+  auto page_of = [&](int k) -> int {
+    const int page_idx = pg0 + k * at_once + group;
+    return k < rounds && page_idx < max_blocks ? block_table[hkv * max_blocks + page_idx] : -1;
+  };
+  auto issue_stage = [&](int phys) {
+    if (stage_bytes == 0 || phys < 0) return;
+    const int64_t tok0 = (int64_t)phys * page_size + sub * seg;
+    const uint32_t dst = smem_u32(stage);
+    const uint8_t* vs = reinterpret_cast<const uint8_t*>(v_pool + tok0 * dh);
+    for (int i = lane * 16; i < c_bytes; i += 512) {
+      cp_async_16(dst + v_bytes + i, theta_codes + tok0 * G_max + i);
+      cp_async_16(dst + v_bytes + c_bytes + i, radius_codes + tok0 * G_max + i);
+    }
+    for (int i = lane * 16; i < v_bytes; i += 512) cp_async_16(dst + i, vs + i);
+  };
+  int phys_next = page_of(0);
+  issue_stage(phys_next);
   for (int i = tid; i < kv_groups * dh; i += blockDim.x) sq[i] = q_all[(int64_t)hq0 * dh + i];
   __syncthreads();
-  // q . centroid tables of every tier; same summation order as decode_kernel.cu:186-188
+  for (int i = pg0 + tid; i < pg_end; i += blockDim.x)
+    if (block_table[hkv * max_blocks + i] >= 0) atomicOr(&s_tiers, 1u << (bits_table[hkv * max_blocks + i] & 31));
+  __syncthreads();
+  // q . centroid tables; same summation order as decode_kernel.cu:186-188.  A thread dots one centroid
+  // row with every query head, so the row is read once.
+  const unsigned tiers = s_tiers;
+  const bool vec4 = (g_max & 3) == 0 && (dh & 3) == 0 && (reinterpret_cast<uintptr_t>(cb_flat) & 15) == 0;
   for (int ti = 0; ti < num_tiers; ++ti) {
+    if (ti < 32 && !((tiers >> ti) & 1)) continue;
     const int G = tier_G_arr[ti], g = tier_g_arr[ti];
     const float* cb_t = cb_flat + ((int64_t)hkv * num_tiers + ti) * G_max * cb_max * g_max;
-    const bool vec4 = ((g | g_max) & 3) == 0 && (reinterpret_cast<uintptr_t>(cb_flat) & 15) == 0;
     float* lt = lut + (int64_t)ti * kv_groups * G_max * cb_max;
-    for (int i = tid; i < kv_groups * G * cb_max; i += blockDim.x) {
-      const int c = i % cb_max, gg = (i / cb_max) % G, h = i / (cb_max * G);
-      const float* qg = sq + h * dh + gg * g;
+    for (int i = tid; i < G * cb_max; i += blockDim.x) {
+      const int c = i % cb_max, gg = i / cb_max;
       const float* cw = cb_t + ((int64_t)gg * cb_max + c) * g_max;
-      float dot = 0.f;
-      if (vec4) {  // same left-to-right order, 16-byte loads
-        for (int d = 0; d < g; d += 4) {
-          const float4 w4 = __ldg(reinterpret_cast<const float4*>(cw + d));
-          dot += qg[d] * w4.x;
-          dot += qg[d + 1] * w4.y;
-          dot += qg[d + 2] * w4.z;
-          dot += qg[d + 3] * w4.w;
+      if (vec4 && (g == 16 || g == 32)) {
+        float4 w4[8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w4[e] = __ldg(reinterpret_cast<const float4*>(cw) + e);
+        if (g == 32) {
+#pragma unroll
+          for (int e = 4; e < 8; ++e) w4[e] = __ldg(reinterpret_cast<const float4*>(cw) + e);
+        }
+        for (int h = 0; h < kv_groups; ++h) {
+          const float4* qg = reinterpret_cast<const float4*>(sq + h * dh + gg * g);
+          float dot = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (e < 4 || g == 32) {
+              const float4 q4 = qg[e];
+              dot += q4.x * w4[e].x;
+              dot += q4.y * w4[e].y;
+              dot += q4.z * w4[e].z;
+              dot += q4.w * w4[e].w;
+            }
+          }
+          lt[(h * G_max + gg) * cb_max + c] = dot;
         }
       } else {
-        for (int d = 0; d < g; ++d) dot += qg[d] * cw[d];
+        for (int h = 0; h < kv_groups; ++h) {
+          float dot = 0.f;
+          for (int d = 0; d < g; ++d) dot += sq[h * dh + gg * g + d] * cw[d];
+          lt[(h * G_max + gg) * cb_max + c] = dot;
+        }
       }
-      lt[(h * G_max + gg) * cb_max + c] = dot;
     }
   }
   __syncthreads();
 
-  const int pg0 = blockIdx.y * kPoolWarps * pages_per_warp;
-  for (int k = 0; k < pages_per_warp; ++k) {
-    const int page_idx = pg0 + warp + k * kPoolWarps;  // warp-uniform
-    if (page_idx >= max_blocks) break;
-    const int phys = block_table[hkv * max_blocks + page_idx];
-    if (phys < 0) {
+  for (int k = 0; k < rounds; ++k) {
+    const int page_idx = pg0 + k * at_once + group;
+    const int phys = phys_next;
+    phys_next = page_of(k + 1);
+    if (page_idx < max_blocks && phys < 0 && sub == 0) {
       for (int h = 0; h < kv_groups; ++h) {
         float* po = partial_out + ((int64_t)(hq0 + h) * max_blocks + page_idx) * (dh + 2);
         if (lane == 0) { po[0] = -INFINITY; po[1] = 0.f; }
         for (int d = lane; d < dh; d += 32) po[2 + d] = 0.f;
       }
-      continue;
     }
-    const int tier_idx = bits_table[hkv * max_blocks + page_idx];
-    const int G = tier_G_arr[tier_idx];
-    const float* lt = lut + (int64_t)tier_idx * kv_groups * G_max * cb_max;
-    __syncwarp();  // the previous page's readers of slog / srs are done
-    for (int i = lane; i < G_max; i += 32) srs[i] = r_scales[(int64_t)phys * G_max + i];
-    __syncwarp();
-    // logits: lane = (token, query head) pairs.  A byte becomes a float by planting it in the
-    // mantissa of 2^23 (exact, and keeps the conversion off the special-function pipe).
-    const bool words = (G_max & 3) == 0;
-    for (int i = lane; i < page_size * kv_groups; i += 32) {
-      const int t = i % page_size, h = i / page_size;
-      const uint8_t* th = theta_codes + ((int64_t)phys * page_size + t) * G_max;
-      const uint8_t* rc = radius_codes + ((int64_t)phys * page_size + t) * G_max;
-      const float* lh = lt + (int64_t)h * G_max * cb_max;
-      float logit_sum = 0.f;
-      if (words) {
-        for (int g0 = 0; g0 < G; g0 += 4) {
-          const uint32_t tw = __ldg(reinterpret_cast<const uint32_t*>(th + g0));
-          const uint32_t rw = __ldg(reinterpret_cast<const uint32_t*>(rc + g0));
+    if (phys >= 0) {
+      const int tier_idx = bits_table[hkv * max_blocks + page_idx];
+      const int G = tier_G_arr[tier_idx];
+      const float* lt = lut + (int64_t)tier_idx * kv_groups * G_max * cb_max;
+      const int64_t tok0 = (int64_t)phys * page_size + sub * seg;
+      __syncwarp();  // the previous page's readers of slog / srs are done
+      for (int i = lane; i < G_max; i += 32) srs[i] = r_scales[(int64_t)phys * G_max + i];
+      const bool staged = stage_bytes > 0;
+      const uint8_t* th_rows = staged ? stage + v_bytes : theta_codes + tok0 * G_max;
+      const uint8_t* rc_rows = staged ? stage + v_bytes + c_bytes : radius_codes + tok0 * G_max;
+      const __half* v_rows = staged ? reinterpret_cast<const __half*>(stage) : v_pool + tok0 * dh;
+      cp_async_wait<0>();
+      __syncwarp();
+      // logits: lane = (token, query head) pairs.  A byte becomes a float by planting it in the
+      // mantissa of 2^23 (exact, and keeps the conversion off the special-function pipe).
+      const bool words = (G_max & 3) == 0;
+      for (int i = lane; i < seg * kv_groups; i += 32) {
+        const int t = i % seg, h = i / seg;
+        const uint8_t* th = th_rows + t * G_max;
+        const uint8_t* rc = rc_rows + t * G_max;
+        const float* lh = lt + (int64_t)h * G_max * cb_max;
+        float logit_sum = 0.f;
+        if (words) {
+          for (int g0 = 0; g0 < G; g0 += 4) {
+            const uint32_t tw = *reinterpret_cast<const uint32_t*>(th + g0);
+            const uint32_t rw = *reinterpret_cast<const uint32_t*>(rc + g0);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (g0 + e < G) {
-              const float rf = __uint_as_float(0x4B000000u | ((rw >> (8 * e)) & 0xFFu)) - 8388608.0f;
-              const float r_hat = srs[g0 + e] * rf / 255.0f;
-              logit_sum += r_hat * lh[(g0 + e) * cb_max + ((tw >> (8 * e)) & 0xFFu)];
+            for (int e = 0; e < 4; ++e) {
+              if (g0 + e < G) {
+                const float rf = __uint_as_float(0x4B000000u | ((rw >> (8 * e)) & 0xFFu)) - 8388608.0f;
+                const float r_hat = srs[g0 + e] * rf / 255.0f;
+                logit_sum += r_hat * lh[(g0 + e) * cb_max + ((tw >> (8 * e)) & 0xFFu)];
+              }
             }
           }
+        } else {
+          for (int gg = 0; gg < G; ++gg) {
+            const float r_hat = srs[gg] * (float)rc[gg] / 255.0f;
+            logit_sum += r_hat * lh[gg * cb_max + th[gg]];
+          }
         }
-      } else {
-        for (int gg = 0; gg < G; ++gg) {
-          const float r_hat = srs[gg] * (float)rc[gg] / 255.0f;
-          logit_sum += r_hat * lh[gg * cb_max + th[gg]];
+        slog[h * seg + t] = (logit_sum == 0.f) ? -1e9f : logit_sum * sm_scale;
+      }
+      __syncwarp();
+      // softmax statistics per head; the logits are replaced in place by exp(logit - max)
+      for (int h = 0; h < kv_groups; ++h) {
+        float* lg = slog + h * seg;
+        float m = -INFINITY;
+        for (int t = lane; t < seg; t += 32) m = fmaxf(m, lg[t]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        float l = 0.f;
+        for (int t = lane; t < seg; t += 32) {
+          const float pt = __expf(lg[t] - m);
+          lg[t] = pt;
+          l += pt;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (lane == 0) {
+          float* po = wpp > 1 ? fold + h * (dh + 2)
+                              : partial_out + ((int64_t)(hq0 + h) * max_blocks + page_idx) * (dh + 2);
+          po[0] = m;
+          po[1] = l;
         }
       }
-      slog[h * page_size + t] = (logit_sum == 0.f) ? -1e9f : logit_sum * sm_scale;
-    }
-    __syncwarp();
-    // softmax statistics per head; the logits are replaced in place by exp(logit - max)
-    for (int h = 0; h < kv_groups; ++h) {
-      float* lg = slog + h * page_size;
-      float m = -INFINITY;
-      for (int t = lane; t < page_size; t += 32) m = fmaxf(m, lg[t]);
+      __syncwarp();
+      // V accumulation: a lane owns 4 dimensions, one pass over the rows feeds four heads
+      for (int h0 = 0; h0 < kv_groups; h0 += 4) {
+        for (int d0 = 4 * lane; d0 < dh; d0 += 128) {
+          float acc[4][4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      float l = 0.f;
-      for (int t = lane; t < page_size; t += 32) {
-        const float pt = __expf(lg[t] - m);
-        lg[t] = pt;
-        l += pt;
-      }
+          for (int hh = 0; hh < 4; ++hh) acc[hh][0] = acc[hh][1] = acc[hh][2] = acc[hh][3] = 0.f;
+          const __half* vp = v_rows + d0;
+#pragma unroll 8
+          for (int t = 0; t < seg; ++t) {
+            const uint2 raw = *reinterpret_cast<const uint2*>(vp + t * dh);
+            const float2 va = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+            const float2 vb = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-      if (lane == 0) {
-        float* po = partial_out + ((int64_t)(hq0 + h) * max_blocks + page_idx) * (dh + 2);
-        po[0] = m;
-        po[1] = l;
-      }
-    }
-    __syncwarp();
-    // V accumulation: a lane owns 4 dimensions, one pass over the rows feeds four heads
-    for (int h0 = 0; h0 < kv_groups; h0 += 4) {
-      for (int d0 = 4 * lane; d0 < dh; d0 += 128) {
-        float acc[4][4];
-#pragma unroll
-        for (int hh = 0; hh < 4; ++hh) acc[hh][0] = acc[hh][1] = acc[hh][2] = acc[hh][3] = 0.f;
-        const __half* vp = v_pool + (int64_t)phys * page_size * dh + d0;
-#pragma unroll 4
-        for (int t = 0; t < page_size; ++t) {
-          const uint2 raw = __ldg(reinterpret_cast<const uint2*>(vp + (int64_t)t * dh));
-          const float2 va = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-          const float2 vb = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+            for (int hh = 0; hh < 4; ++hh) {
+              if (h0 + hh < kv_groups) {
+                const float pt = slog[(h0 + hh) * seg + t];
+                acc[hh][0] += pt * va.x;
+                acc[hh][1] += pt * va.y;
+                acc[hh][2] += pt * vb.x;
+                acc[hh][3] += pt * vb.y;
+              }
+            }
+          }
 #pragma unroll
           for (int hh = 0; hh < 4; ++hh) {
             if (h0 + hh < kv_groups) {
-              const float pt = slog[(h0 + hh) * page_size + t];
-              acc[hh][0] += pt * va.x;
-              acc[hh][1] += pt * va.y;
-              acc[hh][2] += pt * vb.x;
-              acc[hh][3] += pt * vb.y;
+              float* po = (wpp > 1 ? fold + (h0 + hh) * (dh + 2)
+                                   : partial_out + ((int64_t)(hq0 + h0 + hh) * max_blocks + page_idx) * (dh + 2)) + 2 + d0;
+              *reinterpret_cast<float2*>(po) = make_float2(acc[hh][0], acc[hh][1]);
+              *reinterpret_cast<float2*>(po + 2) = make_float2(acc[hh][2], acc[hh][3]);
             }
           }
         }
-#pragma unroll
-        for (int hh = 0; hh < 4; ++hh) {
-          if (h0 + hh < kv_groups) {
-            float* po = partial_out + ((int64_t)(hq0 + h0 + hh) * max_blocks + page_idx) * (dh + 2) + 2 + d0;
-            *reinterpret_cast<float2*>(po) = make_float2(acc[hh][0], acc[hh][1]);
-            *reinterpret_cast<float2*>(po + 2) = make_float2(acc[hh][2], acc[hh][3]);
-          }
+      }
+    }
+    __syncwarp();  // this warp is done with its staged rows
+    issue_stage(phys_next);
+    if (wpp > 1) {  // the page's wpp triples -> one
+      __syncthreads();
+      if (phys >= 0) {
+        const float* f0 = fold_all + (int64_t)group * wpp * kv_groups * (dh + 2);
+        const int64_t fstride = (int64_t)kv_groups * (dh + 2);
+        for (int i = sub * 32 + lane; i < kv_groups * (dh + 1); i += wpp * 32) {
+          const int h = i / (dh + 1), e = i - h * (dh + 1) + 1;  // 1 = the sum, 2 .. the accumulator
+          const float* fh = f0 + h * (dh + 2);
+          float m = fh[0];
+          for (int w = 1; w < wpp; ++w) m = fmaxf(m, fh[w * fstride]);
+          float x = 0.f;
+          for (int w = 0; w < wpp; ++w) x += fh[w * fstride + e] * __expf(fh[w * fstride] - m);
+          float* po = partial_out + ((int64_t)(hq0 + h) * max_blocks + page_idx) * (dh + 2);
+          po[e] = x;
+          if (e == 1) po[0] = m;
         }
       }
+      __syncthreads();
     }
   }
 }
@@ -201,6 +290,8 @@ __global__ void __launch_bounds__(kReduceThreads) pool_reduce_kernel(const float
   __shared__ float s_red[32];
   __shared__ float s_acc[32][33];
   __shared__ float s_l[32];
+  griddep_wait();
+  griddep_launch();
   const float* base = partial_out + (int64_t)hq * max_pages * (dh + 2);
   const int64_t row = dh + 2;
   float M = -INFINITY;
@@ -255,6 +346,8 @@ __global__ void pool_encode_append_kernel(
     uint8_t* __restrict__ radius_codes, float* __restrict__ r_scales, __half* __restrict__ v_pool,
     const int64_t* __restrict__ pids, int slot, int G, int g, int C, int G_max, int dh,
     int page_size, int is_new_page) {
+  griddep_wait();
+  griddep_launch();
   pool_append_token(k_post, v_new, decode_cb, theta_codes, radius_codes, r_scales, v_pool,
                     pids[blockIdx.x], slot, G, g, C, G_max, dh, page_size, is_new_page);
 }
@@ -360,6 +453,111 @@ __global__ void ragged_logits_kernel(const uint8_t* __restrict__ pages,
   }
 }
 
+// The same logits for the shapes models use (dh 64 or 128, g 16 or 32, float4-aligned tables).  The
+// kernel above walks one (token, query head) per thread: every lane gathers its own cos/sin row and
+// codebook row a float at a time, and the query is rotated from global memory for each group.  Here a
+// token's dh dimensions lie across dh / 4 lanes, four each, so a cos, sin or centroid row is one
+// coalesced 16-byte load per lane, the rotation partner of a lane's four dimensions is loaded with them,
+// and four query heads live in registers over all of a warp's tokens.  Per group the (norm, dot) pairs
+// of the four heads are reduced and transposed at once (three shuffles each): lane j of a quad ends with
+// head j and does that head's square root and division.  A CTA covers kRagSlots slots of one page and
+// also writes the zeros of the other heads.  Bound: latency at a few thousand tokens, the cos/sin rows
+// from L2 beyond.  2458 tokens x 8 KV heads, 32 query heads: 167 -> 11 us.
+constexpr int kRagSlots = 32, kRagWarps = 4;
+template <int DH, int LG>  // LG = lanes per group = g / 4
+__global__ void __launch_bounds__(kRagWarps * 32) ragged_logits_rows_kernel(
+    const uint8_t* __restrict__ pages, const int* __restrict__ ptable, const int* __restrict__ head_ids,
+    const int* __restrict__ positions, const float* __restrict__ cos_tbl, const float* __restrict__ sin_tbl,
+    const float* __restrict__ q, const float* __restrict__ codebooks, float* __restrict__ logits_out, int grp,
+    int num_kv, int b_theta, int page_size, int n_pages, int Hq, int table_rows, int radius_fmt) {
+  constexpr int LPT = DH / 4, TPW = 32 / LPT;  // lanes per token, tokens a warp works on at once
+  constexpr int G = LPT / LG, g = 4 * LG;
+  constexpr int kPerWarp = kRagSlots / kRagWarps;      // slots of a warp
+  __shared__ float s_out[4][kRagSlots];
+  const int pg = blockIdx.x, slot0 = blockIdx.y * kRagSlots;
+  const int n_slots = min(kRagSlots, page_size - slot0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int l = lane & (LPT - 1), sub = lane / LPT, d = 4 * l, gg = l / LG, j = l & 3;
+  const int hkv = head_ids[pg];
+  const bool known = hkv >= 0 && hkv < num_kv;
+  const int poff = ptable[3 * pg], toff = ptable[3 * pg + 1], roff = ptable[3 * pg + 2];
+  const int count = pages[poff + 1];
+  const int64_t out_stride = (int64_t)n_pages * page_size;
+  float* out_pg = logits_out + (int64_t)pg * page_size + slot0;
+  // rows of the other KV heads
+  for (int i = threadIdx.x; i < Hq * kRagSlots; i += kRagWarps * 32) {
+    const int hq = i / kRagSlots, t = i & (kRagSlots - 1);
+    if (t < n_slots && !(known && hq / grp == hkv)) out_pg[hq * out_stride + t] = 0.f;
+  }
+  if (!known) return;
+  float sc = 0.f;
+  memcpy(&sc, pages + poff + 8 + 4 * gg, 4);
+  const float* cb = codebooks + (((int64_t)hkv * G + gg) << b_theta) * g + (d & (g - 1));
+  const float inv_sqrt = rsqrtf((float)DH);
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int h0 = 0; h0 < grp; h0 += 4) {
+    float4 qa[4], qb[4];  // the lane's dimensions, and what rotate_half pairs them with
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const float* qh = q + ((int64_t)hkv * grp + h0 + h) * DH;
+      qa[h] = h0 + h < grp ? *reinterpret_cast<const float4*>(qh + d) : zero4;
+      const float4 p = h0 + h < grp ? *reinterpret_cast<const float4*>(qh + (d ^ (DH / 2))) : zero4;
+      qb[h] = d < DH / 2 ? make_float4(-p.x, -p.y, -p.z, -p.w) : p;
+    }
+#pragma unroll 2
+    for (int i = 0; i < kPerWarp; i += TPW) {
+      const int ts = warp * kPerWarp + i + sub, t = slot0 + ts;
+      const int pos = ts < n_slots ? positions[(int64_t)pg * page_size + t] : -1;
+      const bool live = ts < n_slots && t < count && pos >= 0 && pos < table_rows;
+      float4 cs = zero4, sn = zero4, cw = zero4;
+      float rad = 0.f;
+      if (live) {
+        cs = __ldg(reinterpret_cast<const float4*>(cos_tbl + (int64_t)pos * DH + d));
+        sn = __ldg(reinterpret_cast<const float4*>(sin_tbl + (int64_t)pos * DH + d));
+        const int64_t bit = ((int64_t)t * G + gg) * b_theta;
+        const uint32_t w = (uint32_t)pages[toff + (bit >> 3)] | ((uint32_t)pages[toff + (bit >> 3) + 1] << 8);
+        const int code = (int)((w >> (bit & 7)) & ((1u << b_theta) - 1u));
+        cw = __ldg(reinterpret_cast<const float4*>(cb + code * g));
+        if (radius_fmt == SPHKV_RADIUS_F16) {
+          const uint16_t hv = (uint16_t)pages[roff + 2 * (t * G + gg)] |
+                              (uint16_t)((uint16_t)pages[roff + 2 * (t * G + gg) + 1] << 8);
+          rad = __half2float(__ushort_as_half(hv));
+        } else {
+          rad = sc * (float)(int8_t)pages[roff + t * G + gg] / 127.0f;
+        }
+      }
+      float nsq[4], dot[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float x0 = qa[h].x * cs.x - qb[h].x * sn.x, x1 = qa[h].y * cs.y - qb[h].y * sn.y;
+        const float x2 = qa[h].z * cs.z - qb[h].z * sn.z, x3 = qa[h].w * cs.w - qb[h].w * sn.w;
+        nsq[h] = (x0 * x0 + x1 * x1) + (x2 * x2 + x3 * x3);
+        dot[h] = (x0 * cw.x + x1 * cw.y) + (x2 * cw.z + x3 * cw.w);
+      }
+      auto fold = [&](const float (&v)[4]) -> float {  // sum over the group's lanes; lane j keeps head j
+        const bool odd = j & 1, up = j & 2;
+        const float k0 = (odd ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[1], 1);
+        const float k1 = (odd ? v[3] : v[2]) + __shfl_xor_sync(0xffffffffu, odd ? v[2] : v[3], 1);
+        float r = (up ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up ? k0 : k1, 2);
+        if (LG == 8) r += __shfl_xor_sync(0xffffffffu, r, 4);
+        return r;
+      };
+      const float qn = fmaxf(sqrtf(fold(nsq)), 1e-6f);
+      const float cpg = fminf(fmaxf(fold(dot) / qn, -1.f), 1.f);
+      float logit = qn * cpg * rad;
+#pragma unroll
+      for (int o = LG; o < LPT; o <<= 1) logit += __shfl_xor_sync(0xffffffffu, logit, o);
+      if (l < 4) s_out[j][ts] = live ? logit * inv_sqrt : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * kRagSlots; i += kRagWarps * 32) {
+      const int h = i / kRagSlots, t = i & (kRagSlots - 1);
+      if (h0 + h < grp && t < n_slots) out_pg[((int64_t)hkv * grp + h0 + h) * out_stride + t] = s_out[h][t];
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace sphkv
 
 using namespace sphkv;
@@ -393,24 +591,42 @@ extern "C" int sphkv_pool_decode(const float* q_all, const float* cb_flat, const
   SPHKV_REQUIRE((reinterpret_cast<uintptr_t>(v_pool) & 7) == 0 && (reinterpret_cast<uintptr_t>(partial_scratch) & 7) == 0 &&
                     (reinterpret_cast<uintptr_t>(theta_codes) & 3) == 0 && (reinterpret_cast<uintptr_t>(radius_codes) & 3) == 0,
                 SPHKV_E_ALIGN, "pool_decode: v_pool / partial_scratch need 8 B, code arrays 4 B alignment");
-  const size_t smem = ((size_t)kv_groups * dh + (size_t)num_tiers * kv_groups * G_max * cb_max +
-                       (size_t)kPoolWarps * ((size_t)kv_groups * page_size + G_max)) * sizeof(float);
+  auto smem_for = [&](int wpp) -> size_t {
+    return ((size_t)kv_groups * dh + (size_t)num_tiers * kv_groups * G_max * cb_max +
+            (size_t)kPoolWarps * ((size_t)kv_groups * (page_size / wpp) + G_max) +
+            (wpp > 1 ? (size_t)kPoolWarps * kv_groups * (dh + 2) : 0)) * sizeof(float);
+  };
+  // warps that share a page: as many as leave each 16 tokens (and fit shared memory)
+  int wpp = kPoolWarps;
+  while (wpp > 1 && (page_size % wpp != 0 || page_size / wpp < 16 || smem_for(wpp) > 100 * 1024)) wpp >>= 1;
+  size_t smem = smem_for(wpp);
   SPHKV_REQUIRE(smem <= 200 * 1024, SPHKV_E_LIMIT, "pool_decode: needs %zu B shared memory", smem);
+  // asynchronous staging of a warp's rows: 16-byte pieces, and two CTAs per SM have to stay possible
+  const int seg = page_size / wpp;
+  int stage_bytes = seg * dh * 2 + 2 * seg * G_max;
+  if (((seg * G_max) & 15) != 0 || (dh & 7) != 0 || smem + 16 + (size_t)kPoolWarps * stage_bytes > 110 * 1024 ||
+      ((reinterpret_cast<uintptr_t>(v_pool) | reinterpret_cast<uintptr_t>(theta_codes) |
+        reinterpret_cast<uintptr_t>(radius_codes)) & 15) != 0)
+    stage_bytes = 0;
+  if (stage_bytes > 0) smem = (smem + 15) / 16 * 16 + (size_t)kPoolWarps * stage_bytes;
   {
     static SmemOptIn opt_in;
     if (int rc = ensure_dynamic_smem(opt_in, (const void*)pool_page_kernel, (int)smem, "pool_decode")) return rc;
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // pages per warp: up to kMaxPagesPerWarp (amortises the table build), fewer while the grid is small
-  int ppw = (int)(((int64_t)num_kv_heads * max_blocks) / ((int64_t)kPoolWarps * 2 * sphkv_sm_count_or(148)));
-  ppw = ppw < 1 ? 1 : (ppw > kMaxPagesPerWarp ? kMaxPagesPerWarp : ppw);
-  const int ppc = kPoolWarps * ppw;
-  pool_page_kernel<<<dim3(num_kv_heads, (max_blocks + ppc - 1) / ppc), kPoolThreads, smem, st>>>(
+  // rounds of pages per CTA: up to kMaxPageRounds (amortises the table build), fewer while the grid is small
+  const int at_once = kPoolWarps / wpp;
+  int rounds = (int)(((int64_t)num_kv_heads * max_blocks) / ((int64_t)at_once * 2 * sphkv_sm_count_or(148)));
+  rounds = rounds < 1 ? 1 : (rounds > kMaxPageRounds ? kMaxPageRounds : rounds);
+  const int ppc = at_once * rounds;
+  (void)launch_overlapped(pool_page_kernel, dim3(num_kv_heads, (max_blocks + ppc - 1) / ppc), dim3(kPoolThreads), smem, st,
       q_all, cb_flat, tier_G, tier_g, theta_codes, radius_codes, r_scales,
       reinterpret_cast<const __half*>(v_pool), block_table, bits_table, partial_scratch,
-      num_q_heads, kv_groups, num_tiers, max_blocks, page_size, dh, G_max, cb_max, g_max, sm_scale, ppw);
+      num_q_heads, kv_groups, num_tiers, max_blocks, page_size, dh, G_max, cb_max, g_max, sm_scale, wpp, rounds,
+      stage_bytes);
   if (int rc = check_launch("pool_page_kernel")) return rc;
-  pool_reduce_kernel<<<dim3(num_q_heads, (dh + 31) / 32), kReduceThreads, 0, st>>>(partial_scratch, out, dh, max_blocks);
+  (void)launch_overlapped(pool_reduce_kernel, dim3(num_q_heads, (dh + 31) / 32), dim3(kReduceThreads), 0, st,
+                          static_cast<const float*>(partial_scratch), out, dh, max_blocks);
   return check_launch("pool_reduce_kernel");
 }
 
@@ -427,7 +643,7 @@ extern "C" int sphkv_pool_encode_append(const float* k_post, const float* v_new,
                     slot >= 0 && slot < page_size,
                 SPHKV_E_ARG, "encode_append: G=%d g=%d C=%d G_max=%d dh=%d slot=%d page_size=%d", G,
                 g, C, G_max, dh, slot, page_size);
-  pool_encode_append_kernel<<<num_kv, 32 * G, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  (void)launch_overlapped(pool_encode_append_kernel, dim3(num_kv), dim3(32 * G), 0, reinterpret_cast<cudaStream_t>(stream),
       k_post, v_new, decode_cb, theta_codes, radius_codes, r_scales,
       reinterpret_cast<__half*>(v_pool), pids, slot, G, g, C, G_max, dh, page_size, is_new_page);
   return check_launch("pool_encode_append_kernel");
@@ -471,7 +687,20 @@ extern "C" int sphkv_ragged_logits(const uint8_t* pages, const int32_t* ptable,
                     (dh & 1) == 0 && b_theta >= 1 && b_theta <= 8 && page_size > 0 && table_rows > 0,
                 SPHKV_E_ARG, "ragged_logits: bad size (Hq=%d grp=%d num_kv=%d G=%d g=%d dh=%d)", Hq,
                 grp, num_kv, G, g, dh);
-  ragged_logits_kernel<<<n_pages, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  // one coalesced row per token where the rows are float4s across a power-of-two of lanes
+  const bool rows = (dh == 64 || dh == 128) && (g == 16 || g == 32) &&
+                    ((reinterpret_cast<uintptr_t>(cos_tbl) | reinterpret_cast<uintptr_t>(sin_tbl) |
+                      reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(codebooks)) & 15) == 0;
+  if (rows) {
+    const dim3 grid(n_pages, (page_size + kRagSlots - 1) / kRagSlots);
+    auto kern = dh == 128 ? (g == 16 ? ragged_logits_rows_kernel<128, 4> : ragged_logits_rows_kernel<128, 8>)
+                          : (g == 16 ? ragged_logits_rows_kernel<64, 4> : ragged_logits_rows_kernel<64, 8>);
+    kern<<<grid, kRagWarps * 32, 0, st>>>(pages, ptable, head_ids, positions, cos_tbl, sin_tbl, q, codebooks, logits_out, grp,
+                               num_kv, b_theta, page_size, n_pages, Hq, table_rows, radius_fmt);
+    return check_launch("ragged_logits_rows_kernel");
+  }
+  ragged_logits_kernel<<<n_pages, 256, 0, st>>>(
       pages, ptable, head_ids, positions, cos_tbl, sin_tbl, q, codebooks, logits_out, grp, num_kv,
       dh, G, g, b_theta, page_size, n_pages, Hq, table_rows, radius_fmt);
   return check_launch("ragged_logits_kernel");

@@ -1455,31 +1455,12 @@ static int make_v_map(CUtensorMap* map, const sphkv_decode_params& p) {
   return 0;
 }
 
-// Launch with programmatic stream serialization: the grid may become resident while the kernel
-// before it in the stream is still running.  Only for kernels that call griddep_wait() before
-// their first global-memory access.
-template <typename Arg>
-static cudaError_t launch_after_predecessor_starts(void (*kern)(Arg), dim3 grid, dim3 block, size_t smem_bytes,
-                                                   cudaStream_t st, const DecodeArgs& a) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem_bytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a);
-}
-
 template <int DH, typename VT, bool ROT, int MODE, bool PACK>
 static int launch_decode_t(const DecodeArgs& a, int smem_bytes, cudaStream_t st) {
   static SmemOptIn opt_in;
   auto kern = decode_splitk_kernel<DH, VT, ROT, MODE, PACK>;
   if (int rc = ensure_dynamic_smem(opt_in, (const void*)kern, smem_bytes, "decode")) return rc;
-  (void)launch_after_predecessor_starts(kern, dim3(a.n_ctas), dim3(kWarps * 32), smem_bytes, st, a);  // check_launch reports
+  (void)launch_overlapped(kern, dim3(a.n_ctas), dim3(kWarps * 32), smem_bytes, st, a);  // check_launch reports
   return check_launch("decode_splitk_kernel");
 }
 

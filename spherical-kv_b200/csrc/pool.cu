@@ -79,6 +79,8 @@ __global__ void pool_append_step_kernel(
     int n_pool_pages) {
   __shared__ int s_cur, s_used, s_err;
   const int h = blockIdx.x, num_kv = gridDim.x, tid = threadIdx.x;
+  griddep_wait();
+  griddep_launch();
   if (tid == 0) {
     s_cur = state[kStCtx];
     s_used = state[kStUsed];
@@ -162,7 +164,7 @@ extern "C" int sphkv_pool_append_step(const float* k_post, const float* v_new, c
                     page_size > 0 && max_blocks > 0 && n_pool_pages > 0 && dec_tier_idx >= 0,
                 SPHKV_E_ARG, "pool_append_step: G=%d g=%d C=%d G_max=%d dh=%d page_size=%d num_kv=%d", G,
                 g, C, G_max, dh, page_size, num_kv);
-  pool_append_step_kernel<<<num_kv, 32 * G, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  (void)launch_overlapped(pool_append_step_kernel, dim3(num_kv), dim3(32 * G), 0, reinterpret_cast<cudaStream_t>(stream),
       k_post, v_new, decode_cb, theta_codes, radius_codes, r_scales, reinterpret_cast<__half*>(v_pool),
       block_table, bits_table, ctx_lens, pids, state, dec_tier_idx, G, g, C, G_max, dh, page_size,
       max_blocks, n_pool_pages);

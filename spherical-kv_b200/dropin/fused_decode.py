@@ -94,7 +94,7 @@ def fused_decode_ragged(pages_u8, ptable, head_ids, positions, cos_tbl, sin_tbl,
     f32, i32 = torch.float32, torch.int32
     n_pages = ptable.shape[0]
     hq = q.shape[0]
-    out = torch.zeros(hq, n_pages * page_size, dtype=f32, device=q.device)
+    out = torch.empty(hq, n_pages * page_size, dtype=f32, device=q.device)  # the kernel writes every element
     if n_pages == 0:
         return out
     cb = codebooks.contiguous()

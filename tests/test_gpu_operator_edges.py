@@ -1,0 +1,76 @@
+"""GPU: the reference-signature operators at the edges of their dispatch -- warps per page of the pool
+decode, rows-across-lanes ragged logits -- against the CPU restatements."""
+import math
+import os
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_compat import dev, make_pool
+from util import ROOT, load_oracle, load_pkg
+
+pkg = load_pkg()
+orc = load_oracle()
+synth = pkg.synth
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+sys.path.insert(0, os.path.join(ROOT, "spherical-kv_b200", "dropin"))
+
+
+# page sizes that split over 1, 2, 4, 8 warps and one that does not split evenly; 1, 3 and 8 query heads
+@pytest.mark.parametrize("page_size,dh,grp", [(16, 64, 3), (32, 128, 8), (64, 128, 1), (128, 64, 4), (24, 128, 4), (40, 64, 4)])
+def test_pool_decode_page_splits(page_size, dh, grp):
+    import fused_decode
+    Hkv = 2
+    Hq = Hkv * grp
+    pool = make_pool(Hkv, grp, dh, [page_size * 11 + 1, 3], page_size, seed=page_size)
+    G_max, C_max, g_max, max_blocks = pool["dims"]
+    q = torch.randn(Hq, dh, generator=torch.Generator().manual_seed(5))
+    sm = 1.0 / math.sqrt(dh)
+    want, want_part = orc.pool_decode(q, pool["cb_flat"], pool["tier_G"], pool["tier_g"], pool["theta"], pool["radius"],
+                                      pool["scales"], pool["v"], pool["block_table"], pool["bits_table"], sm)
+    d = dev(pool)
+    out, part = torch.zeros(Hq, dh, device=DEV), torch.full((Hq, max_blocks, dh + 2), 7.0, device=DEV)
+    fused_decode.sphkv_decode(q.to(DEV), d["cb_flat"], d["tier_G"], d["tier_g"], d["theta"], d["radius"], d["scales"],
+                              d["v"], d["block_table"], d["bits_table"], d["ctx_lens"], out, part, Hq, Hkv, grp, 3,
+                              max_blocks, page_size, dh, G_max, C_max, g_max, sm, int(pool["ctx_lens"].max()))
+    assert (out.cpu() - want).abs().max().item() <= 2e-4
+    gp, live = part.cpu(), torch.isfinite(want_part[:, :, 0])
+    assert torch.equal(torch.isfinite(gp[:, :, 0]), live) and (gp[:, :, 1:][~live] == 0).all()
+    # fp32 sums of at most page_size terms in another order: a few ulps of the sum of magnitudes
+    assert (gp[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
+
+
+@pytest.mark.parametrize("dh,page_size,tier,grp", [(64, 16, 0, 4), (64, 128, 2, 1), (128, 32, 1, 8), (128, 48, 2, 5)])
+def test_ragged_logits_shapes(dh, page_size, tier, grp):
+    import fused_decode
+    t = pkg.REFERENCE_TIERS[tier]
+    Hkv, ctx = 3, 150
+    Hq, G = Hkv * grp, dh // t.g
+    tiers = pkg.TierSet(dh, [t])
+    K, V, Q, _ = synth.make_kvq(1, Hq, Hkv, dh, ctx, seed=2)
+    cbs = synth.make_codebooks(Hkv, dh, [t], seed=3)
+    assign = synth.make_tier_assign(1, Hkv, ctx, {t.tier_id: 0.6}, seed=4, per_head=True)
+    lists = pkg.build_page_lists(assign, tiers, page_size, page_align=4)
+    pages = np.zeros(lists.pool_bytes + 16, np.uint8)
+    want = torch.zeros(Hq, lists.n_pages * page_size)
+    cos, sin = orc.rope_tables(ctx + 4, dh)
+    for ph in range(lists.n_pages):
+        c, h = int(lists.page_count[ph]), int(lists.page_head[ph])
+        rows = lists.src_index[ph, :c].long()
+        r, th = orc.encode(K.reshape(ctx, Hkv, dh)[rows, h].contiguous(), cbs[0][h])
+        page, _, _ = orc.build_page(r, th, t.b_theta, t.tier_id, 0)
+        po = int(lists.ptable[ph, 0])
+        pages[po:po + page.size] = page
+        _, _, _, th2, r2 = orc.parse_page(pages, *(int(x) for x in lists.ptable[ph]), G, t.b_theta, 0)
+        want[h * grp:(h + 1) * grp, ph * page_size:ph * page_size + c] = orc.backrot_logits(
+            Q[0, h * grp:(h + 1) * grp], torch.from_numpy(r2), torch.from_numpy(th2), lists.positions[ph, :c].long(),
+            cbs[0][h], cos, sin)
+    got = fused_decode.fused_decode_ragged(
+        torch.from_numpy(pages).to(DEV), lists.ptable.to(DEV), lists.page_head.to(DEV),
+        lists.positions.reshape(-1).to(DEV), cos.to(DEV), sin.to(DEV), Q[0].to(DEV), grp, Hkv,
+        torch.cat([cbs[0][h] for h in range(Hkv)], 0).to(DEV), dh, G, t.g, t.b_theta, page_size).cpu()
+    assert (got - want).abs().max().item() <= 2e-4
+    assert torch.equal(got == 0, want == 0)
