@@ -75,7 +75,7 @@ int sphkv_rope_table_build(float* table, int32_t max_pos, int32_t dh, const floa
  * Groups retained tokens into pages on the device: the grouping and sort of
  * _build_per_head_pages (spherical_kv_pipeline.py:1146-1228) and the pointer table of
  * pointer_table.py:4-21 for all units at once.  Two calls, because the sizes of the tables
- * follow from the tiers: sphkv_page_lists_count returns them (it synchronises the stream),
+ * follow from the tiers: sphkv_page_lists_count returns them (it waits for the stream to reach them),
  * sphkv_page_lists_fill writes every table.  Both take the same struct and scratch. */
 typedef struct sphkv_page_lists_params {
   const void* tier_assign;  /* [units][T] tier id per token, contiguous; ids that no slot has:

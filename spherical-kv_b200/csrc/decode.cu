@@ -13,6 +13,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "splitk.cuh"
 
 namespace sphkv {
@@ -82,106 +84,83 @@ __global__ void plan_kernel(const int32_t* __restrict__ num_blocks, int n_units,
   if (threadIdx.x == 0) pfx[n_units] = s_carry;
 }
 
+// grid (unit, importance slices); one thread per (query head, dimension): grp * DH threads.  Bound: memory
+// latencies in a row (span -> rows -> output), so everything that can be is loaded at once.  A step of eight
+// units, dh 64: 5.3 -> 3.7 us; with the importance update of three rows at 128-token pages 12.3 -> 4.9 us.
 template <int DH>
-__global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
-  constexpr int kChunk = 128;  // partial rows combined per pass
+__global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) {
+  constexpr int kChunk = 128;  // partial rows combined per pass (general path)
+  constexpr int kBatch = 16;   // rows' loads in flight at a time
   const sphkv_decode_params& p = a.p;
   const int u = blockIdx.x;  // traversal index: hkv * B + b
   const int hkv = u / p.B, b = u - hkv * p.B;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = threadIdx.x / DH, d = threadIdx.x % DH;  // this thread's query head (warp-uniform) and dimension
   __shared__ float s_M[8], s_L[8];
   __shared__ float s_w[8][kChunk];
-  // The next kernel in the stream -- the next step's decode kernel -- may become resident now; it
-  // waits for this grid to complete before it touches global memory.  (Launching THIS kernel the
-  // same way measured 2 us slower per step, so it is launched plainly.)
+  // launched like the decode kernel: its blocks wait here for it to end, and let the next step's in early
+  griddep_wait();
   griddep_launch();
-  const int32_t* pfx = a.pfx;
-  const int64_t T = pfx[a.n_units];
-  const int64_t ps = pfx[u], pe = pfx[u + 1];
-  // the CTAs whose block ranges meet this unit's (every thread derives them: no barrier, no
-  // shared-memory round trip between the prefix loads and the row loads)
-  int c_lo = 0, c_hi = -1;
-  const UnitSplit us = split_by_unit(pfx, a.n_units, a.n_ctas, p.page_size >> 4, u, -1);
-  if (us.by_unit) {
-    c_lo = us.first;
-    c_hi = us.first + us.count - 1;
-  } else if (pe > ps && T > 0) {
-    c_lo = (int)((ps * a.n_ctas) / T);
-    if (c_lo >= a.n_ctas) c_lo = a.n_ctas - 1;
-    while (c_lo > 0 && cta_range_start(c_lo, a.n_ctas, T) > ps) --c_lo;
-    while (cta_range_start(c_lo + 1, a.n_ctas, T) <= ps) ++c_lo;
-    c_hi = (int)(((pe - 1) * a.n_ctas) / T);
-    if (c_hi >= a.n_ctas) c_hi = a.n_ctas - 1;
-    while (c_hi > c_lo && cta_range_start(c_hi, a.n_ctas, T) >= pe) --c_hi;
-    while (c_hi + 1 < a.n_ctas && cta_range_start(c_hi + 1, a.n_ctas, T) < pe) ++c_hi;
+  const int unit = b * p.Hkv + hkv;
+  // the CTAs that wrote a partial row of this unit, as the decode kernel's CTAs left them
+  int c_lo = 0, nrows = 0;
+  const int nb_unit = min(p.num_blocks[unit], p.max_blocks);
+  const uint32_t span = a.spans[u];
+  if (nb_unit > 0) {
+    c_lo = (int)(span & 0xFFFFu);
+    nrows = (int)(span >> 16);
   }
-  const int nrows = c_hi - c_lo + 1;
-  auto row_exists = [&](int c) -> bool {
-    return us.by_unit || cta_range_start(c, a.n_ctas, T) != cta_range_start(c + 1, a.n_ctas, T);
-  };
-  auto row_m = [&](int n, int c) -> float {  // max of row (c, u) for head n; -inf if no such row
-    if (!row_exists(c)) return -INFINITY;
-    return a.rows[((int64_t)(c + u) * 8 + n) * (DH + 2)];
-  };
-  float o_acc[(8 * DH + 255) / 256];
-#pragma unroll
-  for (int q = 0; q < (8 * DH + 255) / 256; ++q) o_acc[q] = 0.f;
+  const int64_t row_stride = 8 * (DH + 2);
+  const float* rows_n = a.rows + ((int64_t)(c_lo + u) * 8 + n) * (DH + 2);  // row 0 of this thread's head
+  float o_acc = 0.f;
   const bool few_rows = nrows <= 32;
   if (few_rows) {
-    // At most one row per lane (the usual case: units >= CTAs / 32).  A warp covers 32 dimensions
-    // of one head: lane c fetches row c's (max, sum) while the accumulator loads of the first
-    // rows are already in flight, the warp reduces, and every lane then folds the rows of its
-    // dimension with the weights passed around by shuffles -- one memory latency instead of the
-    // four of the general path below, and the same arithmetic in the same order.
+    // At most one row per lane (the usual case: units >= CTAs / 32).  Lane c fetches row c's (max, sum)
+    // while the accumulator loads of the first rows are already in flight, the warp reduces, and every
+    // lane then folds the rows of its dimension with the weights passed around by shuffles -- one memory
+    // latency instead of the four of the general path below, and the same arithmetic in the same order.
+    const bool mine = lane < nrows;
+    const float mr = mine ? rows_n[lane * row_stride] : -INFINITY;
+    const float lr = mine ? rows_n[lane * row_stride + 1] : 0.f;
+    float w = 0.f;
+    for (int ci = 0; ci < max(nrows, 1); ci += kBatch) {
+      float v[kBatch];
 #pragma unroll
-    for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-      const int i = threadIdx.x + q * 256;
-      const int n = i / DH, d = i - n * DH;
-      if (n >= a.grp) continue;  // warp-uniform: DH is a multiple of 32
-      const float* col = a.rows + ((int64_t)(c_lo + u) * 8 + n) * (DH + 2);
-      const bool mine = lane < nrows && row_exists(c_lo + lane);
-      const float mr = mine ? col[(int64_t)lane * 8 * (DH + 2)] : -INFINITY;
-      const float lr = mine ? col[(int64_t)lane * 8 * (DH + 2) + 1] : 0.f;
-      float M = mr;
+      for (int k = 0; k < kBatch; ++k) v[k] = ci + k < nrows ? rows_n[(ci + k) * row_stride + 2 + d] : 0.f;
+      if (ci == 0) {
+        float M = mr;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
-      const float w = (mine && M != -INFINITY) ? exp2f(mr - M) : 0.f;
-      float L = lr * w;
+        for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        w = (mine && M != -INFINITY) ? exp2f(mr - M) : 0.f;
+        float L = lr * w;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
-      if (lane == 0 && d == 0) { s_M[n] = M; s_L[n] = L; }
-      float o = 0.f;
-      for (int ci = 0; ci < nrows; ci += 8) {
-        float v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = ci + k < nrows ? col[(int64_t)(ci + k) * 8 * (DH + 2) + 2 + d] : 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float wk = __shfl_sync(0xffffffffu, w, (ci + k) & 31);
-          o += (ci + k < nrows && wk != 0.f) ? wk * v[k] : 0.f;
-        }
+        for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+        if (d == 0) { s_M[n] = M; s_L[n] = L; }
       }
-      o_acc[q] = o;
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) {
+        const float wk = __shfl_sync(0xffffffffu, w, (ci + k) & 31);
+        o_acc += (ci + k < nrows && wk != 0.f) ? wk * v[k] : 0.f;
+      }
     }
-    __syncthreads();
   } else if (warp < a.grp) {
-    // pass 1: warp n -> global max and sum of head n
+    // pass 1: warp h -> global max and sum of head h
+    const float* rows_h = a.rows + ((int64_t)(c_lo + u) * 8 + warp) * (DH + 2);
     float M = -INFINITY;
-    for (int i = lane; i < nrows; i += 32) M = fmaxf(M, row_m(warp, c_lo + i));
+    for (int i = lane; i < nrows; i += 32) M = fmaxf(M, rows_h[i * row_stride]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
     float L = 0.f;
     if (M != -INFINITY)
       for (int i = lane; i < nrows; i += 32) {
-        const float mw = row_m(warp, c_lo + i);
-        if (mw != -INFINITY)
-          L += a.rows[((int64_t)(c_lo + i + u) * 8 + warp) * (DH + 2) + 1] * exp2f(mw - M);
+        const float mw = rows_h[i * row_stride];
+        if (mw != -INFINITY) L += rows_h[i * row_stride + 1] * exp2f(mw - M);
       }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
     if (lane == 0) { s_M[warp] = M; s_L[warp] = L; }
   }
-  if (!few_rows) __syncthreads();
+  __syncthreads();
   // page-importance EMA (_omega_ema_eager, spherical_kv_pipeline.py:952-987) from the per-tile
   // (max, sum) the split-K kernel left in page_ml: per query head the block weights
   // exp(max(m - m_max, -60)) * l are normalised over the blocks, averaged over the heads of
@@ -190,30 +169,41 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
   // are sums of the same exp(logit - m_max) terms, so no second pass over the blocks is needed
   // (the -60 clamp changes terms below e^-60 of the largest one).
   if (p.omega != nullptr) {
+    // A thread takes one (block, query head), gp = grp rounded up to a power of two of them side by side, and
+    // loads all (at most eight) tiles of the block at once.  The blocks are spread over gridDim.y CTAs of this
+    // unit; each repeats the cheap pass 1.
     const int tpp = p.page_size >> 4;
-    const int unit = b * p.Hkv + hkv;
-    const int nb = min(p.num_blocks[unit], p.max_blocks);
+    const int gp_shift = a.grp <= 1 ? 0 : 32 - __clz(a.grp - 1), gp = 1 << gp_shift;
     const int32_t* bt = p.block_table + (int64_t)unit * p.max_blocks;
     const float one_minus = (1.0f - p.ema_beta) / (float)a.grp;
-    // blocks are spread over gridDim.y CTAs of this unit; each repeats the cheap pass 1
-    for (int blk = blockIdx.y * blockDim.x + threadIdx.x; blk < p.max_blocks; blk += gridDim.y * blockDim.x) {
+    const int h = threadIdx.x & (gp - 1);
+    const int per_cta = blockDim.x >> gp_shift;
+    const float2* ml = reinterpret_cast<const float2*>(p.page_ml) +
+                       ((int64_t)b * p.Hq + (int64_t)hkv * a.grp + min(h, a.grp - 1)) * p.max_blocks * tpp;
+    for (int blk0 = blockIdx.y * per_cta; blk0 < p.max_blocks; blk0 += gridDim.y * per_cta) {
+      const int blk = blk0 + (threadIdx.x >> gp_shift);
+      const bool in = (int)(threadIdx.x >> gp_shift) < per_cta && blk < p.max_blocks;
       float mass = 0.f;
-      if (blk < nb && bt[blk] >= 0) {
-        for (int n = 0; n < a.grp; ++n) {
-          const float* t = p.page_ml +
-                           (((int64_t)b * p.Hq + (int64_t)hkv * a.grp + n) * p.max_blocks + blk) * tpp * 2;
-          float m = -INFINITY;
-          for (int i = 0; i < tpp; ++i)
-            if (t[2 * i + 1] > 0.f) m = fmaxf(m, t[2 * i]);
-          if (m == -INFINITY) continue;
-          float l = 0.f;
-          for (int i = 0; i < tpp; ++i)
-            if (t[2 * i + 1] > 0.f) l += t[2 * i + 1] * __expf(t[2 * i] - m);
-          mass += __expf(fmaxf(m - s_M[n] * kLn2, -60.f)) * l / fmaxf(s_L[n], 1e-12f);
+      if (in && h < a.grp && blk < nb_unit && bt[blk] >= 0) {
+        float2 t[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) t[i] = i < tpp ? ml[(int64_t)blk * tpp + i] : make_float2(-INFINITY, 0.f);
+        float m = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (t[i].y > 0.f) m = fmaxf(m, t[i].x);
+        if (m != -INFINITY) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (t[i].y > 0.f) l += t[i].y * __expf(t[i].x - m);
+          mass = __expf(fmaxf(m - s_M[h] * kLn2, -60.f)) * l / fmaxf(s_L[h], 1e-12f);
         }
       }
-      float* o = p.omega + (int64_t)unit * p.max_blocks + blk;
-      *o = *o * p.ema_beta + mass * one_minus;
+      for (int o = 1; o < gp; o <<= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
+      if (in && h == 0) {
+        float* dst = p.omega + (int64_t)unit * p.max_blocks + blk;
+        *dst = *dst * p.ema_beta + mass * one_minus;
+      }
     }
   }
   if (blockIdx.y != 0) return;  // only the first CTA of a unit writes the attention output
@@ -221,53 +211,37 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
   for (int c0 = 0; c0 < (few_rows ? 0 : nrows); c0 += kChunk) {
     const int nc = min(kChunk, nrows - c0);
     for (int i = threadIdx.x; i < a.grp * nc; i += blockDim.x) {
-      const int n = i / nc, ci = i - n * nc;
-      const float mw = row_m(n, c_lo + c0 + ci);
-      s_w[n][ci] = (mw == -INFINITY || s_M[n] == -INFINITY) ? 0.f : exp2f(mw - s_M[n]);
+      const int h = i / nc, ci = i - h * nc;
+      const float mw = a.rows[((int64_t)(c_lo + c0 + ci + u) * 8 + h) * (DH + 2)];
+      s_w[h][ci] = (mw == -INFINITY || s_M[h] == -INFINITY) ? 0.f : exp2f(mw - s_M[h]);
     }
     __syncthreads();
+    const float* col = rows_n + c0 * row_stride + 2 + d;
+    for (int ci = 0; ci < nc; ci += kBatch) {
+      float v[kBatch];
 #pragma unroll
-    for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-      const int i = threadIdx.x + q * 256;
-      const int n = i / DH, d = i - n * DH;
-      if (n < a.grp) {
-        // eight rows' loads in flight at a time (a unit cut over many CTAs has tens of rows: one
-        // dependent load per row made this loop the whole kernel); a row that does not exist has
-        // weight 0 and whatever the scratch holds there is discarded by the select
-        float o = o_acc[q];
-        const float* col = a.rows + ((int64_t)(c_lo + c0 + u) * 8 + n) * (DH + 2) + 2 + d;
-        for (int ci = 0; ci < nc; ci += 8) {
-          float v[8];
+      for (int k = 0; k < kBatch; ++k) v[k] = ci + k < nc ? col[(ci + k) * row_stride] : 0.f;
 #pragma unroll
-          for (int k = 0; k < 8; ++k) v[k] = ci + k < nc ? col[(int64_t)(ci + k) * 8 * (DH + 2)] : 0.f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float w = ci + k < nc ? s_w[n][ci + k] : 0.f;
-            o += w != 0.f ? w * v[k] : 0.f;
-          }
-        }
-        o_acc[q] = o;
+      for (int k = 0; k < kBatch; ++k) {
+        const float w = ci + k < nc ? s_w[n][ci + k] : 0.f;
+        o_acc += w != 0.f ? w * v[k] : 0.f;
       }
     }
     __syncthreads();
   }
-#pragma unroll
-  for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-    const int i = threadIdx.x + q * 256;
-    const int n = i / DH, d = i - n * DH;
-    if (n >= a.grp) continue;
-    const float M = s_M[n], l = s_L[n], o = o_acc[q];
-    const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
+  const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
+  {
+    const float M = s_M[n], l = s_L[n];
     if (p.out_partial != nullptr) {
       float* dst = p.out_partial + hq * (DH + 2);
       if (d == 0) {
         dst[0] = M * kLn2;
         dst[1] = l;
       }
-      dst[2 + d] = o;
+      dst[2 + d] = o_acc;
     }
     if (p.out != nullptr && p.xchg_world <= 1)
-      store_from_float(p.out, p.out_dtype, hq * DH + d, l > 0.f ? o / l : 0.f);
+      store_from_float(p.out, p.out_dtype, hq * DH + d, l > 0.f ? o_acc / l : 0.f);
   }
   if (p.xchg_world <= 1) return;
 
@@ -278,7 +252,6 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
   //      memory is touched by plain stores only; the words a rank reads are in its own memory.
   __shared__ int s_seq, s_ok;
   __shared__ float s_rm[SPHKV_MAX_XCHG_RANKS][8], s_rl[SPHKV_MAX_XCHG_RANKS][8];
-  const int unit = b * p.Hkv + hkv;
   const int64_t n_rows = (int64_t)p.B * p.Hq;
   if (threadIdx.x == 0) {
     s_seq = p.xchg_seq[unit] + 1;
@@ -291,12 +264,7 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
     const unsigned long long w = ((unsigned long long)seq << 32) | (unsigned long long)__float_as_uint(v);
     asm volatile("st.relaxed.sys.global.b64 [%0], %1;" ::"l"(dst), "l"(w) : "memory");
   };
-#pragma unroll
-  for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-    const int i = threadIdx.x + q * 256;
-    const int n = i / DH, d = i - n * DH;
-    if (n >= a.grp) continue;
-    const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
+  {
     const int64_t off = (slot_base + (int64_t)p.xchg_rank * n_rows + hq) * (DH + 2);
     for (int peer = 0; peer < p.xchg_world; ++peer) {
       unsigned long long* dst = p.xchg_recv[peer] + off;
@@ -304,7 +272,7 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
         put(dst, s_M[n] * kLn2);
         put(dst + 1, s_L[n]);
       }
-      put(dst + 2 + d, o_acc[q]);
+      put(dst + 2 + d, o_acc);
     }
   }
   // Bounded wait, word by word: a word of this step's slot is in when it carries exactly this
@@ -326,22 +294,15 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
     }
   };
   for (int i = threadIdx.x; i < p.xchg_world * a.grp; i += blockDim.x) {
-    const int rr = i / a.grp, n = i - rr * a.grp;
-    const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
-    const unsigned long long* pr = mine + ((int64_t)rr * n_rows + hq) * (DH + 2);
+    const int rr = i / a.grp, h = i - rr * a.grp;
+    const unsigned long long* pr = mine + ((int64_t)rr * n_rows + (int64_t)b * p.Hq + (int64_t)hkv * a.grp + h) * (DH + 2);
     const float pm = get(pr), pl = get(pr + 1);
-    s_rm[rr][n] = pl > 0.f ? pm : -INFINITY;
-    s_rl[rr][n] = pl;
+    s_rm[rr][h] = pl > 0.f ? pm : -INFINITY;
+    s_rl[rr][h] = pl;
   }
   __syncthreads();
-  float res[(8 * DH + 255) / 256];
-#pragma unroll
-  for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-    const int i = threadIdx.x + q * 256;
-    const int n = i / DH, d = i - n * DH;
-    res[q] = 0.f;
-    if (n >= a.grp) continue;
-    const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
+  float res;
+  {
     float M = -INFINITY;
     for (int rr = 0; rr < p.xchg_world; ++rr) M = fmaxf(M, s_rm[rr][n]);
     float l = 0.f, o = 0.f;
@@ -352,21 +313,14 @@ __global__ void __launch_bounds__(256) merge_rows_kernel(const DecodeArgs a) {
       l += s_rl[rr][n] * w;
       o += v * w;
     }
-    res[q] = l > 0.f ? o / l : 0.f;
+    res = l > 0.f ? o / l : 0.f;
   }
   __syncthreads();  // every wait has ended, one way or the other
   if (threadIdx.x == 0) p.xchg_seq[unit] = (int32_t)seq;
   const bool ok = s_ok != 0;
   if (!ok && threadIdx.x == 0 && p.status) atomicOr(p.status, SPHKV_ST_TIMEOUT);  // a rank never published this step
   if (p.out == nullptr) return;
-#pragma unroll
-  for (int q = 0; q < (8 * DH + 255) / 256; ++q) {
-    const int i = threadIdx.x + q * 256;
-    const int n = i / DH, d = i - n * DH;
-    if (n >= a.grp) continue;
-    const int64_t hq = (int64_t)b * p.Hq + (int64_t)hkv * a.grp + n;
-    store_from_float(p.out, p.out_dtype, hq * DH + d, ok ? res[q] : 0.f);  // defined output either way
-  }
+  store_from_float(p.out, p.out_dtype, hq * DH + d, ok ? res : 0.f);  // defined output either way
 }
 
 // ---- merge of R partial sets (cross-GPU split-KV) ----------------------------------------
@@ -518,13 +472,19 @@ extern "C" int sphkv_rope_table_build(float* table, int32_t max_pos, int32_t dh,
   return check_launch("rope_table_kernel");
 }
 
+// Block prefix per unit and the units' spans of CTAs.  One array serves both when the decode kernel derives the
+// prefix itself (it keeps it in shared memory).
+static int64_t prefix_bytes(int64_t n_units) {
+  return align_up((n_units + 1) * 4, 256) * (n_units <= kMaxUnitsInKernelPlan ? 1 : 2);
+}
+
 static int resolve_ctas(int n_ctas) { return n_ctas > 0 ? n_ctas : sm_count_current_device(); }
 
 extern "C" int64_t sphkv_decode_scratch_bytes(int32_t B, int32_t Hkv, int32_t dh, int32_t n_ctas) {
   n_ctas = resolve_ctas(n_ctas);
   if (n_ctas <= 0 || B <= 0 || Hkv <= 0 || dh <= 0) return SPHKV_E_ARG;
   const int64_t n_units = (int64_t)B * Hkv;
-  return align_up((n_units + 1) * 4, 256) + (int64_t)(n_ctas + n_units) * 8 * (dh + 2) * 4;
+  return prefix_bytes(n_units) + (int64_t)(n_ctas + n_units) * 8 * (dh + 2) * 4;
 }
 
 extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
@@ -582,8 +542,10 @@ extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
   SPHKV_REQUIRE(p.scratch_bytes >= need, SPHKV_E_SCRATCH, "decode: scratch %lld B < %lld B",
                 (long long)p.scratch_bytes, (long long)need);
   a.pfx = reinterpret_cast<int32_t*>(p.scratch);
-  a.rows = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.scratch) +
-                                    align_up((int64_t)(a.n_units + 1) * 4, 256));
+  a.rows = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(p.scratch) + prefix_bytes(a.n_units));
+  a.spans = reinterpret_cast<uint32_t*>(p.scratch);
+  if (a.n_units > kMaxUnitsInKernelPlan) a.spans += align_up((int64_t)(a.n_units + 1) * 4, 256) / 4;
+  a.n_ctas = min(a.n_ctas, 0xFFFF);  // a span packs two CTA counts into a word
   a.wide = ((reinterpret_cast<uintptr_t>(p.k_pages) | reinterpret_cast<uintptr_t>(p.positions)) & 15) == 0;
   a.plan_in_kernel = a.n_units <= kMaxUnitsInKernelPlan ? 1 : 0;
   const int pfx_bytes = a.plan_in_kernel ? (a.n_units + 1) * 4 : 0;
@@ -612,11 +574,12 @@ extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
                                 : launch_decode<64, __nv_bfloat16>(a, smem_bytes, st);
   if (rc) return rc;
   // with an importance update, extra CTAs per unit share the walk over the blocks
-  const dim3 mgrid(a.n_units, p.omega ? (unsigned)min(16, (p.max_blocks + 255) / 256) : 1u);
+  const int merge_threads = grp * p.dh;
+  const dim3 mgrid(a.n_units, p.omega ? (unsigned)std::max(1, std::min(16, p.max_blocks * SPHKV_MAX_GQA / merge_threads)) : 1u);
   if (p.dh == 128)
-    merge_rows_kernel<128><<<mgrid, 256, 0, st>>>(a);
+    (void)launch_overlapped(merge_rows_kernel<128>, mgrid, dim3(merge_threads), 0, st, a);
   else
-    merge_rows_kernel<64><<<mgrid, 256, 0, st>>>(a);
+    (void)launch_overlapped(merge_rows_kernel<64>, mgrid, dim3(merge_threads), 0, st, a);
   return check_launch("merge_rows_kernel");
 }
 

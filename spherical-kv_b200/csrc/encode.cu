@@ -410,6 +410,8 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
 template <int GS>
 __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
+  griddep_wait();
+  griddep_launch();
   extern __shared__ __align__(16) uint8_t smem[];
   float* cb_s = reinterpret_cast<float*>(smem);  // [G][C][GS] of the current (head, tier slot)
   const int N = p.page_size, dh = p.dh;
@@ -516,6 +518,8 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
 template <int SRC>
 __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
+  griddep_wait();
+  griddep_launch();
   extern __shared__ __align__(16) uint8_t smem[];
   const int N = p.page_size, dh = p.dh, GST = dh >> 4;
   const int ppb_shift = __clz(N) - 24;  // log2 of the 128 / N pages per bundle (N is 16 .. 128)
@@ -895,7 +899,7 @@ static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaSt
     EncodeArgs b = a;
     b.search_chunk = std::max(1, std::min(8, a.p.n_bundles / (resident * 4)));  // >= 4 chunks per CTA, <= 8 bundles each
     const int grid = std::max(1, std::min((a.p.n_bundles + b.search_chunk - 1) / b.search_chunk, resident));
-    search_bundles_kernel<GS><<<grid, kEncThreads, cb_bytes, st>>>(b);
+    (void)launch_overlapped(search_bundles_kernel<GS>, dim3(grid), dim3(kEncThreads), cb_bytes, st, b);
     return check_launch("search_bundles_kernel");
   }
   const int grid = (a.p.n_bundles + a.bundles_per_cta - 1) / a.bundles_per_cta;
@@ -917,9 +921,9 @@ static int launch_assemble(EncodeArgs& a, bool from_codes, cudaStream_t st) {
   const int64_t ctas = (items + kEncThreads / 32 - 1) / (kEncThreads / 32);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)sm_count_current_device() * 8));
   if (from_codes)
-    assemble_pages_kernel<3><<<grid, kEncThreads, smem_bytes, st>>>(a);
+    (void)launch_overlapped(assemble_pages_kernel<3>, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);
   else
-    assemble_pages_kernel<2><<<grid, kEncThreads, smem_bytes, st>>>(a);
+    (void)launch_overlapped(assemble_pages_kernel<2>, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);
   return check_launch("assemble_pages_kernel");
 }
 

@@ -10,6 +10,8 @@
 // Bound: launches and the one round trip, not bandwidth (a 32768-token, 8-head prompt is 0.26 MB of
 // tiers in and 2.5 MB of tables out).  As array operations the same construction was ~130 launches
 // with 15 synchronising copies, 1.8 ms whatever the prompt's length.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sphkv {
@@ -26,7 +28,8 @@ struct ListArgs {
   int U, Hkv, S, n_chunks, N, n_shift, rb, align;
   int tier_id[SPHKV_MAX_TIER_SLOTS], G[SPHKV_MAX_TIER_SLOTS], bits[SPHKV_MAX_TIER_SLOTS];
   // scratch; run r = slot * U + unit
-  int64_t* totals;     // pages, most blocks of a unit, bundles, pool bytes
+  int64_t* totals;     // pinned host memory: pages, most blocks of a unit, bundles, pool bytes, call number
+  int64_t call;
   int64_t* byte_base;  // [S*U] pool offset of the run's first page
   int32_t* cnt;        // [S*U] tokens
   int32_t* run_base;   // [S*U] first logical page
@@ -43,9 +46,10 @@ struct ListOut {
 };
 
 __device__ __forceinline__ int64_t page_bytes(const ListArgs& a, int s, int count) {
-  const int64_t vals = (int64_t)count * a.G[s];
-  const int64_t b = 8 + 4 * a.G[s] + ((vals * a.bits[s] + 7) >> 3) + vals * a.rb;
-  return (b + a.align - 1) / a.align * a.align;
+  // 32-bit arithmetic: a page is at most a few KB (a 64-bit division here was a third of the scan)
+  const uint32_t vals = (uint32_t)count * a.G[s];
+  const uint32_t b = 8 + 4 * a.G[s] + ((vals * a.bits[s] + 7) >> 3) + vals * a.rb;
+  return (b + a.align - 1) / (uint32_t)a.align * a.align;
 }
 
 // tier ids of this thread's kListPer tokens (consecutive; -1 past the end: ids are compared as int64)
@@ -83,6 +87,7 @@ __global__ void __launch_bounds__(kListThreads) list_count_kernel(const ListArgs
   const int chunk = blockIdx.x, u = blockIdx.y, lane = threadIdx.x & 31;
   if (threadIdx.x < SPHKV_MAX_TIER_SLOTS) s_cnt[threadIdx.x] = 0;
   __syncthreads();
+  griddep_launch();
   int64_t v[kListPer];
   load_tiers(a, u, (int64_t)chunk * kListChunk + threadIdx.x * kListPer, v);
   for (int s = 0; s < a.S; ++s) {
@@ -121,9 +126,10 @@ __device__ __forceinline__ T block_exclusive(T v, T* s_part, T& total) {
 __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs a) {
   __shared__ int64_t s_part[kScanThreads / 32];
   __shared__ int s_max[kScanThreads / 32];
+  griddep_wait();
   const int n_runs = a.S * a.U, ppb = 128 >> a.n_shift;
   int64_t c_pages = 0, c_bundles = 0, c_bytes = 0;
-  for (int r0 = 0; r0 < n_runs; r0 += kScanThreads) {
+  for (int r0 = 0; r0 < n_runs; r0 += blockDim.x) {
     const int r = r0 + threadIdx.x;
     int n = 0;
     if (r < n_runs) {
@@ -159,7 +165,7 @@ __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs 
   }
   __syncthreads();
   int most = 0;
-  for (int u = threadIdx.x; u < a.U; u += kScanThreads) {
+  for (int u = threadIdx.x; u < a.U; u += blockDim.x) {
     int col = 0;
     for (int s = 0; s < a.S; ++s) {
       a.col_base[s * a.U + u] = col;
@@ -171,11 +177,13 @@ __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs 
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = most;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < kScanThreads / 32; ++w) most = max(most, s_max[w]);
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) most = max(most, s_max[w]);
     a.totals[0] = c_pages;
     a.totals[1] = most;
     a.totals[2] = c_bundles;
     a.totals[3] = c_bytes + 16;
+    __threadfence_system();
+    *reinterpret_cast<volatile int64_t*>(a.totals + 4) = a.call;  // the host polls this word
   }
 }
 
@@ -187,6 +195,7 @@ __global__ void __launch_bounds__(kListThreads) list_fill_kernel(const ListArgs 
   __shared__ int s_part[kListThreads / 32];
   const int chunk = blockIdx.x, u = blockIdx.y, tid = threadIdx.x;
   const int N = a.N, ppb = 128 >> a.n_shift;
+  griddep_launch();
   const int64_t t_first = (int64_t)chunk * kListChunk;
   const int64_t row_first = (int64_t)(u / a.Hkv) * a.T;
   int64_t v[kListPer];
@@ -281,12 +290,18 @@ __global__ void __launch_bounds__(kScanThreads) list_offsets_kernel(const ListAr
   }
 }
 
-// The four totals land in pinned host memory: one small buffer per calling thread, freed with it.
+// The scan writes the four totals and a call number straight into pinned host memory: one small buffer per
+// calling thread, freed with it.
 struct PinnedTotals {
   int64_t* p = nullptr;
+  int64_t calls = 0;
   int64_t* get() {
-    if (p == nullptr && cudaHostAlloc(reinterpret_cast<void**>(&p), 4 * sizeof(int64_t), cudaHostAllocPortable) != cudaSuccess)
-      p = nullptr;
+    if (p == nullptr) {
+      if (cudaHostAlloc(reinterpret_cast<void**>(&p), 5 * sizeof(int64_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+        p = nullptr;
+      else
+        p[4] = 0;
+    }
     return p;
   }
   ~PinnedTotals() {
@@ -303,7 +318,7 @@ using namespace sphkv;
 extern "C" int64_t sphkv_page_lists_scratch_bytes(int32_t units, int64_t T, int32_t n_slots) {
   if (units <= 0 || T <= 0 || n_slots <= 0) return SPHKV_E_ARG;
   const int64_t runs = (int64_t)units * n_slots;
-  return 32 + runs * (8 + 16) + runs * list_chunks(T) * 4;
+  return runs * (8 + 16) + runs * list_chunks(T) * 4;
 }
 
 static int list_args(ListArgs& a, const sphkv_page_lists_params* p) {
@@ -332,8 +347,8 @@ static int list_args(ListArgs& a, const sphkv_page_lists_params* p) {
     a.tier_id[s] = p->tier_id[s]; a.G[s] = p->G[s]; a.bits[s] = p->bits[s];
   }
   const int64_t runs = (int64_t)a.U * a.S;
-  a.totals = reinterpret_cast<int64_t*>(p->scratch);
-  a.byte_base = a.totals + 4;
+  a.totals = nullptr;
+  a.byte_base = reinterpret_cast<int64_t*>(p->scratch);
   a.cnt = reinterpret_cast<int32_t*>(a.byte_base + runs);
   a.run_base = a.cnt + runs;
   a.bun_base = a.run_base + runs;
@@ -350,14 +365,21 @@ extern "C" int sphkv_page_lists_count(const sphkv_page_lists_params* p, int64_t*
   int64_t* host = pinned.get();
   SPHKV_REQUIRE(host != nullptr, SPHKV_E_LIMIT, "page_lists_count: no pinned host memory");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  a.totals = host;
+  a.call = ++pinned.calls;
   list_count_kernel<<<dim3(a.n_chunks, a.U), kListThreads, 0, st>>>(a);
-  list_scan_kernel<<<1, kScanThreads, 0, st>>>(a);
+  // as many warps as there are runs for (the prefix over the warps is serial)
+  const int scan_threads = std::min(kScanThreads, (a.S * a.U + 31) / 32 * 32);
+  (void)launch_overlapped(list_scan_kernel, dim3(1), dim3(scan_threads), 0, st, a);
   if (int rc = check_launch("page_lists_count")) return rc;
-  cudaError_t e = cudaMemcpyAsync(host, a.totals, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    set_error("page_lists_count: %s", cudaGetErrorString(e));
-    return (int)e;
+  // The host needs nothing but the totals, so it waits for the word behind them, not for the stream.  An
+  // error, or a stream that has ended without it, ends the wait.
+  for (int64_t spins = 1; __atomic_load_n(host + 4, __ATOMIC_ACQUIRE) != a.call; ++spins) {
+    if (spins % 16384 != 0) continue;
+    const cudaError_t e = cudaStreamQuery(st);
+    if (e == cudaErrorNotReady || __atomic_load_n(host + 4, __ATOMIC_ACQUIRE) == a.call) continue;
+    set_error("page_lists_count: %s", e == cudaSuccess ? "the totals did not arrive" : cudaGetErrorString(e));
+    return e == cudaSuccess ? (int)cudaErrorUnknown : (int)e;
   }
   for (int i = 0; i < 4; ++i) totals[i] = host[i];
   return 0;

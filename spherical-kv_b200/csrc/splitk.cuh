@@ -49,6 +49,7 @@ struct DecodeArgs {
   int wide;              // byte pool and positions start on 16-byte boundaries
   int plan_in_kernel;    // every CTA derives the block prefix itself (n_units small enough)
   int32_t* pfx;
+  uint32_t* spans;  // per unit, for the merge: first CTA with a partial row | number of them << 16
   float* rows;  // [(n_ctas + n_units)][8][dh + 2]
 };
 
@@ -136,15 +137,14 @@ __device__ __forceinline__ int find_unit(const int32_t* pfx, int n, int64_t x) {
 // kSegmentCost tiles of work).  By unit: unit u gets c_u = floor(nb_u n / T) CTAs (at least one) of equal
 // shares, and nobody meets two units.  The second is taken when its largest share is within that
 // cost of T / n: few units of similar size (2048 tokens x 8 heads: a step 22.3 -> 17.2 us, three rows of up
-// to 6001 tokens x 8 heads 40.3 -> 33.1 us; by range half the CTAs met two units).  Both kernels derive the
-// same answer from the block prefix; call with a whole warp.
+// to 6001 tokens x 8 heads 40.3 -> 33.1 us; by range half the CTAs met two units).  Call with a whole warp.
 constexpr int kSegmentCost = 30;
 struct UnitSplit {
   bool by_unit;
-  int u, first, count;  // the unit (given, or the one CTA `want_cta` works for), its first CTA, its CTAs
+  int u, first, count;  // the unit `cta` works for, its first CTA, its CTAs
 };
 __device__ __forceinline__ UnitSplit split_by_unit(const int32_t* pfx, int n_units, int n_ctas, int tiles_per_block,
-                                                   int want_unit, int want_cta) {
+                                                   int cta) {
   UnitSplit r;
   r.by_unit = false; r.first = r.count = 0; r.u = 0;
   const uint32_t T = (uint32_t)pfx[n_units];
@@ -166,8 +166,7 @@ __device__ __forceinline__ UnitSplit split_by_unit(const int32_t* pfx, int n_uni
   r.by_unit = true;
   uint32_t carry = 0;
   for (int base = 0; base < n_units; base += 32) {
-    const int i = base + lane;
-    const uint32_t c = ctas_of(blocks_of(i));
+    const uint32_t c = ctas_of(blocks_of(base + lane));
     uint32_t x = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -175,8 +174,7 @@ __device__ __forceinline__ UnitSplit split_by_unit(const int32_t* pfx, int n_uni
       if (lane >= o) x += y;
     }
     const uint32_t first = carry + x - c;
-    const unsigned hit = __ballot_sync(0xffffffffu, want_unit >= 0 ? i == want_unit
-                                                                   : (uint32_t)want_cta >= first && (uint32_t)want_cta < first + c);
+    const unsigned hit = __ballot_sync(0xffffffffu, (uint32_t)cta >= first && (uint32_t)cta < first + c);
     if (hit) {
       const int src = __ffs(hit) - 1;
       r.u = base + src;
@@ -218,7 +216,7 @@ static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 2
 // keys in flight and nothing else, twelve team warps fit an SM (the mma.sync version it replaced: eight, at
 // 244 registers, and shuffles, ldmatrix and accumulator moves around both products).
 // Bound: instruction issue and the waits between the roles, not HBM.  A 96-bit, 32768-token, batch-8 layer
-// step: 221.6 -> DECODE_US us (2.4 -> DECODE_TBS TB/s of the bytes it has to read).
+// step: 221.6 -> 157 us, merge included (2.5 -> 3.5 TB/s of the bytes it has to read).
 // Lane map of the rebuild (lane = 4 r + j): rows r and r + 8 of a tile are the lane's two tokens; in each
 // rotary half the lane owns the contiguous block of W = dh / 8 dimensions  W j .. W j + W - 1, and in the
 // other half the same block shifted by dh / 2: the RoPE partner of every value a lane holds is in the same
@@ -292,8 +290,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   griddep_wait();
   bool dead = false;  // a bounded wait ran out: stop working, keep meeting the barriers
 
-  // ---- block prefix per unit: computed by warp 0 of every CTA (CTA 0 publishes it for the
-  //      merge kernel), or read from the plan kernel's output when there are many units ----
+  // ---- block prefix per unit: computed by warp 0 of every CTA, or read from the plan kernel's output
+  //      when there are many units ----
   const int32_t* pfx = a.pfx;
   if (a.plan_in_kernel) {
     int32_t* pfx_s = reinterpret_cast<int32_t*>(smem + (cb_u32 - smem0) + a.cb_smem_bytes);
@@ -314,14 +312,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         }
         if (i < a.n_units) {
           pfx_s[i] = carry + x - v;
-          if (blockIdx.x == 0) a.pfx[i] = carry + x - v;
         }
         carry += __shfl_sync(0xffffffffu, x, 31);
       }
-      if (lane == 0) {
-        pfx_s[a.n_units] = carry;
-        if (blockIdx.x == 0) a.pfx[a.n_units] = carry;
-      }
+      if (lane == 0) pfx_s[a.n_units] = carry;
     }
     __syncthreads();
     pfx = pfx_s;
@@ -329,10 +323,12 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   const int64_t T = pfx[a.n_units];
   const int N = FAST ? 16 : p.page_size;
   int64_t start, end;
-  int u;
+  int u, unit_ctas = 0;  // unit_ctas: CTAs of the one unit of this CTA; 0: dealt by range
+  const int n_ctas = (int)min((int64_t)a.n_ctas, T);  // every CTA below has a block
   {
-    const UnitSplit us = split_by_unit(pfx, a.n_units, a.n_ctas, N >> 4, -1, blockIdx.x);
+    const UnitSplit us = split_by_unit(pfx, a.n_units, n_ctas, N >> 4, blockIdx.x);
     if (us.by_unit) {
+      unit_ctas = us.count;
       u = us.u;
       const int64_t first = pfx[u], nb = (int64_t)pfx[u + 1] - first;
       start = end = first;
@@ -341,8 +337,11 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         end = first + share_start(blockIdx.x - us.first + 1, us.count, nb);
       }
     } else {
-      start = cta_range_start(blockIdx.x, a.n_ctas, T);
-      end = cta_range_start(blockIdx.x + 1, a.n_ctas, T);
+      start = end = 0;
+      if ((int)blockIdx.x < n_ctas) {
+        start = cta_range_start(blockIdx.x, n_ctas, T);
+        end = cta_range_start(blockIdx.x + 1, n_ctas, T);
+      }
       u = start < end ? find_unit(pfx, a.n_units, start) : 0;
     }
   }
@@ -401,6 +400,12 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   for (; start < end; start = seg_end, ++u) {
     next_segment();
     const int u_ext = b * p.Hkv + hkv;
+    // the CTA of a unit's first block tells the merge kernel which CTAs the unit has (by range: the last one
+    // is the largest c with c T / n < the unit's end)
+    if (warp == 4 * kTeams + 3 && lane == 0 && lb0 == 0) {
+      const int count = unit_ctas > 0 ? unit_ctas : (int)(((int64_t)pfx[u + 1] * n_ctas - 1) / T) - (int)blockIdx.x + 1;
+      a.spans[u] = (uint32_t)blockIdx.x | ((uint32_t)count << 16);
+    }
     // ---- block table -> pointer table -> page header of 32 tiles at a time (lane = tile), the
     //      three dependent loads in separate rounds so that no round waits for a load it issued itself ----
     const int32_t* bt_row = p.block_table + (int64_t)u_ext * p.max_blocks;

@@ -31,11 +31,15 @@ _lib = _pkg._lib
 _L = _lib.load()
 
 
-def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_st = _lib.stream_ptr
 
 
 def _chk(t: torch.Tensor, dtype: torch.dtype, name: str) -> int:
+    try:  # a decode step checks twenty tensors
+        if t.dtype is dtype and t.is_cuda and t.is_contiguous():
+            return t.data_ptr()
+    except AttributeError:
+        pass
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise RuntimeError(f"{name}: expected a CUDA tensor")
     if t.dtype != dtype:
@@ -94,16 +98,18 @@ def fused_decode_ragged(pages_u8, ptable, head_ids, positions, cos_tbl, sin_tbl,
     f32, i32 = torch.float32, torch.int32
     n_pages = ptable.shape[0]
     hq = q.shape[0]
-    out = torch.empty(hq, n_pages * page_size, dtype=f32, device=q.device)  # the kernel writes every element
+    out = torch.empty((hq, n_pages * page_size), dtype=f32, device=q.device)  # the kernel writes every element
     if n_pages == 0:
         return out
-    cb = codebooks.contiguous()
+    # converted copies are named here: they have to outlive the launch call
+    ptable, head_ids, positions = (t if t.dtype is i32 and t.is_contiguous() else t.to(i32).contiguous()
+                                   for t in (ptable, head_ids, positions))
+    cos_tbl, sin_tbl, q, codebooks = (t if t.is_contiguous() else t.contiguous()
+                                      for t in (cos_tbl, sin_tbl, q, codebooks))
     rc = _L.sphkv_ragged_logits(
-        _chk(pages_u8, torch.uint8, "pages"), _chk(ptable.to(i32).contiguous(), i32, "ptable"),
-        _chk(head_ids.to(i32).contiguous(), i32, "head_ids"),
-        _chk(positions.to(i32).contiguous(), i32, "positions"),
-        _chk(cos_tbl.contiguous(), f32, "cos_tbl"), _chk(sin_tbl.contiguous(), f32, "sin_tbl"),
-        _chk(q.contiguous(), f32, "q"), _chk(cb, f32, "codebooks"), out.data_ptr(),
+        _chk(pages_u8, torch.uint8, "pages"), _chk(ptable, i32, "ptable"), _chk(head_ids, i32, "head_ids"),
+        _chk(positions, i32, "positions"), _chk(cos_tbl, f32, "cos_tbl"), _chk(sin_tbl, f32, "sin_tbl"),
+        _chk(q, f32, "q"), _chk(codebooks, f32, "codebooks"), out.data_ptr(),
         int(grp), int(num_kv), int(dh), int(groups), int(group_size), int(b_theta), int(page_size),
         int(n_pages), int(hq), int(cos_tbl.shape[0]), 0, 0, _st())
     _lib.check(rc, "sphkv_ragged_logits")

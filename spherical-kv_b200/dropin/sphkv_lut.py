@@ -40,8 +40,7 @@ _L = _lib.load()
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 
 
-def _st() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_st = _lib.stream_ptr
 
 
 def _f32_ptr(t, name: str, numel: int) -> int:

@@ -34,7 +34,7 @@ def kmeans_assign(U: torch.Tensor, centers: torch.Tensor, want_sim: bool = True
     counts = torch.empty(K, dtype=torch.int32, device=U.device)
     _lib.check(lib.sphkv_kmeans_assign(U.data_ptr(), N, d, centers.data_ptr(), K, assigns.data_ptr(),
                                        best.data_ptr() if want_sim else None, sums.data_ptr(),
-                                       counts.data_ptr(), torch.cuda.current_stream().cuda_stream),
+                                       counts.data_ptr(), _lib.stream_ptr()),
                "sphkv_kmeans_assign")
     return assigns, best, sums, counts
 

@@ -15,8 +15,7 @@ from .pages import PagedCache, PageLists, TierSet
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_stream = _lib.stream_ptr
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -25,7 +24,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 def _need_cuda(*ts: torch.Tensor) -> None:
     for t in ts:
-        if t is not None and (not t.is_cuda or not t.is_contiguous()):
+        if t is not None and not (t.is_cuda and t.is_contiguous()):
             raise _lib.SphKVError("expected contiguous CUDA tensors")
 
 
@@ -172,6 +171,53 @@ def decode_scratch(cache: PagedCache, n_ctas: int = 0) -> torch.Tensor:
     return torch.empty(nbytes, dtype=torch.uint8, device=cache.k_pages.device)
 
 
+def _decode_template(lib, cache: PagedCache, B: int, Hq: int, dh: int, n_ctas: int, dev) -> "_lib.DecodeParams":
+    """A copy of the parameter struct with everything filled in that belongs to the cache.  The filled struct
+    stays with the cache while nothing it was made from changes (60 ctypes assignments: 10 us a call)."""
+    L, scratch, status = cache.lists, cache.scratch, cache.status
+    if scratch is not None and status is not None:
+        key = (cache.k_pages.data_ptr(), cache.v_pool.data_ptr(), cache.codebooks.data_ptr(), scratch.data_ptr(),
+               scratch.numel(), status.data_ptr(), L.ptable.data_ptr(), L.positions.data_ptr(), L.block_table.data_ptr(),
+               L.bits_table.data_ptr(), L.num_blocks.data_ptr(), L.B, L.Hkv, L.page_size, L.max_blocks, L.n_pages,
+               cache.v_pool.dtype, cache.radius_fmt, id(cache.tiers), B, Hq, dh, n_ctas)
+        plan = cache.extra.get("decode_plan")
+        if plan is not None and plan[0] == key:
+            return _lib.DecodeParams.from_buffer_copy(plan[1])
+    assert B == L.B and dh == cache.dh
+    need = lib.sphkv_decode_scratch_bytes(L.B, L.Hkv, dh, n_ctas)
+    if scratch is None or scratch.numel() < need:
+        cache.scratch = scratch = decode_scratch(cache, n_ctas)
+    if status is None:
+        cache.status = status = torch.zeros(1, dtype=torch.int32, device=dev)
+    p = _lib.DecodeParams()
+    p.k_pages, p.ptable = cache.k_pages.data_ptr(), L.ptable.data_ptr()
+    p.v_pool, p.positions = cache.v_pool.data_ptr(), L.positions.data_ptr()
+    p.block_table, p.bits_table = L.block_table.data_ptr(), L.bits_table.data_ptr()
+    p.num_blocks, p.codebooks = L.num_blocks.data_ptr(), cache.codebooks.data_ptr()
+    p.scratch, p.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    p.status = status.data_ptr()
+    p.B, p.Hq, p.Hkv, p.dh = B, Hq, L.Hkv, dh
+    p.page_size, p.max_blocks, p.n_pages = L.page_size, L.max_blocks, L.n_pages
+    p.v_dtype, p.out_dtype = _DT[cache.v_pool.dtype], _lib.F32
+    p.radius_fmt, p.n_ctas = cache.radius_fmt, n_ctas
+    p.tiers = cache.tiers.to_c()
+    key = (p.k_pages, p.v_pool, p.codebooks, p.scratch, p.scratch_bytes, p.status, p.ptable, p.positions, p.block_table,
+           p.bits_table, p.num_blocks, L.B, L.Hkv, L.page_size, L.max_blocks, L.n_pages, cache.v_pool.dtype,
+           cache.radius_fmt, id(cache.tiers), B, Hq, dh, n_ctas)
+    cache.extra["decode_plan"] = (key, p, cache.tiers)  # the tier set is held: its id stays its own
+    return _lib.DecodeParams.from_buffer_copy(p)
+
+
+def _tile_stats(cache: PagedCache, B: int, Hq: int, dev) -> torch.Tensor:
+    """Workspace for the per-tile (max, sum) of a step that updates omega, kept with the cache."""
+    L = cache.lists
+    n = B * Hq * L.max_blocks * (L.page_size // 16) * 2
+    ws = cache.extra.get("tile_stats")
+    if ws is None or ws.numel() < n:
+        ws = cache.extra["tile_stats"] = torch.empty(n, dtype=torch.float32, device=dev)
+    return ws
+
+
 def decode_paged(q: torch.Tensor, cache: PagedCache, rope: Optional[torch.Tensor],
                  sm_scale: Optional[float] = None, out: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, out_partial: Optional[torch.Tensor] = None,
@@ -188,49 +234,39 @@ def decode_paged(q: torch.Tensor, cache: PagedCache, rope: Optional[torch.Tensor
     `omega` (f32 [B*Hkv, max_blocks]) is the page-importance EMA of
     spherical_kv_pipeline.py:952-987, updated in place inside the merge kernel from the
     per-tile statistics of this step; `page_ml` (f32 [B, Hq, max_blocks, page_size/16, 2]) is
-    allocated when omega is given without it.
+    kept with the cache when omega is given without it.
     `exchange` (split_kv.PeerExchange) turns the call into one rank's part of a split-KV decode:
     `cache` then holds this rank's share of every block list and the merge kernel trades the
     partial rows with the other ranks over peer memory before it writes `out`.
-    The split-K scratch and the status word live in `cache` (grown when a later call needs
+    The split-K scratch, the status word and (with omega alone) the tile statistics live in `cache` (grown when a later call needs
     more): one cache must not be decoded on two streams at once.  The status word is not read
     here (that would synchronise); `check_status(cache)` does it.
     """
     lib = _lib.load()
     L = cache.lists
     B, Hq, dh = q.shape
-    if omega is not None and page_ml is None:
-        page_ml = torch.empty(B, Hq, L.max_blocks, L.page_size // 16, 2, dtype=torch.float32, device=q.device)
-    _need_cuda(q, out, out_partial, page_ml, logits_out, rope, omega)
     if omega is not None:
         assert omega.dtype == torch.float32 and omega.is_contiguous() and omega.numel() == B * L.Hkv * L.max_blocks
-    assert B == L.B and dh == cache.dh
-    need = lib.sphkv_decode_scratch_bytes(L.B, L.Hkv, cache.dh, n_ctas)
-    if cache.scratch is None or cache.scratch.numel() < need:
-        cache.scratch = decode_scratch(cache, n_ctas)
-    if cache.status is None:
-        cache.status = torch.zeros(1, dtype=torch.int32, device=q.device)
+        if page_ml is None:  # consumed inside the call
+            page_ml = _tile_stats(cache, B, Hq, q.device)
+    _need_cuda(q, out, out_partial, page_ml, logits_out, rope, omega)
+    p = _decode_template(lib, cache, B, Hq, dh, n_ctas, q.device)
     if out is None and want_out:
-        out = torch.empty(B, Hq, dh, dtype=out_dtype or q.dtype, device=q.device)
-    p = _lib.DecodeParams()
-    p.q, p.k_pages, p.ptable = q.data_ptr(), cache.k_pages.data_ptr(), L.ptable.data_ptr()
-    p.v_pool, p.positions = cache.v_pool.data_ptr(), L.positions.data_ptr()
-    p.block_table, p.bits_table = L.block_table.data_ptr(), L.bits_table.data_ptr()
-    p.num_blocks, p.codebooks = L.num_blocks.data_ptr(), cache.codebooks.data_ptr()
-    p.rope_table = _ptr(rope)
-    p.out, p.out_partial, p.page_ml = _ptr(out), _ptr(out_partial), _ptr(page_ml)
-    p.logits_out = _ptr(logits_out)
-    p.scratch, p.scratch_bytes = cache.scratch.data_ptr(), cache.scratch.numel()
-    p.status = cache.status.data_ptr()
-    p.omega, p.ema_beta = _ptr(omega), ema_beta
-    p.B, p.Hq, p.Hkv, p.dh = B, Hq, L.Hkv, dh
-    p.page_size, p.max_blocks, p.n_pages = L.page_size, L.max_blocks, L.n_pages
-    p.max_pos = 0 if rope is None else rope.shape[0]
-    p.q_dtype, p.v_dtype = _DT[q.dtype], _DT[cache.v_pool.dtype]
-    p.out_dtype = _DT[out.dtype] if out is not None else _lib.F32
-    p.radius_fmt, p.n_ctas = cache.radius_fmt, n_ctas
-    p.sm_scale = (1.0 / math.sqrt(dh)) if sm_scale is None else sm_scale
-    p.tiers = cache.tiers.to_c()
+        out = torch.empty((B, Hq, dh), dtype=out_dtype or q.dtype, device=q.device)
+    p.q, p.q_dtype = q.data_ptr(), _DT[q.dtype]
+    if out is not None:
+        p.out, p.out_dtype = out.data_ptr(), _DT[out.dtype]
+    if rope is not None:
+        p.rope_table, p.max_pos = rope.data_ptr(), rope.shape[0]
+    if out_partial is not None:
+        p.out_partial = out_partial.data_ptr()
+    if page_ml is not None:
+        p.page_ml = page_ml.data_ptr()
+    if logits_out is not None:
+        p.logits_out = logits_out.data_ptr()
+    if omega is not None:
+        p.omega, p.ema_beta = omega.data_ptr(), ema_beta
+    p.sm_scale = 1.0 / math.sqrt(dh) if sm_scale is None else sm_scale
     if exchange is not None and exchange.world > 1:
         exchange.check_shape(B, Hq, L.Hkv, dh)
         p.xchg_recv = exchange.recv_ptrs.data_ptr()

@@ -53,6 +53,7 @@ class TierSet:
         for t in self.tiers:
             if t.g not in (16, 32) or dh % (2 * t.g) or not 1 <= t.b_theta <= 6:
                 raise ValueError(f"unsupported tier {t} for dh={dh}")
+        self._c = None
         self.G_max = max(dh // t.g for t in self.tiers)
         self.C_max = max(t.codebook_size for t in self.tiers)
         self.g_max = max(t.g for t in self.tiers)
@@ -70,11 +71,15 @@ class TierSet:
         return self.dh // self.tiers[slot].g
 
     def to_c(self) -> "_lib.Tiers":
+        """The C struct (one object per set: a set does not change; callers copy or only read it)."""
+        if self._c is not None:
+            return self._c
         c = _lib.Tiers()
         c.n_slots = len(self.tiers)
         c.G_max, c.C_max, c.g_max = self.G_max, self.C_max, self.g_max
         for s, t in enumerate(self.tiers):
             c.g[s], c.bits[s], c.tier_id[s] = t.g, t.b_theta, t.tier_id
+        self._c = c
         return c
 
     def pack_codebooks(self, per_tier: Sequence[torch.Tensor]) -> torch.Tensor:
@@ -125,6 +130,8 @@ class PageLists:
 
 
 _NATIVE_IDS = (torch.uint8, torch.int32, torch.int64)
+_TABLES = ("positions", "src_index", "page_head", "page_slot", "page_count", "ptable", "block_table", "bits_table",
+           "num_blocks", "bundles")
 
 
 def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fmt: int, page_align: int,
@@ -133,7 +140,7 @@ def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fm
     with a page permutation).  32768 tokens x 8 heads: 1.8 ms as array operations."""
     B, Hkv, T = ta.shape
     U, N, S, dev = B * Hkv, page_size, len(tiers), ta.device
-    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    lib, st = _lib.load(), _lib.stream_ptr()
     ta = ta.contiguous()
     p = _lib.PageListsParams()
     need = lib.sphkv_page_lists_scratch_bytes(U, T, S)
@@ -154,19 +161,27 @@ def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fm
     perm = None
     if shuffle_seed is not None:
         perm = torch.randperm(P, generator=torch.Generator().manual_seed(shuffle_seed)).to(dev)
-    new = lambda *shape: torch.empty(shape, dtype=torch.int32, device=dev)  # noqa: E731
-    L = PageLists(page_size=N, n_pages=P, positions=new(P, N), src_index=new(P, N), page_head=new(P), page_slot=new(P),
-                  page_count=new(P), ptable=new(P, 3), block_table=new(U, max_blocks), bits_table=new(U, max_blocks),
-                  num_blocks=new(U), bundles=new(n_bundles, 8), pool_bytes=pool_bytes, B=B, Hkv=Hkv,
-                  max_blocks=max_blocks, covers_pool=True)
+    # one allocation for the ten tables (an allocator call each was a third of a short prompt's host time), each
+    # on a 256-byte boundary
+    shapes = ((P, N), (P, N), (P,), (P,), (P,), (P, 3), (U, max_blocks), (U, max_blocks), (U,), (n_bundles, 8))
+    cuts, at = [], 0
+    for f, shape in zip(_TABLES, shapes):
+        n = shape[0] * shape[1] if len(shape) == 2 else shape[0]
+        room = (n + 63) // 64 * 64
+        cuts += (n, room - n)
+        setattr(p, f, at * 4)  # offset for now
+        at += room
+    buf = torch.empty(at, dtype=torch.int32, device=dev)
+    base, parts = buf.data_ptr(), buf.split(cuts)
+    tables = {}
+    for i, (f, shape) in enumerate(zip(_TABLES, shapes)):
+        setattr(p, f, base + (getattr(p, f) or 0))
+        tables[f] = parts[2 * i].view(shape) if len(shape) == 2 else parts[2 * i]
     p.n_pages, p.max_blocks = P, max_blocks
     p.perm = None if perm is None else perm.data_ptr()
-    p.positions, p.src_index = L.positions.data_ptr(), L.src_index.data_ptr()
-    p.page_head, p.page_slot, p.page_count = L.page_head.data_ptr(), L.page_slot.data_ptr(), L.page_count.data_ptr()
-    p.ptable, p.block_table, p.bits_table = L.ptable.data_ptr(), L.block_table.data_ptr(), L.bits_table.data_ptr()
-    p.num_blocks, p.bundles = L.num_blocks.data_ptr(), L.bundles.data_ptr()
     _lib.check(lib.sphkv_page_lists_fill(C.byref(p), st), "sphkv_page_lists_fill")
-    return L
+    return PageLists(page_size=N, n_pages=P, pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks,
+                     covers_pool=True, **tables)
 
 
 def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
@@ -190,8 +205,11 @@ def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
     # sizes and id types that the kernels do not take.
     if (dev.type == "cuda" and N in (16, 32, 64, 128) and tier_assign.dtype in _NATIVE_IDS and T > 0
             and 0 < B * Hkv <= 65535 and extra_blocks >= 0):
+        args = (tier_assign, tiers, N, radius_fmt, page_align, shuffle_seed, extra_blocks)
+        if torch.cuda.current_device() == dev.index:
+            return _build_on_device(*args)
         with torch.cuda.device(dev):
-            return _build_on_device(tier_assign, tiers, N, radius_fmt, page_align, shuffle_seed, extra_blocks)
+            return _build_on_device(*args)
     U = B * Hkv
     rb = 2 if radius_fmt == _lib.RADIUS_F16 else 1
     ppb = 128 // N
