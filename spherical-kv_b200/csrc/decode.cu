@@ -89,7 +89,7 @@ __global__ void plan_kernel(const int32_t* __restrict__ num_blocks, int n_units,
 // units, dh 64: 5.3 -> 3.7 us; with the importance update of three rows at 128-token pages 12.3 -> 4.9 us.
 template <int DH>
 __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) {
-  constexpr int kChunk = 128;  // partial rows combined per pass (general path)
+  constexpr int kChunk = 32;   // partial rows combined per pass (general path); shared memory is kept small: see kSmemMax
   constexpr int kBatch = 16;   // rows' loads in flight at a time
   const sphkv_decode_params& p = a.p;
   const int u = blockIdx.x;  // traversal index: hkv * B + b
@@ -97,7 +97,11 @@ __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = threadIdx.x / DH, d = threadIdx.x % DH;  // this thread's query head (warp-uniform) and dimension
   __shared__ float s_M[8], s_L[8];
-  __shared__ float s_w[8][kChunk];
+  __shared__ union {
+    float w[8][kChunk];
+    struct { float m[SPHKV_MAX_XCHG_RANKS][8], l[SPHKV_MAX_XCHG_RANKS][8]; } rank;  // exchange: the ranks' rows
+  } s_u;
+  auto& s_w = s_u.w;
   // launched like the decode kernel: its blocks wait here for it to end, and let the next step's in early
   griddep_wait();
   griddep_launch();
@@ -251,7 +255,8 @@ __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) 
   //      validates itself: no fence, no separate flag, one NVLink crossing per value.  Peer
   //      memory is touched by plain stores only; the words a rank reads are in its own memory.
   __shared__ int s_seq, s_ok;
-  __shared__ float s_rm[SPHKV_MAX_XCHG_RANKS][8], s_rl[SPHKV_MAX_XCHG_RANKS][8];
+  auto& s_rm = s_u.rank.m;
+  auto& s_rl = s_u.rank.l;
   const int64_t n_rows = (int64_t)p.B * p.Hq;
   if (threadIdx.x == 0) {
     s_seq = p.xchg_seq[unit] + 1;
@@ -405,18 +410,18 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// V pool viewed as a 2-D tensor [n_pages * page_size rows][dh] of 16-bit elements; a box is 16
-// rows x 64 elements (128 bytes, the widest row the 128-byte swizzle takes).  Encoding is host
-// arithmetic only (no device memory, no driver state).
+// V pool viewed as a 3-D tensor [dh / 64][n_pages * page_size rows][64] of 16-bit elements; a box is all the
+// 64-element slices (128 bytes, the widest row the 128-byte swizzle takes) of 16 rows, so a tile is one
+// copy.  Encoding is host arithmetic only (no device memory, no driver state).
 static int make_v_map(CUtensorMap* map, const sphkv_decode_params& p) {
   EncodeTiledFn fn = encode_tiled_fn();
   SPHKV_REQUIRE(fn != nullptr, SPHKV_E_ARG, "decode: cuTensorMapEncodeTiled is not available from this driver");
-  const cuuint64_t dims[2] = {(cuuint64_t)p.dh, (cuuint64_t)p.n_pages * (cuuint64_t)p.page_size};
-  const cuuint64_t strides[1] = {(cuuint64_t)p.dh * 2};
-  const cuuint32_t box[2] = {64, 16};
-  const cuuint32_t estr[2] = {1, 1};
+  const cuuint64_t dims[3] = {64, (cuuint64_t)p.n_pages * (cuuint64_t)p.page_size, (cuuint64_t)p.dh / 64};
+  const cuuint64_t strides[2] = {(cuuint64_t)p.dh * 2, 128};
+  const cuuint32_t box[3] = {64, 16, (cuuint32_t)p.dh / 64};
+  const cuuint32_t estr[3] = {1, 1, 1};
   const CUresult rc = fn(map, p.v_dtype == SPHKV_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                         2, const_cast<void*>(p.v_pool), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         3, const_cast<void*>(p.v_pool), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   SPHKV_REQUIRE(rc == CUDA_SUCCESS, SPHKV_E_ARG, "decode: cuTensorMapEncodeTiled failed (%d) for the V pool", (int)rc);
@@ -549,15 +554,18 @@ extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
   a.wide = ((reinterpret_cast<uintptr_t>(p.k_pages) | reinterpret_cast<uintptr_t>(p.positions)) & 15) == 0;
   a.plan_in_kernel = a.n_units <= kMaxUnitsInKernelPlan ? 1 : 0;
   const int pfx_bytes = a.plan_in_kernel ? (a.n_units + 1) * 4 : 0;
+  // a little less than an SM has, so that this kernel's blocks become resident beside the merge blocks of the
+  // step before (which keep 2 KB) and set themselves up while those finish
+  constexpr int kSmemMax = 230272;  // 228 KB less 1 KB per block and the merge kernel's 1.1
   int smem_bytes = 0;
   for (a.teams = kTeams; a.teams >= 1; --a.teams) {
     const int fixed_bytes = smem_fixed_bytes(p.dh, a.teams) + pfx_bytes;
-    a.cb_smem_bytes = smem_cb_layout(p.tiers, p.dh, 227 * 1024 - fixed_bytes, a.cb_smem_off, a.cb_dup);
+    a.cb_smem_bytes = smem_cb_layout(p.tiers, p.dh, kSmemMax - fixed_bytes, a.cb_smem_off, a.cb_dup);
     smem_bytes = fixed_bytes + a.cb_smem_bytes;
-    if (smem_bytes <= 227 * 1024) break;
+    if (smem_bytes <= kSmemMax) break;
   }
   SPHKV_REQUIRE(a.teams >= 1, SPHKV_E_LIMIT,
-                "decode: codebooks need %d B of shared memory (limit %d)", smem_bytes, 227 * 1024);
+                "decode: codebooks need %d B of shared memory (limit %d)", smem_bytes, kSmemMax);
   if (int rc = make_v_map(&a.v_map, p)) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 

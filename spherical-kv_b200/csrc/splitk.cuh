@@ -12,19 +12,23 @@ constexpr int kTeams = 3;
 constexpr int kTeamThreads = 4 * kTeams * 32, kDecodeThreads = kTeamThreads + 4 * 32;
 constexpr int kMacroTiles = 8;   // 16-token tiles per macro tile (128 rows)
 constexpr int kMetaRing = 64;    // tiles of metadata per team, refilled 32 at a time
-constexpr int kKStages = 2;      // macro tiles of page bytes per team
+// Macro tiles of page bytes per team.  Three when a tile's stage is small enough (int8 radii): a copy issued
+// while the teams weigh macro tile k has to land before they finish rebuilding the first half of k + 1,
+// which two stages leave no room for under load.
+constexpr int kKStages = 3;
 // Registers: the launch gives every thread 128; the drivers return theirs to the teams
 // (3 * 152 + 56 = 4 * 128 per four warps).
 constexpr int kTeamRegs = 152, kDriverRegs = 56;
 static_assert(kTeams * kTeamRegs + kDriverRegs <= 4 * 128 && kTeams == 3, "register split exceeds the launch");
 // tensor memory columns of a team: rebuilt keys (hi | lo), logits, output accumulator
 constexpr int kColKeys = 0, kColLogits = 128, kColOut = 144, kTeamCols = 160, kTmemCols = 512;
+static_assert(kKStages <= 3 && kMetaRing == 8 * kMacroTiles, "metadata is ready three macro tiles ahead");
 static_assert(kTeams * kTeamCols <= kTmemCols, "tensor memory");
 
 // One 16-token tile, computed by the driver for 32 tiles at a time (16 bytes in the metadata ring)
 struct TileMeta {
   int phys;        // physical page id; -1 hole / invalid page, -2 no such tile
-  uint32_t where;  // tokens of the tile | tier slot << 8 | stage byte offsets: header << 12, theta << 16
+  uint32_t where;  // tokens of the tile, at most | tier slot << 8 | stage byte offsets: header << 12, theta << 16
                    // (bytes; 9 bits); sub tile of the page << 28
   uint32_t rad;    // stage byte offset of the tile's first radius byte | (theta - page) << 9 | (radii - theta) << 16
   int poff;        // page offset in the byte pool
@@ -37,7 +41,7 @@ __device__ __forceinline__ uint32_t meta_radius(const TileMeta& m) { return m.ra
 __device__ __forceinline__ int meta_sub(const TileMeta& m) { return m.where >> 28; }
 
 struct DecodeArgs {
-  alignas(64) CUtensorMap v_map;  // V pool as [pages * page_size rows][dh], 16 x 64 boxes, 128-byte swizzle
+  alignas(64) CUtensorMap v_map;  // V pool as [dh / 64][pages * page_size rows][64], boxes of 16 rows, 128-byte swizzle
   sphkv_decode_params p;
   int cb_smem_off[SPHKV_MAX_TIER_SLOTS];  // byte offset of each slot's codebook in smem
   int cb_dup[SPHKV_MAX_TIER_SLOTS];       // 1: two copies at a 128-byte row pitch
@@ -57,9 +61,9 @@ struct DecodeArgs {
 // metadata, query operand, barriers; then codebooks and the block prefix
 __host__ __device__ constexpr int smem_v_bytes(int dh) { return kMacroTiles * 16 * dh * 2; }  // per team
 constexpr int kSmemP = kMacroTiles * 512;                                                      // per team
-constexpr int kSmemK = kKStages * kMacroTiles * 512;                                           // per team
+constexpr int kSmemK = 3 * kMacroTiles * 384;                                                  // per team (f16 radii: 2 x 512)
 constexpr int kSmemMeta = kMetaRing * 16;                                                      // per team
-constexpr int kSmemBars = 2048;
+constexpr int kSmemBars = 1792;
 __host__ __device__ constexpr int smem_q_bytes(int dh) { return dh / 16 * 512; }
 __host__ __device__ constexpr int smem_fixed_bytes(int dh, int teams) {
   return teams * (smem_v_bytes(dh) + kSmemP + kSmemK + kSmemMeta) + smem_q_bytes(dh) + kSmemBars;
@@ -193,18 +197,17 @@ __device__ __forceinline__ int64_t share_start(int i, int n, int64_t nb) { retur
 // A 16-token page is staged whole; of a larger page the header + group scales, the slice of the theta
 // bit stream of the tile's 16 tokens and the slice of their radius bytes go to fixed offsets; plus the
 // tile's 16 positions.  Every piece keeps the phase inside 16 bytes that it has in the pool.
-constexpr int kKStageBytes = 512;
 constexpr int kKHdr = 0;    // 8 header bytes + up to 8 scales = 40, + 12 phase
 constexpr int kKTh = 64;    // 16 tokens x 8 groups x 6 bits = 96 bytes + 15 phase
-constexpr int kKRd = 176;   // 16 tokens x 8 groups x 2 bytes = 256 bytes + 15 phase
-constexpr int kKPos = 448;  // 16 words
-static_assert(kKTh + 112 <= kKRd && kKRd + 272 <= kKPos && kKPos + 64 <= kKStageBytes, "K stage layout");
-// the largest 16-token page, 8 + 32 + 96 + 256 bytes + 12 phase, ends before the positions as well
+constexpr int kKRd = 176;   // 16 tokens x 8 groups x 1 or 2 bytes + 15 phase
+// int8 radii: stages of 384 bytes, positions in the last 64; f16: 512
+static_assert(kKTh + 112 <= kKRd && kKRd + 128 + 16 <= 384 - 64 && kKRd + 256 + 16 <= 512 - 64, "K stage layout");
+// the largest 16-token page, 8 + 32 + 96 + 128 (256) bytes + 12 phase, ends before the positions as well
 
 // barriers of a team (8 bytes each, kBarStride per team)
 enum { kBarKFull = 0, kBarKeys = kKStages, kBarKeys2, kBarLogits, kBarWeights, kBarV, kBarOut, kBarVote, kBarCount };
 constexpr int kBarStride = 128;
-static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 256 + 32) + 16 <= kSmemBars, "barrier block");
+static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 256 + 32) + 64 <= kSmemBars, "barrier block");
 
 // A team of four warps rebuilds 128 keys (eight 16-token tiles) into tensor memory, its driver warp --
 // which also fetches everything -- issues the two contractions:
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + (bar_all - smem0) + kSmemBars - 16);
   const uint32_t cb_u32 = bar_all + kSmemBars;
 
-  // ---- set-up: barriers, tensor memory, the zero columns of the weights ----
+  // ---- set-up: barriers, tensor memory, the zero columns of the weights and of the query operand ----
   if (driver && in_use && lane == 0) {
     for (int i = 0; i < kKStages; ++i) mbar_init(bar + 8 * (kBarKFull + i), 33);  // 32 copy arrivals + plain stores
     mbar_init(bar + 8 * kBarKeys, 4);
@@ -273,8 +276,11 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     mbar_init(bar + 8 * kBarOut, 1);
     mbar_init(bar + 8 * kBarVote, 4);
   }
-  if (!driver && in_use)
-    for (int i = threadIdx.x & 127; i < kSmemP / 16; i += 128) sts128(p_buf + 16 * i, 0, 0, 0, 0);
+  if (!driver) {
+    if (in_use)
+      for (int i = threadIdx.x & 127; i < kSmemP / 16; i += 128) sts128(p_buf + 16 * i, 0, 0, 0, 0);
+    for (int i = threadIdx.x; i < smem_q_bytes(DH) / 16; i += kTeamThreads) sts128(q_u32 + 16 * i, 0, 0, 0, 0);
+  }
   if (warp == 4 * kTeams + 3) {
     if (lane == 0) shared_words[1] = 0;
     tmem_alloc(smem_u32(const_cast<uint32_t*>(shared_words)), kTmemCols);
@@ -297,23 +303,27 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     int32_t* pfx_s = reinterpret_cast<int32_t*>(smem + (cb_u32 - smem0) + a.cb_smem_bytes);
     if (warp == 0) {
       int carry = 0;
-      for (int base = 0; base < a.n_units; base += 32) {
-        const int i = base + lane;
-        int v = 0;
-        if (i < a.n_units) {
-          v = p.num_blocks[(i % p.B) * p.Hkv + i / p.B];
-          v = v < 0 ? 0 : (v > p.max_blocks ? p.max_blocks : v);
-        }
-        int x = v;
+      for (int base = 0; base < a.n_units; base += 128) {
+        int v[4];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, x, o);
-          if (lane >= o) x += y;
+        for (int q = 0; q < 4; ++q) {  // four loads in flight
+          const int i = base + 32 * q + lane;
+          v[q] = i < a.n_units ? p.num_blocks[(i % p.B) * p.Hkv + i / p.B] : 0;
         }
-        if (i < a.n_units) {
-          pfx_s[i] = carry + x - v;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = base + 32 * q + lane;
+          if (base + 32 * q >= a.n_units) break;
+          v[q] = v[q] < 0 ? 0 : (v[q] > p.max_blocks ? p.max_blocks : v[q]);
+          int x = v[q];
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+          }
+          if (i < a.n_units) pfx_s[i] = carry + x - v[q];
+          carry += __shfl_sync(0xffffffffu, x, 31);
         }
-        carry += __shfl_sync(0xffffffffu, x, 31);
       }
       if (lane == 0) pfx_s[a.n_units] = carry;
     }
@@ -350,6 +360,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   const int tpp_shift = 31 - __clz(TPP);
   const int fmt = FAST ? SPHKV_RADIUS_I8 : p.radius_fmt;
   const uint32_t rb = fmt == SPHKV_RADIUS_F16 ? 2u : 1u;
+  const uint32_t kst_bytes = rb == 2 ? 512 : 384, kst_pos = kst_bytes - 64;  // K stage of a tile, its positions
+  const int n_stages = rb == 2 ? 2 : kKStages;
   // per tier slot: b_theta | log2(g) << 8 | duplicated << 12 | codebook offset in shared
   // memory << 13, held by lanes 0..3 and read with a shuffle
   uint32_t tier_word = 0;
@@ -406,8 +418,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       const int count = unit_ctas > 0 ? unit_ctas : (int)(((int64_t)pfx[u + 1] * n_ctas - 1) / T) - (int)blockIdx.x + 1;
       a.spans[u] = (uint32_t)blockIdx.x | ((uint32_t)count << 16);
     }
-    // ---- block table -> pointer table -> page header of 32 tiles at a time (lane = tile), the
-    //      three dependent loads in separate rounds so that no round waits for a load it issued itself ----
+    // ---- block table -> pointer table of 32 tiles at a time (lane = tile), the dependent loads in separate
+    //      rounds so that no round waits for a load it issued itself.  How many tokens the page can hold
+    //      follows from the size of its theta stream; the header's count is applied by the teams, from
+    //      the staged bytes (reading it here would be one more memory latency before the page copies) ----
     const int32_t* bt_row = p.block_table + (int64_t)u_ext * p.max_blocks;
     const int32_t* st_row = p.bits_table + (int64_t)u_ext * p.max_blocks;
     int mf_phys = -2, mf_slot = 0, mf_poff = 0, mf_toff = 0, mf_roff = 0;
@@ -437,15 +451,14 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       mf_toff = p.ptable[3 * (int64_t)mf_phys + 1];
       mf_roff = p.ptable[3 * (int64_t)mf_phys + 2];
     };
-    auto meta_headers = [&](int kb) {
+    auto meta_store = [&](int kb) {
       TileMeta m;
       m.phys = mf_phys; m.poff = mf_poff; m.where = m.rad = 0;
       if (mf_phys >= 0) {
-        const uint32_t hdr = *reinterpret_cast<const uint32_t*>(p.k_pages + mf_poff);
-        const int count = min((int)((hdr >> 8) & 0xFFu), N);
         const int sub = (first_tile(kb + (lane >> 3)) + (lane & 7)) & (TPP - 1);
         const uint32_t bits = p.tiers.bits[mf_slot], G = DH / p.tiers.g[mf_slot];
         const uint32_t phase = (uint32_t)mf_poff & 15u;
+        const int th_bytes = mf_roff - mf_toff;
         uint32_t th, rd;
         if (TPP == 1) {
           th = phase + (uint32_t)(mf_toff - mf_poff);
@@ -454,14 +467,17 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           th = kKTh + (((uint32_t)mf_toff + ((16u * sub * G * bits) >> 3)) & 15u);
           rd = kKRd + (((uint32_t)mf_roff + 16u * sub * G * rb) & 15u);
         }
-        if (mf_toff - mf_poff != (int)(8 + 4 * G) || mf_roff < mf_toff || mf_roff - mf_toff > N * 6) {
+        if (mf_toff - mf_poff != (int)(8 + 4 * G) || th_bytes < 0 || th_bytes > N * 6) {
           // the pointer table disagrees with the page format: not a page this kernel can read
           if (p.status) atomicOr(p.status, SPHKV_ST_BAD_BLOCK);
           m.phys = -1;
         } else {
+          int count = min(N, (int)((uint32_t)th_bytes * 8u / (G * bits)));
+          if (G * bits < 8)  // several counts share a stream size: the header it is
+            count = min(count, (int)p.k_pages[mf_poff + 1]);
           const int tokens = min(16, max(0, count - 16 * sub));
           m.where = (uint32_t)tokens | ((uint32_t)mf_slot << 8) | (phase << 12) | (th << 16) | ((uint32_t)sub << 28);
-          m.rad = rd | ((uint32_t)(mf_toff - mf_poff) << 9) | ((uint32_t)(mf_roff - mf_toff) << 16);
+          m.rad = rd | ((uint32_t)(mf_toff - mf_poff) << 9) | ((uint32_t)th_bytes << 16);
         }
       }
       sts_meta(meta + ((kb * kMacroTiles + lane) & (kMetaRing - 1)) * 16, m);
@@ -469,7 +485,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     };
     auto get_meta = [&](int k, int x) { return lds_meta(meta + ((k * kMacroTiles + x) & (kMetaRing - 1)) * 16); };
 
-    // V tiles of macro tile k: one or two boxes of 16 rows x 128 bytes per tile through the tensor map,
+    // V tiles of macro tile k: one box of dh / 64 x 16 rows x 128 bytes per tile through the tensor map,
     // hardware swizzle = chunk ^ (row & 7).  Returns the tiles that hold tokens.
     auto issue_v = [&](int k) -> unsigned {
       TileMeta m;
@@ -486,9 +502,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       __syncwarp();
       if (have) {
         const int y = m.phys * N + 16 * meta_sub(m);
-#pragma unroll
-        for (int h = 0; h < DH / 64; ++h)
-          tma_load_2d(v_buf + lane * V_TILE + h * 2048, &a.v_map, 64 * h, y, bar + 8 * kBarV, v_policy);
+        tma_load_3d(v_buf + lane * V_TILE, &a.v_map, 0, y, 0, bar + 8 * kBarV, v_policy);
       }
       return mask;
     };
@@ -497,13 +511,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     // hold it (it keeps its byte phase inside the first), its last, partial chunk as words: nothing past
     // the piece's last word is read.  16-token pages are one piece; of larger ones the header, the
     // tile's slice of the theta stream and of the radii.  Pools off a 16-byte boundary: words only.
-    auto issue_k = [&](int k) {
-      const int stage = k & (kKStages - 1), x = lane >> 2, q = lane & 3;
+    auto issue_k = [&](int k, int stage) {
+      const int x = lane >> 2, q = lane & 3;
       TileMeta m;
       m.phys = -2; m.poff = 0; m.where = 0; m.rad = 0;
       if (x < width) m = get_meta(k, x);
       const uint32_t tw = tier_of(meta_slot(m));
-      const uint32_t kb = k_ring + (stage * kMacroTiles + x) * kKStageBytes;
+      const uint32_t kb = k_ring + (stage * kMacroTiles + x) * kst_bytes;
       auto piece = [&](uint32_t dst, uint32_t src, uint32_t stop) {
         const uint32_t s0 = src & ~15u;
         uint32_t o = src & ~3u;
@@ -530,14 +544,14 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         if (ROT) {
           const int32_t* ps = p.positions + ((uint32_t)m.phys * (uint32_t)N + 16u * sub + 4 * q);
           if (a.wide) {
-            cp_async_16(kb + kKPos + 16 * q, ps);
+            cp_async_16(kb + kst_pos + 16 * q, ps);
           } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cp_async_4(kb + kKPos + 16 * q + 4 * e, ps + e);
+            for (int e = 0; e < 4; ++e) cp_async_4(kb + kst_pos + 16 * q + 4 * e, ps + e);
           }
         }
       } else if (ROT && x < width) {
-        sts128(kb + kKPos + 16 * q, ~0u, ~0u, ~0u, ~0u);  // no page: its positions read as "no token"
+        sts128(kb + kst_pos + 16 * q, ~0u, ~0u, ~0u, ~0u);  // no page: its positions read as "no token"
       }
       cp_async_arrive(bar + 8 * (kBarKFull + stage));
       __syncwarp();
@@ -548,21 +562,23 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     if (rounds > 0) {
       meta_blocks(0);
       meta_pointers();
-      meta_headers(0);
-      issue_k(0);
-      if (rounds > 1) issue_k(1);
+      meta_store(0);
+      for (int i = 0; i < min(rounds, n_stages); ++i) issue_k(i, i);
       v_tiles = issue_v(0);
+      meta_blocks(4);
     }
     bool started = false;
     const uint64_t q_desc = smem_desc(q_u32, 128, 256, 0), p_desc = smem_desc(p_buf, 128, 256, 0);
     const uint64_t v_desc = smem_desc(v_buf, DH == 128 ? 2048 : 0, 1024, 2);
-    for (int k = 0; k < rounds; ++k) {
-      {  // the next four macro tiles' metadata
-        const int ph = k & 3, kb = (k & ~3) + 4;
-        if (ph == 0) meta_blocks(kb);
-        else if (ph == 1) meta_pointers();
-        else if (ph == 2) meta_headers(kb);
-      }
+    for (int k = 0, st = 0; k < rounds; ++k) {
+      // the metadata of the next four macro tiles, stored before the first of them is fetched (k + 3 at most)
+      // and after the teams have finished what it replaces in the ring (k - 5 and before)
+      if ((k & 3) == 0)
+        meta_pointers();
+      else if ((k & 3) == 1)
+        meta_store(k + 3);
+      else if ((k & 3) == 3)
+        meta_blocks(k + 5);
       // the first chunks of the keys are multiplied while the teams rebuild the last
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
@@ -578,7 +594,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       if (dead) break;
       par_keys ^= 1;
       __syncwarp();
-      if (k + kKStages < rounds) issue_k(k + kKStages);  // the team has read macro tile k's stage
+      if (k + n_stages < rounds) issue_k(k + n_stages, st);  // the team has read macro tile k's stage
+      if (++st == n_stages) st = 0;
       const bool got = mbar_wait(bar + 8 * kBarWeights, par_weights) && mbar_wait(bar + 8 * kBarV, par_v);
       if (!__all_sync(0xffffffffu, got)) { dead = true; break; }
       par_weights ^= 1;
@@ -619,16 +636,17 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       const int dup = a.cb_dup[s];
       const float* src = p.codebooks + ((int64_t)(hkv * tg.n_slots + s) * tg.G_max) * tg.C_max * tg.g_max;
       const uint32_t dst = cb_u32 + a.cb_smem_off[s];
-      const int chunks = (G << bits) * cpr;
+      const int lc = g == 32 ? 3 : 2;  // log2 of the chunks per row
+      const int chunks = (G << bits) << lc;
       // asynchronous 16-byte copies: every chunk of the codebook is in flight at once instead
       // of one load-store round trip per loop iteration (the caller waits for the group)
       for (int i = threadIdx.x; i < chunks; i += kTeamThreads) {
-        const int c4 = i % cpr, row = i / cpr;
+        const int c4 = i & (cpr - 1), row = i >> lc;
         const int c = row & ((1 << bits) - 1), gam = row >> bits;
         const int to = c4 ^ ((((gam * g + c4 * 4) & (DH / 2 - 1)) / W) & (NCH - 1));
         const int gh = gam >= (G >> 1) ? gam - (G >> 1) : gam;
         const uint32_t at = dst + gh * 16 + (gam >= (G >> 1) ? 64 : 0);
-        const float4* sp = reinterpret_cast<const float4*>(src + ((int64_t)gam * tg.C_max + c) * tg.g_max) + c4;
+        const float4* sp = reinterpret_cast<const float4*>(src + (gam * tg.C_max + c) * tg.g_max) + c4;
         if (dup) {
           cp_async_16(at + (row * 8 + to) * 16, sp);
           cp_async_16(at + (row * 8 + 4 + to) * 16, sp);
@@ -641,27 +659,41 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   };
   // Query operand of a unit: bf16 hi (truncated) and lo parts of q * sm_scale * log2(e), 16 columns x 16
   // dims per block, K-major, no swizzle: 8-column groups at 256 bytes, 8-dim groups at 128.  Block
-  // half * NCH + i holds, for lane quad member j, the four dims of chunk i: k = 4 j + e.
-  auto stage_query = [&]() {
-    const float qscale = p.sm_scale * kLog2e;
-    for (int i = threadIdx.x; i < DH * 16; i += kTeamThreads) {
-      const int k = i & 15, n = (i >> 4) & 15, blk = i >> 8;
-      const int d = (blk / NCH) * (DH / 2) + lane_freq(DH, blk % NCH, k >> 2, k & 3);
-      const int head = n & (HEADS - 1), part = n / HEADS;
-      float v = 0.f;
-      if (head < a.grp && part < 2) {
-        const float x = load_as_float(p.q, p.q_dtype, ((int64_t)b * p.Hq + (int64_t)hkv * a.grp + head) * DH + d) * qscale;
-        const float hi = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
-        v = part ? x - hi : hi;
-      }
-      const __nv_bfloat16 w = __float2bfloat16_rn(v);  // exact for the hi part
-      reinterpret_cast<__nv_bfloat16*>(smem + (q_u32 - smem0) + blk * 512 + (n >> 3) * 256 + (k >> 3) * 128)[(n & 7) * 8 + (k & 7)] = w;
+  // half * NCH + i holds, for lane quad member j, the four dims of chunk i: k = 4 j + e.  A thread loads its
+  // (at most three) values at once, before the codebooks, and stores both parts of each after them.
+  constexpr int kQLoads = (HEADS * DH + kTeamThreads - 1) / kTeamThreads;
+  float q_val[kQLoads];
+  auto load_query = [&]() {
+    const int64_t q0 = ((int64_t)b * p.Hq + (int64_t)hkv * a.grp) * DH;
+#pragma unroll
+    for (int l = 0; l < kQLoads; ++l) {
+      const int i = threadIdx.x + l * kTeamThreads;
+      q_val[l] = i < a.grp * DH ? load_as_float(p.q, p.q_dtype, q0 + i) : 0.f;
     }
   };
-  uint32_t par_k[kKStages] = {}, par_logits = 0, par_out = 0, par_vote = 0;
+  auto stage_query = [&]() {
+    const float qscale = p.sm_scale * kLog2e;
+#pragma unroll
+    for (int l = 0; l < kQLoads; ++l) {
+      const int i = threadIdx.x + l * kTeamThreads;
+      if (i >= a.grp * DH) break;
+      const int head = i / DH, d = i % DH, half = d / (DH / 2), f = d % (DH / 2);
+      const int j = f / W, chunk = ((f % W) >> 2) ^ (j & (NCH - 1)), k = 4 * j + (f & 3);
+      const float x = q_val[l] * qscale;
+      const float hi = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
+      auto put = [&](int n, float v) {
+        reinterpret_cast<__nv_bfloat16*>(smem + (q_u32 - smem0) + (half * NCH + chunk) * 512 + (n >> 3) * 256 +
+                                         (k >> 3) * 128)[(n & 7) * 8 + (k & 7)] = __float2bfloat16_rn(v);
+      };
+      put(head, hi);  // exact
+      put(head + HEADS, x - hi);
+    }
+  };
+  uint32_t par_k = 0, par_logits = 0, par_out = 0, par_vote = 0;
   for (; start < end; start = seg_end, ++u) {
     next_segment();
     const int64_t ml_head = (int64_t)p.max_blocks * TPP * 2;
+    load_query();
     stage_codebooks();
     cp_async_commit();
     stage_query();
@@ -729,7 +761,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
 #pragma unroll
           for (int tk = 0; tk < 2; ++tk)
             cs_src[tk] = reinterpret_cast<const float4*>(p.rope_table) +
-                         (clamp_pos((int)lds32(st + kKPos + 4 * r + 32 * tk)) * (DH / 4) + j * 2);
+                         (clamp_pos((int)lds32(st + kst_pos + 4 * r + 32 * tk)) * (DH / 4) + j * 2);
         }
       };
       auto issue_cs_chunk = [&](int i) {
@@ -742,15 +774,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
                          : "l"(cs_src[tk] + i * 8));
         }
       };
-      auto stage_of = [&](int k, int x) { return k_ring + ((k & (kKStages - 1)) * kMacroTiles + x) * kKStageBytes; };
+      // K stage of tile x in ring slot `slot`; parities of the slots are bits of par_k
+      auto stage_at = [&](int slot, int x) { return k_ring + (slot * kMacroTiles + x) * kst_bytes; };
       auto meta_of = [&](int k, int x) { return lds_meta(meta + ((k * kMacroTiles + x) & (kMetaRing - 1)) * 16); };
-      auto wait_k = [&](int k) -> bool {
-        const int s = k & (kKStages - 1);
-        uint32_t par = 0;
-#pragma unroll
-        for (int i = 0; i < kKStages; ++i)
-          if (i == s) { par = par_k[i]; par_k[i] ^= 1; }
-        return __all_sync(0xffffffffu, mbar_wait(bar + 8 * (kBarKFull + s), par));
+      auto wait_k = [&](int slot) -> bool {
+        const uint32_t par = (par_k >> slot) & 1u;
+        par_k ^= 1u << slot;
+        return __all_sync(0xffffffffu, mbar_wait(bar + 8 * (kBarKFull + slot), par));
       };
       // Centroid rows (shared-memory addresses) and radii of this lane's tokens r, r + 8 in the tiles of
       // both passes, [pass][2 token + half]; taken from the page bytes while the tensor core multiplies
@@ -758,7 +788,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       uint32_t row[2][4];
       float rad[2][4];
       bool have[2];
-      auto extract = [&](int k) {
+      auto extract = [&](int k, int slot) {
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
           const int x = w + 4 * pass;
@@ -768,7 +798,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           have[pass] = meta_tokens(m) != 0;
           if (!have[pass]) continue;
           if (meta_slot(m) != c_slot) load_slot_constants(meta_slot(m));
-          const uint32_t kst = stage_of(k, x);
+          const uint32_t kst = stage_at(slot, x);
           const uint32_t hd_ad = kst + meta_hdr(m), rd_ad = kst + meta_radius(m) + c_rad0;
           const uint32_t bit0 = 8 * (FAST ? meta_hdr(m) : meta_theta(m)) + c_bit0;
           float scl[2] = {1.f, 1.f};
@@ -805,22 +835,23 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       dead = !wait_k(0);
       if (!dead) {
         if (w < width) {
-          cs_rows(stage_of(0, w));
+          cs_rows(stage_at(0, w));
 #pragma unroll
           for (int i = 0; i < NCH; ++i) issue_cs_chunk(i);
         }
-        extract(0);
+        extract(0, 0);
       }
-      for (int k = 0; k < rounds && !dead; ++k) {
+      for (int k = 0, slot = 0, slot_n = 0; k < rounds && !dead; ++k, slot = slot_n) {
+        slot_n = slot + 1 == n_stages ? 0 : slot + 1;  // the next macro tile's
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
           // the pass after this one: its positions decide the cos/sin rows fetched below
           bool more = w + 4 < width;
-          uint32_t st_next = stage_of(k, w + 4);
+          uint32_t st_next = stage_at(slot, w + 4);
           if (pass == 1) {
             more = k + 1 < rounds && w < width;
-            st_next = stage_of(k + 1, w);
-            if (k + 1 < rounds && !wait_k(k + 1)) { dead = true; break; }
+            st_next = stage_at(slot_n, w);
+            if (k + 1 < rounds && !wait_k(slot_n)) { dead = true; break; }
           }
           if (more) cs_rows(st_next);
           if (have[pass]) {
@@ -889,13 +920,14 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         if (xs < width) ms = meta_of(k, xs);
         // rows without a token (past the page's count, or position -1) take no part
         bool valid = tok < meta_tokens(ms);
+        if (valid) valid = 16 * meta_sub(ms) + tok < (int)lds_u8(stage_at(slot, xs) + meta_hdr(ms) + 1);
         if (ROT && valid) {
-          const int pos = (int)lds32(stage_of(k, xs) + kKPos + 4 * tok);
+          const int pos = (int)lds32(stage_at(slot, xs) + kst_pos + 4 * tok);
           if (pos >= p.max_pos && p.status) atomicOr(p.status, SPHKV_ST_BAD_POSITION);
           valid = pos >= 0;
         }
         keys_ready(kBarKeys2);
-        if (k + 1 < rounds) extract(k + 1);
+        if (k + 1 < rounds) extract(k + 1, slot_n);
         if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * kBarLogits, par_logits))) { dead = true; break; }
         par_logits ^= 1;
         tc_fence_after();
@@ -1068,28 +1100,34 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     dead = dead || shared_words[1] != 0;
     {
       float* out_row = a.rows + (int64_t)(blockIdx.x + u) * 8 * (DH + 2);
-      for (int i = threadIdx.x; i < a.grp * (DH + 2); i += kTeamThreads) {
-        const int n = i / (DH + 2), e = i - n * (DH + 2);
-        float M = -INFINITY;
-        for (int t = 0; t < a.teams; ++t)
+      for (int i = threadIdx.x; i < a.grp * DH; i += kTeamThreads) {
+        const int n = i / DH, d = i % DH;
+        float M = -INFINITY, L = 0.f, o = 0.f;
 #pragma unroll
-          for (int w = 0; w < 4; ++w) M = fmaxf(M, stats_all[((t * 4 + w) * 8 + n) * 2 + 1]);
-        float outv = e == 0 ? M : 0.f;
-        if (e != 0 && M != -INFINITY) {
-          for (int t = 0; t < a.teams; ++t) {
+        for (int tw = 0; tw < 4 * kTeams; ++tw)
+          if (tw < 4 * a.teams) M = fmaxf(M, stats_all[(tw * 8 + n) * 2 + 1]);
+        if (M != -INFINITY) {
+#pragma unroll
+          for (int t = 0; t < kTeams; ++t) {
+            if (t >= a.teams) break;
             const float mw = mref_all[t * 8 + n];
             if (mw == -INFINITY) continue;
-            float val = 0.f;
-            if (e == 1) {
+            const float sc = fast_exp2(mw - M);
+            o += *acc_at(t, i) * sc;
+            if (d == 0) {
+              float l = 0.f;
 #pragma unroll
-              for (int w = 0; w < 4; ++w) val += stats_all[((t * 4 + w) * 8 + n) * 2];
-            } else {
-              val = *acc_at(t, n * DH + e - 2);
+              for (int w = 0; w < 4; ++w) l += stats_all[((t * 4 + w) * 8 + n) * 2];
+              L += l * sc;
             }
-            outv += val * fast_exp2(mw - M);
           }
         }
-        out_row[i] = outv;
+        float* dst = out_row + n * (DH + 2);
+        dst[2 + d] = o;
+        if (d == 0) {
+          dst[0] = M;
+          dst[1] = L;
+        }
       }
     }
   }
