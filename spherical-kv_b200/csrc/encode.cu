@@ -24,7 +24,8 @@ namespace sphkv {
 struct EncodeArgs {
   sphkv_encode_params p;
   int bundles_per_cta;
-  int warp_smem_bytes;  // page assembly: shared memory of one warp
+  int page_smem_bytes;  // page assembly: shared memory of one page
+  int wpp_shift;        // page assembly: log2 of the warps of a page
   int search_chunk;     // search launch: consecutive bundles a CTA takes at a time (1 .. 8)
 };
 
@@ -507,14 +508,15 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
   }
 }
 
-// ---- page assembly, one warp per page -----------------------------------------------------
+// ---- page assembly, `wpp` warps per page ------------------------------------------------------
 // Builds page images from per-(token, group) radii and centroid indices that already exist:
 // SRC 2 = the scratch arrays the search launch wrote ([(page * N + slot) * (dh / 16) + group]),
 // SRC 3 = a per-token code cache (sphkv_encode_codes) gathered through src_index, i.e. re-paging
-// after a tier change without touching the dense keys.  A warp owns a page from the first
-// lookup to the last byte, so there is no CTA barrier and the only dependent global loads are
-// page index -> src_index row -> code; with 64 warps per SM thousands of pages are in flight.
-// Per-warp shared memory: rows i32[N] | r f32[N*G] | scale f32[8] | theta u8[N*G] | page image.
+// after a tier change without touching the dense keys.  The warps of a page own it from the first lookup
+// to the last byte; the only dependent global loads are page index -> src_index row -> code.  16-token
+// pages take a warp each (no barrier at all; thousands in flight); a 128-token page is eight warps' work:
+// with one, the 440 pages of an 8190-token prompt kept three warps per SM busy (62 us), so ASM_US us.
+// Shared memory of a page: rows i32[N] | r f32[N*G] | scale f32[8] | theta u8[N*G] | page image.
 template <int SRC>
 __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
@@ -523,8 +525,16 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
   extern __shared__ __align__(16) uint8_t smem[];
   const int N = p.page_size, dh = p.dh, GST = dh >> 4;
   const int ppb_shift = __clz(N) - 24;  // log2 of the 128 / N pages per bundle (N is 16 .. 128)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* mine = smem + (size_t)warp * a.warp_smem_bytes;
+  const int wpp_shift = a.wpp_shift, team = threadIdx.x >> (5 + wpp_shift);
+  const int nt = 32 << wpp_shift, t0 = threadIdx.x & (nt - 1), lane = threadIdx.x & 31;  // threads of the page, this one
+  const int pages_at_once = (kEncThreads / 32) >> wpp_shift;
+  auto page_sync = [&]() {
+    if (wpp_shift == 0)
+      __syncwarp();
+    else
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(nt) : "memory");
+  };
+  uint8_t* mine = smem + (size_t)team * a.page_smem_bytes;
   int* rows_w = reinterpret_cast<int*>(mine);
   float* r_w = reinterpret_cast<float*>(rows_w + N);
   float* scale_w = r_w + N * GST;
@@ -534,7 +544,7 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
   const uint8_t* scr_t = reinterpret_cast<const uint8_t*>(p.scratch) + (int64_t)p.n_pages * N * GST * 4;
   const int rb = p.radius_fmt == SPHKV_RADIUS_F16 ? 2 : 1;
   const int64_t items = (int64_t)p.n_bundles << ppb_shift;
-  for (int64_t it = (int64_t)blockIdx.x * (kEncThreads / 32) + warp; it < items; it += (int64_t)gridDim.x * (kEncThreads / 32)) {
+  for (int64_t it = (int64_t)blockIdx.x * pages_at_once + team; it < items; it += (int64_t)gridDim.x * pages_at_once) {
     const int page = p.bundles[8 * (it >> ppb_shift) + (it & ((1 << ppb_shift) - 1))];
     if (page < 0) continue;
     const int head = p.page_head[page], slot = p.page_slot[page];
@@ -543,59 +553,58 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
     const int G = dh / gs, g_shift = 31 - __clz(G);
     const float* code_r = SRC == 3 ? p.code_r[slot] + (int64_t)head * p.code_rows * G : nullptr;
     const uint8_t* code_t = SRC == 3 ? p.code_theta[slot] + (int64_t)head * p.code_rows * G : nullptr;
-    __syncwarp();  // the previous page's image has been copied out
-    // ---- source rows and the valid-token count (valid slots form a prefix) -------------------
+    page_sync();  // the previous page's image has been copied out
+    // ---- source rows and the valid-token count (valid slots form a prefix); every warp counts all ----
     int cnt = 0;
-    for (int t0 = 0; t0 < N; t0 += 32) {
-      const int row = t0 + lane < N ? p.src_index[(int64_t)page * N + t0 + lane] : -1;
-      if (t0 + lane < N) rows_w[t0 + lane] = row;
+    for (int s0 = 0; s0 < N; s0 += 32) {
+      const int row = s0 + lane < N ? p.src_index[(int64_t)page * N + s0 + lane] : -1;
+      if (s0 + lane < N && t0 < 32) rows_w[s0 + lane] = row;
       cnt += __popc(__ballot_sync(0xffffffffu, row >= 0));
     }
-    __syncwarp();
-    // ---- radii and centroid indices of the page -----------------------------------------------
-    for (int i = lane; i < N * G; i += 32) {
-      const int tin = i >> g_shift, gq = i & (G - 1);
-      float rv = 0.f;
-      uint8_t tv = 0;
-      if (SRC == 2) {
-        const int64_t si = ((int64_t)page * N + tin) * GST + gq;
-        rv = scr_r[si];
-        tv = scr_t[si];
-      } else {
-        const int row = rows_w[tin];
-        if (row >= 0) {
-          rv = code_r[(int64_t)row * G + gq];
-          tv = code_t[(int64_t)row * G + gq];
-        }
-      }
-      r_w[i] = rv;
-      th_w[i] = tv;
-    }
-    __syncwarp();
-    // ---- per-group scale = max radius over the page's tokens ----------------------------------
+    if (t0 < 8) scale_w[t0] = 0.f;
+    page_sync();
+    // ---- radii and centroid indices of the page; per-group scale = max radius over its tokens.  A thread's
+    //      items all belong to one group (32 is a multiple of G) ----
     {
-      const int gq = lane & 7, tq = lane >> 3;
       float mx = 0.f;
-      if (gq < G)
-        for (int t = tq; t < cnt; t += 4) mx = fmaxf(mx, r_w[t * G + gq]);
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-      if (lane < 8) scale_w[lane] = mx;
+#pragma unroll 4
+      for (int i = t0; i < N * G; i += nt) {
+        const int tin = i >> g_shift, gq = i & (G - 1);
+        float rv = 0.f;
+        uint8_t tv = 0;
+        if (SRC == 2) {
+          const int64_t si = ((int64_t)page * N + tin) * GST + gq;
+          rv = scr_r[si];
+          tv = scr_t[si];
+        } else {
+          const int row = rows_w[tin];
+          if (row >= 0) {
+            rv = code_r[(int64_t)row * G + gq];
+            tv = code_t[(int64_t)row * G + gq];
+          }
+        }
+        r_w[i] = rv;
+        th_w[i] = tv;
+        if (tin < cnt) mx = fmaxf(mx, rv);
+      }
+      for (int o = G; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      // radii are not negative: their bit patterns order as integers
+      if (lane < G) atomicMax(reinterpret_cast<int*>(scale_w + lane), __float_as_int(mx));
     }
-    __syncwarp();
+    page_sync();
     if (cnt > 0) {
       // ---- header, scales, LSB-first theta words ----------------------------------------------
       const int hdr = 8 + 4 * G;
       const int nvals = cnt * G;
       const int th_bytes = (nvals * bits + 7) >> 3;
       const int th_words = (th_bytes + 3) >> 2;
-      if (lane < 2)
-        reinterpret_cast<uint32_t*>(img)[lane] =
-            lane == 0 ? (uint32_t)(p.tiers.tier_id[slot] & 0xFF) | ((uint32_t)(cnt & 0xFF) << 8) |
-                            ((uint32_t)(p.radius_fmt & 0xFF) << 16)
-                      : 0u;
-      if (lane < G) reinterpret_cast<float*>(img + 8)[lane] = scale_w[lane];
-      for (int w = lane; w < th_words; w += 32) {
+      if (t0 < 2)
+        reinterpret_cast<uint32_t*>(img)[t0] =
+            t0 == 0 ? (uint32_t)(p.tiers.tier_id[slot] & 0xFF) | ((uint32_t)(cnt & 0xFF) << 8) |
+                          ((uint32_t)(p.radius_fmt & 0xFF) << 16)
+                    : 0u;
+      if (t0 < G) reinterpret_cast<float*>(img + 8)[t0] = scale_w[t0];
+      for (int w = t0; w < th_words; w += nt) {
         const int bit0 = w * 32;
         const int i0 = bit0 / bits;                             // first value overlapping this word
         const int i1 = min(nvals, (bit0 + 31) / bits + 1);      // one past the last
@@ -606,10 +615,10 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
         for (int i = i0; i < i1; ++i, sh += bits) acc |= (unsigned long long)th_w[i] << sh;
         reinterpret_cast<uint32_t*>(img + hdr)[w] = (uint32_t)(acc >> 8);
       }
-      __syncwarp();
+      page_sync();
       // ---- radii (may overlay the zero tail of the last theta word) ---------------------------
       uint8_t* rad = img + hdr + th_bytes;
-      for (int i = lane; i < nvals; i += 32) {
+      for (int i = t0; i < nvals; i += nt) {
         const float rr = r_w[i];
         if (rb == 1) {
           const float safe = fmaxf(scale_w[i & (G - 1)], 1e-8f);
@@ -617,33 +626,44 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
           qv = fminf(fmaxf(qv, -127.f), 127.f);
           rad[i] = (uint8_t)(int8_t)(int)qv;
         } else {
-          // the half's bit pattern goes over the radius slot as a 32-bit word (this lane read it
+          // the half's bit pattern goes over the radius slot as a 32-bit word (this thread read it
           // just above); its two bytes are laid into the image below
           reinterpret_cast<uint32_t*>(r_w)[i] = (uint32_t)__half_as_ushort(__float2half_rn(rr));
         }
       }
-      __syncwarp();
+      page_sync();
       if (rb == 2) {
         const uint8_t* hb = reinterpret_cast<const uint8_t*>(r_w);
-        for (int b2 = lane; b2 < 2 * nvals; b2 += 32) rad[b2] = hb[(b2 >> 1) * 4 + (b2 & 1)];
-        __syncwarp();
+        for (int b2 = t0; b2 < 2 * nvals; b2 += nt) rad[b2] = hb[(b2 >> 1) * 4 + (b2 & 1)];
+        page_sync();
       }
       // ---- copy the image out ----------------------------------------------------------------
       const int bytes = hdr + th_bytes + nvals * rb;
-      for (int w = lane; w < (bytes >> 2); w += 32)
+      for (int w = t0; w < (bytes >> 2); w += nt)
         reinterpret_cast<uint32_t*>(p.k_pages + poff)[w] = reinterpret_cast<const uint32_t*>(img)[w];
-      if (lane < (bytes & 3)) p.k_pages[poff + (bytes & ~3) + lane] = img[(bytes & ~3) + lane];
+      if (t0 < (bytes & 3)) p.k_pages[poff + (bytes & ~3) + t0] = img[(bytes & ~3) + t0];
     }
-    // ---- dense V page (16-bit), empty slots zero-filled ---------------------------------------
+    // ---- dense V page (16-bit), empty slots zero-filled; four chunks in flight per thread -------
     if (p.v_src != nullptr && p.v_pool != nullptr) {
+      constexpr int kInFlight = 4;
       const int pr_shift = 31 - __clz(dh >> 3);  // 16-byte chunks per row (dh / 8, a power of two)
       const bool same = p.v_src_dtype == p.v_pool_dtype;
-      for (int i = lane; i < (N << pr_shift); i += 32) {
-        const int tin = i >> pr_shift, d = (i & ((1 << pr_shift) - 1)) * 8;
-        const int row = rows_w[tin];
-        uint4 o = make_uint4(0u, 0u, 0u, 0u);
-        if (row >= 0) o = load_v_chunk(p, same, (int64_t)row * p.v_row_stride + (int64_t)head * p.v_head_stride + d);
-        reinterpret_cast<uint4*>(p.v_pool)[(((int64_t)page * N + tin) * dh + d) >> 3] = o;
+      const int chunks = N << pr_shift;
+      for (int i0 = t0; i0 < chunks; i0 += nt * kInFlight) {
+        uint4 o[kInFlight];
+#pragma unroll
+        for (int e = 0; e < kInFlight; ++e) {
+          const int i = i0 + e * nt;
+          o[e] = make_uint4(0u, 0u, 0u, 0u);
+          if (i >= chunks) continue;
+          const int tin = i >> pr_shift, d = (i & ((1 << pr_shift) - 1)) * 8;
+          const int row = rows_w[tin];
+          if (row >= 0) o[e] = load_v_chunk(p, same, (int64_t)row * p.v_row_stride + (int64_t)head * p.v_head_stride + d);
+        }
+#pragma unroll
+        for (int e = 0; e < kInFlight; ++e)
+          if (i0 + e * nt < chunks)
+            reinterpret_cast<uint4*>(p.v_pool)[(((int64_t)page * N * dh) >> 3) + i0 + e * nt] = o[e];
       }
     }
   }
@@ -907,18 +927,21 @@ static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaSt
   return check_launch("encode_bundle_kernel");
 }
 
-// One warp per page of the bundle list, every tier slot in the same launch.
+// Every page of the bundle list, every tier slot in the same launch: a warp per 16 tokens, so that large pages
+// fill the GPU as small ones do.
 static int launch_assemble(EncodeArgs& a, bool from_codes, cudaStream_t st) {
   const sphkv_encode_params& p = a.p;
   const int N = p.page_size, GST = p.dh >> 4;
   const int img = ((8 + 4 * GST + N * GST + N * GST * 2) + 15) & ~15;  // 8-bit codes, f16 radii: the largest image
-  a.warp_smem_bytes = 4 * N + 4 * N * GST + 32 + N * GST + img;
-  const int smem_bytes = a.warp_smem_bytes * (kEncThreads / 32);
+  a.page_smem_bytes = 4 * N + 4 * N * GST + 32 + N * GST + img;
+  a.wpp_shift = N == 16 ? 0 : N == 32 ? 1 : N == 64 ? 2 : 3;
+  const int at_once = (kEncThreads / 32) >> a.wpp_shift;
+  const int smem_bytes = a.page_smem_bytes * at_once;
   static SmemOptIn opt_in[2];
   const void* fn = from_codes ? (const void*)assemble_pages_kernel<3> : (const void*)assemble_pages_kernel<2>;
   if (int rc = ensure_dynamic_smem(opt_in[from_codes], fn, smem_bytes, "assemble_pages")) return rc;
   const int64_t items = (int64_t)p.n_bundles * (128 / N);
-  const int64_t ctas = (items + kEncThreads / 32 - 1) / (kEncThreads / 32);
+  const int64_t ctas = (items + at_once - 1) / at_once;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)sm_count_current_device() * 8));
   if (from_codes)
     (void)launch_overlapped(assemble_pages_kernel<3>, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);

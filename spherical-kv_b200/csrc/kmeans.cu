@@ -5,50 +5,60 @@
 // are visited in ascending order and the first maximum wins (torch.argmax convention).
 //
 // One thread holds kPts points in registers and walks the centroids out of shared memory
-// (one broadcast 16-byte load feeds 16 or 8 FMAs).  The accumulation uses no float atomics:
-// per pass of 1024 (512) points a CTA counting-sorts the point ids by cluster in shared memory
-// (integer atomics give each point its rank), then every (cluster, dimension) pair is summed
-// by one thread walking its cluster's id list and re-reading the rows (L1/L2 hits).  The
-// rank order inside a cluster is not fixed, so -- as with index_add_ on a GPU -- sums agree to
-// rounding while assignments and counts are exact.  Per-CTA sums go to global memory once.
+// (one broadcast 16-byte load feeds 16 or 8 FMAs).  The accumulation uses no float atomics and no
+// barrier: every warp keeps sums of its own in shared memory, 32 / D sets of [K][D] (`ways`; one when they would
+// not fit), and walks its points D lanes to a row -- lane = dimension, one add per row and lane, the rows
+// turned through a 32-row tile of shared memory -- so lanes never meet in an address.  Warps and CTAs are
+// folded at the end.  Sums agree to rounding, as with index_add_ on a GPU; assignments and counts are
+// exact.  Bound: fp32 FMA issue for K = 64, then the shared-memory adds.  4M points, d 16, K 64: KM64A -> KM64B us;
+// K 16, 2.3M points: 96 -> KM16B us (a counting sort per 1024 points with six barriers before).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sphkv {
 
 constexpr int kKmThreads = 256;
+constexpr int kKmWarps = kKmThreads / 32;
 // points per thread: 4 (2 for 32-dim points) keeps the kernel at two CTAs per SM
 __host__ __device__ constexpr int pts_for(int d) { return d >= 32 ? 2 : 4; }
 
+// a CTA takes passes of kKmThreads * pts_for(D) points; its warps walk them without meeting
 template <int D>
 __global__ void __launch_bounds__(kKmThreads, 2) kmeans_assign_kernel(
     const float* __restrict__ U, int64_t N, const float* __restrict__ centers, int K,
     int32_t* __restrict__ assigns, float* __restrict__ best_sim, float* __restrict__ sums,
-    int32_t* __restrict__ counts, int64_t pts_per_cta) {
+    int32_t* __restrict__ counts, int ways) {
   constexpr int kPts = pts_for(D);
-  constexpr int P = kKmThreads * kPts;  // points per pass
+  constexpr int kWarpPts = 32 * kPts;           // points of a warp per pass
   extern __shared__ __align__(16) float sm[];
-  float* c_s = sm;                                      // [K][D] centres
-  float* sum_s = sm + K * D;                            // [K][D] this CTA's sums
-  int* cnt_s = reinterpret_cast<int*>(sum_s + K * D);   // [K] counts of the current pass
-  int* tot_s = cnt_s + K;                               // [K] counts of all passes
-  int* off_s = tot_s + K;                               // [K + 1] start of each cluster's id list
-  uint16_t* order_s = reinterpret_cast<uint16_t*>(off_s + K + 1);  // [P] point ids sorted by cluster
-  for (int i = threadIdx.x; i < K * D; i += blockDim.x) {
-    c_s[i] = centers[i];
-    sum_s[i] = 0.f;
-  }
-  for (int i = threadIdx.x; i < K; i += blockDim.x) cnt_s[i] = tot_s[i] = 0;
+  float* c_s = sm;                                            // [K][D] centres
+  float* sum_s = sm + K * D;                                  // [warps][ways][K][D] sums
+  int* cnt_s = reinterpret_cast<int*>(sum_s + kKmWarps * ways * K * D);  // [K] counts of this CTA
+  uint8_t* code_s = reinterpret_cast<uint8_t*>(cnt_s + K);               // [warps][32]
+  for (int i = threadIdx.x; i < K * D; i += kKmThreads) c_s[i] = centers[i];
+  for (int i = threadIdx.x; i < kKmWarps * ways * K * D; i += kKmThreads) sum_s[i] = 0.f;
+  for (int i = threadIdx.x; i < K; i += kKmThreads) cnt_s[i] = 0;
   __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* my_codes = code_s + warp * 32;
+  // 32 rows of points, 16-byte chunk q of row p at chunk q ^ turn(p): neither the row-per-lane stores nor the
+  // dimension-per-lane loads meet in a bank
+  float* tile = reinterpret_cast<float*>(sm + K * D + kKmWarps * ways * K * D + ((K + 3) & ~3) + kKmWarps * 8) + warp * 32 * D;
+  auto turn = [](int p) { return (p >> (D == 32 ? 0 : D == 16 ? 1 : 2)) & (D / 4 - 1); };
+  // adding: lane = (way, dimension); with one way the first D lanes work
+  const int dim = lane & (D - 1), way = lane / D;
+  const bool adds = way < ways;
+  float* my_sums = sum_s + ((int64_t)warp * ways + (adds ? way : 0)) * K * D + dim;
 
-  const int64_t first = (int64_t)blockIdx.x * pts_per_cta;
-  const int64_t last = first + pts_per_cta < N ? first + pts_per_cta : N;
-  for (int64_t base = first; base < last; base += P) {
+  const int64_t stride = (int64_t)gridDim.x * kKmWarps * kWarpPts;
+  for (int64_t base = ((int64_t)blockIdx.x * kKmWarps + warp) * kWarpPts; base < N; base += stride) {
     float u[kPts][D];
     bool live[kPts];
 #pragma unroll
     for (int h = 0; h < kPts; ++h) {
-      const int64_t idx = base + threadIdx.x + h * kKmThreads;  // coalesced across the CTA
-      live[h] = idx < last;
+      const int64_t idx = base + lane + 32 * h;
+      live[h] = idx < N;
       if (live[h]) {
         const float4* src = reinterpret_cast<const float4*>(U + idx * D);
 #pragma unroll
@@ -86,56 +96,62 @@ __global__ void __launch_bounds__(kKmThreads, 2) kmeans_assign_kernel(
       for (int h = 0; h < kPts; ++h)
         if (acc[h] > best[h]) { best[h] = acc[h]; code[h] = c; }
     }
-    // rank of each point inside its cluster, results out
-    int rank[kPts];
 #pragma unroll
     for (int h = 0; h < kPts; ++h) {
-      rank[h] = 0;
+      const int64_t idx = base + lane + 32 * h;
+      __syncwarp();  // the adds before have read the tile
+      my_codes[lane] = (uint8_t)code[h];
+#pragma unroll
+      for (int q = 0; q < D / 4; ++q)
+        *reinterpret_cast<float4*>(tile + lane * D + 4 * (q ^ turn(lane))) =
+            make_float4(u[h][4 * q], u[h][4 * q + 1], u[h][4 * q + 2], u[h][4 * q + 3]);
       if (live[h]) {
-        const int64_t idx = base + threadIdx.x + h * kKmThreads;
         assigns[idx] = code[h];
         if (best_sim != nullptr) best_sim[idx] = best[h];
-        rank[h] = atomicAdd(&cnt_s[code[h]], 1);
+        atomicAdd(&cnt_s[code[h]], 1);
       }
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {  // exclusive prefix of the K counts by one warp
-      int carry = 0;
-      for (int k0 = 0; k0 < K; k0 += 32) {
-        const int k = k0 + threadIdx.x;
-        const int v = k < K ? cnt_s[k] : 0;
-        int incl = v;
+      __syncwarp();
+      if (adds) {  // rows past the end are zero and add nothing
+        for (int p0 = 0; p0 < 32; p0 += 8 * ways) {
+          float v[8];
+          int c[8];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int t = __shfl_up_sync(0xffffffffu, incl, o);
-          if ((int)threadIdx.x >= o) incl += t;
+          for (int e = 0; e < 8; ++e) {
+            const int p = p0 + e * ways + way;
+            v[e] = tile[p * D + 4 * ((dim >> 2) ^ turn(p)) + (dim & 3)];
+            c[e] = my_codes[p];
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) my_sums[c[e] * D] += v[e];
         }
-        if (k < K) off_s[k] = carry + incl - v;
-        carry += __shfl_sync(0xffffffffu, incl, 31);
       }
-      if (threadIdx.x == 0) off_s[K] = carry;
     }
-    __syncthreads();
-#pragma unroll
-    for (int h = 0; h < kPts; ++h)
-      if (live[h]) order_s[off_s[code[h]] + rank[h]] = (uint16_t)(threadIdx.x + h * kKmThreads);
-    __syncthreads();
-    for (int q = threadIdx.x; q < K * D; q += blockDim.x) {
-      const int k = q / D, i = q - k * D;
-      float acc = 0.f;
-      for (int jj = off_s[k]; jj < off_s[k + 1]; ++jj) acc += __ldg(U + (base + order_s[jj]) * D + i);
-      sum_s[q] += acc;
-    }
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-      tot_s[k] += cnt_s[k];
-      cnt_s[k] = 0;
-    }
-    __syncthreads();
   }
-  for (int i = threadIdx.x; i < K * D; i += blockDim.x)
-    if (sum_s[i] != 0.f) atomicAdd(sums + i, sum_s[i]);
-  for (int i = threadIdx.x; i < K; i += blockDim.x)
-    if (tot_s[i] != 0) atomicAdd(counts + i, tot_s[i]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < K * D; i += kKmThreads) {
+    float t = 0.f;
+    for (int w = 0; w < kKmWarps * ways; ++w) t += sum_s[(int64_t)w * K * D + i];
+    if (t != 0.f) atomicAdd(sums + i, t);
+  }
+  for (int i = threadIdx.x; i < K; i += kKmThreads)
+    if (cnt_s[i] != 0) atomicAdd(counts + i, cnt_s[i]);
+}
+
+template <int D>
+static int launch_kmeans(const float* U, int64_t N, const float* centers, int K, int32_t* assigns, float* best_sim, float* sums,
+                         int32_t* counts, int sms, cudaStream_t st) {
+  // a set of sums for every D lanes of a warp while two CTAs fit an SM, else one per warp
+  auto bytes = [&](int ways) {
+    return ((size_t)K * D * (1 + kKmWarps * ways) + ((K + 3) & ~3) + kKmWarps * 8 + kKmWarps * 32 * D) * sizeof(float);
+  };
+  int ways = 32 / D;
+  if (bytes(ways) > 110 * 1024) ways = 1;
+  static SmemOptIn opt_in;
+  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_assign_kernel<D>, (int)bytes(ways), "kmeans_assign")) return rc;
+  const int64_t pass = (int64_t)kKmThreads * pts_for(D);
+  const int64_t ctas = std::min<int64_t>((N + pass - 1) / pass, (int64_t)sms * (bytes(ways) <= 110 * 1024 ? 2 : 1));
+  kmeans_assign_kernel<D><<<(unsigned)ctas, kKmThreads, bytes(ways), st>>>(U, N, centers, K, assigns, best_sim, sums, counts, ways);
+  return check_launch("kmeans_assign_kernel");
 }
 
 }  // namespace sphkv
@@ -151,13 +167,6 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
   SPHKV_REQUIRE((reinterpret_cast<uintptr_t>(U) & 15) == 0, SPHKV_E_ARG, "kmeans_assign: U must be 16-byte aligned");
   const int sms = sphkv_sm_count();
   SPHKV_REQUIRE(sms > 0, SPHKV_E_ARG, "kmeans_assign: cannot resolve the SM count");
-  // a few CTAs per SM, each over a contiguous run of points that is a multiple of one pass
-  const int64_t pass = (int64_t)kKmThreads * pts_for(d);
-  int64_t ctas = (N + pass - 1) / pass;
-  if (ctas < 1) ctas = 1;  // N == 0 returns after the memsets below
-  if (ctas > (int64_t)sms * 8) ctas = (int64_t)sms * 8;
-  const int64_t per = ((N + ctas - 1) / ctas + pass - 1) / pass * pass;
-  ctas = (N + per - 1) / per;
   const size_t smem = (size_t)K * d * 8 + (size_t)(3 * K + 1) * 4 + (size_t)kKmThreads * pts_for(d) * 2;
   SPHKV_REQUIRE(smem <= 48 * 1024, SPHKV_E_LIMIT, "kmeans_assign: K=%d x d=%d needs %zu B of shared memory (limit 49152)",
                 K, d, smem);
@@ -169,11 +178,8 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
     return (int)e;
   }
   if (N == 0) return SPHKV_OK;
-  if (d == 8)
-    kmeans_assign_kernel<8><<<(unsigned)ctas, kKmThreads, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, per);
-  else if (d == 16)
-    kmeans_assign_kernel<16><<<(unsigned)ctas, kKmThreads, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, per);
-  else
-    kmeans_assign_kernel<32><<<(unsigned)ctas, kKmThreads, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, per);
-  return check_launch("kmeans_assign_kernel");
+  return d == 8    ? launch_kmeans<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
+         : d == 16 ? launch_kmeans<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
+                   : launch_kmeans<32>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
 }
+
