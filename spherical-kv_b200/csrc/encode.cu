@@ -26,6 +26,7 @@ struct EncodeArgs {
   int bundles_per_cta;
   int page_smem_bytes;  // page assembly: shared memory of one page
   int wpp_shift;        // page assembly: log2 of the warps of a page
+  int search_kbuf;      // search launch: byte offset of the staged rows
   int search_chunk;     // search launch: consecutive bundles a CTA takes at a time (1 .. 8)
 };
 
@@ -134,21 +135,22 @@ __device__ __forceinline__ void search_four_tokens(const float (&k)[4][GS], cons
   }
 }
 
-// The codebook of one (KV head, tier slot), [G][C][GS] packed, global -> shared memory.
+// The codebook of one (KV head, tier slot), [G][C][GS] packed, global -> shared memory: every 16-byte copy of
+// the CTA in flight at once.  The caller's barrier publishes it.
 template <int GS>
 __device__ __forceinline__ void stage_slot_codebook(const sphkv_encode_params& p, int head, int slot, float* cb_s) {
   const int bits = p.tiers.bits[slot], G = p.dh / GS;
-  const float4* src = reinterpret_cast<const float4*>(
-      p.codebooks + ((int64_t)(head * p.tiers.n_slots + slot) * p.tiers.G_max) * p.tiers.C_max * p.tiers.g_max);
-  float4* dst = reinterpret_cast<float4*>(cb_s);
+  const float* src = p.codebooks + ((int64_t)(head * p.tiers.n_slots + slot) * p.tiers.G_max) * p.tiers.C_max * p.tiers.g_max;
+  const uint32_t dst = smem_u32(cb_s);
   constexpr int Q4 = GS / 4;
   const int total = (G << bits) * Q4;
-  const int row_stride4 = p.tiers.g_max >> 2;
   for (int i = threadIdx.x; i < total; i += blockDim.x) {
     const int q4 = i % Q4, row = i / Q4;
     const int c = row & ((1 << bits) - 1), gam = row >> bits;
-    dst[i] = __ldg(src + ((int64_t)gam * p.tiers.C_max + c) * row_stride4 + q4);
+    cp_async_16(dst + i * 16, src + (gam * p.tiers.C_max + c) * p.tiers.g_max + 4 * q4);
   }
+  cp_async_commit();
+  cp_async_wait<0>();
 }
 
 // Everything in one kernel (the route without scratch): search, page images and V pages per bundle.
@@ -408,7 +410,12 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
 // lane = four token slots.  The only barrier is the codebook change between (head, tier) keys;
 // otherwise a warp walks its bundles alone, and while it searches one bundle the page ids and
 // source rows of the next are already loaded and its key rows are on their way to L2.
-template <int GS>
+// STAGED: a warp's slices of the next bundle's rows travel to shared memory by 16-byte asynchronous copies, the
+// lanes of a row slice side by side, while the current bundle is searched; as one row per lane, every 128-bit
+// load fetched 32 sectors and used half of each (GS 16: 106 -> 90 us for a 32768-token prompt).  Chunk c
+// of row s is stored at chunk c ^ turn(s), so neither the copies nor the row-per-lane reads meet in a bank.
+// Not STAGED: slices off a 16-byte boundary.
+template <int GS, bool STAGED>
 __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
   griddep_wait();
@@ -433,6 +440,24 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
       row[h] = pg[h] >= 0 ? p.src_index[(int64_t)pg[h] * N + (ts & (N - 1))] : -1;
     }
   };
+  // 16-byte chunks of a row slice: GS / 4 (fp32) or GS / 8
+  const int ch_shift = (GS == 32 ? 3 : 2) - (esize == 2 ? 1 : 0), ch = 1 << ch_shift;
+  const uint32_t kbuf = smem_u32(smem + a.search_kbuf) + warp * (128 * GS * 4);
+  auto turn = [&](int s) { return (s >> (3 - ch_shift)) & (ch - 1); };
+  auto issue_rows = [&](const int (&row)[4], int head) {
+    const int s_l = lane >> ch_shift, c = lane & (ch - 1), rows_per = 32 >> ch_shift;
+    const char* base = reinterpret_cast<const char*>(p.k_src) + ((int64_t)head * p.k_head_stride + warp * GS) * esize + c * 16;
+    const int64_t row_bytes = p.k_row_stride * esize;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      for (int i = 0; i < ch; ++i) {  // 32 rows of quarter h, rows_per at a time
+        const int s = i * rows_per + s_l;
+        const int r = __shfl_sync(0xffffffffu, row[h], s);
+        cp_async_16_zfill(kbuf + (((32 * h + s) << ch_shift) + (c ^ turn(s))) * 16, r >= 0 ? base + r * row_bytes : reinterpret_cast<const char*>(p.k_src),
+                          r >= 0 ? 16 : 0);
+      }
+    cp_async_commit();
+  };
   int loaded_key = -1;
   for (int64_t chunk = blockIdx.x; chunk * chunk_len < p.n_bundles; chunk += gridDim.x) {
     // lane q < chunk_len looks at bundle q of the chunk: which (head, tier slot), and is it of this
@@ -453,7 +478,10 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
     }
     unsigned todo = __ballot_sync(0xffffffffu, my_head >= 0 && p.tiers.g[my_slot] == GS);  // same in every warp
     int pg_n[4], row_n[4];
-    if (todo) lookup(chunk * chunk_len + (__ffs(todo) - 1), pg_n, row_n);
+    if (todo) {
+      lookup(chunk * chunk_len + (__ffs(todo) - 1), pg_n, row_n);
+      if (STAGED && warp < G) issue_rows(row_n, __shfl_sync(0xffffffffu, my_head, __ffs(todo) - 1));
+    }
     while (todo) {
       const int q = __ffs(todo) - 1;
       todo &= todo - 1;
@@ -474,24 +502,50 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
         __syncthreads();
       }
       if (warp >= G) continue;
-      if (head_n >= 0) {
-#pragma unroll
-        for (int h = 0; h < 4; ++h)
-          if (row_n[h] >= 0)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(
-                reinterpret_cast<const char*>(p.k_src) +
-                ((int64_t)row_n[h] * p.k_row_stride + (int64_t)head_n * p.k_head_stride + warp * GS) * esize));
-      }
       const int bits = p.tiers.bits[slot];
       float k[4][GS];
+      if (STAGED) {
+        cp_async_wait<0>();
+        __syncwarp();
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        if (row[h] >= 0) {
-          load_group<GS>(p.k_src, p.k_dtype,
-                         (int64_t)row[h] * p.k_row_stride + (int64_t)head * p.k_head_stride + warp * GS, k[h]);
-        } else {
+        for (int h = 0; h < 4; ++h) {
+          const uint32_t src = kbuf + (((32 * h + lane) << ch_shift) * 16);
+          if (esize == 4) {
 #pragma unroll
-          for (int i = 0; i < GS; ++i) k[h][i] = 0.f;
+            for (int c = 0; c < GS / 4; ++c) {
+              const float4 v = lds_f4(src + ((c ^ turn(lane)) << 4));
+              k[h][4 * c] = v.x; k[h][4 * c + 1] = v.y; k[h][4 * c + 2] = v.z; k[h][4 * c + 3] = v.w;
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < GS / 8; ++c) {
+              const float4 v = lds_f4(src + ((c ^ turn(lane)) << 4));
+              const uint32_t w[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) unpack16(w[e], p.k_dtype, k[h][8 * c + 2 * e], k[h][8 * c + 2 * e + 1]);
+            }
+          }
+        }
+        __syncwarp();
+        if (head_n >= 0) issue_rows(row_n, head_n);
+      } else {
+        if (head_n >= 0) {
+#pragma unroll
+          for (int h = 0; h < 4; ++h)
+            if (row_n[h] >= 0)
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                  reinterpret_cast<const char*>(p.k_src) +
+                  ((int64_t)row_n[h] * p.k_row_stride + (int64_t)head_n * p.k_head_stride + warp * GS) * esize));
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          if (row[h] >= 0) {
+            load_group<GS>(p.k_src, p.k_dtype,
+                           (int64_t)row[h] * p.k_row_stride + (int64_t)head * p.k_head_stride + warp * GS, k[h]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < GS; ++i) k[h][i] = 0.f;
+          }
         }
       }
       float nsq[4];
@@ -515,7 +569,7 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
 // after a tier change without touching the dense keys.  The warps of a page own it from the first lookup
 // to the last byte; the only dependent global loads are page index -> src_index row -> code.  16-token
 // pages take a warp each (no barrier at all; thousands in flight); a 128-token page is eight warps' work:
-// with one, the 440 pages of an 8190-token prompt kept three warps per SM busy (62 us), so ASM_US us.
+// with one, the 440 pages of an 8190-token prompt kept three warps per SM busy (60 us), so 13 us.
 // Shared memory of a page: rows i32[N] | r f32[N*G] | scale f32[8] | theta u8[N*G] | page image.
 template <int SRC>
 __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const EncodeArgs a) {
@@ -912,14 +966,21 @@ template <int GS>
 static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaStream_t st) {
   if (split) {
     // persistent: as many CTAs as are resident at once, each striding over chunks of bundles
-    static SmemOptIn opt_in;
-    const int cb_bytes = a.p.dh * a.p.tiers.C_max * 4;
-    if (int rc = ensure_dynamic_smem(opt_in, (const void*)search_bundles_kernel<GS>, cb_bytes, "encode search")) return rc;
+    static SmemOptIn opt_in[2];
+    const sphkv_encode_params& p = a.p;
+    const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
+    const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
+                        (p.k_head_stride * esize) % 16 == 0;
+    const int cb_bytes = p.dh * p.tiers.C_max * 4;
+    const int smem = cb_bytes + (staged ? p.dh / GS * 128 * GS * 4 : 0);
+    auto kern = staged ? search_bundles_kernel<GS, true> : search_bundles_kernel<GS, false>;
+    if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem, "encode search")) return rc;
     const int resident = sm_count_current_device() * (GS == 16 ? 2 : 1);
     EncodeArgs b = a;
+    b.search_kbuf = cb_bytes;
     b.search_chunk = std::max(1, std::min(8, a.p.n_bundles / (resident * 4)));  // >= 4 chunks per CTA, <= 8 bundles each
     const int grid = std::max(1, std::min((a.p.n_bundles + b.search_chunk - 1) / b.search_chunk, resident));
-    (void)launch_overlapped(search_bundles_kernel<GS>, dim3(grid), dim3(kEncThreads), cb_bytes, st, b);
+    (void)launch_overlapped(kern, dim3(grid), dim3(kEncThreads), smem, st, b);
     return check_launch("search_bundles_kernel");
   }
   const int grid = (a.p.n_bundles + a.bundles_per_cta - 1) / a.bundles_per_cta;
