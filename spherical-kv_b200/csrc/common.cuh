@@ -13,11 +13,7 @@
 #ifndef SPHKV_SEARCH_UNROLL
 #define SPHKV_SEARCH_UNROLL 2
 #endif
-// all-tier code kernel: tokens per thread (4 = one CTA of 8 warps per SM, 232 registers; 2 = two
-// CTAs per SM) and the unroll factor of its centroid loop
-#ifndef SPHKV_CODE_TOKENS
-#define SPHKV_CODE_TOKENS 4
-#endif
+// all-tier code kernel: unroll factor of its centroid loop
 #ifndef SPHKV_CODE_UNROLL
 #define SPHKV_CODE_UNROLL 4
 #endif

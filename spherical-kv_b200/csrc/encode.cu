@@ -744,10 +744,7 @@ struct CodesArgs {
   sphkv_tiers tiers;
 };
 
-// tokens per thread of the code-cache kernel
-constexpr int kCodeTok = SPHKV_CODE_TOKENS;
-
-template <int OFF, int GS>
+template <int OFF, int GS, int kCodeTok>
 __device__ __forceinline__ void search_slice(const float (&k)[kCodeTok][32], const float* __restrict__ cbg, int C,
                                              int (&code)[kCodeTok]) {
   float best[kCodeTok];
@@ -776,8 +773,6 @@ __device__ __forceinline__ void search_slice(const float (&k)[kCodeTok][32], con
   }
 }
 
-// CTAs per SM of the code-cache kernel (2 tokens per thread fit 128 registers, 4 need 232)
-constexpr int kCodeCtasPerSm = kCodeTok <= 2 ? 2 : 1;
 #ifndef SPHKV_CODE_WARPS
 #define SPHKV_CODE_WARPS 8
 #endif
@@ -792,8 +787,10 @@ constexpr int kCodeThreads = SPHKV_CODE_WARPS * 32;  // a multiple of four warps
 // and the later one-row-per-lane 128-bit reads touch every bank once.  Not STAGED (slices not
 // 16-byte aligned, or no room beside the codebooks): each lane loads its own rows and asks L2
 // for the next block's rows a block ahead.
-template <bool STAGED>
-__global__ void __launch_bounds__(kCodeThreads, kCodeCtasPerSm) encode_codes_kernel(const CodesArgs a) {
+// kCodeTok tokens per thread: four feed 16 fmas from every centroid load (232 registers); with two or one a small
+// input reaches more SMs and waits for a shorter pass (419 tokens x 8 heads: 27 -> 14 us; 2048: 27 -> 19).
+template <bool STAGED, int kCodeTok>
+__global__ void __launch_bounds__(kCodeThreads, 1) encode_codes_kernel(const CodesArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   float* cb_s = reinterpret_cast<float*>(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -932,8 +929,8 @@ __global__ void __launch_bounds__(kCodeThreads, kCodeCtasPerSm) encode_codes_ker
         // both 16-dim halves of the slice, stored as one 8-byte radius pair and one 2-byte code pair
         const int G = a.dh >> 4;
         int code_a[kCodeTok], code_b[kCodeTok];
-        search_slice<0, 16>(k, cb_s + a.cb_off[s] + ((2 * grp) << bits) * 16, C, code_a);
-        search_slice<16, 16>(k, cb_s + a.cb_off[s] + ((2 * grp + 1) << bits) * 16, C, code_b);
+        search_slice<0, 16, kCodeTok>(k, cb_s + a.cb_off[s] + ((2 * grp) << bits) * 16, C, code_a);
+        search_slice<16, 16, kCodeTok>(k, cb_s + a.cb_off[s] + ((2 * grp + 1) << bits) * 16, C, code_b);
 #pragma unroll
         for (int h = 0; h < kCodeTok; ++h) {
           if (!have[h]) continue;
@@ -943,7 +940,7 @@ __global__ void __launch_bounds__(kCodeThreads, kCodeCtasPerSm) encode_codes_ker
         }
       } else {
         int code[kCodeTok];
-        search_slice<0, 32>(k, cb_s + a.cb_off[s] + (grp << bits) * 32, C, code);
+        search_slice<0, 32, kCodeTok>(k, cb_s + a.cb_off[s] + (grp << bits) * 32, C, code);
 #pragma unroll
         for (int h = 0; h < kCodeTok; ++h) {
           if (!have[h]) continue;
@@ -1129,24 +1126,37 @@ extern "C" int sphkv_encode_codes(const void* k_src, int32_t k_dtype, int64_t k_
   // row blocks staged through shared memory when every 32-element slice starts on a 16-byte
   // boundary and the blocks fit beside the codebooks
   const int esz = k_dtype == SPHKV_F32 ? 4 : 2;
-  const int kbuf_bytes = (kCodeThreads / 32) * 32 * kCodeTok * 128;
-  const bool staged = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 &&
-                      (k_head_stride * esz) % 16 == 0 && (off * 4 + kbuf_bytes) * kCodeCtasPerSm <= 220 * 1024;
+  const bool aligned = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 &&
+                       (k_head_stride * esz) % 16 == 0;
   a.kbuf_off = off * 4;
-  const int smem_bytes = off * 4 + (staged ? kbuf_bytes : 0);
-  {
+  const int64_t sms = sm_count_current_device();
+  const int row_sets = (kCodeThreads / 32) / (dh >> 5);  // warps' row sets of a CTA
+  auto launch = [&](auto tok) -> int {
+    constexpr int TOK = decltype(tok)::value;
+    const int kbuf_bytes = (kCodeThreads / 32) * 32 * TOK * 128;
+    const bool staged = aligned && off * 4 + kbuf_bytes <= 220 * 1024;
+    const int smem_bytes = off * 4 + (staged ? kbuf_bytes : 0);
+    auto kern = staged ? encode_codes_kernel<true, TOK> : encode_codes_kernel<false, TOK>;
     static SmemOptIn opt_in[2];
-    const void* fn = staged ? (const void*)encode_codes_kernel<true> : (const void*)encode_codes_kernel<false>;
-    if (int rc = ensure_dynamic_smem(opt_in[staged], fn, smem_bytes, "encode_codes")) return rc;
-  }
-  const int per_cta = (kCodeThreads / 32) / (dh >> 5) * 32 * kCodeTok;  // rows per CTA and pass
-  a.units_per_head = (rows + per_cta - 1) / per_cta;
-  a.n_units = a.units_per_head * Hkv;
-  const int64_t resident = (int64_t)sm_count_current_device() * kCodeCtasPerSm;  // CTAs that fit at once
-  const dim3 grid((unsigned)std::max<int64_t>(1, std::min(a.n_units, resident)));
-  if (staged)
-    encode_codes_kernel<true><<<grid, kCodeThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-  else
-    encode_codes_kernel<false><<<grid, kCodeThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+    if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem_bytes, "encode_codes")) return rc;
+    const int per_cta = row_sets * 32 * TOK;  // rows per CTA and pass
+    a.units_per_head = (rows + per_cta - 1) / per_cta;
+    a.n_units = a.units_per_head * Hkv;
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min(a.n_units, sms)));
+    kern<<<grid, kCodeThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+    return 0;
+  };
+  // Tokens per thread: the fewest microseconds of passes per CTA.  A pass of 4 / 2 / 1 tokens per thread was
+  // measured at 24 / 13 / 9 us (three reference tiers; the ratio is what counts): two or one win where four
+  // would leave SMs without a unit or the last pass nearly empty.
+  auto passes = [&](int tok) {
+    const int64_t units = (rows + row_sets * 32 * tok - 1) / (row_sets * 32 * tok) * Hkv;
+    return (units + sms - 1) / sms;
+  };
+  const int64_t t4 = passes(4) * 24, t2 = passes(2) * 13, t1 = passes(1) * 9;
+  const int rc = t4 <= t2 && t4 <= t1 ? launch(std::integral_constant<int, 4>())
+                 : t2 <= t1           ? launch(std::integral_constant<int, 2>())
+                                      : launch(std::integral_constant<int, 1>());
+  if (rc) return rc;
   return check_launch("encode_codes_kernel");
 }

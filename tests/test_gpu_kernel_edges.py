@@ -1,0 +1,120 @@
+"""GPU: edges of the dispatch rules and tiles of the decode, encode and k-means kernels."""
+import pytest
+import torch
+
+from test_gpu_decode import DEV, build, check_against_oracle
+from util import load_pkg
+
+pkg = load_pkg()
+synth = pkg.synth
+pytestmark = pytest.mark.gpu
+T1, T2, T3 = pkg.REFERENCE_TIERS
+
+
+# tiles per segment around the 24 of a round of three teams and the 8 of a macro tile; blocks dealt by unit (few
+# units) and by range (more units than CTAs divide evenly, uneven rows); a tier whose theta stream holds
+# fewer than eight bits per token (dh 64, tier 3)
+@pytest.mark.parametrize("B,Hkv,dh,ctx,page,specs,fr", [
+    (1, 1, 128, 16, 16, (T1,), {1: 1.0}),
+    (1, 2, 128, 129, 16, (T1,), {1: 1.0}),
+    (1, 1, 64, 385, 16, (T2, T3), {2: 0.5, 3: 0.5}),
+    (1, 3, 64, 4000, 64, (T1, T3), {1: 0.3, 3: 0.6}),
+    (19, 8, 64, 150, 32, (T1, T2), {1: 0.4, 2: 0.4}),
+    (5, 8, 128, 700, 16, (T1, T2, T3), {1: 0.2, 2: 0.3, 3: 0.3}),
+])
+@pytest.mark.parametrize("radius_fmt", [0, 1])
+def test_decode_segment_shapes(B, Hkv, dh, ctx, page, specs, fr, radius_fmt):
+    cache, cbs, K, V, Q, _ = build(B, 2 * Hkv, Hkv, dh, ctx, page, specs, fr, radius_fmt=radius_fmt, seed=ctx)
+    check_against_oracle(cache, cbs, Q, ctx, dh)
+
+
+def test_decode_many_partial_rows_and_idle_ctas():
+    """more than 32 partial rows per unit (the merge's general path), and CTAs without a block"""
+    cache, cbs, K, V, Q, _ = build(1, 4, 1, 128, 2300, 16, (T1, T2), {1: 0.3, 2: 0.6}, seed=3)
+    for n_ctas in (40, 131, 400):
+        cache.scratch = None
+        check_against_oracle(cache, cbs, Q, 2300, 128, n_ctas=n_ctas)
+
+
+@pytest.mark.parametrize("page", [16, 64])
+def test_decode_pool_off_a_16_byte_boundary(page):
+    """byte pool and positions at 4-byte alignment take word copies; the result does not change"""
+    cache, cbs, K, V, Q, _ = build(2, 8, 2, 128, 500, page, (T1, T2), {1: 0.4, 2: 0.4}, seed=5)
+    rope = pkg.rope_table(512, 128, device=DEV)
+    want = pkg.decode_paged(Q.to(DEV), cache, rope).clone()
+    flat = torch.zeros(cache.k_pages.numel() + 16, dtype=torch.uint8, device=DEV)
+    flat[4:4 + cache.k_pages.numel()] = cache.k_pages
+    L = cache.lists
+    pos = torch.zeros(L.positions.numel() + 4, dtype=torch.int32, device=DEV)
+    pos[1:1 + L.positions.numel()] = L.positions.reshape(-1)
+    L.positions = pos[1:1 + L.positions.numel()].view(L.positions.shape)
+    cache.k_pages = flat[4:4 + cache.k_pages.numel()]
+    assert torch.equal(pkg.decode_paged(Q.to(DEV), cache, rope), want)
+    pkg.check_status(cache)
+
+
+@pytest.mark.parametrize("page", [16, 128])
+def test_decode_honours_the_header_count(page):
+    """a page whose header counts fewer tokens than its theta stream has room for"""
+    cache, cbs, K, V, Q, _ = build(1, 8, 2, 128, 400, page, (T1, T2), {1: 0.4, 2: 0.5}, seed=9)
+    L = cache.lists
+    rope = pkg.rope_table(512, 128, device=DEV)
+    fewer = torch.clamp(L.page_count - 5, min=1)
+    slot = torch.arange(page, device=DEV)
+    held, L.positions = L.positions, torch.where(slot[None] < fewer[:, None], L.positions, torch.full_like(L.positions, -1))
+    want = pkg.decode_paged(Q.to(DEV), cache, rope).clone()
+    L.positions = held
+    cache.k_pages[L.ptable[:, 0].long() + 1] = fewer.to(torch.uint8)
+    assert torch.equal(pkg.decode_paged(Q.to(DEV), cache, rope), want)
+
+
+# one, two and four tokens per thread; staged and direct loads
+@pytest.mark.parametrize("T,Hkv,dh", [(2047, 8, 128), (4097, 8, 128), (9001, 8, 128), (6001, 8, 64)])
+@pytest.mark.parametrize("dtype,shift", [(torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)])
+def test_codes_do_not_depend_on_tokens_per_thread(T, Hkv, dh, dtype, shift):
+    """large inputs equal the codes of 64-row slices of them (one token per thread, checked against the oracle)"""
+    tiers = pkg.TierSet(dh)
+    cb = tiers.pack_codebooks(synth.make_codebooks(Hkv, dh, pkg.REFERENCE_TIERS[:2], seed=T)).to(DEV)
+    flat = torch.randn(T * Hkv * dh + 8, generator=torch.Generator(device=DEV).manual_seed(T), device=DEV).to(dtype)
+    K = flat[shift:shift + T * Hkv * dh].view(T, Hkv, dh)
+    got = pkg.encode_codes(K, cb, tiers)
+    for t0 in (0, 64 * (T // 128), T - 64):
+        part = pkg.encode_codes(K[t0:t0 + 64], cb, tiers)
+        for s in range(2):
+            assert torch.equal(got.r[s][:, t0:t0 + 64].view(torch.int32), part.r[s].view(torch.int32))
+            assert torch.equal(got.theta[s][:, t0:t0 + 64], part.theta[s])
+
+
+@pytest.mark.parametrize("dh,dtype", [(128, torch.float32), (64, torch.float16), (128, torch.bfloat16)])
+def test_encode_pages_of_keys_off_a_16_byte_boundary(dh, dtype):
+    Hkv, T, tiers = 3, 900, pkg.TierSet(dh, pkg.REFERENCE_TIERS)
+    cb = tiers.pack_codebooks(synth.make_codebooks(Hkv, dh, pkg.REFERENCE_TIERS, seed=2)).to(DEV)
+    assign = synth.make_tier_assign(1, Hkv, T, {1: 0.3, 2: 0.3, 3: 0.3}, seed=1, per_head=True).to(DEV)
+    lists = pkg.build_page_lists(assign, tiers, 32)
+    K = torch.randn(T, Hkv, dh, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV).to(dtype)
+    flat = torch.zeros(K.numel() + 8, dtype=dtype, device=DEV)
+    off = flat[1:1 + K.numel()].view(K.shape)
+    off.copy_(K)
+    a, b = pkg.encode_pages(K, K, lists, cb, tiers), pkg.encode_pages(off, off, lists, cb, tiers)
+    c = pkg.encode_pages(K, K, lists, cb, tiers, use_scratch=False)
+    for other in (b, c):
+        assert torch.equal(a.k_pages, other.k_pages) and torch.equal(a.v_pool, other.v_pool)
+
+
+@pytest.mark.parametrize("N", [1, 31, 1025, 70001])
+@pytest.mark.parametrize("d,K", [(8, 256), (16, 64), (16, 200), (32, 8), (32, 170)])
+def test_kmeans_sums_and_counts(N, d, K):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    U = torch.nn.functional.normalize(torch.randn(N, d, generator=g, device=DEV), dim=1)
+    C = torch.nn.functional.normalize(torch.randn(K, d, generator=g, device=DEV), dim=1)
+    assigns, best, sums, counts = pkg.kmeans_assign(U, C)
+    sims = U.double() @ C.double().T
+    # the winner of the fp32 chain is within its rounding (16 or 32 terms of magnitude below 1) of the exact maximum
+    picked = sims.gather(1, assigns.long()[:, None])[:, 0]
+    assert (sims.max(1).values - picked).max().item() <= 4 * d * 2.0 ** -24
+    assert (best.double() - picked).abs().max().item() <= 2 * d * 2.0 ** -24
+    assert torch.equal(counts.long(), torch.bincount(assigns.long(), minlength=K))
+    want = torch.zeros(K, d, dtype=torch.float64, device=DEV).index_add_(0, assigns.long(), U.double())
+    # sums of at most n_k numbers below 1 in any order: n_k * n_k * 2^-24 is the worst case, sqrt(n_k) steps typical
+    bound = (counts.double().clamp(min=1) * 2.0 ** -22)[:, None]
+    assert ((sums.double() - want).abs() <= bound).all()
