@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
 // pages take a warp each (no barrier at all; thousands in flight); a 128-token page is eight warps' work:
 // with one, the 440 pages of an 8190-token prompt kept three warps per SM busy (60 us), so 13 us.
 // Shared memory of a page: rows i32[N] | r f32[N*G] | scale f32[8] | theta u8[N*G] | page image.
-template <int SRC>
+template <int SRC, bool ONE_WARP>
 __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
   griddep_wait();
@@ -579,11 +579,11 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
   extern __shared__ __align__(16) uint8_t smem[];
   const int N = p.page_size, dh = p.dh, GST = dh >> 4;
   const int ppb_shift = __clz(N) - 24;  // log2 of the 128 / N pages per bundle (N is 16 .. 128)
-  const int wpp_shift = a.wpp_shift, team = threadIdx.x >> (5 + wpp_shift);
+  const int wpp_shift = ONE_WARP ? 0 : a.wpp_shift, team = threadIdx.x >> (5 + wpp_shift);
   const int nt = 32 << wpp_shift, t0 = threadIdx.x & (nt - 1), lane = threadIdx.x & 31;  // threads of the page, this one
   const int pages_at_once = (kEncThreads / 32) >> wpp_shift;
   auto page_sync = [&]() {
-    if (wpp_shift == 0)
+    if (ONE_WARP)
       __syncwarp();
     else
       asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(nt) : "memory");
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
       if (s0 + lane < N && t0 < 32) rows_w[s0 + lane] = row;
       cnt += __popc(__ballot_sync(0xffffffffu, row >= 0));
     }
-    if (t0 < 8) scale_w[t0] = 0.f;
+    if (!ONE_WARP && t0 < 8) scale_w[t0] = 0.f;
     page_sync();
     // ---- radii and centroid indices of the page; per-group scale = max radius over its tokens.  A thread's
     //      items all belong to one group (32 is a multiple of G) ----
@@ -642,8 +642,12 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
         if (tin < cnt) mx = fmaxf(mx, rv);
       }
       for (int o = G; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      // radii are not negative: their bit patterns order as integers
-      if (lane < G) atomicMax(reinterpret_cast<int*>(scale_w + lane), __float_as_int(mx));
+      if (lane < G) {
+        if (ONE_WARP)
+          scale_w[lane] = mx;
+        else  // radii are not negative: their bit patterns order as integers
+          atomicMax(reinterpret_cast<int*>(scale_w + lane), __float_as_int(mx));
+      }
     }
     page_sync();
     if (cnt > 0) {
@@ -995,16 +999,15 @@ static int launch_assemble(EncodeArgs& a, bool from_codes, cudaStream_t st) {
   a.wpp_shift = N == 16 ? 0 : N == 32 ? 1 : N == 64 ? 2 : 3;
   const int at_once = (kEncThreads / 32) >> a.wpp_shift;
   const int smem_bytes = a.page_smem_bytes * at_once;
-  static SmemOptIn opt_in[2];
-  const void* fn = from_codes ? (const void*)assemble_pages_kernel<3> : (const void*)assemble_pages_kernel<2>;
-  if (int rc = ensure_dynamic_smem(opt_in[from_codes], fn, smem_bytes, "assemble_pages")) return rc;
+  static SmemOptIn opt_in[2][2];
+  const bool one = a.wpp_shift == 0;
+  auto kern = from_codes ? (one ? assemble_pages_kernel<3, true> : assemble_pages_kernel<3, false>)
+                         : (one ? assemble_pages_kernel<2, true> : assemble_pages_kernel<2, false>);
+  if (int rc = ensure_dynamic_smem(opt_in[from_codes][one], (const void*)kern, smem_bytes, "assemble_pages")) return rc;
   const int64_t items = (int64_t)p.n_bundles * (128 / N);
   const int64_t ctas = (items + at_once - 1) / at_once;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ctas, (int64_t)sm_count_current_device() * 8));
-  if (from_codes)
-    (void)launch_overlapped(assemble_pages_kernel<3>, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);
-  else
-    (void)launch_overlapped(assemble_pages_kernel<2>, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);
+  (void)launch_overlapped(kern, dim3(grid), dim3(kEncThreads), smem_bytes, st, a);
   return check_launch("assemble_pages_kernel");
 }
 
