@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsphkv_b200.so")
+HOST_PATH = os.path.join(HERE, "host_tables.so")
 
 F32, BF16, F16 = 0, 1, 2
 RADIUS_I8, RADIUS_F16 = 0, 1
@@ -113,6 +114,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class SphKVError(RuntimeError):
@@ -142,6 +144,20 @@ def load() -> C.CDLL:
                              f"{lib.sphkv_struct_size(which)} B, binding {C.sizeof(st)} B")
     _lib = lib
     return lib
+
+
+def host_tables():
+    """The module of csrc/host_tables.cpp; raises if it is missing (no fallback exists)."""
+    global _host
+    if _host is None:
+        import importlib.util
+        if not os.path.exists(HOST_PATH):
+            raise SphKVError(f"{HOST_PATH} is missing: build it with `python -c \"import __graft_entry__ as g; g.build()\"`")
+        spec = importlib.util.spec_from_file_location("host_tables", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def stream_ptr() -> int:

@@ -1,4 +1,5 @@
-"""Builds libsphkv_b200.so (sm_100a) in-tree with nvcc.  No GPU is needed to build."""
+"""Builds libsphkv_b200.so (sm_100a) with nvcc and the host module host_tables.so with g++, in-tree.  No GPU is
+needed to build."""
 from __future__ import annotations
 
 import os
@@ -10,6 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libsphkv_b200.so")
+HOST_PATH = os.path.join(HERE, "host_tables.so")
 SOURCES = ["capi.cu", "decode.cu", "encode.cu", "lists.cu", "compat.cu", "pool.cu", "kmeans.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -31,8 +33,24 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_module(force: bool) -> "subprocess.Popen | None":
+    """Starts the compilation of csrc/host_tables.cpp against the installed torch and Python."""
+    import sysconfig
+
+    import torch
+    src = os.path.join(CSRC, "host_tables.cpp")
+    if not (force or _stale(HOST_PATH, [src])):
+        return None
+    root = os.path.dirname(torch.__file__)
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-isystem", sysconfig.get_paths()["include"], src, "-o", HOST_PATH,
+           "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile every .cu under csrc/ and link the shared library.  Returns its path."""
+    """Compile every .cu under csrc/ and link the shared library, and the host module.  Returns the library's path."""
     nvcc = _nvcc()
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(INCLUDE, "sphkv.h"))
@@ -40,6 +58,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(objdir, exist_ok=True)
     objs = []
     procs = []
+    host = _host_module(force)
+    if host is not None:
+        procs.append(("host_tables.cpp", host))
     for src in SOURCES:
         sp = os.path.join(CSRC, src)
         if not os.path.exists(sp):
@@ -57,7 +78,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose or pr.returncode != 0:
             sys.stdout.write(out.decode())
         if pr.returncode != 0:
-            raise RuntimeError(f"nvcc failed on {src}")
+            raise RuntimeError(f"compilation of {src} failed")
     if force or _stale(LIB_PATH, objs):
         cmd = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
         subprocess.check_call(cmd)

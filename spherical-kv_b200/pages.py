@@ -130,11 +130,7 @@ class PageLists:
 
 
 _NATIVE_IDS = (torch.uint8, torch.int32, torch.int64)
-
-
-def _room(n: int) -> int:
-    """n i32 values rounded up to 256 bytes."""
-    return (n + 63) // 64 * 64
+_POINTERS = _lib.PageListsParams.positions.offset  # of the ten tables, in the order of PageLists
 
 
 def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fmt: int, page_align: int,
@@ -164,29 +160,14 @@ def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fm
     perm = None
     if shuffle_seed is not None:
         perm = torch.randperm(P, generator=torch.Generator().manual_seed(shuffle_seed)).to(dev)
-    # One allocation for the ten tables (an allocator call each was a third of a short prompt's host time), each on
-    # a 256-byte boundary, and one strided view per table, made after the fill launch: with split() and a reshape per
-    # piece the lists and pages of 8 heads x 777 tokens took 94 us, like this 73.
-    pn, pr, ub = _room(P * N), _room(P), _room(U * max_blocks)
-    src, head = pn, 2 * pn
-    slot, count, ptab = head + pr, head + 2 * pr, head + 3 * pr
-    block = ptab + _room(3 * P)
-    bits, nblk = block + ub, block + 2 * ub
-    bun = nblk + _room(U)
-    buf = torch.empty(bun + 8 * n_bundles, dtype=torch.int32, device=dev)
-    base, cut = buf.data_ptr(), buf.as_strided
-    p.positions, p.src_index, p.page_head, p.page_slot = base, base + 4 * src, base + 4 * head, base + 4 * slot
-    p.page_count, p.ptable, p.block_table = base + 4 * count, base + 4 * ptab, base + 4 * block
-    p.bits_table, p.num_blocks, p.bundles = base + 4 * bits, base + 4 * nblk, base + 4 * bun
+    # One allocation for the ten tables, each on a 256-byte boundary, cut by the host module: the lists and pages of
+    # 8 heads x 777 tokens took 94 us with split() and a reshape per piece, 73 with a strided view per table made
+    # from Python, 62 like this.
+    tables = _lib.host_tables().make(C.addressof(p) + _POINTERS, dev.index, P, N, U, max_blocks, n_bundles)
     p.n_pages, p.max_blocks = P, max_blocks
     p.perm = None if perm is None else perm.data_ptr()
     _lib.check(lib.sphkv_page_lists_fill(C.byref(p), st), "sphkv_page_lists_fill")
-    return PageLists(page_size=N, n_pages=P, positions=cut((P, N), (N, 1)), src_index=cut((P, N), (N, 1), src),
-                     page_head=cut((P,), (1,), head), page_slot=cut((P,), (1,), slot), page_count=cut((P,), (1,), count),
-                     ptable=cut((P, 3), (3, 1), ptab), block_table=cut((U, max_blocks), (max_blocks, 1), block),
-                     bits_table=cut((U, max_blocks), (max_blocks, 1), bits), num_blocks=cut((U,), (1,), nblk),
-                     bundles=cut((n_bundles, 8), (8, 1), bun), pool_bytes=pool_bytes, B=B, Hkv=Hkv,
-                     max_blocks=max_blocks, covers_pool=True)
+    return PageLists(N, P, *tables, pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks, covers_pool=True)
 
 
 def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
