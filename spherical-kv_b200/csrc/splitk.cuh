@@ -857,8 +857,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           if (have[pass]) {
             // ---- rebuild and rotate the keys chunk by chunk; bf16 hi | lo parts to tensor memory ----
             // Operand split: hi = the upper 16 bits of the fp32 value (a bf16 number, by truncation: one
-            // byte permute packs two of them), lo = the value minus hi, again truncated to bf16; hi + lo
-            // carries 16 mantissa bits, products are accumulated in fp32.
+            // byte permute packs two of them), lo = the value minus hi, rounded to bf16; hi + lo carries 16
+            // mantissa bits without a bias (a truncated lo: twice the error), products are accumulated in fp32.
             const uint32_t ta = tmem_rows + ((uint32_t)(16 * pass) << 16) + kColKeys;
 #pragma unroll
             for (int i = 0; i < NCH; ++i) {
@@ -895,7 +895,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
                     const uint32_t h0 = a0 & 0xFFFF0000u, h1 = a1 & 0xFFFF0000u;
                     const float2 l = __ffma2_rn(f2(__uint_as_float(h0), __uint_as_float(h1)), f2(-1.f, -1.f), v[hf][e2]);
                     pk[4 * hf + 2 * tk + e2] = __byte_perm(a0, a1, 0x7632);
-                    pk[8 + 4 * hf + 2 * tk + e2] = __byte_perm(__float_as_uint(l.x), __float_as_uint(l.y), 0x7632);
+                    const __nv_bfloat162 lb = __floats2bfloat162_rn(l.x, l.y);
+                    pk[8 + 4 * hf + 2 * tk + e2] = *reinterpret_cast<const uint32_t*>(&lb);
                   }
               }
               // this chunk's cos/sin registers are free: fetch the next pass's
@@ -1026,23 +1027,19 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           }
         }
         // ---- weights into the MN-major operand layout: token rows of 16 bytes (eight columns), 8-token
-        //      groups at 128 bytes, the second eight columns at 256 ----
+        //      groups at 128 bytes, the second eight columns at 256.  Hi + lo parts for either type of V: against
+        //      a lagging reference maximum not even the largest weight is exactly 1, and 11 bits of it showed
+        //      (error of a three-row step with f16 V against float64: 1.4e-4, so 1.3e-5; 24.6 -> 25.1 us) ----
 #pragma unroll
         for (int h = 0; h < HEADS; ++h) l_run[h] += pv[h];
         if (xs < width) {
           uint32_t hi[HEADS / 2], lo[HEADS / 2];
 #pragma unroll
           for (int h = 0; h < HEADS; h += 2) {
-            if (kBf16) {
-              const __nv_bfloat162 hb = __floats2bfloat162_rn(pv[h], pv[h + 1]);
-              const float2 hf = __bfloat1622float2(hb);
-              const __nv_bfloat162 lb = __floats2bfloat162_rn(pv[h] - hf.x, pv[h + 1] - hf.y);
-              hi[h / 2] = *reinterpret_cast<const uint32_t*>(&hb);
-              lo[h / 2] = *reinterpret_cast<const uint32_t*>(&lb);
-            } else {
-              hi[h / 2] = pack_f16x2(pv[h], pv[h + 1]);
-              lo[h / 2] = 0;
-            }
+            if (kBf16)
+              split_bf16x2(pv[h], pv[h + 1], hi[h / 2], lo[h / 2]);
+            else
+              split_f16x2(pv[h], pv[h + 1], hi[h / 2], lo[h / 2]);
           }
           const uint32_t dst = p_buf + xs * 512 + (tok >> 3) * 128 + (tok & 7) * 16;
           if (PACK) {
