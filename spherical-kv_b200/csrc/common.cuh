@@ -112,10 +112,12 @@ __device__ __forceinline__ float4 lds_f4(uint32_t smem_addr) {
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_addr));
   return v;
 }
+// Copies belong to a group once they are committed: cp_async_wait<N>() waits until at most the N newest groups are
+// in flight, and not for copies that were never committed.
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 // Programmatic dependent launch.  A kernel launched with the stream-serialization attribute may
 // become resident while the kernel before it in the stream is still running; it must not touch

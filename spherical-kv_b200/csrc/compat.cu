@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
       cp_async_16(dst + v_bytes + c_bytes + i, radius_codes + tok0 * G_max + i);
     }
     for (int i = lane * 16; i < v_bytes; i += 512) cp_async_16(dst + i, vs + i);
+    cp_async_commit();
   };
   int phys_next = page_of(0);
   issue_stage(phys_next);

@@ -74,3 +74,44 @@ def test_ragged_logits_shapes(dh, page_size, tier, grp):
         torch.cat([cbs[0][h] for h in range(Hkv)], 0).to(DEV), dh, G, t.g, t.b_theta, page_size).cpu()
     assert (got - want).abs().max().item() <= 2e-4
     assert torch.equal(got == 0, want == 0)
+
+
+# CTAs that take several rounds of pages, restaging their rows between them: a warp per page (16-token pages) and eight
+# warps per page; holes, a last round that is partly empty, and a second pool so that what the first call left in
+# shared memory cannot match
+@pytest.mark.parametrize("page_size,grp", [(16, 2), (128, 1)])
+@pytest.mark.parametrize("rounds", [1, 2, 3, 4])
+def test_pool_decode_rounds(page_size, grp, rounds):
+    import fused_decode
+    Hkv, dh = 8, 128
+    tiers = pkg.TierSet(dh, pkg.REFERENCE_TIERS)
+    at_once = 8 if page_size == 16 else 1
+    max_blocks = -(-rounds * at_once * 2 * pkg._lib.load().sphkv_sm_count() // Hkv) + 3
+    for seed in (1, 2):
+        g = torch.Generator().manual_seed(10 * rounds + seed)
+        cbs = synth.make_codebooks(Hkv, dh, pkg.REFERENCE_TIERS, seed=seed)
+        P = 150                                              # pages may repeat in the lists: they are only read
+        bits = torch.randint(0, 3, (Hkv, max_blocks), generator=g, dtype=torch.int32)
+        table = torch.randint(0, P // 3, (Hkv, max_blocks), generator=g, dtype=torch.int32) * 3 + bits
+        table[torch.rand(Hkv, max_blocks, generator=g) < 0.05] = -1
+        C = torch.tensor([1 << t.b_theta for t in pkg.REFERENCE_TIERS])[torch.arange(P) % 3]
+        theta = (torch.rand(P, page_size, tiers.G_max, generator=g) * C[:, None, None]).to(torch.uint8)
+        radius = torch.randint(0, 256, theta.shape, generator=g).to(torch.uint8)
+        scales = torch.rand(P, tiers.G_max, generator=g) + 0.5
+        v = torch.randn(P, page_size, dh, generator=g).half()
+        tier_G = torch.tensor([dh // t.g for t in pkg.REFERENCE_TIERS], dtype=torch.int32)
+        tier_g = torch.tensor([t.g for t in pkg.REFERENCE_TIERS], dtype=torch.int32)
+        cb = tiers.pack_codebooks(cbs)
+        Hq, sm = Hkv * grp, 1.0 / math.sqrt(dh)
+        q = torch.randn(Hq, dh, generator=g)
+        want, want_part = orc.pool_decode(q, cb, tier_G, tier_g, theta, radius, scales, v, table, bits, sm)
+        out, part = torch.zeros(Hq, dh, device=DEV), torch.full((Hq, max_blocks, dh + 2), 7.0, device=DEV)
+        ctx = torch.full((Hkv,), max_blocks * page_size, dtype=torch.int32, device=DEV)
+        fused_decode.sphkv_decode(q.to(DEV), cb.to(DEV), tier_G.to(DEV), tier_g.to(DEV), theta.to(DEV), radius.to(DEV),
+                                  scales.to(DEV), v.to(DEV), table.to(DEV), bits.to(DEV), ctx, out, part, Hq, Hkv, grp, 3,
+                                  max_blocks, page_size, dh, tiers.G_max, tiers.C_max, tiers.g_max, sm, max_blocks * page_size)
+        gp, live = part.cpu(), torch.isfinite(want_part[:, :, 0])
+        assert torch.equal(torch.isfinite(gp[:, :, 0]), live) and (gp[:, :, 1:][~live] == 0).all()
+        # fp32 sums of at most page_size terms in another order: a few ulps of the sum of magnitudes
+        assert (gp[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
+        assert (out.cpu() - want).abs().max().item() <= 2e-4
