@@ -18,41 +18,40 @@
 
 namespace sphkv {
 
-constexpr int kKmThreads = 256;
-constexpr int kKmWarps = kKmThreads / 32;
 // points per thread: 4 (2 for 32-dim points) keeps the kernel at two CTAs per SM
 __host__ __device__ constexpr int pts_for(int d) { return d >= 32 ? 2 : 4; }
 
-// a CTA takes passes of kKmThreads * pts_for(D) points; its warps walk them without meeting
-template <int D>
-__global__ void __launch_bounds__(kKmThreads, 2) kmeans_assign_kernel(
+// a CTA takes passes of 32 * pts_for(D) points per warp; its warps walk them without meeting
+template <int D, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 2) kmeans_assign_kernel(
     const float* __restrict__ U, int64_t N, const float* __restrict__ centers, int K,
     int32_t* __restrict__ assigns, float* __restrict__ best_sim, float* __restrict__ sums,
     int32_t* __restrict__ counts, int ways) {
   constexpr int kPts = pts_for(D);
   constexpr int kWarpPts = 32 * kPts;           // points of a warp per pass
   extern __shared__ __align__(16) float sm[];
+  constexpr int threads = 32 * WARPS;
   float* c_s = sm;                                            // [K][D] centres
   float* sum_s = sm + K * D;                                  // [warps][ways][K][D] sums
-  int* cnt_s = reinterpret_cast<int*>(sum_s + kKmWarps * ways * K * D);  // [K] counts of this CTA
+  int* cnt_s = reinterpret_cast<int*>(sum_s + WARPS * ways * K * D);     // [K] counts of this CTA
   uint8_t* code_s = reinterpret_cast<uint8_t*>(cnt_s + K);               // [warps][32]
-  for (int i = threadIdx.x; i < K * D; i += kKmThreads) c_s[i] = centers[i];
-  for (int i = threadIdx.x; i < kKmWarps * ways * K * D; i += kKmThreads) sum_s[i] = 0.f;
-  for (int i = threadIdx.x; i < K; i += kKmThreads) cnt_s[i] = 0;
+  for (int i = threadIdx.x; i < K * D; i += threads) c_s[i] = centers[i];
+  for (int i = threadIdx.x; i < WARPS * ways * K * D; i += threads) sum_s[i] = 0.f;
+  for (int i = threadIdx.x; i < K; i += threads) cnt_s[i] = 0;
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* my_codes = code_s + warp * 32;
   // 32 rows of points, 16-byte chunk q of row p at chunk q ^ turn(p): neither the row-per-lane stores nor the
   // dimension-per-lane loads meet in a bank
-  float* tile = reinterpret_cast<float*>(sm + K * D + kKmWarps * ways * K * D + ((K + 3) & ~3) + kKmWarps * 8) + warp * 32 * D;
+  float* tile = reinterpret_cast<float*>(sm + K * D + WARPS * ways * K * D + ((K + 3) & ~3) + WARPS * 8) + warp * 32 * D;
   auto turn = [](int p) { return (p >> (D == 32 ? 0 : D == 16 ? 1 : 2)) & (D / 4 - 1); };
   // adding: lane = (way, dimension); with one way the first D lanes work
   const int dim = lane & (D - 1), way = lane / D;
   const bool adds = way < ways;
   float* my_sums = sum_s + ((int64_t)warp * ways + (adds ? way : 0)) * K * D + dim;
 
-  const int64_t stride = (int64_t)gridDim.x * kKmWarps * kWarpPts;
-  for (int64_t base = ((int64_t)blockIdx.x * kKmWarps + warp) * kWarpPts; base < N; base += stride) {
+  const int64_t stride = (int64_t)gridDim.x * WARPS * kWarpPts;
+  for (int64_t base = ((int64_t)blockIdx.x * WARPS + warp) * kWarpPts; base < N; base += stride) {
     float u[kPts][D];
     bool live[kPts];
 #pragma unroll
@@ -128,29 +127,34 @@ __global__ void __launch_bounds__(kKmThreads, 2) kmeans_assign_kernel(
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < K * D; i += kKmThreads) {
+  for (int i = threadIdx.x; i < K * D; i += threads) {
     float t = 0.f;
-    for (int w = 0; w < kKmWarps * ways; ++w) t += sum_s[(int64_t)w * K * D + i];
+    for (int w = 0; w < WARPS * ways; ++w) t += sum_s[(int64_t)w * K * D + i];
     if (t != 0.f) atomicAdd(sums + i, t);
   }
-  for (int i = threadIdx.x; i < K; i += kKmThreads)
+  for (int i = threadIdx.x; i < K; i += threads)
     if (cnt_s[i] != 0) atomicAdd(counts + i, cnt_s[i]);
 }
 
-template <int D>
+template <int D, int WARPS = 8>
 static int launch_kmeans(const float* U, int64_t N, const float* centers, int K, int32_t* assigns, float* best_sim, float* sums,
                          int32_t* counts, int sms, cudaStream_t st) {
   // a set of sums for every D lanes of a warp while two CTAs fit an SM, else one per warp
   auto bytes = [&](int ways) {
-    return ((size_t)K * D * (1 + kKmWarps * ways) + ((K + 3) & ~3) + kKmWarps * 8 + kKmWarps * 32 * D) * sizeof(float);
+    return ((size_t)K * D * (1 + WARPS * ways) + ((K + 3) & ~3) + WARPS * 8 + WARPS * 32 * D) * sizeof(float);
   };
   int ways = 32 / D;
   if (bytes(ways) > 110 * 1024) ways = 1;
+  const size_t smem = bytes(ways);
+  // eight warps' sums are more than a CTA can have from K 173 on at d 32: seven (a runtime warp count cost every
+  // size 1 to 4 %)
+  if constexpr (WARPS == 8 && D == 32)
+    if (smem > 227 * 1024) return launch_kmeans<D, 7>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
   static SmemOptIn opt_in;
-  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_assign_kernel<D>, (int)bytes(ways), "kmeans_assign")) return rc;
-  const int64_t pass = (int64_t)kKmThreads * pts_for(D);
-  const int64_t ctas = std::min<int64_t>((N + pass - 1) / pass, (int64_t)sms * (bytes(ways) <= 110 * 1024 ? 2 : 1));
-  kmeans_assign_kernel<D><<<(unsigned)ctas, kKmThreads, bytes(ways), st>>>(U, N, centers, K, assigns, best_sim, sums, counts, ways);
+  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_assign_kernel<D, WARPS>, (int)smem, "kmeans_assign")) return rc;
+  const int64_t pass = (int64_t)32 * WARPS * pts_for(D);
+  const int64_t ctas = std::min<int64_t>((N + pass - 1) / pass, (int64_t)sms * (smem <= 110 * 1024 ? 2 : 1));
+  kmeans_assign_kernel<D, WARPS><<<(unsigned)ctas, 32 * WARPS, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, ways);
   return check_launch("kmeans_assign_kernel");
 }
 
@@ -167,9 +171,10 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
   SPHKV_REQUIRE((reinterpret_cast<uintptr_t>(U) & 15) == 0, SPHKV_E_ARG, "kmeans_assign: U must be 16-byte aligned");
   const int sms = sphkv_sm_count();
   SPHKV_REQUIRE(sms > 0, SPHKV_E_ARG, "kmeans_assign: cannot resolve the SM count");
-  const size_t smem = (size_t)K * d * 8 + (size_t)(3 * K + 1) * 4 + (size_t)kKmThreads * pts_for(d) * 2;
-  SPHKV_REQUIRE(smem <= 48 * 1024, SPHKV_E_LIMIT, "kmeans_assign: K=%d x d=%d needs %zu B of shared memory (limit 49152)",
-                K, d, smem);
+  // the sizes the call takes (8 and 16: every K; 32: K up to 179); all of them fit with one set of sums per warp
+  const int per_pass = 256 * pts_for(d) * 2;
+  SPHKV_REQUIRE(K * d * 8 + (3 * K + 1) * 4 + per_pass <= 48 * 1024, SPHKV_E_LIMIT,
+                "kmeans_assign: K=%d x d=%d is beyond the sizes it takes (K * d * 8 + 12 * K + %d <= 49152)", K, d, 4 + per_pass);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(float) * K * d, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, sizeof(int32_t) * K, st);
@@ -182,4 +187,3 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
          : d == 16 ? launch_kmeans<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
                    : launch_kmeans<32>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
 }
-

@@ -118,3 +118,15 @@ def test_kmeans_sums_and_counts(N, d, K):
     # sums of at most n_k numbers below 1 in any order: n_k * n_k * 2^-24 is the worst case, sqrt(n_k) steps typical
     bound = (counts.double().clamp(min=1) * 2.0 ** -22)[:, None]
     assert ((sums.double() - want).abs() <= bound).all()
+
+
+# the largest codebooks of 32-dim points: eight, then seven sets of sums per CTA
+@pytest.mark.parametrize("K", [172, 173, 179])
+def test_kmeans_largest_codebooks(K):
+    test_kmeans_sums_and_counts(5001, 32, K)
+
+
+def test_kmeans_refuses_what_it_refused():
+    U, C = torch.zeros(8, 32, device=DEV), torch.zeros(180, 32, device=DEV)
+    with pytest.raises(pkg.SphKVError, match="K=180 x d=32"):
+        pkg.kmeans_assign(U, C)
