@@ -130,3 +130,9 @@ def test_kmeans_refuses_what_it_refused():
     U, C = torch.zeros(8, 32, device=DEV), torch.zeros(180, 32, device=DEV)
     with pytest.raises(pkg.SphKVError, match="K=180 x d=32"):
         pkg.kmeans_assign(U, C)
+
+
+# 8-dim points: four, two and one set of sums per warp
+@pytest.mark.parametrize("K", [98, 99, 190, 191])
+def test_kmeans_sets_of_sums(K):
+    test_kmeans_sums_and_counts(9001, 8, K)
