@@ -29,11 +29,14 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
   return ok;
 }
 // Bounded wait: what a warp waits for is work of this CTA, done within microseconds; a phase that has not
-// completed after 2^25 tries (a second or more: a try suspends the warp for a while) is lost.  The
-// caller then raises a status bit and its warps stop working instead of spinning for ever.  (A bound by
-// clock64() cost 15 % of the decode step: the clock is read on every entry that does not succeed at once.)
+// completed after kWaitTries is lost.  The caller then raises a status bit and its warps stop working instead of
+// spinning for ever.  A try on a phase that does not complete holds the warp for 4.0 us on this part (measured,
+// with and without a suspend-time hint), so 2^18 of them are 1.05 s.  The bound is a count because reading a clock
+// in this loop, even once in 4096 tries, costs the decode step 7 to 20 % (8 x 32768: 151 -> 161 .. 181 us).
+constexpr int kWaitTries = 1 << 18;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < (1 << 25); ++i)
+#pragma unroll 1
+  for (int i = 0; i < kWaitTries; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
