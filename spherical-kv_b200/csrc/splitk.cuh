@@ -205,7 +205,7 @@ static_assert(kKTh + 112 <= kKRd && kKRd + 128 + 16 <= 384 - 64 && kKRd + 256 + 
 // the largest 16-token page, 8 + 32 + 96 + 128 (256) bytes + 12 phase, ends before the positions as well
 
 // barriers of a team (8 bytes each, kBarStride per team)
-enum { kBarKFull = 0, kBarKeys = kKStages, kBarKeys2, kBarLogits, kBarWeights, kBarV, kBarOut, kBarVote, kBarCount };
+enum { kBarKFull = 0, kBarKeys = kKStages, kBarKeys2, kBarLogits, kBarWeights, kBarV, kBarOut, kBarVote, kBarDrain, kBarCount };
 constexpr int kBarStride = 128;
 static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 256 + 32) + 64 <= kSmemBars, "barrier block");
 
@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     mbar_init(bar + 8 * kBarV, 1);
     mbar_init(bar + 8 * kBarOut, 1);
     mbar_init(bar + 8 * kBarVote, 4);
+    mbar_init(bar + 8 * kBarDrain, 1);
   }
   if (!driver) {
     if (in_use)
@@ -408,6 +409,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   if (driver) {
   regs_down<kDriverRegs>();
   uint32_t par_keys = 0, par_weights = 0, par_v = 0, par_out = 0;
+  bool v_pending = false;  // V tiles issued, their arrival not seen yet
+  bool drained = false;
   const uint64_t v_policy = policy_evict_first();  // V is read once per step, the cos/sin rows many times
   for (; start < end; start = seg_end, ++u) {
     next_segment();
@@ -504,6 +507,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         const int y = m.phys * N + 16 * meta_sub(m);
         tma_load_3d(v_buf + lane * V_TILE, &a.v_map, 0, y, 0, bar + 8 * kBarV, v_policy);
       }
+      v_pending = true;
       return mask;
     };
 
@@ -600,6 +604,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       if (!__all_sync(0xffffffffu, got)) { dead = true; break; }
       par_weights ^= 1;
       par_v ^= 1;
+      v_pending = false;
       tc_fence_after();
       if (elect_one()) {
         // A = V^T: 64-dim halves 2048 bytes apart (dh 64: the second half repeats the first, its rows of
@@ -617,7 +622,20 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       par_out ^= 1;
       if (k + 1 < rounds) v_tiles = issue_v(k + 1);
     }
-    if (dead) give_up();
+    if (dead && !drained) {
+      give_up();
+      // nothing that this warp started may still write when the CTA's memory is given back: page bytes, V tiles
+      // and products, each awaited within the same bound (a dead driver issues nothing in later segments)
+      drained = true;
+      cp_async_wait_all();
+      if (v_pending) (void)mbar_wait(bar + 8 * kBarV, par_v);
+      __syncwarp();
+      if (in_use) {
+        if (elect_one()) mma_commit(bar + 8 * kBarDrain);
+        __syncwarp();
+        (void)mbar_wait(bar + 8 * kBarDrain, 0);
+      }
+    }
     dead = dead || shared_words[1] != 0;
   }
   } else {
@@ -1058,6 +1076,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * kBarOut, par_out))) dead = true;
         par_out ^= 1;
       }
+      if (dead) tmem_wait_st();  // this warp's stores to tensor memory
     }
     if (dead) give_up();
 

@@ -47,6 +47,9 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
 __device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* gptr) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr), "l"(gptr));
 }
+__device__ __forceinline__ void cp_async_wait_all() {  // this thread's copies, committed to a group or not
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
 __device__ __forceinline__ void fence_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
