@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) 
     const float one_minus = (1.0f - p.ema_beta) / (float)a.grp;
     const int h = threadIdx.x & (gp - 1);
     const int per_cta = blockDim.x >> gp_shift;
-    const float2* ml = reinterpret_cast<const float2*>(p.page_ml) +
-                       ((int64_t)b * p.Hq + (int64_t)hkv * a.grp + min(h, a.grp - 1)) * p.max_blocks * tpp;
+    // (max, sum) pairs as two 4-byte loads: page_ml is the caller's and need not start on 8 bytes
+    const float* ml = p.page_ml + ((int64_t)b * p.Hq + (int64_t)hkv * a.grp + min(h, a.grp - 1)) * p.max_blocks * tpp * 2;
     for (int blk0 = blockIdx.y * per_cta; blk0 < p.max_blocks; blk0 += gridDim.y * per_cta) {
       const int blk = blk0 + (threadIdx.x >> gp_shift);
       const bool in = (int)(threadIdx.x >> gp_shift) < per_cta && blk < p.max_blocks;
@@ -191,7 +191,10 @@ __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) 
       if (in && h < a.grp && blk < nb_unit && bt[blk] >= 0) {
         float2 t[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) t[i] = i < tpp ? ml[(int64_t)blk * tpp + i] : make_float2(-INFINITY, 0.f);
+        for (int i = 0; i < 8; ++i) {
+          const float* pair = ml + 2 * ((int64_t)blk * tpp + i);
+          t[i] = i < tpp ? make_float2(pair[0], pair[1]) : make_float2(-INFINITY, 0.f);
+        }
         float m = -INFINITY, l = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i)

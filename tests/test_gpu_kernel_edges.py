@@ -139,3 +139,18 @@ def test_kmeans_refuses_what_it_refused():
 @pytest.mark.parametrize("K", [98, 99, 190, 191])
 def test_kmeans_sets_of_sums(K):
     test_kmeans_sums_and_counts(9001, 8, K)
+
+
+@pytest.mark.parametrize("page", [16, 64])
+def test_importance_update_with_statistics_off_an_8_byte_boundary(page):
+    cache, cbs, K, V, Q, _ = build(2, 8, 2, 128, 500, page, (T1, T2), {1: 0.4, 2: 0.4}, seed=5)
+    L, rope, q = cache.lists, pkg.rope_table(512, 128, device=DEV), Q.to(DEV)
+    n = 2 * 8 * L.max_blocks * (page // 16) * 2
+    got = []
+    for shift in (0, 1):
+        ml = torch.zeros(n + 1, device=DEV)[shift:shift + n].view(2, 8, L.max_blocks, page // 16, 2)
+        omega = torch.full((4, L.max_blocks), 0.5, device=DEV)
+        got.append((pkg.decode_paged(q, cache, rope, page_ml=ml, omega=omega).clone(), omega, ml.clone()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    pkg.check_status(cache)
