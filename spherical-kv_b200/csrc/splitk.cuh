@@ -409,8 +409,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   if (driver) {
   regs_down<kDriverRegs>();
   uint32_t par_keys = 0, par_weights = 0, par_v = 0, par_out = 0;
-  bool v_pending = false;  // V tiles issued, their arrival not seen yet
-  bool drained = false;
   const uint64_t v_policy = policy_evict_first();  // V is read once per step, the cos/sin rows many times
   for (; start < end; start = seg_end, ++u) {
     next_segment();
@@ -507,7 +505,6 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         const int y = m.phys * N + 16 * meta_sub(m);
         tma_load_3d(v_buf + lane * V_TILE, &a.v_map, 0, y, 0, bar + 8 * kBarV, v_policy);
       }
-      v_pending = true;
       return mask;
     };
 
@@ -571,6 +568,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       v_tiles = issue_v(0);
       meta_blocks(4);
     }
+    int lost = 0;  // a wait ran out: 1 with V tiles on their way, 2 without
     bool started = false;
     const uint64_t q_desc = smem_desc(q_u32, 128, 256, 0), p_desc = smem_desc(p_buf, 128, 256, 0);
     const uint64_t v_desc = smem_desc(v_buf, DH == 128 ? 2048 : 0, 1024, 2);
@@ -586,7 +584,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       // the first chunks of the keys are multiplied while the teams rebuild the last
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
-        if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * (kBarKeys + part), par_keys))) { dead = true; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * (kBarKeys + part), par_keys))) { lost = 1; break; }
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
@@ -595,16 +593,15 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           if (part == 1) mma_commit(bar + 8 * kBarLogits);
         }
       }
-      if (dead) break;
+      if (lost) break;
       par_keys ^= 1;
       __syncwarp();
       if (k + n_stages < rounds) issue_k(k + n_stages, st);  // the team has read macro tile k's stage
       if (++st == n_stages) st = 0;
       const bool got = mbar_wait(bar + 8 * kBarWeights, par_weights) && mbar_wait(bar + 8 * kBarV, par_v);
-      if (!__all_sync(0xffffffffu, got)) { dead = true; break; }
+      if (!__all_sync(0xffffffffu, got)) { lost = 1; break; }
       par_weights ^= 1;
       par_v ^= 1;
-      v_pending = false;
       tc_fence_after();
       if (elect_one()) {
         // A = V^T: 64-dim halves 2048 bytes apart (dh 64: the second half repeats the first, its rows of
@@ -618,23 +615,22 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       }
       started = started || v_tiles != 0;
       __syncwarp();
-      if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * kBarOut, par_out))) { dead = true; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(bar + 8 * kBarOut, par_out))) { lost = 2; break; }
       par_out ^= 1;
       if (k + 1 < rounds) v_tiles = issue_v(k + 1);
     }
-    if (dead && !drained) {
+    if (lost) {
+      // Nothing that this driver started may still write when the CTA's memory is given back: page bytes, V tiles
+      // and products are awaited, each within the same bound.  Reached once at most: it has no rounds in later
+      // segments.
+      dead = true;
       give_up();
-      // nothing that this warp started may still write when the CTA's memory is given back: page bytes, V tiles
-      // and products, each awaited within the same bound (a dead driver issues nothing in later segments)
-      drained = true;
       cp_async_wait_all();
-      if (v_pending) (void)mbar_wait(bar + 8 * kBarV, par_v);
+      if (lost == 1) (void)mbar_wait(bar + 8 * kBarV, par_v);
       __syncwarp();
-      if (in_use) {
-        if (elect_one()) mma_commit(bar + 8 * kBarDrain);
-        __syncwarp();
-        (void)mbar_wait(bar + 8 * kBarDrain, 0);
-      }
+      if (elect_one()) mma_commit(bar + 8 * kBarDrain);
+      __syncwarp();
+      (void)mbar_wait(bar + 8 * kBarDrain, 0);
     }
     dead = dead || shared_words[1] != 0;
   }
