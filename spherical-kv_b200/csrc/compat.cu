@@ -49,7 +49,8 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
   extern __shared__ __align__(16) uint8_t smem_raw[];
   float* sq = reinterpret_cast<float*>(smem_raw);                 // [kv_groups][dh]
   float* lut = sq + kv_groups * dh;                                // [num_tiers][kv_groups][G_max][cb_max]
-  float* slog_all = lut + num_tiers * kv_groups * G_max * cb_max;  // [warps][kv_groups][seg]
+  // an even number of floats: the accumulators of fold_all are stored in 8-byte pieces
+  float* slog_all = lut + ((num_tiers * kv_groups * G_max * cb_max + 1) & ~1);  // [warps][kv_groups][seg]
   float* srs_all = slog_all + kPoolWarps * kv_groups * seg;        // [warps][G_max]
   float* fold_all = srs_all + kPoolWarps * G_max;                  // wpp > 1: [warps][kv_groups][dh + 2]
   float* slog = slog_all + warp * kv_groups * seg;
@@ -593,7 +594,7 @@ extern "C" int sphkv_pool_decode(const float* q_all, const float* cb_flat, const
                     (reinterpret_cast<uintptr_t>(theta_codes) & 3) == 0 && (reinterpret_cast<uintptr_t>(radius_codes) & 3) == 0,
                 SPHKV_E_ALIGN, "pool_decode: v_pool / partial_scratch need 8 B, code arrays 4 B alignment");
   auto smem_for = [&](int wpp) -> size_t {
-    return ((size_t)kv_groups * dh + (size_t)num_tiers * kv_groups * G_max * cb_max +
+    return ((size_t)kv_groups * dh + (((size_t)num_tiers * kv_groups * G_max * cb_max + 1) & ~(size_t)1) +
             (size_t)kPoolWarps * ((size_t)kv_groups * (page_size / wpp) + G_max) +
             (wpp > 1 ? (size_t)kPoolWarps * kv_groups * (dh + 2) : 0)) * sizeof(float);
   };

@@ -115,3 +115,46 @@ def test_pool_decode_rounds(page_size, grp, rounds):
         # fp32 sums of at most page_size terms in another order: a few ulps of the sum of magnitudes
         assert (gp[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
         assert (out.cpu() - want).abs().max().item() <= 2e-4
+
+
+def random_pool(seed, Hkv, dh, page_size, max_blocks, g, C, n_tiers=1, P=20):
+    """A LayerPool of one group size and C centroids per group, random codes and a hole per head."""
+    gen = torch.Generator().manual_seed(seed)
+    G = dh // g
+    cb = torch.nn.functional.normalize(torch.randn(Hkv, n_tiers, G, C, g, generator=gen), dim=-1)
+    table = torch.randint(0, P, (Hkv, max_blocks), generator=gen, dtype=torch.int32)
+    table[:, 1] = -1
+    return dict(cb=cb, table=table, bits=torch.randint(0, n_tiers, (Hkv, max_blocks), generator=gen, dtype=torch.int32),
+                theta=torch.randint(0, C, (P, page_size, G), generator=gen).to(torch.uint8),
+                radius=torch.randint(1, 256, (P, page_size, G), generator=gen).to(torch.uint8),
+                scales=torch.rand(P, G, generator=gen) + 0.5, v=torch.randn(P, page_size, dh, generator=gen).half(),
+                tier_G=torch.full((n_tiers,), G, dtype=torch.int32), tier_g=torch.full((n_tiers,), g, dtype=torch.int32))
+
+
+def run_pool(pool, q, grp):
+    import fused_decode
+    Hkv, max_blocks = pool["table"].shape
+    _, n_tiers, G, C, g = pool["cb"].shape
+    Hq, dh = q.shape
+    page_size, sm = pool["theta"].shape[1], 1.0 / math.sqrt(dh)
+    out, part = torch.zeros(Hq, dh, device=DEV), torch.full((Hq, max_blocks, dh + 2), 7.0, device=DEV)
+    d = {k: x.to(DEV) for k, x in pool.items()}
+    fused_decode.sphkv_decode(q.to(DEV), d["cb"], d["tier_G"], d["tier_g"], d["theta"], d["radius"], d["scales"], d["v"],
+                              d["table"], d["bits"], torch.full((Hkv,), max_blocks * page_size, dtype=torch.int32, device=DEV),
+                              out, part, Hq, Hkv, grp, n_tiers, max_blocks, page_size, dh, G, C, g, sm, max_blocks * page_size)
+    want, want_part = orc.pool_decode(q, pool["cb"], pool["tier_G"], pool["tier_g"], pool["theta"], pool["radius"],
+                                      pool["scales"], pool["v"], pool["table"], pool["bits"], sm)
+    return out.cpu(), part.cpu(), want, want_part
+
+
+# tables of an odd number of floats in front of the pieces that are stored eight bytes at a time
+@pytest.mark.parametrize("page_size", [16, 32, 128])
+@pytest.mark.parametrize("dh,g,C,n_tiers,grp", [(48, 16, 5, 1, 1), (48, 16, 7, 3, 3), (80, 16, 3, 1, 5)])
+def test_pool_decode_odd_table_sizes(page_size, dh, g, C, n_tiers, grp):
+    pool = random_pool(dh + C, 2, dh, page_size, 7, g, C, n_tiers)
+    q = torch.randn(2 * grp, dh, generator=torch.Generator().manual_seed(1))
+    out, part, want, want_part = run_pool(pool, q, grp)
+    live = torch.isfinite(want_part[:, :, 0])
+    assert (out - want).abs().max().item() <= 2e-4
+    # fp32 sums of at most page_size terms in another order: a few ulps of the sum of magnitudes
+    assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
