@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         float l = 0.f;
         for (int t = lane; t < seg; t += 32) {
-          const float pt = __expf(lg[t] - m);
+          // a warp's share may be all -inf beside finite logits of the page's other warps: it weighs nothing
+          const float pt = wpp > 1 && lg[t] == -INFINITY ? 0.f : __expf(lg[t] - m);
           lg[t] = pt;
           l += pt;
         }

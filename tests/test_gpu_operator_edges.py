@@ -158,3 +158,21 @@ def test_pool_decode_odd_table_sizes(page_size, dh, g, C, n_tiers, grp):
     assert (out - want).abs().max().item() <= 2e-4
     # fp32 sums of at most page_size terms in another order: a few ulps of the sum of magnitudes
     assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
+
+
+# a warp's 16 tokens all at -inf, and single tokens at -inf, beside finite logits in the same page
+@pytest.mark.parametrize("page_size", [32, 128])
+def test_pool_decode_tokens_at_minus_infinity(page_size):
+    pool = random_pool(3, 2, 64, page_size, 5, 16, 2)
+    pool["cb"][..., 0, 0], pool["cb"][..., 1, 0] = -1000.0, 1e-36   # times 3e38 / 255: overflows, and about one
+    pool["scales"][:, 0], pool["scales"][:, 1:], pool["radius"][:] = 3e38, 0.0, 1
+    pool["theta"][:] = 1
+    pool["theta"][:, :16] = 0
+    pool["theta"][:, 20] = 0
+    q = torch.zeros(2, 64)
+    q[:, 0] = 1.0
+    out, part, want, want_part = run_pool(pool, q, 1)
+    live = torch.isfinite(want_part[:, :, 0])
+    assert torch.isfinite(want).all() and live.sum() == 8
+    assert (out - want).abs().max().item() <= 2e-4
+    assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
