@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
   for (int i = pg0 + tid; i < pg_end; i += blockDim.x)
     if (block_table[hkv * max_blocks + i] >= 0) atomicOr(&s_tiers, 1u << (bits_table[hkv * max_blocks + i] & 31));
   __syncthreads();
-  // q . centroid tables; same summation order as decode_kernel.cu:186-188.  A thread dots one centroid
-  // row with every query head, so the row is read once.
+  // q . centroid tables; same summation order as decode_kernel.cu:186-188.  Groups of 16 and 32: a thread dots one
+  // centroid row with every query head, so the row is read once.
   const unsigned tiers = s_tiers;
   const bool vec4 = (g_max & 3) == 0 && (dh & 3) == 0 && (reinterpret_cast<uintptr_t>(cb_flat) & 15) == 0;
   for (int ti = 0; ti < num_tiers; ++ti) {
@@ -100,10 +100,10 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
     const int G = tier_G_arr[ti], g = tier_g_arr[ti];
     const float* cb_t = cb_flat + ((int64_t)hkv * num_tiers + ti) * G_max * cb_max * g_max;
     float* lt = lut + (int64_t)ti * kv_groups * G_max * cb_max;
-    for (int i = tid; i < G * cb_max; i += blockDim.x) {
-      const int c = i % cb_max, gg = i / cb_max;
-      const float* cw = cb_t + ((int64_t)gg * cb_max + c) * g_max;
-      if (vec4 && (g == 16 || g == 32)) {
+    if (vec4 && (g == 16 || g == 32)) {
+      for (int i = tid; i < G * cb_max; i += blockDim.x) {
+        const int c = i % cb_max, gg = i / cb_max;
+        const float* cw = cb_t + ((int64_t)gg * cb_max + c) * g_max;
         float4 w4[8];
 #pragma unroll
         for (int e = 0; e < 4; ++e) w4[e] = __ldg(reinterpret_cast<const float4*>(cw) + e);
@@ -126,12 +126,26 @@ __global__ void __launch_bounds__(kPoolThreads) pool_page_kernel(
           }
           lt[(h * G_max + gg) * cb_max + c] = dot;
         }
-      } else {
-        for (int h = 0; h < kv_groups; ++h) {
-          float dot = 0.f;
-          for (int d = 0; d < g; ++d) dot += sq[h * dh + gg * g + d] * cw[d];
-          lt[(h * G_max + gg) * cb_max + c] = dot;
+      }
+    } else {  // other group sizes: a thread per (query head, centroid), 16-byte pieces where rows allow it
+      const bool pieces = vec4 && (g & 3) == 0;
+      for (int i = tid; i < kv_groups * G * cb_max; i += blockDim.x) {
+        const int c = i % cb_max, gg = (i / cb_max) % G, h = i / (cb_max * G);
+        const float* qg = sq + h * dh + gg * g;
+        const float* cw = cb_t + ((int64_t)gg * cb_max + c) * g_max;
+        float dot = 0.f;
+        if (pieces) {
+          for (int d = 0; d < g; d += 4) {
+            const float4 w = __ldg(reinterpret_cast<const float4*>(cw + d));
+            dot += qg[d] * w.x;
+            dot += qg[d + 1] * w.y;
+            dot += qg[d + 2] * w.z;
+            dot += qg[d + 3] * w.w;
+          }
+        } else {
+          for (int d = 0; d < g; ++d) dot += qg[d] * cw[d];
         }
+        lt[(h * G_max + gg) * cb_max + c] = dot;
       }
     }
   }

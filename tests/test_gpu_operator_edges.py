@@ -176,3 +176,14 @@ def test_pool_decode_tokens_at_minus_infinity(page_size):
     assert torch.isfinite(want).all() and live.sum() == 8
     assert (out - want).abs().max().item() <= 2e-4
     assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
+
+
+# group sizes beside the reference's 16 and 32: tables built in 16-byte pieces, and element by element
+@pytest.mark.parametrize("dh,g,C", [(128, 8, 64), (128, 64, 64), (120, 10, 16), (128, 4, 16)])
+def test_pool_decode_other_group_sizes(dh, g, C):
+    pool = random_pool(g, 2, dh, 32, 9, g, C, 2)
+    q = torch.randn(8, dh, generator=torch.Generator().manual_seed(1))
+    out, part, want, want_part = run_pool(pool, q, 4)
+    live = torch.isfinite(want_part[:, :, 0])
+    assert (out - want).abs().max().item() <= 2e-4
+    assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
