@@ -12,6 +12,8 @@
 // division, running-max radius scale with in-place re-quantisation); the work split is
 // new: one CTA serves all query heads of a KV head per page through a q.centroid look-up
 // table instead of staging a 64 KiB codebook per (query head, page).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sphkv {
@@ -635,6 +637,7 @@ extern "C" int sphkv_pool_decode(const float* q_all, const float* cb_flat, const
   const int at_once = kPoolWarps / wpp;
   int rounds = (int)(((int64_t)num_kv_heads * max_blocks) / ((int64_t)at_once * 2 * sphkv_sm_count_or(148)));
   rounds = rounds < 1 ? 1 : (rounds > kMaxPageRounds ? kMaxPageRounds : rounds);
+  rounds = std::max(rounds, (int)((max_blocks + (int64_t)at_once * 65535 - 1) / ((int64_t)at_once * 65535)));  // grid.y
   const int ppc = at_once * rounds;
   (void)launch_overlapped(pool_page_kernel, dim3(num_kv_heads, (max_blocks + ppc - 1) / ppc), dim3(kPoolThreads), smem, st,
       q_all, cb_flat, tier_G, tier_g, theta_codes, radius_codes, r_scales,

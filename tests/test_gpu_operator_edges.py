@@ -187,3 +187,18 @@ def test_pool_decode_other_group_sizes(dh, g, C):
     live = torch.isfinite(want_part[:, :, 0])
     assert (out - want).abs().max().item() <= 2e-4
     assert (part[live] - want_part[live]).abs().max().item() <= 1e-4 * want_part[live].abs().max().item()
+
+
+def test_pool_decode_of_more_pages_than_a_grid_has_rows():
+    """128-token pages, one page per CTA at a time: four rounds of them leave more CTAs than a grid's second dimension"""
+    mb = 4 * 65535 + 1000
+    pool = random_pool(7, 1, 16, 128, mb, 16, 4)
+    live = torch.tensor([0, 5, 4 * 65535 - 1, 4 * 65535, mb - 1])
+    table = torch.full((1, mb), -1, dtype=torch.int32)
+    table[0, live] = torch.arange(5, dtype=torch.int32)
+    pool["table"] = table
+    q = torch.randn(1, 16, generator=torch.Generator().manual_seed(1))
+    out, part, want, want_part = run_pool(pool, q, 1)
+    assert (out - want).abs().max().item() <= 2e-4
+    assert torch.equal(torch.isfinite(part[0, :, 0]), table[0] >= 0)
+    assert (part[0, live] - want_part[0, live]).abs().max().item() <= 1e-4 * want_part[0, live].abs().max().item()
