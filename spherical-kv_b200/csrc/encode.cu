@@ -970,10 +970,11 @@ static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaSt
     static SmemOptIn opt_in[2];
     const sphkv_encode_params& p = a.p;
     const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
+    const int cb_bytes = p.dh * p.tiers.C_max * 4, row_bytes = p.dh / GS * 128 * GS * 4;
+    // staged rows need aligned slices, and room beside a codebook tensor of any C_max (dh 128: up to 326)
     const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
-                        (p.k_head_stride * esize) % 16 == 0;
-    const int cb_bytes = p.dh * p.tiers.C_max * 4;
-    const int smem = cb_bytes + (staged ? p.dh / GS * 128 * GS * 4 : 0);
+                        (p.k_head_stride * esize) % 16 == 0 && cb_bytes + row_bytes <= 227 * 1024;
+    const int smem = cb_bytes + (staged ? row_bytes : 0);
     auto kern = staged ? search_bundles_kernel<GS, true> : search_bundles_kernel<GS, false>;
     if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem, "encode search")) return rc;
     const int resident = sm_count_current_device() * (GS == 16 ? 2 : 1);

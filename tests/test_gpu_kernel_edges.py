@@ -154,3 +154,18 @@ def test_importance_update_with_statistics_off_an_8_byte_boundary(page):
     for a, b in zip(*got):
         assert torch.equal(a, b)
     pkg.check_status(cache)
+
+
+def test_encode_with_a_wide_codebook_tensor():
+    """codebook tensors of any C_max that the encoder takes: rows are staged beside the codebook while they fit"""
+    Hkv, T, dh = 2, 700, 128
+    K = torch.randn(T, Hkv, dh, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV)
+    assign = synth.make_tier_assign(1, Hkv, T, {1: 0.5, 2: 0.3}, seed=1, per_head=True).to(DEV)
+    cbs = synth.make_codebooks(Hkv, dh, (T1, T2), seed=2)
+    got = []
+    for c_max in (64, 326, 327, 430):
+        tiers = pkg.TierSet(dh, (T1, T2))
+        tiers.C_max = c_max
+        got.append(pkg.encode_pages(K, K, pkg.build_page_lists(assign, tiers, 16), tiers.pack_codebooks(cbs).to(DEV), tiers))
+    for other in got[1:]:
+        assert torch.equal(other.k_pages, got[0].k_pages) and torch.equal(other.v_pool, got[0].v_pool)
