@@ -49,6 +49,7 @@ int ensure_dynamic_smem(SmemOptIn& st, const void* kernel, int bytes, const char
   if (st.bytes[dev] >= bytes) return 0;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();  // reported here; left behind, the next launch would report it as its own
     set_error("%s: cudaFuncSetAttribute(%d B of dynamic shared memory): %s", what, bytes, cudaGetErrorString(e));
     return (int)e;
   }

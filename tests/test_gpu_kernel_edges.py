@@ -169,3 +169,18 @@ def test_encode_with_a_wide_codebook_tensor():
         got.append(pkg.encode_pages(K, K, pkg.build_page_lists(assign, tiers, 16), tiers.pack_codebooks(cbs).to(DEV), tiers))
     for other in got[1:]:
         assert torch.equal(other.k_pages, got[0].k_pages) and torch.equal(other.v_pool, got[0].v_pool)
+
+
+def test_a_refused_size_does_not_fail_the_next_call():
+    Hkv, T, dh = 2, 300, 128
+    K = torch.randn(T, Hkv, dh, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV)
+    tiers, wide = pkg.TierSet(dh, (T1, T2)), pkg.TierSet(dh, (T1, T2))
+    wide.C_max = 460
+    cbs = synth.make_codebooks(Hkv, dh, (T1, T2), seed=2)
+    lists = pkg.build_page_lists(torch.ones(1, Hkv, T, dtype=torch.uint8, device=DEV), tiers, 16)
+    want = pkg.encode_pages(K, K, lists, tiers.pack_codebooks(cbs).to(DEV), tiers)
+    with pytest.raises(pkg.SphKVError, match="shared memory"):
+        pkg.encode_pages(K, K, lists, wide.pack_codebooks(cbs).to(DEV), wide)
+    pkg.kmeans_assign(K.view(-1, 16), K.view(-1, 16)[:8].contiguous())
+    got = pkg.encode_pages(K, K, lists, tiers.pack_codebooks(cbs).to(DEV), tiers)
+    assert torch.equal(got.k_pages, want.k_pages)
