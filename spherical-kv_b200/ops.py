@@ -173,39 +173,39 @@ def decode_scratch(cache: PagedCache, n_ctas: int = 0) -> torch.Tensor:
 
 def _decode_template(lib, cache: PagedCache, B: int, Hq: int, dh: int, n_ctas: int, dev) -> "_lib.DecodeParams":
     """A copy of the parameter struct with everything filled in that belongs to the cache.  The filled struct
-    stays with the cache while nothing it was made from changes (60 ctypes assignments: 10 us a call)."""
-    L, scratch, status = cache.lists, cache.scratch, cache.status
-    if scratch is not None and status is not None:
-        key = (cache.k_pages.data_ptr(), cache.v_pool.data_ptr(), cache.codebooks.data_ptr(), scratch.data_ptr(),
-               scratch.numel(), status.data_ptr(), L.ptable.data_ptr(), L.positions.data_ptr(), L.block_table.data_ptr(),
-               L.bits_table.data_ptr(), L.num_blocks.data_ptr(), L.B, L.Hkv, L.page_size, L.max_blocks, L.n_pages,
-               cache.v_pool.dtype, cache.radius_fmt, id(cache.tiers), B, Hq, dh, n_ctas)
+    stays with the cache, as bytes beside the values that it was made from, and serves again while all of those
+    are the same (60 ctypes assignments: 10 us a call)."""
+    L, tiers = cache.lists, cache.tiers.to_c()
+
+    def values():
+        return (cache.k_pages.data_ptr(), cache.v_pool.data_ptr(), cache.codebooks.data_ptr(), cache.scratch.data_ptr(),
+                cache.scratch.numel(), cache.status.data_ptr(), L.ptable.data_ptr(), L.positions.data_ptr(),
+                L.block_table.data_ptr(), L.bits_table.data_ptr(), L.num_blocks.data_ptr(), L.B, L.Hkv, L.page_size,
+                L.max_blocks, L.n_pages, cache.v_pool.dtype, cache.radius_fmt, bytes(tiers), cache.dh, B, Hq, dh, n_ctas)
+    if cache.scratch is not None and cache.status is not None:
         plan = cache.extra.get("decode_plan")
-        if plan is not None and plan[0] == key:
+        if plan is not None and plan[0] == values():
             return _lib.DecodeParams.from_buffer_copy(plan[1])
     assert B == L.B and dh == cache.dh
     need = lib.sphkv_decode_scratch_bytes(L.B, L.Hkv, dh, n_ctas)
-    if scratch is None or scratch.numel() < need:
-        cache.scratch = scratch = decode_scratch(cache, n_ctas)
-    if status is None:
-        cache.status = status = torch.zeros(1, dtype=torch.int32, device=dev)
+    if cache.scratch is None or cache.scratch.numel() < need:
+        cache.scratch = decode_scratch(cache, n_ctas)
+    if cache.status is None:
+        cache.status = torch.zeros(1, dtype=torch.int32, device=dev)
     p = _lib.DecodeParams()
     p.k_pages, p.ptable = cache.k_pages.data_ptr(), L.ptable.data_ptr()
     p.v_pool, p.positions = cache.v_pool.data_ptr(), L.positions.data_ptr()
     p.block_table, p.bits_table = L.block_table.data_ptr(), L.bits_table.data_ptr()
     p.num_blocks, p.codebooks = L.num_blocks.data_ptr(), cache.codebooks.data_ptr()
-    p.scratch, p.scratch_bytes = scratch.data_ptr(), scratch.numel()
-    p.status = status.data_ptr()
+    p.scratch, p.scratch_bytes = cache.scratch.data_ptr(), cache.scratch.numel()
+    p.status = cache.status.data_ptr()
     p.B, p.Hq, p.Hkv, p.dh = B, Hq, L.Hkv, dh
     p.page_size, p.max_blocks, p.n_pages = L.page_size, L.max_blocks, L.n_pages
     p.v_dtype, p.out_dtype = _DT[cache.v_pool.dtype], _lib.F32
     p.radius_fmt, p.n_ctas = cache.radius_fmt, n_ctas
-    p.tiers = cache.tiers.to_c()
-    key = (p.k_pages, p.v_pool, p.codebooks, p.scratch, p.scratch_bytes, p.status, p.ptable, p.positions, p.block_table,
-           p.bits_table, p.num_blocks, L.B, L.Hkv, L.page_size, L.max_blocks, L.n_pages, cache.v_pool.dtype,
-           cache.radius_fmt, id(cache.tiers), B, Hq, dh, n_ctas)
-    cache.extra["decode_plan"] = (key, p, cache.tiers)  # the tier set is held: its id stays its own
-    return _lib.DecodeParams.from_buffer_copy(p)
+    p.tiers = tiers
+    cache.extra["decode_plan"] = (values(), bytes(p))
+    return p
 
 
 def _tile_stats(cache: PagedCache, B: int, Hq: int, dev) -> torch.Tensor:

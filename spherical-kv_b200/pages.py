@@ -45,6 +45,16 @@ REFERENCE_TIERS = (TierSpec(1, 16, 6), TierSpec(2, 16, 4), TierSpec(3, 32, 3))
 class TierSet:
     """Active tiers in slot (rank) order, the order of make_tier_idx_map (sphkv_lut.py:7-14)."""
 
+    _c = None  # the C struct, made on first use; not part of the set's state
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name != "_c":
+            object.__setattr__(self, "_c", None)
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_c"}
+
     def __init__(self, dh: int, tiers: Sequence[TierSpec] = REFERENCE_TIERS[:2]):
         if not 1 <= len(tiers) <= _lib.MAX_TIER_SLOTS:
             raise ValueError(f"1..{_lib.MAX_TIER_SLOTS} tiers, got {len(tiers)}")
@@ -53,7 +63,6 @@ class TierSet:
         for t in self.tiers:
             if t.g not in (16, 32) or dh % (2 * t.g) or not 1 <= t.b_theta <= 6:
                 raise ValueError(f"unsupported tier {t} for dh={dh}")
-        self._c = None
         self.G_max = max(dh // t.g for t in self.tiers)
         self.C_max = max(t.codebook_size for t in self.tiers)
         self.g_max = max(t.g for t in self.tiers)
@@ -71,7 +80,7 @@ class TierSet:
         return self.dh // self.tiers[slot].g
 
     def to_c(self) -> "_lib.Tiers":
-        """The C struct (one object per set: a set does not change; callers copy or only read it)."""
+        """The C struct, kept until an attribute of the set is assigned; callers copy or only read it."""
         if self._c is not None:
             return self._c
         c = _lib.Tiers()
