@@ -208,16 +208,6 @@ def _decode_template(lib, cache: PagedCache, B: int, Hq: int, dh: int, n_ctas: i
     return p
 
 
-def _tile_stats(cache: PagedCache, B: int, Hq: int, dev) -> torch.Tensor:
-    """Workspace for the per-tile (max, sum) of a step that updates omega, kept with the cache."""
-    L = cache.lists
-    n = B * Hq * L.max_blocks * (L.page_size // 16) * 2
-    ws = cache.extra.get("tile_stats")
-    if ws is None or ws.numel() < n:
-        ws = cache.extra["tile_stats"] = torch.empty(n, dtype=torch.float32, device=dev)
-    return ws
-
-
 def decode_paged(q: torch.Tensor, cache: PagedCache, rope: Optional[torch.Tensor],
                  sm_scale: Optional[float] = None, out: Optional[torch.Tensor] = None,
                  out_dtype: Optional[torch.dtype] = None, out_partial: Optional[torch.Tensor] = None,
@@ -234,11 +224,11 @@ def decode_paged(q: torch.Tensor, cache: PagedCache, rope: Optional[torch.Tensor
     `omega` (f32 [B*Hkv, max_blocks]) is the page-importance EMA of
     spherical_kv_pipeline.py:952-987, updated in place inside the merge kernel from the
     per-tile statistics of this step; `page_ml` (f32 [B, Hq, max_blocks, page_size/16, 2]) is
-    kept with the cache when omega is given without it.
+    allocated when omega is given without it.
     `exchange` (split_kv.PeerExchange) turns the call into one rank's part of a split-KV decode:
     `cache` then holds this rank's share of every block list and the merge kernel trades the
     partial rows with the other ranks over peer memory before it writes `out`.
-    The split-K scratch, the status word and (with omega alone) the tile statistics live in `cache` (grown when a later call needs
+    The split-K scratch and the status word live in `cache` (grown when a later call needs
     more): one cache must not be decoded on two streams at once.  The status word is not read
     here (that would synchronise); `check_status(cache)` does it.
     """
@@ -248,7 +238,7 @@ def decode_paged(q: torch.Tensor, cache: PagedCache, rope: Optional[torch.Tensor
     if omega is not None:
         assert omega.dtype == torch.float32 and omega.is_contiguous() and omega.numel() == B * L.Hkv * L.max_blocks
         if page_ml is None:  # consumed inside the call
-            page_ml = _tile_stats(cache, B, Hq, q.device)
+            page_ml = torch.empty(B * Hq * L.max_blocks * (L.page_size // 16) * 2, dtype=torch.float32, device=q.device)
     _need_cuda(q, out, out_partial, page_ml, logits_out, rope, omega)
     p = _decode_template(lib, cache, B, Hq, dh, n_ctas, q.device)
     if out is None and want_out:

@@ -184,3 +184,16 @@ def test_a_refused_size_does_not_fail_the_next_call():
     pkg.kmeans_assign(K.view(-1, 16), K.view(-1, 16)[:8].contiguous())
     got = pkg.encode_pages(K, K, lists, tiers.pack_codebooks(cbs).to(DEV), tiers)
     assert torch.equal(got.k_pages, want.k_pages)
+
+
+def test_importance_update_keeps_no_workspace_that_copies_would_share():
+    """a cache and its dataclasses.replace() share their `extra`: nothing that a step writes may live there"""
+    import dataclasses
+    cache, cbs, K, V, Q, _ = build(1, 8, 2, 128, 400, 16, (T1, T2), {1: 0.4, 2: 0.4}, seed=5)
+    rope = pkg.rope_table(512, 128, device=DEV)
+    before = {k for k, v in cache.extra.items() if isinstance(v, torch.Tensor)}
+    pkg.decode_paged(Q.to(DEV), cache, rope, omega=torch.zeros(2, cache.lists.max_blocks, device=DEV))
+    other = dataclasses.replace(cache, scratch=None, status=None)
+    pkg.decode_paged(Q.to(DEV), other, rope, omega=torch.zeros(2, cache.lists.max_blocks, device=DEV))
+    assert other.extra is cache.extra and other.scratch.data_ptr() != cache.scratch.data_ptr()
+    assert {k for k, v in cache.extra.items() if isinstance(v, torch.Tensor)} == before
