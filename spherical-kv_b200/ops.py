@@ -51,7 +51,7 @@ def rope_table(max_pos: int, dh: int, base: float = 500000.0, device="cuda",
 def _new_cache(lists: PageLists, tiers: TierSet, codebooks: torch.Tensor, dh: int, has_v: bool, v_dtype: torch.dtype,
                radius_fmt: int, dev) -> PagedCache:
     """Pools for `lists`: zeroed, except a V pool of which the kernels write every slot (zeros included)."""
-    make = torch.empty if has_v and lists.covers_pool else torch.zeros
+    make = torch.empty if has_v and lists.encode_fills_pool() else torch.zeros
     return PagedCache(tiers=tiers, lists=lists, codebooks=codebooks,
                       k_pages=torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev),
                       v_pool=make(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev), radius_fmt=radius_fmt)

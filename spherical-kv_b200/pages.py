@@ -135,7 +135,21 @@ class PageLists:
     B: int
     Hkv: int
     max_blocks: int
-    covers_pool: bool = False    # every page is in `bundles`: an encode writes every V slot
+    covers_pool: Optional[tuple] = None  # what encode_fills_pool() compares; set by build_page_lists
+
+    def encode_fills_pool(self) -> bool:
+        """Whether every page is in `bundles`, so that an encode writes every V slot: they are the bundles that
+        build_page_lists made for these pages, and unchanged (assigned, sliced, moved or written to, they are not)."""
+        return isinstance(self.covers_pool, tuple) and self.covers_pool[0] is self.bundles and self._cover() == self.covers_pool[1:]
+
+    def _cover(self) -> Optional[tuple]:
+        # an inference tensor has no version counter: nothing can be promised about it
+        return None if self.bundles.is_inference() else (self.bundles._version, self.n_pages, self.page_size)
+
+    def _covered(self) -> "PageLists":
+        cover = self._cover()
+        self.covers_pool = None if cover is None else (self.bundles, *cover)
+        return self
 
 
 _NATIVE_IDS = (torch.uint8, torch.int32, torch.int64)
@@ -176,7 +190,7 @@ def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fm
     p.n_pages, p.max_blocks = P, max_blocks
     p.perm = None if perm is None else perm.data_ptr()
     _lib.check(lib.sphkv_page_lists_fill(C.byref(p), st), "sphkv_page_lists_fill")
-    return PageLists(N, P, *tables, pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks, covers_pool=True)
+    return PageLists(N, P, *tables, pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks)._covered()
 
 
 def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
@@ -298,7 +312,7 @@ def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
                      page_head=page_head, page_slot=page_slot, page_count=page_count,
                      ptable=ptable.contiguous(), block_table=block_table, bits_table=bits_table,
                      num_blocks=blocks_per_unit.to(torch.int32), bundles=torch.cat(bundle_rows, 0),
-                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks, covers_pool=True)
+                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks)._covered()
 
 
 @dataclass
