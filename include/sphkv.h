@@ -176,7 +176,10 @@ typedef struct sphkv_decode_params {
   const void* q;              /* [B][Hq][dh] q_dtype, post-RoPE at the query position */
   const uint8_t* k_pages;     /* byte pool, readable up to the next multiple of 4 bytes
                                  past the end of its last page                        */
-  const int32_t* ptable;      /* [P][3]                                               */
+  const int32_t* ptable;      /* [P][3]: sections may be padded where page_size > 16 or
+                                 radii are f16 (theta_off within 1023 bytes of the page,
+                                 16-token pages within 432 bytes in all); radii of every
+                                 token that the theta stream has room for are readable */
   const void* v_pool;         /* [P][page_size][dh] v_dtype (F16/BF16); slots past a
                                  page's count must hold finite values (zero-filled)   */
   const int32_t* positions;   /* [P][page_size] key positions, -1 = empty             */

@@ -29,8 +29,9 @@ static_assert(kTeams * kTeamCols <= kTmemCols, "tensor memory");
 struct TileMeta {
   int phys;        // physical page id; -1 hole / invalid page, -2 no such tile
   uint32_t where;  // tokens of the tile, at most | tier slot << 8 | stage byte offsets: header << 12, theta << 16
-                   // (bytes; 9 bits); sub tile of the page << 28
-  uint32_t rad;    // stage byte offset of the tile's first radius byte | (theta - page) << 9 | (radii - theta) << 16
+                   // (bytes; 9 bits); (theta - page) >> 7 << 25; sub tile of the page << 28
+  uint32_t rad;    // stage byte offset of the tile's first radius byte | (theta - page) & 127 << 9 |
+                   // (radii - theta) << 16
   int poff;        // page offset in the byte pool
 };
 __device__ __forceinline__ int meta_tokens(const TileMeta& m) { return m.where & 0xFF; }
@@ -468,17 +469,23 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           th = kKTh + (((uint32_t)mf_toff + ((16u * sub * G * bits) >> 3)) & 15u);
           rd = kKRd + (((uint32_t)mf_roff + 16u * sub * G * rb) & 15u);
         }
-        if (mf_toff - mf_poff != (int)(8 + 4 * G) || th_bytes < 0 || th_bytes > N * 6) {
+        // Sections may be padded: 16-token pages are staged whole and have to fit, of larger ones each section is
+        // found by itself.  With int8 radii 16-token pages start their theta stream right behind the scales.
+        const int lead = mf_toff - mf_poff;
+        const bool fits = TPP == 1 ? rd + 16 * G * rb <= kst_pos && rd < 512 : lead < 1024 && th_bytes < 65536;
+        if ((FAST ? lead != (int)(8 + 4 * G) : lead < (int)(8 + 4 * G)) || th_bytes < 0 || !fits) {
           // the pointer table disagrees with the page format: not a page this kernel can read
           if (p.status) atomicOr(p.status, SPHKV_ST_BAD_BLOCK);
           m.phys = -1;
         } else {
           int count = min(N, (int)((uint32_t)th_bytes * 8u / (G * bits)));
-          if (G * bits < 8)  // several counts share a stream size: the header it is
+          if (G * bits < 8 || (int)(((uint32_t)count * G * bits + 7) >> 3) != th_bytes)
+            // several counts share a stream size, or the stream is padded: the header it is
             count = min(count, (int)p.k_pages[mf_poff + 1]);
           const int tokens = min(16, max(0, count - 16 * sub));
           m.where = (uint32_t)tokens | ((uint32_t)mf_slot << 8) | (phase << 12) | (th << 16) | ((uint32_t)sub << 28);
-          m.rad = rd | ((uint32_t)(mf_toff - mf_poff) << 9) | ((uint32_t)th_bytes << 16);
+          m.rad = rd | ((uint32_t)(lead & 0x7F) << 9) | ((uint32_t)th_bytes << 16);
+          if (!FAST) m.where |= (uint32_t)(lead >> 7) << 25;  // read for pages of more than one tile only
         }
       }
       sts_meta(meta + ((kb * kMacroTiles + lane) & (kMetaRing - 1)) * 16, m);
@@ -537,7 +544,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           piece(kb, poff, poff - meta_hdr(m) + meta_radius(m) + (uint32_t)meta_tokens(m) * G * rb);
         } else {
           const uint32_t t0 = 16u * sub, t1 = t0 + (uint32_t)meta_tokens(m);
-          const uint32_t toff = poff + ((m.rad >> 9) & 0x7F), roff = toff + (m.rad >> 16);
+          const uint32_t toff = poff + (((m.rad >> 9) & 0x7F) | (((m.where >> 25) & 0x7) << 7)), roff = toff + (m.rad >> 16);
           piece(kb + kKHdr, poff, poff + 8 + 4 * G);
           piece(kb + kKTh, toff + ((t0 * G * bits) >> 3), toff + ((t1 * G * bits + 7) >> 3));
           piece(kb + kKRd, roff + t0 * G * rb, roff + t1 * G * rb);

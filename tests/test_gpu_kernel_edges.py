@@ -197,3 +197,36 @@ def test_importance_update_keeps_no_workspace_that_copies_would_share():
     pkg.decode_paged(Q.to(DEV), other, rope, omega=torch.zeros(2, cache.lists.max_blocks, device=DEV))
     assert other.extra is cache.extra and other.scratch.data_ptr() != cache.scratch.data_ptr()
     assert {k for k, v in cache.extra.items() if isinstance(v, torch.Tensor)} == before
+
+
+def padded_pages(cache, lead, pad):
+    """The same pages with `lead` bytes from a page to its theta stream (0: as it is) and the stream padded to `pad`."""
+    L, tiers, rb = cache.lists, cache.tiers, 2 if cache.radius_fmt == 1 else 1
+    old, pt = cache.k_pages.cpu(), L.ptable.cpu().tolist()
+    slots, counts = L.page_slot.cpu().tolist(), L.page_count.cpu().tolist()
+    pieces, table, at = [], [], 0
+    for (po, to, ro), s, n in zip(pt, slots, counts):
+        G = tiers.G(s)
+        to2 = at + (lead or to - po)
+        ro2 = to2 + -(-(ro - to) // pad) * pad
+        end = ro2 + n * G * rb
+        page = torch.full((-(-(end - at) // 16) * 16,), 0xEE, dtype=torch.uint8)
+        page[:8 + 4 * G] = old[po:po + 8 + 4 * G]
+        page[to2 - at:to2 - at + ro - to] = old[to:ro]
+        page[ro2 - at:end - at] = old[ro:ro + n * G * rb]
+        pieces.append(page)
+        table.append((at, to2, ro2))
+        at += page.numel()
+    cache.k_pages = torch.cat(pieces + [torch.zeros(16, dtype=torch.uint8)]).to(DEV)
+    L.ptable = torch.tensor(table, dtype=torch.int32, device=DEV)
+
+
+# page, radius format, lead, padding: pointer tables whose sections do not lie back to back
+@pytest.mark.parametrize("page,fmt,lead,pad", [(64, 0, 64, 16), (32, 0, 44, 1), (128, 1, 1020, 256), (16, 1, 64, 16), (16, 0, 0, 16)])
+def test_decode_of_padded_sections(page, fmt, lead, pad):
+    cache, cbs, K, V, Q, _ = build(2, 8, 2, 128, 500, page, (T1, T2, T3), {1: 0.3, 2: 0.3, 3: 0.2}, radius_fmt=fmt, seed=5)
+    rope = pkg.rope_table(512, 128, device=DEV)
+    want = pkg.decode_paged(Q.to(DEV), cache, rope).clone()
+    padded_pages(cache, lead, pad)
+    assert torch.equal(pkg.decode_paged(Q.to(DEV), cache, rope), want)
+    pkg.check_status(cache)
