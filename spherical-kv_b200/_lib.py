@@ -10,7 +10,6 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsphkv_b200.so")
-HOST_PATH = os.path.join(HERE, "host_tables.so")
 
 F32, BF16, F16 = 0, 1, 2
 RADIUS_I8, RADIUS_F16 = 0, 1
@@ -146,14 +145,24 @@ def load() -> C.CDLL:
     return lib
 
 
+def host_path() -> str:
+    """The host module's file.  It is compiled against torch and Python themselves, so its name says which: another
+    version of either finds no file and asks for a build instead of loading one that does not fit."""
+    import sys
+
+    import torch
+    return os.path.join(HERE, "host_tables.%s.torch-%s.so" % (sys.implementation.cache_tag, torch.__version__))
+
+
 def host_tables():
     """The module of csrc/host_tables.cpp; raises if it is missing (no fallback exists)."""
     global _host
     if _host is None:
         import importlib.util
-        if not os.path.exists(HOST_PATH):
-            raise SphKVError(f"{HOST_PATH} is missing: build it with `python -c \"import __graft_entry__ as g; g.build()\"`")
-        spec = importlib.util.spec_from_file_location("host_tables", HOST_PATH)
+        path = host_path()
+        if not os.path.exists(path):
+            raise SphKVError(f"{path} is missing: build it with `python -c \"import __graft_entry__ as g; g.build()\"`")
+        spec = importlib.util.spec_from_file_location("host_tables", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         _host = module

@@ -1,4 +1,4 @@
-"""Builds libsphkv_b200.so (sm_100a) with nvcc and the host module host_tables.so with g++, in-tree.  No GPU is
+"""Builds libsphkv_b200.so (sm_100a) with nvcc and the host module host_tables.*.so with g++, in-tree.  No GPU is
 needed to build."""
 from __future__ import annotations
 
@@ -11,7 +11,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libsphkv_b200.so")
-HOST_PATH = os.path.join(HERE, "host_tables.so")
 SOURCES = ["capi.cu", "decode.cu", "encode.cu", "lists.cu", "compat.cu", "pool.cu", "kmeans.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -33,18 +32,27 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_path() -> str:
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("sphkv_lib_paths", os.path.join(HERE, "_lib.py"))
+    lib = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(lib)
+    return lib.host_path()
+
+
 def _host_module(force: bool) -> "subprocess.Popen | None":
     """Starts the compilation of csrc/host_tables.cpp against the installed torch and Python."""
     import sysconfig
 
     import torch
     src = os.path.join(CSRC, "host_tables.cpp")
-    if not (force or _stale(HOST_PATH, [src])):
+    target = _host_path()
+    if not (force or _stale(target, [src, os.path.abspath(__file__)])):
         return None
     root = os.path.dirname(torch.__file__)
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           "-isystem", sysconfig.get_paths()["include"], src, "-o", HOST_PATH,
+           "-isystem", sysconfig.get_paths()["include"], src, "-o", target,
            "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
     return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)
 

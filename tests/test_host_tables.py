@@ -21,3 +21,14 @@ def test_tables_lie_side_by_side_on_256_byte_boundaries(P, N, U, mb, nb):
     for i, t in enumerate(tables):
         t.fill_(i)
     assert all(bool((t == i).all()) for i, t in enumerate(tables))
+
+
+def test_the_module_is_named_after_what_it_was_built_against(monkeypatch):
+    import sys
+    path = pkg._lib.host_path()
+    assert sys.implementation.cache_tag in path and torch.__version__ in path
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    monkeypatch.setattr(pkg._lib, "_host", None)
+    assert pkg._lib.host_path() != path
+    with pytest.raises(pkg.SphKVError, match="is missing"):
+        pkg._lib.host_tables()
