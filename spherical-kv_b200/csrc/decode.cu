@@ -89,7 +89,7 @@ __global__ void plan_kernel(const int32_t* __restrict__ num_blocks, int n_units,
 // units, dh 64: 5.3 -> 3.7 us; with the importance update of three rows at 128-token pages 12.3 -> 4.9 us.
 template <int DH>
 __global__ void __launch_bounds__(8 * DH) merge_rows_kernel(const DecodeArgs a) {
-  constexpr int kChunk = 32;   // partial rows combined per pass (general path); shared memory is kept small: see kSmemMax
+  constexpr int kChunk = 32;   // partial rows combined per pass (general path)
   constexpr int kBatch = 16;   // rows' loads in flight at a time
   const sphkv_decode_params& p = a.p;
   const int u = blockIdx.x;  // traversal index: hkv * B + b
@@ -557,9 +557,9 @@ extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
   a.wide = ((reinterpret_cast<uintptr_t>(p.k_pages) | reinterpret_cast<uintptr_t>(p.positions)) & 15) == 0;
   a.plan_in_kernel = a.n_units <= kMaxUnitsInKernelPlan ? 1 : 0;
   const int pfx_bytes = a.plan_in_kernel ? (a.n_units + 1) * 4 : 0;
-  // a little less than an SM has, so that this kernel's blocks become resident beside the merge blocks of the
-  // step before (which keep 2 KB) and set themselves up while those finish
-  constexpr int kSmemMax = 230272;  // 228 KB less 1 KB per block and the merge kernel's 1.1
+  // all that a block can have: this kernel's 512 threads launch with every register of an SM, so its blocks never
+  // share one with the merge blocks of the step before, and overlap with them on the SMs that have none
+  constexpr int kSmemMax = 227 * 1024;
   int smem_bytes = 0;
   for (a.teams = kTeams; a.teams >= 1; --a.teams) {
     const int fixed_bytes = smem_fixed_bytes(p.dh, a.teams) + pfx_bytes;
