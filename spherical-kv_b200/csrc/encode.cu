@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
 // source rows of the next are already loaded and its key rows are on their way to L2.
 // STAGED: a warp's slices of the next bundle's rows travel to shared memory by 16-byte asynchronous copies, the
 // lanes of a row slice side by side, while the current bundle is searched; as one row per lane, every 128-bit
-// load fetched 32 sectors and used half of each (GS 16: 106 -> 90 us for a 32768-token prompt).  Chunk c
+// load fetched 32 sectors and used half of each (GS 16: 106 -> 86 us for a 32768-token prompt).  Chunk c
 // of row s is stored at chunk c ^ turn(s), so neither the copies nor the row-per-lane reads meet in a bank.
 // Not STAGED: slices off a 16-byte boundary.
 template <int GS, bool STAGED>

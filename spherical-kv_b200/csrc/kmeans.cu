@@ -6,10 +6,10 @@
 //
 // One thread holds kPts points in registers and walks the centroids out of shared memory
 // (one broadcast 16-byte load feeds 16 or 8 FMAs).  The accumulation uses no float atomics and no
-// barrier: every warp keeps sums of its own in shared memory, 32 / D sets of [K][D] (`ways`; one when they would
-// not fit), and walks its points D lanes to a row -- lane = dimension, one add per row and lane, the rows
-// turned through a 32-row tile of shared memory -- so lanes never meet in an address.  Warps and CTAs are
-// folded at the end.  Sums agree to rounding, as with index_add_ on a GPU; assignments and counts are
+// barrier until the end: every warp keeps sums of its own in shared memory, 32 / D sets of [K][D] (`ways`; fewer
+// when they would not fit), and walks its points D lanes to a row -- lane = dimension, one add per row and lane, the rows
+// turned through a 32-row tile of shared memory -- so lanes never meet in an address.  At the end the
+// warps' sets are added up and every CTA adds its sums to the output with float atomics, in no fixed order.  Sums agree to rounding, as with index_add_ on a GPU; assignments and counts are
 // exact.  Bound: fp32 FMA issue for K = 64, then the shared-memory adds.  4M points, d 16, K 64: 324 -> 254 us;
 // K 16, 2.3M points: 95 -> 76 us (a counting sort per 1024 points with six barriers before).
 #include <algorithm>

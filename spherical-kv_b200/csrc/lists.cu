@@ -52,7 +52,8 @@ __device__ __forceinline__ int64_t page_bytes(const ListArgs& a, int s, int coun
   return (b + a.align - 1) / (uint32_t)a.align * a.align;
 }
 
-// tier ids of this thread's kListPer tokens (consecutive; -1 past the end: ids are compared as int64)
+// tier ids of this thread's kListPer tokens (consecutive; INT64_MIN past the end: ids are
+// compared as int64, and no slot's 32-bit id equals it)
 __device__ __forceinline__ void load_tiers(const ListArgs& a, int u, int64_t t0, int64_t (&v)[kListPer]) {
   const int64_t base = (int64_t)u * a.T + t0;
   const char* p = reinterpret_cast<const char*>(a.assign) + base * a.elem_size;

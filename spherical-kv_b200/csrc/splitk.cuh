@@ -220,7 +220,8 @@ static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 2
 // keys in flight and nothing else, twelve team warps fit an SM (the mma.sync version it replaced: eight, at
 // 244 registers, and shuffles, ldmatrix and accumulator moves around both products).
 // Bound: instruction issue and the waits between the roles, not HBM.  A 96-bit, 32768-token, batch-8 layer
-// step: 221.6 -> 157 us, merge included (2.5 -> 3.5 TB/s of the bytes it has to read).
+// step, merge included: 223 -> 178 us in a long loop under the power cap, 153 us in a burst (2.4 -> 3.0 and
+// 3.5 TB/s of the bytes it has to read).
 // Lane map of the rebuild (lane = 4 r + j): rows r and r + 8 of a tile are the lane's two tokens; in each
 // rotary half the lane owns the contiguous block of W = dh / 8 dimensions  W j .. W j + W - 1, and in the
 // other half the same block shifted by dh / 2: the RoPE partner of every value a lane holds is in the same
