@@ -140,16 +140,14 @@ class PageLists:
     def encode_fills_pool(self) -> bool:
         """Whether every page is in `bundles`, so that an encode writes every V slot: they are the bundles that
         build_page_lists made for these pages, and unchanged (assigned, sliced, moved or written to, they are not)."""
-        return isinstance(self.covers_pool, tuple) and self.covers_pool[0] is self.bundles and self._cover() == self.covers_pool[1:]
+        c, b = self.covers_pool, self.bundles
+        return (isinstance(c, tuple) and c[0] is b and c[1] == b._version and c[2] == self.n_pages
+                and c[3] == self.page_size)
 
-    def _cover(self) -> Optional[tuple]:
-        # an inference tensor has no version counter: nothing can be promised about it
-        return None if self.bundles.is_inference() else (self.bundles._version, self.n_pages, self.page_size)
 
-    def _covered(self) -> "PageLists":
-        cover = self._cover()
-        self.covers_pool = None if cover is None else (self.bundles, *cover)
-        return self
+def _cover(bundles: torch.Tensor, n_pages: int, page_size: int) -> Optional[tuple]:
+    # an inference tensor has no version counter: nothing can be promised about it
+    return None if bundles.is_inference() else (bundles, bundles._version, n_pages, page_size)
 
 
 _NATIVE_IDS = (torch.uint8, torch.int32, torch.int64)
@@ -190,7 +188,7 @@ def _build_on_device(ta: torch.Tensor, tiers: TierSet, page_size: int, radius_fm
     p.n_pages, p.max_blocks = P, max_blocks
     p.perm = None if perm is None else perm.data_ptr()
     _lib.check(lib.sphkv_page_lists_fill(C.byref(p), st), "sphkv_page_lists_fill")
-    return PageLists(N, P, *tables, pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks)._covered()
+    return PageLists(N, P, *tables, pool_bytes, B, Hkv, max_blocks, _cover(tables[9], P, N))
 
 
 def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
@@ -308,11 +306,13 @@ def build_page_lists(tier_assign: torch.Tensor, tiers: TierSet, page_size: int,
     radius_off = theta_off + (page_count.long() * Gs * bts + 7) // 8
     ptable = torch.stack([page_off, theta_off, radius_off], 1).to(torch.int32)
 
+    bundles = torch.cat(bundle_rows, 0)
     return PageLists(page_size=N, n_pages=P, positions=positions, src_index=src_index,
                      page_head=page_head, page_slot=page_slot, page_count=page_count,
                      ptable=ptable.contiguous(), block_table=block_table, bits_table=bits_table,
-                     num_blocks=blocks_per_unit.to(torch.int32), bundles=torch.cat(bundle_rows, 0),
-                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks)._covered()
+                     num_blocks=blocks_per_unit.to(torch.int32), bundles=bundles,
+                     pool_bytes=pool_bytes, B=B, Hkv=Hkv, max_blocks=max_blocks,
+                     covers_pool=_cover(bundles, P, N))
 
 
 @dataclass
