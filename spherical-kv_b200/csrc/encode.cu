@@ -17,7 +17,8 @@
 // The similarity is taken on the un-normalised group vector: dividing by r first
 // (spherical_kv_pipeline.py:1138) scales every sim_c by the same positive factor.
 #include <algorithm>
-#include "common.cuh"
+
+#include "search.cuh"
 
 namespace sphkv {
 
@@ -730,12 +731,9 @@ __global__ void __launch_bounds__(kEncThreads) assemble_pages_kernel(const Encod
 // ---- all-tier code cache ---------------------------------------------------------------------
 // Radius and nearest centroid of every (token, KV head, group) for EVERY tier slot in one pass
 // over the keys (the pre-encode of spherical_kv_pipeline.py:1535-1553, which calls
-// _encode_keys_with_codebooks once per tier).  A thread holds four tokens' 32-dim slice; the two
-// 16-dim halves serve the g = 16 tiers, the whole slice the g = 32 tiers, and the squared norm
-// of the 32-dim group continues the fma chain of its first half, so every value equals what
-// the per-tier encoder computes (same fixed order).  Output per slot s, head-major like the
+// _encode_keys_with_codebooks once per tier).  Output per slot s, head-major like the
 // reference's per-(layer, head) cache: r[s][head][row][G_s] f32, theta[s][head][row][G_s] u8.
-struct CodesArgs {
+struct ChainArgs {
   const void* k_src;
   const float* codebooks;
   float* r_out[SPHKV_MAX_TIER_SLOTS];
@@ -780,8 +778,11 @@ __device__ __forceinline__ void search_slice(const float (&k)[kCodeTok][32], con
 #ifndef SPHKV_CODE_WARPS
 #define SPHKV_CODE_WARPS 8
 #endif
-constexpr int kCodeThreads = SPHKV_CODE_WARPS * 32;  // a multiple of four warps: dh / 32 warps share a token set
+constexpr int kChainThreads = SPHKV_CODE_WARPS * 32;  // a multiple of four warps: dh / 32 warps share a token set
 
+// Few centroids (see the rule at the launch): the chains on the fp32 pipe.  A thread holds four tokens' 32-dim slice; the two
+// 16-dim halves serve the g = 16 tiers, the whole slice the g = 32 tiers, and the squared norm of the 32-dim group
+// continues the fma chain of its first half, so every value equals what the per-tier encoder computes.
 // Persistent: the (head, row block) units are dealt out in contiguous runs, one run per resident
 // CTA.  A CTA stages a head's codebooks when its run enters that head (once or twice per CTA) and
 // has no other barrier, so the warps of an SM drift apart and one warp's key loads hide under the
@@ -794,13 +795,13 @@ constexpr int kCodeThreads = SPHKV_CODE_WARPS * 32;  // a multiple of four warps
 // kCodeTok tokens per thread: four feed 16 fmas from every centroid load (232 registers); with two or one a small
 // input reaches more SMs and waits for a shorter pass (419 tokens x 8 heads: 27 -> 14 us; 2048: 27 -> 19).
 template <bool STAGED, int kCodeTok>
-__global__ void __launch_bounds__(kCodeThreads, 1) encode_codes_kernel(const CodesArgs a) {
+__global__ void __launch_bounds__(kChainThreads, 1) codes_chains_kernel(const ChainArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   float* cb_s = reinterpret_cast<float*>(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G32 = a.dh >> 5;                  // 32-dim groups per head: 2 or 4
   const int grp = warp % G32, set = warp / G32;
-  const int sets = (kCodeThreads / 32) / G32;  // token sets of 32 * kCodeTok per CTA
+  const int sets = (kChainThreads / 32) / G32;  // token sets of 32 * kCodeTok per CTA
   constexpr int kBlockRows = 32 * kCodeTok;
   const int esize = a.k_dtype == SPHKV_F32 ? 4 : 2;
   const int64_t u_lo = a.n_units * blockIdx.x / gridDim.x, u_hi = a.n_units * (blockIdx.x + 1) / gridDim.x;
@@ -957,6 +958,393 @@ __global__ void __launch_bounds__(kCodeThreads, 1) encode_codes_kernel(const Cod
   }
 }
 
+// ---- the same on the tensor cores ----
+struct CodesArgs {
+  const void* k_src;
+  const float* codebooks;
+  float* r_out[SPHKV_MAX_TIER_SLOTS];
+  uint8_t* th_out[SPHKV_MAX_TIER_SLOTS];
+  int64_t k_row_stride, k_head_stride, rows;
+  int64_t n_units, units_per_head;  // unit = 128 rows of one head
+  int k_dtype, dh;
+  int kbuf_off;  // byte offset of the staged rows
+  int wide;      // outputs start on 16 (r) and 4 bytes (theta)
+  sphkv_tiers tiers;
+  SearchPlan plan;
+};
+
+// Row slices of 32 dims wait in shared memory, 128 (fp32) or 64 bytes a row, a 4 KB block per warp and stage; chunk c of
+// row r is stored at chunk c ^ (r & 7), or c ^ (r >> 1 & 3): neither the copies (the lanes of a row side by side) nor
+// the row-per-lane reads meet in a bank.
+constexpr int kSliceBlock = 4096;
+__device__ __forceinline__ int staged_chunk(bool k32, int r, int c) { return k32 ? c ^ (r & 7) : c ^ ((r >> 1) & 3); }
+__device__ __forceinline__ void read_staged_row(uint32_t block, int dtype, float (&k)[32]) {
+  const int lane = threadIdx.x & 31;
+  if (dtype == SPHKV_F32) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float4 v = lds_f4(block + lane * 128 + (staged_chunk(true, lane, c) << 4));
+      k[4 * c] = v.x; k[4 * c + 1] = v.y; k[4 * c + 2] = v.z; k[4 * c + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4 v = lds_f4(block + lane * 64 + (staged_chunk(false, lane, c) << 4));
+      const uint32_t x[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) unpack16(x[e], dtype, k[8 * c + 2 * e], k[8 * c + 2 * e + 1]);
+    }
+  }
+}
+__device__ __forceinline__ void group_barrier(int group) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kSearchWarps * 32) : "memory");
+}
+// `count` (1, 2 or 4) neighbouring radii and codes (a byte each); 16- and 4-byte stores where `wide`
+__device__ __forceinline__ void store_groups(float* r, uint8_t* theta, int count, bool wide, float4 v, uint32_t codes) {
+  if (count == 4 && wide) {
+    *reinterpret_cast<float4*>(r) = v;
+    *reinterpret_cast<uint32_t*>(theta) = codes;
+  } else if (count >= 2) {
+    *reinterpret_cast<float2*>(r) = make_float2(v.x, v.y);
+    *reinterpret_cast<uint16_t*>(theta) = (uint16_t)codes;
+    if (count == 4) {
+      *reinterpret_cast<float2*>(r + 2) = make_float2(v.z, v.w);
+      *reinterpret_cast<uint16_t*>(theta + 2) = (uint16_t)(codes >> 16);
+    }
+  } else {
+    *r = v.x;
+    *theta = (uint8_t)codes;
+  }
+}
+
+// the fma chains' answer for the lanes in `open`: group `gamma` of key row `row`
+template <int GS>
+__device__ __noinline__ int settle(const CodesArgs& p, int head, int s, int gamma, int64_t row, unsigned open, int code) {
+  const sphkv_tiers& t = p.tiers;
+  const float* cb = p.codebooks + (((int64_t)(head * t.n_slots + s) * t.G_max + gamma) * t.C_max) * t.g_max;
+  return exact_search<GS>([&](int64_t off, float (&k)[GS]) { load_group<GS>(p.k_src, p.k_dtype, off, k); },
+                          row * p.k_row_stride + (int64_t)head * p.k_head_stride + gamma * GS, cb, t.g_max, 1 << t.bits[s], open, code);
+}
+
+constexpr int kCodeStages = 4;                                  // slices in flight
+
+constexpr int kCodeTail = 256;  // norms, barriers, tensor memory base
+
+// A set of tiers that the kernel below is compiled for: centroid bits of two 16-dim slots and one 32-dim slot (0: none),
+// in that order.  Its sums are a slice's columns [16-dim slots | the same, second half | 32-dim slot], all loaded at once.
+template <int B0, int B1, int B2>
+struct FixedTiers {
+  static constexpr bool kFixed = B0 > 0;
+  static constexpr int kSlots = (B0 > 0) + (B1 > 0) + (B2 > 0);
+  static constexpr int C0 = B0 ? 1 << B0 : 0, C1 = B1 ? 1 << B1 : 0, C2 = B2 ? 1 << B2 : 0;
+  static constexpr int kHalf = (C0 + C1 + 15) / 16 * 16;  // columns of a half
+  static bool match(const sphkv_tiers& t, unsigned wanted) {
+    if (!kFixed || t.n_slots != kSlots || wanted != (1u << kSlots) - 1) return false;
+    const int bits[3] = {B0, B1, B2}, g[3] = {16, 16, 32};
+    for (int s = 0; s < kSlots; ++s)
+      if (t.bits[s] != bits[s] || t.g[s] != g[s]) return false;
+    return true;
+  }
+};
+using AnyTiers = FixedTiers<0, 0, 0>;
+
+// Persistent: the (head, 128-row block) units are dealt out in contiguous runs, one run per CTA; a CTA lays a head's
+// centroids out for the tensor cores when its run enters that head.  Its two search groups share every unit: each takes
+// half of the 32-dim slices, so the groups never wait for one another between heads and small inputs spread over
+// more SMs.  Thread = row = lane of tensor memory; slice by slice: the sums into registers, so that the tensor cores can
+// multiply the next slice at once; their searches; the slice after that from shared memory, its norms' fma chains, its
+// bf16 pairs to tensor memory.  STAGED: rows travel global -> shared memory by 16-byte asynchronous copies four slices
+// ahead.  Not STAGED (slices off a 16-byte boundary, or no room beside the centroids): each lane loads its own row.
+// AnyTiers: slots of any number and size, in passes of what fits, branch by branch; the instructions around the searches are
+// then as many as those of the searches.
+template <bool STAGED, typename Fix>
+__global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const __grid_constant__ CodesArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int group = warp / kSearchWarps, w = warp % kSearchWarps;
+  float* most = reinterpret_cast<float*>(smem + a.plan.bytes);
+  const uint32_t bars = smem_u32(smem + a.plan.bytes + 128), bar = bars + 8 * group;
+  volatile uint32_t* tmem_word = reinterpret_cast<volatile uint32_t*>(smem + a.plan.bytes + 128 + 8 * kSearchGroups);
+  if (warp == 0) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_word)), kSearchGroups * kGroupCols);
+  if (threadIdx.x < kSearchGroups) mbar_init(bars + 8 * threadIdx.x, 1);
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_word[0], 0);
+  const uint32_t tmem = tmem_base + group * kGroupCols, my_rows = tmem + ((uint32_t)(32 * w) << 16);
+
+  const int64_t u_lo = a.n_units * blockIdx.x / gridDim.x, u_hi = a.n_units * (blockIdx.x + 1) / gridDim.x;
+  const int per = a.dh / 32 / kSearchGroups;   // slices of this group: 1 or 2
+  const int slice0 = group * per;
+  const int n_q = (int)(u_hi - u_lo) * per;    // (unit, slice) pairs this group walks
+  const bool k32 = a.k_dtype == SPHKV_F32, lows = a.k_dtype != SPHKV_BF16;
+  const int esz = k32 ? 4 : 2, ch_shift = k32 ? 3 : 2;  // 16-byte chunks of a row slice: 8 or 4
+  // Where a (unit, slice) pair lies.  Three of these walk the pairs: rows are fetched kCodeStages pairs ahead of the split,
+  // which is two pairs ahead of the search (dividing for each cost a third of the kernel's instructions).
+  struct Place {
+    int q, slice, head;
+    int64_t row0;  // first row of the warp's 32
+  };
+  Place at0;
+  at0.q = 0;
+  at0.slice = slice0;
+  at0.head = (int)(u_lo / a.units_per_head);
+  at0.row0 = (u_lo - at0.head * a.units_per_head) * 128 + 32 * w;
+  const int64_t head_rows = a.units_per_head * 128;
+  auto advance = [&](Place& p) {
+    ++p.q;
+    if (++p.slice < slice0 + per) return;
+    p.slice = slice0;
+    p.row0 += 128;
+    if (p.row0 >= head_rows) {
+      p.row0 -= head_rows;
+      ++p.head;
+    }
+  };
+  const uint32_t kbuf = smem_u32(smem + a.kbuf_off) + warp * (kCodeStages * kSliceBlock);
+  Place fetch = at0;
+  const int r_l = lane >> ch_shift, c_l = lane & ((1 << ch_shift) - 1);  // this lane's first row of a block, its chunk
+  const int64_t row_bytes = a.k_row_stride * esz, src_step = row_bytes * (32 >> ch_shift);
+  auto fetch_base = [&]() {
+    return reinterpret_cast<const char*>(a.k_src) + (fetch.row0 + r_l) * row_bytes + ((int64_t)fetch.head * a.k_head_stride + fetch.slice * 32) * esz +
+           c_l * 16;
+  };
+  const char* fetch_src = fetch_base();
+  // (four 128-byte rows a step flip bit 2 of the chunk on odd steps, eight 64-byte rows do not)
+  const uint32_t to_even = ((r_l << ch_shift) + staged_chunk(k32, r_l, c_l)) * 16, to_odd = k32 ? to_even ^ 64 : to_even;
+  auto issue_rows = [&]() {
+    if (fetch.q < n_q) {
+      const uint32_t dst = kbuf + (fetch.q & (kCodeStages - 1)) * kSliceBlock;
+      const char* src = fetch_src;
+      if (a.rows - fetch.row0 >= 32) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (i < 4 || k32) cp_async_16(dst + ((i & 1) ? to_odd : to_even) + i * 512, src);
+          src += src_step;
+        }
+      } else {
+        const int left = (int)max((int64_t)-64, a.rows - fetch.row0) - r_l;  // rows from this lane's first on
+        for (int i = 0; i < (1 << ch_shift); ++i) {
+          const bool in = (i << (5 - ch_shift)) < left;
+          cp_async_16_zfill(dst + ((i & 1) ? to_odd : to_even) + i * 512, in ? src : reinterpret_cast<const char*>(a.k_src), in ? 16 : 0);
+          src += src_step;
+        }
+      }
+      const int head = fetch.head, slice = fetch.slice;
+      advance(fetch);
+      fetch_src = fetch.head != head ? fetch_base() : fetch_src + (fetch.slice - slice) * 32 * esz + (fetch.slice <= slice ? 128 * row_bytes : 0);
+    }
+    cp_async_commit();
+  };
+
+  Place next = at0;
+  auto convert = [&]() -> SliceNorms {  // the pair `next`
+    float k[32];
+    if (STAGED) {
+      cp_async_wait<kCodeStages - 1>();
+      __syncwarp();
+      read_staged_row(kbuf + (next.q & (kCodeStages - 1)) * kSliceBlock, a.k_dtype, k);
+      __syncwarp();
+      issue_rows();
+    } else if (next.row0 + lane < a.rows) {
+      load_group<32>(a.k_src, a.k_dtype, (next.row0 + lane) * a.k_row_stride + (int64_t)next.head * a.k_head_stride + next.slice * 32, k);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) k[i] = 0.f;
+    }
+    const SliceNorms nn = store_slice(k, my_rows + kKeyCols + (next.q & 1) * 32, lows);
+    advance(next);
+    return nn;
+  };
+  const uint32_t op = smem_u32(smem);
+  Place cur = at0;
+  auto products = [&](int ps) {  // of the pair `cur`, by the group's first warp, after the group's barrier
+    if (w != 0) return;
+    tc_fence_after();
+    if (elect_one()) {
+      const uint32_t keys = tmem + kKeyCols + (cur.q & 1) * 32;
+      if constexpr (Fix::kFixed) {
+        constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);  // fp32 sums, bf16 x bf16, 128 rows
+        constexpr uint32_t k16 = kIdesc | (Fix::kHalf / 8) << 17, k32 = kIdesc | 2u << 17;
+        constexpr uint32_t kRows = 2 * Fix::kHalf + (Fix::C2 ? 32 : 0), kLo = kRows * 2;  // operand rows of a part; 16-byte units
+        const uint64_t b = smem_desc(op, 128, 256, 0) + (uint32_t)(cur.slice * 2 * kRows * 2);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint64_t hi = b + half * Fix::kHalf * 2;
+          const uint32_t d = tmem + half * Fix::kHalf;
+          mma_ts(d, keys + 8 * half, hi, k16, false);
+          if (lows) mma_ts(d, keys + 16 + 8 * half, hi, k16, true);
+          mma_ts(d, keys + 8 * half, hi + kLo, k16, true);
+        }
+        if constexpr (Fix::C2 > 0) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const uint64_t hi = b + (2 * Fix::kHalf + 16 * half) * 2;
+            const uint32_t d = tmem + 2 * Fix::kHalf;
+            mma_ts(d, keys + 8 * half, hi, k32, half > 0);
+            if (lows) mma_ts(d, keys + 16 + 8 * half, hi, k32, true);
+            mma_ts(d, keys + 8 * half, hi + kLo, k32, true);
+          }
+        }
+      } else {
+        issue_products(a.plan, a.tiers, ps, tmem, keys, op + a.plan.base[ps] + cur.slice * 2 * a.plan.rows[ps] * 32, lows);
+      }
+      mma_commit(bar);
+    }
+    __syncwarp();
+  };
+  auto enter_head = [&](int head) {  // between barriers of the whole CTA
+    stage_centroids(a.plan, a.tiers, a.codebooks, head, a.dh, smem, most);
+  };
+
+  if (n_q > 0) {
+    if (STAGED)
+      for (int i = 0; i < kCodeStages; ++i) issue_rows();
+    int head_at = cur.head;
+    enter_head(head_at);
+    SliceNorms n0 = convert(), n1 = {};  // of the pair that is searched next, and of the one after
+    if (next.q < n_q) n1 = convert();
+    tc_fence_before();
+    __syncthreads();
+    products(0);
+    bool lost = false;  // a wait for the tensor cores ran out: the chains decide everything from here on
+    uint32_t parity = 0, codes_before[3] = {0, 0, 0};
+    SliceNorms before = {};
+    for (int ps = 0;;) {
+      const bool last_pass = Fix::kFixed || ps + 1 == a.plan.n_pass;
+      lost = lost || !__all_sync(0xffffffffu, mbar_wait(bar, parity));
+      parity ^= 1;
+      tc_fence_after();
+      const int slice = cur.slice, head = cur.head;
+      const int64_t row = cur.row0 + lane;
+      const bool have = row < a.rows;
+      constexpr int kC0 = Fix::kFixed ? Fix::C0 : 16, kC1 = Fix::C1 ? Fix::C1 : 16, kC2 = Fix::C2 ? Fix::C2 : 16;
+      float s0a[kC0 < 16 ? 16 : kC0], s0b[kC0 < 16 ? 16 : kC0], s1a[kC1 < 16 ? 16 : kC1], s1b[kC1 < 16 ? 16 : kC1], s2[kC2 < 16 ? 16 : kC2];
+      float2 far0, far1;
+      float far2;
+      if constexpr (Fix::kFixed) {
+        tmem_ld_row<kC0>(my_rows, s0a);
+        tmem_ld_row<kC0>(my_rows + Fix::kHalf, s0b);
+        far0 = *reinterpret_cast<const float2*>(most + 2 * slice);
+        if constexpr (Fix::C1 > 0) {
+          tmem_ld_row<kC1>(my_rows + Fix::C0, s1a);
+          tmem_ld_row<kC1>(my_rows + Fix::kHalf + Fix::C0, s1b);
+          far1 = *reinterpret_cast<const float2*>(most + 8 + 2 * slice);
+        }
+        if constexpr (Fix::C2 > 0) {
+          tmem_ld_row<kC2>(my_rows + 2 * Fix::kHalf, s2);
+          far2 = most[8 * (Fix::kSlots - 1) + slice];
+        }
+        tmem_wait_ld();
+      } else {
+        for (int li = a.plan.first[ps]; li < a.plan.first[ps + 1]; ++li) {
+          const int s = a.plan.list[li], bits = a.tiers.bits[s];
+          const bool two = a.tiers.g[s] == 16;
+          const uint32_t sums = my_rows + a.plan.col[s];
+          RowSums v;
+          load_sums(v, sums, sums + a.plan.n16[ps], bits, two);
+          int ca, cb;
+          bool sa, sb;
+          search_sums(v, bits, two, two ? n0.a : n0.ab, n0.b, most[s * 8 + (two ? 2 * slice : slice)], most[s * 8 + (two ? 2 * slice + 1 : 0)], ca, cb, sa, sb);
+          if (__any_sync(0xffffffffu, have && (lost || !(sa && sb)))) {
+            const unsigned open_a = __ballot_sync(0xffffffffu, have && (lost || !sa)), open_b = __ballot_sync(0xffffffffu, have && (lost || !sb));
+            if (two) {
+              if (open_a) ca = settle<16>(a, head, s, 2 * slice, row, open_a, ca);
+              if (open_b) cb = settle<16>(a, head, s, 2 * slice + 1, row, open_b, cb);
+            } else {
+              ca = settle<32>(a, head, s, slice, row, open_a, ca);
+            }
+          }
+          if (have) {
+            const int G = two ? a.dh >> 4 : a.dh >> 5;
+            const int64_t o = ((int64_t)head * a.rows + row) * G + (two ? 2 * slice : slice);
+            store_groups(a.r_out[s] + o, a.th_out[s] + o, two ? 2 : 1, false, two ? make_float4(n0.a, n0.b, 0.f, 0.f) : make_float4(n0.ab, 0.f, 0.f, 0.f),
+                         two ? ca | (cb << 8) : ca);
+          }
+        }
+      }
+      // the sums have been read: the next products
+      tc_fence_before();
+      ++ps;
+      if (last_pass) {
+        advance(cur);
+        ps = 0;
+      }
+      const bool more = cur.q < n_q;
+      if (more) {
+        if (cur.head != head_at) {  // both groups walk the same units, so they meet here
+          head_at = cur.head;
+          __syncthreads();
+          enter_head(head_at);
+          __syncthreads();
+        } else {
+          group_barrier(group);
+        }
+        products(ps);
+      }
+      if constexpr (Fix::kFixed) {
+        int c[5] = {0, 0, 0, 0, 0};
+        bool sure[5] = {true, true, true, true, true};
+        sure[0] = nearest_column<kC0>(s0a, n0.a, far0.x, c[0]);
+        sure[1] = nearest_column<kC0>(s0b, n0.b, far0.y, c[1]);
+        if constexpr (Fix::C1 > 0) {
+          sure[2] = nearest_column<kC1>(s1a, n0.a, far1.x, c[2]);
+          sure[3] = nearest_column<kC1>(s1b, n0.b, far1.y, c[3]);
+        }
+        if constexpr (Fix::C2 > 0) sure[4] = nearest_column<kC2>(s2, n0.ab, far2, c[4]);
+        if (__any_sync(0xffffffffu, have && (lost || !(sure[0] && sure[1] && sure[2] && sure[3] && sure[4])))) {
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            const int s = i == 4 ? Fix::kSlots - 1 : i >> 1;
+            if ((i >= 2 && i < 4 && Fix::C1 == 0) || (i == 4 && Fix::C2 == 0)) continue;
+            const unsigned open = __ballot_sync(0xffffffffu, have && (lost || !sure[i]));
+            if (open) {
+              if (i == 4)
+                c[i] = settle<32>(a, head, s, slice, row, open, c[i]);
+              else
+                c[i] = settle<16>(a, head, s, 2 * slice + (i & 1), row, open, c[i]);
+            }
+          }
+        }
+        const uint32_t codes[3] = {(uint32_t)(c[0] | (c[1] << 8)), (uint32_t)(c[2] | (c[3] << 8)), (uint32_t)c[4]};
+        if (per == 1 || slice != slice0) {  // the group's slices of a row side by side
+          if (have) {
+            const int64_t at = (int64_t)head * a.rows + row;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              if ((i == 1 && Fix::C1 == 0) || (i == 2 && Fix::C2 == 0)) continue;
+              const int s = i == 2 ? Fix::kSlots - 1 : i;
+              const int64_t o = i == 2 ? at * (a.dh >> 5) + slice0 : at * (a.dh >> 4) + 2 * slice0;
+              const float4 r = per == 1 ? (i == 2 ? make_float4(n0.ab, 0.f, 0.f, 0.f) : make_float4(n0.a, n0.b, 0.f, 0.f))
+                                        : (i == 2 ? make_float4(before.ab, n0.ab, 0.f, 0.f) : make_float4(before.a, before.b, n0.a, n0.b));
+              store_groups(a.r_out[s] + o, a.th_out[s] + o, per * (i == 2 ? 1 : 2), a.wide, r,
+                           per == 1 ? codes[i] : codes_before[i] | codes[i] << (i == 2 ? 8 : 16));
+            }
+          }
+        } else {
+          before = n0;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) codes_before[i] = codes[i];
+        }
+      }
+      if (last_pass) {
+        n0 = n1;
+        if (next.q < n_q) n1 = convert();
+      }
+      if (!more) break;
+    }
+    if (lost) (void)mbar_wait(bar, parity);
+  }
+  cp_async_wait<0>();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kSearchGroups * kGroupCols);
+  }
+}
+
 int validate_tiers(const sphkv_tiers& t, int dh);
 
 }  // namespace sphkv
@@ -1095,6 +1483,56 @@ extern "C" int sphkv_pages_from_codes(const sphkv_encode_params* p, void* stream
   return encode_impl(p, stream, true);
 }
 
+static int launch_codes_chains(const CodesArgs& n, int Hkv, cudaStream_t st) {
+  ChainArgs a;
+  a.k_src = n.k_src; a.codebooks = n.codebooks;
+  a.k_row_stride = n.k_row_stride; a.k_head_stride = n.k_head_stride; a.rows = n.rows;
+  a.k_dtype = n.k_dtype; a.dh = n.dh; a.tiers = n.tiers;
+  int off = 0;
+  for (int s = 0; s < SPHKV_MAX_TIER_SLOTS; ++s) {
+    a.r_out[s] = n.r_out[s];
+    a.th_out[s] = n.th_out[s];
+    a.cb_off[s] = off;
+    if (s < a.tiers.n_slots) off += a.dh << a.tiers.bits[s];  // G_s * C_s * g_s floats
+  }
+  // row blocks staged through shared memory when every 32-element slice starts on a 16-byte
+  // boundary and the blocks fit beside the codebooks
+  const int esz = a.k_dtype == SPHKV_F32 ? 4 : 2;
+  const bool aligned = (reinterpret_cast<uintptr_t>(a.k_src) & 15) == 0 && (a.k_row_stride * esz) % 16 == 0 &&
+                       (a.k_head_stride * esz) % 16 == 0;
+  a.kbuf_off = off * 4;
+  const int64_t sms = sm_count_current_device();
+  const int row_sets = (kChainThreads / 32) / (a.dh >> 5);  // warps' row sets of a CTA
+  auto launch = [&](auto tok) -> int {
+    constexpr int TOK = decltype(tok)::value;
+    const int kbuf_bytes = (kChainThreads / 32) * 32 * TOK * 128;
+    const bool staged = aligned && off * 4 + kbuf_bytes <= 220 * 1024;
+    const int smem_bytes = off * 4 + (staged ? kbuf_bytes : 0);
+    auto kern = staged ? codes_chains_kernel<true, TOK> : codes_chains_kernel<false, TOK>;
+    static SmemOptIn opt_in[2];
+    if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem_bytes, "encode_codes")) return rc;
+    const int per_cta = row_sets * 32 * TOK;  // rows per CTA and pass
+    a.units_per_head = (a.rows + per_cta - 1) / per_cta;
+    a.n_units = a.units_per_head * Hkv;
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min(a.n_units, sms)));
+    kern<<<grid, kChainThreads, smem_bytes, st>>>(a);
+    return 0;
+  };
+  // Tokens per thread: the fewest microseconds of passes per CTA.  A pass of 4 / 2 / 1 tokens per thread was
+  // measured at 24 / 13 / 9 us (three reference tiers; the ratio is what counts): two or one win where four
+  // would leave SMs without a unit or the last pass nearly empty.
+  auto passes = [&](int tok) {
+    const int64_t units = (a.rows + row_sets * 32 * tok - 1) / (row_sets * 32 * tok) * Hkv;
+    return (units + sms - 1) / sms;
+  };
+  const int64_t t4 = passes(4) * 24, t2 = passes(2) * 13, t1 = passes(1) * 9;
+  const int rc = t4 <= t2 && t4 <= t1 ? launch(std::integral_constant<int, 4>())
+                 : t2 <= t1           ? launch(std::integral_constant<int, 2>())
+                                      : launch(std::integral_constant<int, 1>());
+  if (rc) return rc;
+  return check_launch("codes_chains_kernel");
+}
+
 extern "C" int sphkv_encode_codes(const void* k_src, int32_t k_dtype, int64_t k_row_stride,
                                   int64_t k_head_stride, int64_t rows, int32_t Hkv, int32_t dh,
                                   const float* codebooks, const sphkv_tiers* tiers, float* const* r_out,
@@ -1110,57 +1548,52 @@ extern "C" int sphkv_encode_codes(const void* k_src, int32_t k_dtype, int64_t k_
   a.k_src = k_src; a.codebooks = codebooks;
   a.k_row_stride = k_row_stride; a.k_head_stride = k_head_stride; a.rows = rows;
   a.k_dtype = k_dtype; a.dh = dh; a.tiers = *tiers;
-  int off = 0;
-  bool any = false;
+  unsigned wanted = 0;
+  uintptr_t ends = 0;
   for (int s = 0; s < SPHKV_MAX_TIER_SLOTS; ++s) {
     a.r_out[s] = s < tiers->n_slots ? r_out[s] : nullptr;
     a.th_out[s] = s < tiers->n_slots ? theta_out[s] : nullptr;
-    a.cb_off[s] = off;
     if (s < tiers->n_slots) {
       SPHKV_REQUIRE((a.r_out[s] == nullptr) == (a.th_out[s] == nullptr), SPHKV_E_ARG,
                     "encode_codes: slot %d needs both r_out and theta_out (or neither)", s);
-      any = any || a.r_out[s] != nullptr;
+      if (a.r_out[s] != nullptr) {
+        wanted |= 1u << s;
+        ends |= reinterpret_cast<uintptr_t>(a.r_out[s]) | reinterpret_cast<uintptr_t>(a.th_out[s]) << 2;
+      }
       SPHKV_REQUIRE((reinterpret_cast<uintptr_t>(a.r_out[s]) & 7) == 0 && (reinterpret_cast<uintptr_t>(a.th_out[s]) & 1) == 0,
                     SPHKV_E_ARG, "encode_codes: slot %d outputs must be 8-byte (r) and 2-byte (theta) aligned", s);
-      off += dh << tiers->bits[s];  // G_s * C_s * g_s floats
     }
   }
-  SPHKV_REQUIRE(any, SPHKV_E_ARG, "encode_codes: no output requested");
-  SPHKV_REQUIRE(off * 4 <= 200 * 1024, SPHKV_E_LIMIT, "encode_codes: codebooks need %d B of shared memory", off * 4);
-  // row blocks staged through shared memory when every 32-element slice starts on a 16-byte
-  // boundary and the blocks fit beside the codebooks
-  const int esz = k_dtype == SPHKV_F32 ? 4 : 2;
-  const bool aligned = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 &&
-                       (k_head_stride * esz) % 16 == 0;
-  a.kbuf_off = off * 4;
-  const int64_t sms = sm_count_current_device();
-  const int row_sets = (kCodeThreads / 32) / (dh >> 5);  // warps' row sets of a CTA
-  auto launch = [&](auto tok) -> int {
-    constexpr int TOK = decltype(tok)::value;
-    const int kbuf_bytes = (kCodeThreads / 32) * 32 * TOK * 128;
-    const bool staged = aligned && off * 4 + kbuf_bytes <= 220 * 1024;
-    const int smem_bytes = off * 4 + (staged ? kbuf_bytes : 0);
-    auto kern = staged ? encode_codes_kernel<true, TOK> : encode_codes_kernel<false, TOK>;
-    static SmemOptIn opt_in[2];
-    if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem_bytes, "encode_codes")) return rc;
-    const int per_cta = row_sets * 32 * TOK;  // rows per CTA and pass
-    a.units_per_head = (rows + per_cta - 1) / per_cta;
-    a.n_units = a.units_per_head * Hkv;
-    const dim3 grid((unsigned)std::max<int64_t>(1, std::min(a.n_units, sms)));
-    kern<<<grid, kCodeThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
-    return 0;
-  };
-  // Tokens per thread: the fewest microseconds of passes per CTA.  A pass of 4 / 2 / 1 tokens per thread was
-  // measured at 24 / 13 / 9 us (three reference tiers; the ratio is what counts): two or one win where four
-  // would leave SMs without a unit or the last pass nearly empty.
-  auto passes = [&](int tok) {
-    const int64_t units = (rows + row_sets * 32 * tok - 1) / (row_sets * 32 * tok) * Hkv;
-    return (units + sms - 1) / sms;
-  };
-  const int64_t t4 = passes(4) * 24, t2 = passes(2) * 13, t1 = passes(1) * 9;
-  const int rc = t4 <= t2 && t4 <= t1 ? launch(std::integral_constant<int, 4>())
-                 : t2 <= t1           ? launch(std::integral_constant<int, 2>())
-                                      : launch(std::integral_constant<int, 1>());
-  if (rc) return rc;
+  SPHKV_REQUIRE(wanted != 0, SPHKV_E_ARG, "encode_codes: no output requested");
+  // The chains cost 1.2 instructions per centroid and dim, the tensor-core kernel a fixed 45 us for 32768 tokens x 8 heads whatever
+  // it searches: centroids per dim 8 (one 32-dim slot) 32 us against 45, 16 49 / 50, 24 64 / 64, 32 74 / 55, 64 124 / 67,
+  // 88 (the three reference tiers) 170 / 75; of 500 tokens 4 / 8, 5 / 9, 7 / 10, 7 / 10, 11 / 12, 14 / 14.
+  int centroids = 0;
+  for (int s = 0; s < tiers->n_slots; ++s) centroids += (wanted >> s) & 1u ? 1 << tiers->bits[s] : 0;
+  if (centroids < 48) return launch_codes_chains(a, Hkv, reinterpret_cast<cudaStream_t>(stream));
+  a.wide = (ends & 15) == 0;
+  a.plan = plan_search(*tiers, dh, wanted);
+  a.kbuf_off = a.plan.bytes + kCodeTail;
+  // rows staged through shared memory when every 32-element slice starts on a 16-byte boundary and they fit beside
+  // the centroids (not with four 64-centroid slots)
+  const int esz = k_dtype == SPHKV_F32 ? 4 : 2, staged_bytes = kSearchThreads / 32 * kCodeStages * kSliceBlock;
+  const bool staged = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 &&
+                      (k_head_stride * esz) % 16 == 0 && a.kbuf_off + staged_bytes <= 227 * 1024;
+  const int smem_bytes = a.kbuf_off + (staged ? staged_bytes : 0);
+  // The reference's tiers (its first two, or all three) have a kernel of their own: 172 us with the chains, 89 us with branches
+  // and loops over the slots, 79 us with their sums in registers at once (32768 fp32 tokens x 8 heads, three tiers).
+  using Two = FixedTiers<6, 4, 0>;
+  using Three = FixedTiers<6, 4, 3>;
+  const int which = !staged ? 0 : Three::match(*tiers, wanted) ? 3 : Two::match(*tiers, wanted) ? 2 : 1;
+  auto kern = which == 3   ? encode_codes_kernel<true, Three>
+              : which == 2 ? encode_codes_kernel<true, Two>
+              : which == 1 ? encode_codes_kernel<true, AnyTiers>
+                           : encode_codes_kernel<false, AnyTiers>;
+  static SmemOptIn opt_in[4];
+  if (int rc = ensure_dynamic_smem(opt_in[which], (const void*)kern, smem_bytes, "encode_codes")) return rc;
+  a.units_per_head = (rows + 127) / 128;
+  a.n_units = a.units_per_head * Hkv;
+  const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(a.n_units, sm_count_current_device())));
+  kern<<<grid, kSearchThreads, smem_bytes, reinterpret_cast<cudaStream_t>(stream)>>>(a);
   return check_launch("encode_codes_kernel");
 }

@@ -1,0 +1,66 @@
+"""GPU: the code cache's tensor-core search against the fused encoder, whose searches are the fp32 fma chains themselves.
+Bytes have to be equal: for keys where the sums do not decide (ties, near ties, zeros, norms out of range), for tiers with
+a kernel of their own and without, in one pass and in several."""
+import pytest
+import torch
+
+from util import load_pkg
+
+pkg = load_pkg()
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+REF = pkg.REFERENCE_TIERS
+T = pkg.pages.TierSpec
+SETS = {
+    "reference": REF,
+    "first two": REF[:2],
+    "32 dims": (T(3, 32, 3),),
+    "small and odd": (T(1, 16, 1), T(2, 32, 2), T(3, 16, 5), T(4, 32, 6)),
+    "two passes": (T(1, 16, 6), T(2, 16, 5), T(3, 32, 6)),
+    "four passes, rows not staged": (T(1, 16, 6), T(2, 16, 6), T(3, 16, 6), T(4, 16, 6)),
+}
+
+
+def keys(kind, rows, hkv, dh, cbs, g):
+    k = torch.randn(rows, hkv, dh, generator=g, device=DEV)
+    if kind == "near ties":  # the mean of two centroids of the first slot, and a little more of one of them
+        c = cbs[0]
+        G, C, gs = c.shape[1:]
+        i, j = (torch.randint(C, (rows, hkv, G, 1, 1), generator=g, device=DEV) for _ in range(2))
+        pick = lambda n: torch.take_along_dim(c[None].expand(rows, -1, -1, -1, -1), n, 3)[:, :, :, 0]  # noqa: E731
+        eps = torch.randint(-3, 4, (rows, hkv, G, 1), generator=g, device=DEV) * 2.0 ** -23
+        k = (pick(i) * (1 + eps) + pick(j)).reshape(rows, hkv, dh)
+    elif kind == "zeros":
+        k[::3] = 0
+        k[1::3, :, ::2] = 0
+    elif kind == "scales":  # from underflow to overflow of the squares
+        k *= 10.0 ** torch.randint(-38, 38, (rows, 1, 1), generator=g, device=DEV).float()
+    elif kind == "not finite":
+        k[::5, :, 3] = float("inf")
+        k[1::5, :, 17] = float("nan")
+        k[2::5, :, 40] = -float("inf")
+    return k
+
+
+@pytest.mark.parametrize("kind", ["random", "near ties", "zeros", "scales", "not finite"])
+@pytest.mark.parametrize("tiers", SETS)
+@pytest.mark.parametrize("dh,rows,dtype", [(128, 129, torch.float32), (64, 300, torch.float32), (128, 127, torch.bfloat16),
+                                           (64, 128, torch.float16)])
+def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
+    specs, hkv = SETS[tiers], 2
+    g = torch.Generator(device=DEV).manual_seed(rows + dh)
+    cbs = []
+    for t in specs:
+        c = torch.randn(hkv, dh // t.g, t.codebook_size, t.g, generator=g, device=DEV)
+        cbs.append(c / c.norm(dim=-1, keepdim=True))
+    cbs[0][:, 0, -1] = cbs[0][:, 0, 0]  # two equal centroids, and one of zeros
+    cbs[0][:, 1, 0] = 0
+    ts = pkg.TierSet(dh, specs)
+    cb = ts.pack_codebooks(cbs)
+    K = keys(kind, rows, hkv, dh, cbs, g).to(dtype)
+    codes = pkg.encode_codes(K, cb, ts)
+    for t in specs:
+        lists = pkg.build_page_lists(torch.full((1, hkv, rows), t.tier_id, dtype=torch.uint8, device=DEV), ts, 16)
+        want = pkg.encode_pages(K, None, lists, cb, ts, use_scratch=False)
+        got = pkg.pages_from_codes(codes, None, lists, cb)
+        assert torch.equal(got.k_pages, want.k_pages)
