@@ -2,19 +2,17 @@
 // (codebooks/generate.py:47-58): sims = U @ centers^T, assigns = argmax, per-cluster vector
 // sums and counts.  The similarity search is the one of the page encoder: the dot product
 // of a point with a centroid is an fp32 fma chain over d = 0..g-1 starting from 0, centroids
-// are visited in ascending order and the first maximum wins (torch.argmax convention).
+// are visited in ascending order and the first maximum wins (torch.argmax convention) -- found on the tensor cores
+// and settled by the chains where that does not decide (search.cuh).
 //
-// One thread holds kPts points in registers and walks the centroids out of shared memory
-// (one broadcast 16-byte load feeds 16 or 8 FMAs).  The accumulation uses no float atomics and no
-// barrier until the end: every warp keeps sums of its own in shared memory, 32 / D sets of [K][D] (`ways`; fewer
-// when they would not fit), and walks its points D lanes to a row -- lane = dimension, one add per row and lane, the rows
-// turned through a 32-row tile of shared memory -- so lanes never meet in an address.  At the end the
-// warps' sets are added up and every CTA adds its sums to the output with float atomics, in no fixed order.  Sums agree to rounding, as with index_add_ on a GPU; assignments and counts are
-// exact.  Bound: fp32 FMA issue for K = 64, then the shared-memory adds.  4M points, d 16, K 64: 324 -> 254 us;
-// K 16, 2.3M points: 95 -> 76 us (a counting sort per 1024 points with six barriers before).
+// The accumulation uses no float atomics and no barrier until the end: every warp keeps sums of its own in
+// shared memory, 32 / D sets of [K][D] (`ways`; fewer when they would not fit), and walks its points D lanes to a row
+// -- lane = dimension, one add per row and lane, the rows as they were staged -- so lanes never meet in an address.  At the
+// end the warps' sets are added up and every CTA adds its sums to the output with float atomics, in no fixed order.
+// Sums agree to rounding, as with index_add_ on a GPU; assignments and counts are exact.
 #include <algorithm>
 
-#include "common.cuh"
+#include "search.cuh"
 
 namespace sphkv {
 
@@ -23,7 +21,7 @@ __host__ __device__ constexpr int pts_for(int d) { return d >= 32 ? 2 : 4; }
 
 // a CTA takes passes of 32 * pts_for(D) points per warp; its warps walk them without meeting
 template <int D, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, 2) kmeans_assign_kernel(
+__global__ void __launch_bounds__(32 * WARPS, 2) kmeans_chains_kernel(
     const float* __restrict__ U, int64_t N, const float* __restrict__ centers, int K,
     int32_t* __restrict__ assigns, float* __restrict__ best_sim, float* __restrict__ sums,
     int32_t* __restrict__ counts, int ways) {
@@ -137,7 +135,7 @@ __global__ void __launch_bounds__(32 * WARPS, 2) kmeans_assign_kernel(
 }
 
 template <int D, int WARPS = 8>
-static int launch_kmeans(const float* U, int64_t N, const float* centers, int K, int32_t* assigns, float* best_sim, float* sums,
+static int launch_chains(const float* U, int64_t N, const float* centers, int K, int32_t* assigns, float* best_sim, float* sums,
                          int32_t* counts, int sms, cudaStream_t st) {
   // a set of sums for every D lanes of a warp, or for fewer of them, while two CTAs fit an SM: with d 8 and K 128 two
   // sets fit where four do not (1M points: 86.4 us with one set, 80.4 with two)
@@ -150,13 +148,341 @@ static int launch_kmeans(const float* U, int64_t N, const float* centers, int K,
   // eight warps' sums are more than a CTA can have from K 173 on at d 32: seven (a runtime warp count cost every
   // size 1 to 4 %)
   if constexpr (WARPS == 8 && D == 32)
-    if (smem > 227 * 1024) return launch_kmeans<D, 7>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
+    if (smem > 227 * 1024) return launch_chains<D, 7>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
   static SmemOptIn opt_in;
-  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_assign_kernel<D, WARPS>, (int)smem, "kmeans_assign")) return rc;
+  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_chains_kernel<D, WARPS>, (int)smem, "kmeans_assign")) return rc;
   const int64_t pass = (int64_t)32 * WARPS * pts_for(D);
   const int64_t ctas = std::min<int64_t>((N + pass - 1) / pass, (int64_t)sms * (smem <= 110 * 1024 ? 2 : 1));
-  kmeans_assign_kernel<D, WARPS><<<(unsigned)ctas, 32 * WARPS, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, ways);
-  return check_launch("kmeans_assign_kernel");
+  kmeans_chains_kernel<D, WARPS><<<(unsigned)ctas, 32 * WARPS, smem, st>>>(U, N, centers, K, assigns, best_sim, sums, counts, ways);
+  return check_launch("kmeans_chains_kernel");
+}
+
+// ---- search on the tensor cores ----
+struct KmeansArgs {
+  const float* U;
+  int64_t N;
+  const float* centers;
+  int K;
+  int32_t* assigns;
+  float* best_sim;
+  float* sums;
+  int32_t* counts;
+  int ways;        // sets of sums per warp
+  int cols;        // tensor memory columns of a group
+  int sum_cols;    // K rounded up to 16
+  int off_centers, off_sums, off_points, off_small;  // byte offsets in shared memory (the centroids' operand at 0)
+};
+
+// batches of 128 points in flight per group, the one whose rows are being added included
+__host__ __device__ constexpr int kmeans_stages(int d) { return d >= 32 ? 3 : 4; }
+__host__ __device__ constexpr int kmeans_key_cols(int d) { return d >= 32 ? 32 : 16; }  // hi | lo of a point
+constexpr int kKmeansGroups = 3;
+
+__device__ __forceinline__ float lds_f1(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+// A CTA has up to three search groups (four warps, thread = point = lane of tensor memory), each striding over batches
+// of 128 points; a warp stages, splits, searches and adds its 32 points by itself and meets the group's other warps
+// once per batch, before the products.
+template <int D>
+__global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(const __grid_constant__ KmeansArgs a) {
+  constexpr int kStages = kmeans_stages(D), kKeys = kmeans_key_cols(D), kParts = D >= 32 ? 2 : 1;
+  constexpr int kRowChunks = D / 4;  // 16-byte chunks of a point
+  extern __shared__ __align__(16) uint8_t smem[];
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int group = warp >> 2, w = warp & 3, groups = blockDim.x >> 7, K = a.K;
+  float* c_s = reinterpret_cast<float*>(smem + a.off_centers);           // [K][D]
+  float* sum_s = reinterpret_cast<float*>(smem + a.off_sums);            // [warps][ways][K][D]
+  int* cnt_s = reinterpret_cast<int*>(smem + a.off_small);               // [K]
+  int* most_s = cnt_s + ((K + 3) & ~3);                                  // largest |c|^2
+  const uint32_t bars = smem_u32(most_s + 2), bar = bars + 8 * group;
+  volatile uint32_t* tmem_word = reinterpret_cast<volatile uint32_t*>(most_s + 2 + 2 * kKmeansGroups);
+  const uint32_t points = smem_u32(smem + a.off_points) + warp * (kStages * 32 * D * 4);
+  // chunk q of row p is stored at chunk q ^ turn(p): neither row-per-lane nor dimension-per-lane accesses meet in a bank
+  auto turn = [](int p) { return (p >> (D == 32 ? 0 : D == 16 ? 1 : 2)) & (kRowChunks - 1); };
+
+  const int64_t stride = (int64_t)gridDim.x * groups * 128;
+  const int64_t first = ((int64_t)blockIdx.x * groups + group) * 128;
+  int64_t fetch_at = first + 32 * w;
+  int fetch_stage = 0;
+  auto fetch = [&]() {  // the warp's 32 rows of the next batch
+    if (fetch_at - 32 * w < a.N) {  // the group's batch; rows past the end are zero
+      const float* src = a.U + fetch_at * D;
+      const int chunks = (int)max((int64_t)0, min((int64_t)32, a.N - fetch_at)) * kRowChunks;
+      const uint32_t dst = points + fetch_stage * (32 * D * 4);
+#pragma unroll
+      for (int i = 0; i < kRowChunks; ++i) {
+        const int c = lane + 32 * i, p = c / kRowChunks, q = c % kRowChunks;
+        const bool in = c < chunks;
+        cp_async_16_zfill(dst + p * (D * 4) + (q ^ turn(p)) * 16, in ? src + 4 * c : a.U, in ? 16 : 0);
+      }
+    }
+    cp_async_commit();
+    fetch_at += stride;
+    fetch_stage = fetch_stage + 1 == kStages ? 0 : fetch_stage + 1;
+  };
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) fetch();
+
+  if (warp == 0) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_word)), 512);
+  if ((int)threadIdx.x < groups) mbar_init(bars + 8 * threadIdx.x, 1);
+  if (threadIdx.x == 0) *most_s = 0;
+  for (int i = threadIdx.x; i < K * D; i += blockDim.x) c_s[i] = a.centers[i];
+  for (int i = threadIdx.x; i < (int)(blockDim.x >> 5) * a.ways * K * D; i += blockDim.x) sum_s[i] = 0.f;
+  for (int i = threadIdx.x; i < K; i += blockDim.x) cnt_s[i] = 0;
+  __syncthreads();
+  // operand of the centroids: per part (hi, lo) and 16 dims, rows of 32 bytes, 8-row groups 256 bytes apart, 8-dim
+  // groups 128; points of 8 dims are padded with zeros
+  const int part_bytes = a.sum_cols * 32 * kParts;
+  for (int i = threadIdx.x; i < K * kParts; i += blockDim.x) {
+    const int c = i / kParts, kc = i % kParts;
+    uint8_t* hi_at = smem + kc * a.sum_cols * 32 + (c >> 3) * 256 + (c & 7) * 16;
+    uint32_t hi[8], lo[8];
+    float nsq = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float x = 2 * e < D ? c_s[c * D + 16 * kc + 2 * e] : 0.f, y = 2 * e < D ? c_s[c * D + 16 * kc + 2 * e + 1] : 0.f;
+      split_bf16x2(x, y, hi[e], lo[e]);
+    }
+    *reinterpret_cast<uint4*>(hi_at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4*>(hi_at + 128) = make_uint4(hi[4], hi[5], hi[6], hi[7]);
+    *reinterpret_cast<uint4*>(hi_at + part_bytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    *reinterpret_cast<uint4*>(hi_at + part_bytes + 128) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+    if (kc == 0) {
+      for (int e = 0; e < D; ++e) nsq += c_s[c * D + e] * c_s[c * D + e];
+      atomicMax(most_s, __float_as_int(nsq) & 0x7fffffff);  // bit patterns order as integers, a NaN above infinity
+    }
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const float most_sq = __int_as_float(*most_s);
+  const float most = most_sq >= 8.6736174e-19f && most_sq <= 1.1529215e18f ? sqrtf(most_sq) : __int_as_float(0x7fc00000);
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_word[0], 0);
+  const uint32_t tmem = tmem_base + group * a.cols, my_rows = tmem + ((uint32_t)(32 * w) << 16);
+  constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);  // fp32 sums, bf16 x bf16, 128 rows
+  const uint32_t idesc = kIdesc | ((uint32_t)(a.sum_cols >> 3) << 17);
+  const uint64_t op = smem_desc(smem_u32(smem), 128, 256, 0);
+
+  float norm_n = 0.f;
+  int conv_stage = 0, keys = 0;
+  auto convert = [&]() {  // the next staged batch's rows as bf16 pairs in tensor memory
+    cp_async_wait<kStages - 2>();
+    __syncwarp();
+    const uint32_t src = points + conv_stage * (32 * D * 4) + lane * (D * 4);
+    float k[D < 16 ? 16 : D];
+#pragma unroll
+    for (int q = 0; q < kRowChunks; ++q) {
+      const float4 v = lds_f4(src + ((q ^ turn(lane)) << 4));
+      k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+    }
+#pragma unroll
+    for (int i = D; i < 16; ++i) k[i] = 0.f;
+    float n0 = 0.f, n1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; i += 2) { n0 = __fmaf_rn(k[i], k[i], n0); n1 = __fmaf_rn(k[i + 1], k[i + 1], n1); }
+    norm_n = sqrtf(n0 + n1);
+    constexpr int kWords = (D < 16 ? 16 : D) / 2;
+    uint32_t hi[kWords], lo[kWords];
+    split_pairs(k, hi, lo);
+    const uint32_t dst = my_rows + a.sum_cols + keys * kKeys;
+    if constexpr (kWords == 16) {
+      tmem_st_x16(dst, hi);
+      tmem_st_x16(dst + 16, lo);
+    } else {
+      tmem_st_x8(dst, hi);
+      tmem_st_x8(dst + 8, lo);
+    }
+    tmem_wait_st();
+    conv_stage = conv_stage + 1 == kStages ? 0 : conv_stage + 1;
+  };
+  auto products = [&]() {
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+    if (w == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t k0 = tmem + a.sum_cols + keys * kKeys;
+#pragma unroll
+        for (int kc = 0; kc < kParts; ++kc) {
+          const uint64_t hi = op + (uint32_t)(kc * a.sum_cols * 2), lo = hi + (uint32_t)(part_bytes >> 4);
+          mma_ts(tmem, k0 + 8 * kc, hi, idesc, kc > 0);
+          mma_ts(tmem, k0 + kKeys / 2 + 8 * kc, hi, idesc, true);
+          mma_ts(tmem, k0 + 8 * kc, lo, idesc, true);
+        }
+        mma_commit(bar);
+      }
+      __syncwarp();
+    }
+    keys ^= 1;
+  };
+  // adding: lane = (way, dimension); with one way the first D lanes work
+  const int dim = lane & (D - 1), way = lane / D;
+  const bool adds = way < a.ways;
+  float* my_sums = sum_s + ((int64_t)warp * a.ways + (adds ? way : 0)) * K * D + dim;
+
+  if (first < a.N) {
+    convert();
+    tc_fence_before();
+    products();
+  }
+  bool lost = false;  // a wait for the tensor cores ran out: the chains decide everything from here on
+  uint32_t parity = 0;
+  int stage = 0;
+  for (int64_t base = first; base < a.N; base += stride) {
+    const float norm = norm_n;
+    const bool more = base + stride < a.N;
+    fetch();
+    if (more) convert();
+    lost = lost || !__all_sync(0xffffffffu, mbar_wait(bar, parity));
+    parity ^= 1;
+    tc_fence_after();
+    const int64_t idx = base + 32 * w + lane;
+    const bool live = idx < a.N;
+    int code;
+    bool sure;
+    auto whole = [&](auto n) {  // all sums of a point at once
+      constexpr int C = decltype(n)::value;
+      float v[C < 16 ? 16 : C];
+      tmem_ld_row<C>(my_rows, v);
+      tmem_wait_ld();
+      sure = nearest_column<C>(v, norm, most, code);
+    };
+    if (K == 64) {
+      whole(std::integral_constant<int, 64>());
+    } else if (K == 16) {
+      whole(std::integral_constant<int, 16>());
+    } else if (K == 8) {
+      whole(std::integral_constant<int, 8>());
+    } else {  // sixteen columns at a time, twice: the largest, then what comes near it
+      float top = -INFINITY;
+      auto columns = [&](int c0, float (&v)[16]) {
+        tmem_ld_x16(my_rows + c0, v);
+        tmem_wait_ld();
+        if (c0 + 16 > K) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            if (c0 + c >= K) v[c] = -INFINITY;
+        }
+      };
+      for (int c0 = 0; c0 < K; c0 += 16) {
+        float v[16];
+        columns(c0, v);
+        top = fmaxf(top, largest_of<16>(v));
+      }
+      const Lead l = lead_of(top, norm, most);
+      float all = 0.f;
+      int base_of = 0;
+      for (int c0 = 0; c0 < K; c0 += 16) {
+        float v[16];
+        columns(c0, v);
+        const float some = count_leaders<16>(v, l);
+        all += some;
+        if (some > 0.f) base_of = c0;
+      }
+      code = leader_of(all) + base_of;
+      sure = l.fit && one_leader(all);
+    }
+    tc_fence_before();
+    if (more) products();  // runs while this batch is added up
+    const unsigned open = __ballot_sync(0xffffffffu, live && (lost || !sure));
+    const uint32_t rows = points + stage * (32 * D * 4);
+    if (open)
+      code = exact_search<D>([&](int64_t off, float (&k)[D]) {
+#pragma unroll
+        for (int q = 0; q < kRowChunks; ++q) {
+          const float4 v = *reinterpret_cast<const float4*>(a.U + off + 4 * q);
+          k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+        }
+      }, idx * D, c_s, D, K, open, code);
+    if (!live) code = 0;
+    if (live) {
+      a.assigns[idx] = code;
+      if (a.best_sim != nullptr) {  // the chain of the winner
+        float s = 0.f;
+        const float4* c = reinterpret_cast<const float4*>(c_s + code * D);
+#pragma unroll
+        for (int q = 0; q < kRowChunks; ++q) {
+          const float4 v = lds_f4(rows + lane * (D * 4) + ((q ^ turn(lane)) << 4)), x = c[q];
+          s = __fmaf_rn(v.x, x.x, s);
+          s = __fmaf_rn(v.y, x.y, s);
+          s = __fmaf_rn(v.z, x.z, s);
+          s = __fmaf_rn(v.w, x.w, s);
+        }
+        a.best_sim[idx] = s;
+      }
+      atomicAdd(&cnt_s[code], 1);
+    }
+    // rows past the end are zero and add nothing.  Two rows at a time: if they are of one cluster, the second sum
+    // follows from the first
+    const int at = code * D;
+    for (int p0 = 0; p0 < 32; p0 += 8 * a.ways) {
+      float v[8];
+      int c[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int p = p0 + e * a.ways + (adds ? way : 0);
+        c[e] = __shfl_sync(0xffffffffu, at, p & 31);
+        v[e] = lds_f1(rows + p * (D * 4) + (((dim >> 2) ^ turn(p)) << 4) + (dim & 3) * 4);
+      }
+      if (adds) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          const float s0 = my_sums[c[e]], s1 = my_sums[c[e + 1]];
+          const float t0 = s0 + v[e], t1 = (c[e] == c[e + 1] ? t0 : s1) + v[e + 1];
+          my_sums[c[e]] = t0;
+          my_sums[c[e + 1]] = t1;
+        }
+      }
+    }
+    __syncwarp();
+    stage = stage + 1 == kStages ? 0 : stage + 1;
+  }
+  if (lost) (void)mbar_wait(bar, parity);
+  cp_async_wait<0>();
+  tc_fence_before();
+  __syncthreads();
+  for (int i = threadIdx.x; i < K * D; i += blockDim.x) {
+    float t = 0.f;
+    for (int s = 0; s < (int)(blockDim.x >> 5) * a.ways; ++s) t += sum_s[(int64_t)s * K * D + i];
+    if (t != 0.f) atomicAdd(a.sums + i, t);
+  }
+  for (int i = threadIdx.x; i < K; i += blockDim.x)
+    if (cnt_s[i] != 0) atomicAdd(a.counts + i, cnt_s[i]);
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <int D>
+static int launch_search(KmeansArgs a, int sms, cudaStream_t st) {
+  a.sum_cols = (a.K + 15) & ~15;
+  a.cols = a.sum_cols + 2 * kmeans_key_cols(D);
+  const int set = a.K * D * 4, parts = D >= 32 ? 2 : 1;
+  const int small = ((a.K + 3) & ~3) * 4 + 8 + 8 * kKmeansGroups + 16;
+  auto bytes = [&](int groups, int ways) {
+    a.off_centers = a.sum_cols * 32 * parts * 2;
+    a.off_sums = a.off_centers + (set + 15) / 16 * 16;
+    a.off_points = a.off_sums + (4 * groups * ways * set + 15) / 16 * 16;
+    a.off_small = a.off_points + 4 * groups * kmeans_stages(D) * 32 * D * 4;
+    return a.off_small + small;
+  };
+  // as many groups as tensor memory and shared memory have room for, then as many sets of sums
+  int groups = kKmeansGroups, ways = 1;
+  while (groups > 1 && (groups * a.cols > 512 || bytes(groups, 1) > 227 * 1024)) --groups;
+  for (int more = 32 / D; more > ways; more >>= 1)
+    if (bytes(groups, more) <= 227 * 1024) ways = more;
+  const int smem = bytes(groups, ways);
+  a.ways = ways;
+  static SmemOptIn opt_in;
+  if (int rc = ensure_dynamic_smem(opt_in, (const void*)kmeans_search_kernel<D>, smem, "kmeans_assign")) return rc;
+  const int64_t ctas = std::min<int64_t>((a.N + 128 * groups - 1) / (128 * groups), sms);
+  kmeans_search_kernel<D><<<(unsigned)ctas, 128 * groups, smem, st>>>(a);
+  return check_launch("kmeans_search_kernel");
 }
 
 }  // namespace sphkv
@@ -172,8 +498,8 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
   SPHKV_REQUIRE((reinterpret_cast<uintptr_t>(U) & 15) == 0, SPHKV_E_ARG, "kmeans_assign: U must be 16-byte aligned");
   const int sms = sphkv_sm_count();
   SPHKV_REQUIRE(sms > 0, SPHKV_E_ARG, "kmeans_assign: cannot resolve the SM count");
-  // the sizes the call takes (8 and 16: every K; 32: K up to 179); all of them fit with one set of sums per warp
-  const int per_pass = 256 * pts_for(d) * 2;
+  // the sizes the call takes (8 and 16: every K; 32: K up to 179); all of them fit with one group and one set of sums per warp
+  const int per_pass = 256 * (d >= 32 ? 2 : 4) * 2;
   SPHKV_REQUIRE(K * d * 8 + (3 * K + 1) * 4 + per_pass <= 48 * 1024, SPHKV_E_LIMIT,
                 "kmeans_assign: K=%d x d=%d is beyond the sizes it takes (K * d * 8 + 12 * K + %d <= 49152)", K, d, 4 + per_pass);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -184,7 +510,15 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
     return (int)e;
   }
   if (N == 0) return SPHKV_OK;
-  return d == 8    ? launch_kmeans<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
-         : d == 16 ? launch_kmeans<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
-                   : launch_kmeans<32>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
+  // The chains cost K fmas per value, the tensor cores hardly anything, but that kernel has fewer warps to hide the sums behind:
+  // 4M points (2M of 32 dims), chains / tensor cores: d 8: K 32 97 / 114 us, 48 126 / 125, 64 156 / 116; d 16: K 16 120 / 140,
+  // 32 163 / 165, 48 210 / 180, 64 255 / 171, 256 917 / 627; d 32: K 8 130 / 123, 64 289 / 182.
+  if (d < 32 && K < 48) {
+    return d == 8 ? launch_chains<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
+                  : launch_chains<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
+  }
+  KmeansArgs a = {};
+  a.U = U; a.N = N; a.centers = centers; a.K = K;
+  a.assigns = assigns; a.best_sim = best_sim; a.sums = sums; a.counts = counts;
+  return d == 8 ? launch_search<8>(a, sms, st) : d == 16 ? launch_search<16>(a, sms, st) : launch_search<32>(a, sms, st);
 }
