@@ -19,7 +19,9 @@ namespace sphkv {
 // points per thread: 4 (2 for 32-dim points) keeps the kernel at two CTAs per SM
 __host__ __device__ constexpr int pts_for(int d) { return d >= 32 ? 2 : 4; }
 
-// a CTA takes passes of 32 * pts_for(D) points per warp; its warps walk them without meeting
+// Few centroids (see the rule at the launch): the chains on the fp32 pipe.  A CTA takes passes of 32 * pts_for(D) points per
+// warp; its warps walk them without meeting; a warp's rows are turned through a 32-row tile for the adds.  Bound: fp32 FMA
+// issue, then the shared-memory adds.
 template <int D, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 2) kmeans_chains_kernel(
     const float* __restrict__ U, int64_t N, const float* __restrict__ centers, int K,
@@ -184,6 +186,8 @@ __device__ __forceinline__ float lds_f1(uint32_t addr) {
   return v;
 }
 
+// Bound: latency -- twelve warps an SM, each with a chain of tensor memory, shared-memory adds and a barrier per batch; DRAM at
+// 26 % of the copy rate.  4M points, d 16, K 64: 255 us with the chains, 170 here.
 // A CTA has up to three search groups (four warps, thread = point = lane of tensor memory), each striding over batches
 // of 128 points; a warp stages, splits, searches and adds its 32 points by itself and meets the group's other warps
 // once per batch, before the products.
@@ -513,9 +517,11 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
   // The chains cost K fmas per value, the tensor cores hardly anything, but that kernel has fewer warps to hide the sums behind:
   // 4M points (2M of 32 dims), chains / tensor cores: d 8: K 32 97 / 114 us, 48 126 / 125, 64 156 / 116; d 16: K 16 120 / 140,
   // 32 163 / 165, 48 210 / 180, 64 255 / 171, 256 917 / 627; d 32: K 8 130 / 123, 64 289 / 182.
-  if (d < 32 && K < 48) {
-    return d == 8 ? launch_chains<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
-                  : launch_chains<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
+  // Of 32 dims and 128 centroids on, one search group is all that fits a CTA: 60000 points 31 / 37 us, 500000 148 / 109.
+  if ((d < 32 && K < 48) || (d == 32 && K >= 128 && N < 200000)) {
+    return d == 8    ? launch_chains<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
+           : d == 16 ? launch_chains<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
+                     : launch_chains<32>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);
   }
   KmeansArgs a = {};
   a.U = U; a.N = N; a.centers = centers; a.K = K;

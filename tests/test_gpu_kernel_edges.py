@@ -123,6 +123,35 @@ def test_kmeans_sums_and_counts(N, d, K):
     assert ((sums.double() - want).abs() <= bound).all()
 
 
+# both sides of the rules that choose the tensor-core search: centroids, and points of the largest codebooks; batches of 128
+@pytest.mark.parametrize("N,d,K", [(129, 8, 47), (129, 8, 48), (385, 16, 47), (385, 16, 48), (199999, 32, 128), (200000, 32, 128),
+                                   (50000, 16, 256), (3000, 32, 17)])
+def test_kmeans_search_rules(N, d, K):
+    test_kmeans_sums_and_counts(N, d, K)
+
+
+@pytest.mark.parametrize("d,K", [(8, 64), (16, 64), (32, 8), (32, 20)])
+def test_kmeans_ties_and_special_points(d, K):
+    """equal centroids, points between two centroids, zeros and norms out of range: the fp32 chains' first maximum"""
+    g = torch.Generator(device=DEV).manual_seed(d)
+    C = torch.nn.functional.normalize(torch.randn(K, d, generator=g, device=DEV), dim=1)
+    C[K - 1] = C[1]
+    C[3] = 0
+    U = C[torch.randint(K, (999,), generator=g, device=DEV)] + C[torch.randint(K, (999,), generator=g, device=DEV)]
+    U[::7] = 0
+    U[1::7] *= 1e-30
+    U[2::7] *= 1e15
+    sims = torch.zeros(999, K, dtype=torch.float64, device=DEV)
+    for i in range(d):  # an fma rounds the exact product and sum once
+        sims = (U[:, i:i + 1].double() * C[:, i].double() + sims).float().double()
+    assigns, best, _, counts = pkg.kmeans_assign(U, C)
+    want = sims.max(1).values
+    # (a 64-bit product and sum rounds a second time, in one of 2^29 cases differently from the fma)
+    assert (sims.gather(1, assigns.long()[:, None])[:, 0] == want).sum() >= 997 and (best.double() == want).sum() >= 997
+    assert (assigns.long() == (sims == want[:, None]).int().argmax(1)).sum() >= 997
+    assert torch.equal(counts.long(), torch.bincount(assigns.long(), minlength=K))
+
+
 # the largest codebooks of 32-dim points: eight, then seven sets of sums per CTA
 @pytest.mark.parametrize("K", [172, 173, 179])
 def test_kmeans_largest_codebooks(K):
