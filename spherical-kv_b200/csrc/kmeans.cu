@@ -179,6 +179,8 @@ struct KmeansArgs {
 __host__ __device__ constexpr int kmeans_stages(int d) { return d >= 32 ? 3 : 4; }
 __host__ __device__ constexpr int kmeans_key_cols(int d) { return d >= 32 ? 32 : 16; }  // hi | lo of a point
 constexpr int kKmeansGroups = 3;
+// floats from one centroid to the next in shared memory: lanes that read rows of their own spread over all banks
+__host__ __device__ constexpr int kmeans_pitch(int d) { return d + 4; }
 
 __device__ __forceinline__ float lds_f1(uint32_t addr) {
   float v;
@@ -187,7 +189,7 @@ __device__ __forceinline__ float lds_f1(uint32_t addr) {
 }
 
 // Bound: latency -- twelve warps an SM, each with a chain of tensor memory, shared-memory adds and a barrier per batch; DRAM at
-// 26 % of the copy rate.  4M points, d 16, K 64: 255 us with the chains, 170 here.
+// 30 % of the copy rate.  4M points, d 16, K 64: 255 us with the chains, 170 here, 148 without bank conflicts on the winners.
 // A CTA has up to three search groups (four warps, thread = point = lane of tensor memory), each striding over batches
 // of 128 points; a warp stages, splits, searches and adds its 32 points by itself and meets the group's other warps
 // once per batch, before the products.
@@ -198,7 +200,8 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int group = warp >> 2, w = warp & 3, groups = blockDim.x >> 7, K = a.K;
-  float* c_s = reinterpret_cast<float*>(smem + a.off_centers);           // [K][D]
+  constexpr int kPitch = kmeans_pitch(D);
+  float* c_s = reinterpret_cast<float*>(smem + a.off_centers);           // [K][kPitch]
   float* sum_s = reinterpret_cast<float*>(smem + a.off_sums);            // [warps][ways][K][D]
   int* cnt_s = reinterpret_cast<int*>(smem + a.off_small);               // [K]
   int* most_s = cnt_s + ((K + 3) & ~3);                                  // largest |c|^2
@@ -234,7 +237,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
   if (warp == 0) tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_word)), 512);
   if ((int)threadIdx.x < groups) mbar_init(bars + 8 * threadIdx.x, 1);
   if (threadIdx.x == 0) *most_s = 0;
-  for (int i = threadIdx.x; i < K * D; i += blockDim.x) c_s[i] = a.centers[i];
+  for (int i = threadIdx.x; i < K * D; i += blockDim.x) c_s[i / D * kPitch + i % D] = a.centers[i];
   for (int i = threadIdx.x; i < (int)(blockDim.x >> 5) * a.ways * K * D; i += blockDim.x) sum_s[i] = 0.f;
   for (int i = threadIdx.x; i < K; i += blockDim.x) cnt_s[i] = 0;
   __syncthreads();
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     float nsq = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float x = 2 * e < D ? c_s[c * D + 16 * kc + 2 * e] : 0.f, y = 2 * e < D ? c_s[c * D + 16 * kc + 2 * e + 1] : 0.f;
+      const float x = 2 * e < D ? c_s[c * kPitch + 16 * kc + 2 * e] : 0.f, y = 2 * e < D ? c_s[c * kPitch + 16 * kc + 2 * e + 1] : 0.f;
       split_bf16x2(x, y, hi[e], lo[e]);
     }
     *reinterpret_cast<uint4*>(hi_at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     *reinterpret_cast<uint4*>(hi_at + part_bytes) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     *reinterpret_cast<uint4*>(hi_at + part_bytes + 128) = make_uint4(lo[4], lo[5], lo[6], lo[7]);
     if (kc == 0) {
-      for (int e = 0; e < D; ++e) nsq += c_s[c * D + e] * c_s[c * D + e];
+      for (int e = 0; e < D; ++e) nsq += c_s[c * kPitch + e] * c_s[c * kPitch + e];
       atomicMax(most_s, __float_as_int(nsq) & 0x7fffffff);  // bit patterns order as integers, a NaN above infinity
     }
   }
@@ -401,13 +404,13 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
           const float4 v = *reinterpret_cast<const float4*>(a.U + off + 4 * q);
           k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
         }
-      }, idx * D, c_s, D, K, open, code);
+      }, idx * D, c_s, kPitch, K, open, code);
     if (!live) code = 0;
     if (live) {
       a.assigns[idx] = code;
       if (a.best_sim != nullptr) {  // the chain of the winner
         float s = 0.f;
-        const float4* c = reinterpret_cast<const float4*>(c_s + code * D);
+        const float4* c = reinterpret_cast<const float4*>(c_s + code * kPitch);
 #pragma unroll
         for (int q = 0; q < kRowChunks; ++q) {
           const float4 v = lds_f4(rows + lane * (D * 4) + ((q ^ turn(lane)) << 4)), x = c[q];
@@ -470,7 +473,7 @@ static int launch_search(KmeansArgs a, int sms, cudaStream_t st) {
   const int small = ((a.K + 3) & ~3) * 4 + 8 + 8 * kKmeansGroups + 16;
   auto bytes = [&](int groups, int ways) {
     a.off_centers = a.sum_cols * 32 * parts * 2;
-    a.off_sums = a.off_centers + (set + 15) / 16 * 16;
+    a.off_sums = a.off_centers + a.K * kmeans_pitch(D) * 4;
     a.off_points = a.off_sums + (4 * groups * ways * set + 15) / 16 * 16;
     a.off_small = a.off_points + 4 * groups * kmeans_stages(D) * 32 * D * 4;
     return a.off_small + small;
