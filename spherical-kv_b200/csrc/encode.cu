@@ -1581,7 +1581,7 @@ extern "C" int sphkv_encode_codes(const void* k_src, int32_t k_dtype, int64_t k_
                       (k_head_stride * esz) % 16 == 0 && a.kbuf_off + staged_bytes <= 227 * 1024;
   const int smem_bytes = a.kbuf_off + (staged ? staged_bytes : 0);
   // The reference's tiers (its first two, or all three) have a kernel of their own: 172 us with the chains, 89 us with branches
-  // and loops over the slots, 79 us with their sums in registers at once, 85 with the wider kGap (32768 fp32 tokens x 8 heads, three tiers).
+  // and loops over the slots, 79 us with their sums in registers at once (32768 fp32 tokens x 8 heads, three tiers).
   using Two = FixedTiers<6, 4, 0>;
   using Three = FixedTiers<6, 4, 3>;
   const int which = !staged ? 0 : Three::match(*tiers, wanted) ? 3 : Two::match(*tiers, wanted) ? 2 : 1;

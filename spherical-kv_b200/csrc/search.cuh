@@ -5,20 +5,22 @@
 // (16-dim group, centroid).  Here the tensor cores compute every product sum from bf16 pairs (key = hi + lo,
 // centroid = hi + lo, three products, fp32 accumulators in tensor memory), a thread looks at its token's row of
 // approximate sums at 2.5 instructions per centroid, and the answer is taken only where the largest one leads by
-// more than twice what the approximation can be off; where it does not (some 0.2 % of the searches) the
+// more than twice what the approximation can be off; where it does not (some 0.1 % of the searches) the
 // chains decide.  The result is that of the chains, bit for bit.
 //
-// Error of an approximate sum, relative to |k| |c|: a value less its two bf16 parts 2^-18, for the key and
-// for the centroid; the product lo * lo that is left out 2^-18; the tensor core's sums of at most 6 x 16 products
-// plus the accumulator, should each lose 2^-22 of the largest, 102 x 2^-22; the chains themselves at most 32 x
-// 2^-24.  Together 3.8e-5, and twice that is below kGap.  Norms outside 2^-30 .. 2^30 (underflow, overflow, infinities,
-// NaN) are never decided here.
+// Error of an approximate sum, relative to |k| |c|: a value less its two bf16 parts 2^-18, for the key and for the
+// centroid; the product lo * lo that is left out 2^-18; the chains themselves at most 32 x 2^-24; and the tensor core's sums.
+// Measured on this part (one term 1, fifteen of 2^-18 .. 2^-29): a product's addends are cut off below 2^-25 of the
+// largest, the sum at fp32, so six products of 16 addends and the accumulator lose at most 6 x (17 x 2^-25 + 2^-23) =
+// 3.8e-6 (seen on random vectors: 2^-21.2).  Together 1.7e-5, and twice that is 0.56 of kGap.  Norms outside 2^-30 .. 2^30
+// (underflow, overflow, infinities, NaN) are never decided here.  With kGap at 2^-13 the chains' extra work takes the
+// code cache of 32768 tokens x 8 heads from 79 to 85 us.
 #pragma once
 #include "tcgen05.cuh"
 
 namespace sphkv {
 
-constexpr float kGap = 1.f / 8192.f;        // lead over the runner-up, relative to |k| max |c|, that settles a search
+constexpr float kGap = 1.f / 16384.f;       // lead over the runner-up, relative to |k| max |c|, that settles a search
 constexpr int kSearchWarps = 4;             // warps of a search group: the 128 lanes (token rows) of tensor memory
 constexpr int kSearchGroups = 2;            // search groups of a CTA
 constexpr int kSearchThreads = kSearchGroups * kSearchWarps * 32;
