@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
           s = __fmaf_rn(v.z, x.z, s);
           s = __fmaf_rn(v.w, x.w, s);
         }
-        a.best_sim[idx] = s;
+        a.best_sim[idx] = s > -INFINITY ? s : -INFINITY;  // a point whose sums are all NaN has none: -inf, as in the chains' kernel
       }
       atomicAdd(&cnt_s[code], 1);
     }

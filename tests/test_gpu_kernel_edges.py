@@ -152,6 +152,28 @@ def test_kmeans_ties_and_special_points(d, K):
     assert torch.equal(counts.long(), torch.bincount(assigns.long(), minlength=K))
 
 
+# both kernels: the chains (few centroids; few points of the largest codebooks) and the tensor-core search
+@pytest.mark.parametrize("d,K", [(8, 47), (8, 64), (16, 16), (16, 64), (16, 200), (32, 8), (32, 64), (32, 128)])
+def test_kmeans_points_that_are_not_finite(d, K):
+    """sums that are NaN never win; a point that has no other gets cluster 0 and a similarity of -inf"""
+    g = torch.Generator(device=DEV).manual_seed(d + K)
+    U = torch.randn(300, d, generator=g, device=DEV)
+    C = torch.randn(K, d, generator=g, device=DEV)
+    C[::3, 2] = 0  # inf * 0 is NaN: such a point has sums of both kinds
+    U[::4, 1] = float("nan")
+    U[1::4, 2] = float("inf")
+    U[2::8, 2] = -float("inf")
+    U[2::16, 5] = float("inf")
+    sims = torch.zeros(300, K, dtype=torch.float64, device=DEV)
+    for i in range(d):  # an fma rounds the exact product and sum once
+        sims = (U[:, i:i + 1].double() * C[:, i].double() + sims).float().double()
+    want = torch.where(sims.isnan(), -torch.inf, sims)
+    assigns, best, _, counts = pkg.kmeans_assign(U, C)
+    first = (want == want.max(1).values[:, None]).int().argmax(1)
+    assert torch.equal(best.double(), want.max(1).values) and torch.equal(assigns.long(), first)
+    assert torch.equal(counts.long(), torch.bincount(first, minlength=K))
+
+
 # the largest codebooks of 32-dim points: eight, then seven sets of sums per CTA
 @pytest.mark.parametrize("K", [172, 173, 179])
 def test_kmeans_largest_codebooks(K):
