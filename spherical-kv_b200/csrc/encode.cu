@@ -1159,8 +1159,10 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
   };
   const uint32_t op = smem_u32(smem);
   Place cur = at0;
+  ProductWaits waits;  // once one ran out the chains decide everything
+  auto wait = [&](uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
   auto products = [&](int ps) {  // of the pair `cur`, by the group's first warp, after the group's barrier
-    if (w != 0) return;
+    if (w != 0 || waits.lost) return;
     tc_fence_after();
     if (elect_one()) {
       const uint32_t keys = tmem + kKeyCols + (cur.q & 1) * 32;
@@ -1208,13 +1210,12 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
     tc_fence_before();
     __syncthreads();
     products(0);
-    bool lost = false;  // a wait for the tensor cores ran out: the chains decide everything from here on
-    uint32_t parity = 0, codes_before[3] = {0, 0, 0};
+    uint32_t codes_before[3] = {0, 0, 0};
     SliceNorms before = {};
     for (int ps = 0;;) {
       const bool last_pass = Fix::kFixed || ps + 1 == a.plan.n_pass;
-      lost = lost || !__all_sync(0xffffffffu, mbar_wait(bar, parity));
-      parity ^= 1;
+      waits.next(wait);
+      const bool lost = waits.lost;
       tc_fence_after();
       const int slice = cur.slice, head = cur.head;
       const int64_t row = cur.row0 + lane;
@@ -1334,7 +1335,7 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
       }
       if (!more) break;
     }
-    if (lost) (void)mbar_wait(bar, parity);
+    if (w == 0) waits.leave(wait);
   }
   cp_async_wait<0>();
   tc_fence_before();

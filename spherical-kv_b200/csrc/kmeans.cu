@@ -307,9 +307,11 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     tmem_wait_st();
     conv_stage = conv_stage + 1 == kStages ? 0 : conv_stage + 1;
   };
+  ProductWaits waits;  // once one ran out the chains decide everything
+  auto wait = [&](uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0; };
   auto products = [&]() {
     asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
-    if (w == 0) {
+    if (w == 0 && !waits.lost) {
       tc_fence_after();
       if (elect_one()) {
         const uint32_t k0 = tmem + a.sum_cols + keys * kKeys;
@@ -336,16 +338,13 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     tc_fence_before();
     products();
   }
-  bool lost = false;  // a wait for the tensor cores ran out: the chains decide everything from here on
-  uint32_t parity = 0;
   int stage = 0;
   for (int64_t base = first; base < a.N; base += stride) {
     const float norm = norm_n;
     const bool more = base + stride < a.N;
     fetch();
     if (more) convert();
-    lost = lost || !__all_sync(0xffffffffu, mbar_wait(bar, parity));
-    parity ^= 1;
+    waits.next(wait);
     tc_fence_after();
     const int64_t idx = base + 32 * w + lane;
     const bool live = idx < a.N;
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     }
     tc_fence_before();
     if (more) products();  // runs while this batch is added up
-    const unsigned open = __ballot_sync(0xffffffffu, live && (lost || !sure));
+    const unsigned open = __ballot_sync(0xffffffffu, live && (waits.lost || !sure));
     const uint32_t rows = points + stage * (32 * D * 4);
     if (open)
       code = exact_search<D>([&](int64_t off, float (&k)[D]) {
@@ -448,7 +447,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     __syncwarp();
     stage = stage + 1 == kStages ? 0 : stage + 1;
   }
-  if (lost) (void)mbar_wait(bar, parity);
+  if (w == 0) waits.leave(wait);
   cp_async_wait<0>();
   tc_fence_before();
   __syncthreads();

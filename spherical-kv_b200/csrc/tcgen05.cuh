@@ -40,6 +40,25 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
+// A warp's waits for products that are issued one batch at a time, each batch completing one phase of a barrier.  After a wait
+// that ran out the warp waits for no later phase, and the warp that issues the batches issues no more (`lost`): the phase of
+// `parity` is then the last one that anything can still complete, and leave() awaits it, within the same bound, before the
+// CTA's shared and tensor memory are given back.
+struct ProductWaits {
+  uint32_t parity = 0;
+  bool lost = false;
+#pragma nv_exec_check_disable
+  template <typename Wait>
+  __host__ __device__ __forceinline__ void next(Wait wait) {
+    if (!lost) lost = !wait(parity);
+    if (!lost) parity ^= 1;
+  }
+#pragma nv_exec_check_disable
+  template <typename Wait>
+  __host__ __device__ __forceinline__ void leave(Wait wait) const {
+    if (lost) (void)wait(parity);
+  }
+};
 // arrives on `bar` once this thread's earlier cp.async copies have landed
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
