@@ -1178,6 +1178,7 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
           mma_ts(d, keys + 8 * half, hi, k16, false);
           if (lows) mma_ts(d, keys + 16 + 8 * half, hi, k16, true);
           mma_ts(d, keys + 8 * half, hi + kLo, k16, true);
+          if (lows) mma_ts(d, keys + 16 + 8 * half, hi + kLo, k16, true);
         }
         if constexpr (Fix::C2 > 0) {
 #pragma unroll
@@ -1187,6 +1188,7 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
             mma_ts(d, keys + 8 * half, hi, k32, half > 0);
             if (lows) mma_ts(d, keys + 16 + 8 * half, hi, k32, true);
             mma_ts(d, keys + 8 * half, hi + kLo, k32, true);
+            if (lows) mma_ts(d, keys + 16 + 8 * half, hi + kLo, k32, true);
           }
         }
       } else {

@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
           mma_ts(tmem, k0 + 8 * kc, hi, idesc, kc > 0);
           mma_ts(tmem, k0 + kKeys / 2 + 8 * kc, hi, idesc, true);
           mma_ts(tmem, k0 + 8 * kc, lo, idesc, true);
+          mma_ts(tmem, k0 + kKeys / 2 + 8 * kc, lo, idesc, true);
         }
         mma_commit(bar);
       }

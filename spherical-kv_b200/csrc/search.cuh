@@ -3,24 +3,28 @@
 // What the encoders and k-means promise is the first maximum of fp32 fma chains (k . c over d = 0 .. g-1 from
 // 0).  As chains on the fp32 pipe the search costs 16 fmas and three compare / select instructions per
 // (16-dim group, centroid).  Here the tensor cores compute every product sum from bf16 pairs (key = hi + lo,
-// centroid = hi + lo, three products, fp32 accumulators in tensor memory), a thread looks at its token's row of
+// centroid = hi + lo, four products, fp32 accumulators in tensor memory), a thread looks at its token's row of
 // approximate sums at 2.5 instructions per centroid, and the answer is taken only where the largest one leads by
 // more than twice what the approximation can be off; where it does not (some 0.1 % of the searches) the
 // chains decide.  The result is that of the chains, bit for bit.
 //
-// Error of an approximate sum, relative to |k| |c|: a value less its two bf16 parts 2^-18, for the key and for the
-// centroid; the product lo * lo that is left out 2^-18; the chains themselves at most 32 x 2^-24; and the tensor core's sums.
-// Measured on this part (one term 1, fifteen of 2^-18 .. 2^-29): a product's addends are cut off below 2^-25 of the
-// largest, the sum at fp32, so six products of 16 addends and the accumulator lose at most 6 x (17 x 2^-25 + 2^-23) =
-// 3.8e-6 (seen on random vectors: 2^-21.2).  Together 1.7e-5, and twice that is 0.56 of kGap.  Norms outside 2^-30 .. 2^30
-// (underflow, overflow, infinities, NaN) are never decided here.  With kGap at 2^-13 the chains' extra work takes the
-// code cache of 32768 tokens x 8 heads from 79 to 85 us.
+// Error of an approximate sum, relative to |k| |c| (Cauchy-Schwarz over the dims): a value less its two bf16 parts
+// (kPairError), for the key and for the centroid; the chains' own rounding (kChainError); and the tensor core's sums (kSumError).
+// Twice all of it is 0.98 kGap; without the product lo * lo, up to 2^-16, it would be 1.6 kGap.  The tensor core, measured on this part
+// (one term 1, fifteen of 2^-18 .. 2^-29): a product's addends are cut off below 2^-25 of the largest, the sum at
+// fp32, so a product of 16 addends and the accumulator lose at most 17 x 2^-25 + 2^-23 (seen on random vectors: 2^-21.2 in
+// all).  Norms outside 2^-30 .. 2^30 (underflow, overflow, infinities, NaN) are never decided here.
 #pragma once
 #include "tcgen05.cuh"
 
 namespace sphkv {
 
-constexpr float kGap = 1.f / 16384.f;       // lead over the runner-up, relative to |k| max |c|, that settles a search
+constexpr float kGap = 3.f / 65536.f;       // lead over the runner-up, relative to |k| max |c|, that settles a search
+constexpr double kPairError = 1. / (1 << 17);                                // half a place of lo, which is at most 2^-8
+constexpr double kSumError = 8 * (17. / (1 << 25) + 1. / (1 << 23));         // four products of two halves of 32 dims
+constexpr double kChainError = 32. / (1 << 24);
+constexpr double kRestError = 1. / (1 << 23);                                // of norms, t and products of two remainders
+static_assert(2 * (2 * kPairError + kSumError + kChainError + kRestError) < kGap, "the lead covers both sums' errors");
 constexpr int kSearchWarps = 4;             // warps of a search group: the 128 lanes (token rows) of tensor memory
 constexpr int kSearchGroups = 2;            // search groups of a CTA
 constexpr int kSearchThreads = kSearchGroups * kSearchWarps * 32;
@@ -28,7 +32,7 @@ constexpr int kGroupCols = 256;             // tensor memory columns of a group 
 constexpr int kSumCols = 192;               // ... of which the sums take up to 192,
 constexpr int kKeyCols = 192;               // and two buffers of 32 the key pairs of a 32-dim slice (hi x 16 | lo x 16)
 
-// bf16 pairs of N fp32 values: hi = rounded, lo = rounded rest; word i holds values 2 i and 2 i + 1
+// bf16 pairs of N fp32 values: hi = rounded, lo = rounded rest (off by kPairError at most); word i holds values 2 i and 2 i + 1
 template <int N>
 __device__ __forceinline__ void split_pairs(const float (&k)[N], uint32_t (&hi)[N / 2], uint32_t (&lo)[N / 2]) {
 #pragma unroll
@@ -327,6 +331,7 @@ __device__ __forceinline__ void issue_products(const SearchPlan& pl, const sphkv
     mma_ts(d, keys + 8 * half, hi, idesc, more);
     if (lows) mma_ts(d, keys + 16 + 8 * half, hi, idesc, true);
     mma_ts(d, keys + 8 * half, lo, idesc, true);
+    if (lows) mma_ts(d, keys + 16 + 8 * half, lo, idesc, true);
   };
   const int n16 = pl.n16[ps];
   if (n16 > 0)

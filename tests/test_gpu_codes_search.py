@@ -30,6 +30,9 @@ def keys(kind, rows, hkv, dh, cbs, g):
         pick = lambda n: torch.take_along_dim(c[None].expand(rows, -1, -1, -1, -1), n, 3)[:, :, :, 0]  # noqa: E731
         eps = torch.randint(-3, 4, (rows, hkv, G, 1), generator=g, device=DEV) * 2.0 ** -23
         k = (pick(i) * (1 + eps) + pick(j)).reshape(rows, hkv, dh)
+    elif kind == "worst mantissas":  # where a value is farthest from its bf16 pair; sums around 0, relative to the norms
+        k = (1 + 2.0 ** -8 - 2.0 ** -16 + 2.0 ** -17) * torch.randint(0, 2, k.shape, generator=g, device=DEV).float().mul(2).sub(1)
+        k *= 2.0 ** torch.randint(-2, 3, (rows, hkv, 1), generator=g, device=DEV).float()
     elif kind == "zeros":
         k[::3] = 0
         k[1::3, :, ::2] = 0
@@ -42,7 +45,7 @@ def keys(kind, rows, hkv, dh, cbs, g):
     return k
 
 
-@pytest.mark.parametrize("kind", ["random", "near ties", "zeros", "scales", "not finite"])
+@pytest.mark.parametrize("kind", ["random", "near ties", "worst mantissas", "zeros", "scales", "not finite"])
 @pytest.mark.parametrize("tiers", SETS)
 @pytest.mark.parametrize("dh,rows,dtype", [(128, 129, torch.float32), (64, 300, torch.float32), (128, 127, torch.bfloat16),
                                            (64, 128, torch.float16)])
@@ -53,6 +56,10 @@ def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
     for t in specs:
         c = torch.randn(hkv, dh // t.g, t.codebook_size, t.g, generator=g, device=DEV)
         cbs.append(c / c.norm(dim=-1, keepdim=True))
+    if kind == "worst mantissas":
+        for c in cbs:
+            c[:] = (1 + 2.0 ** -8 - 2.0 ** -16 + 2.0 ** -17) * torch.randint(0, 2, c.shape, generator=g, device=DEV).float().mul(2).sub(1)
+            c[:, :, 1::2] = -c[:, :, ::2] * (1 + 2.0 ** -7 * torch.randint(0, 2, c[:, :, ::2].shape, generator=g, device=DEV))
     cbs[0][:, 0, -1] = cbs[0][:, 0, 0]  # two equal centroids, and one of zeros
     cbs[0][:, 1, 0] = 0
     ts = pkg.TierSet(dh, specs)
