@@ -1017,13 +1017,30 @@ __device__ __forceinline__ void store_groups(float* r, uint8_t* theta, int count
   }
 }
 
-// the fma chains' answer for the lanes in `open`: group `gamma` of key row `row`
+// The fma chains' answer for the lanes in `open`: group `gamma` of key row `row`; kFirstWins (low byte 0) for a vector of zeros, or
+// with a NaN, where many lanes are open.  Bound by what it reads: keys and centroids come from L2, row by row.  32768 tokens x 8 heads,
+// three tiers, by the data (every lane walking all centroids of an open search before / now / the chains' kernel): random 76 / 77 / 170
+// us; a third of the keys' mean as spread 124 / 114 / 170, a tenth 396 / 227 / 170; zeros 870 / 140 / 174; every search a tie
+// 865 / 790 / 170.  Columns instead of lanes (as k-means does) take registers that the searches need: 81 to 92 us for random keys.
+constexpr int kFirstWins = 256;
 template <int GS>
 __device__ __noinline__ int settle(const CodesArgs& p, int head, int s, int gamma, int64_t row, unsigned open, int code) {
   const sphkv_tiers& t = p.tiers;
   const float* cb = p.codebooks + (((int64_t)(head * t.n_slots + s) * t.G_max + gamma) * t.C_max) * t.g_max;
-  return exact_search<GS>([&](int64_t off, float (&k)[GS]) { load_group<GS>(p.k_src, p.k_dtype, off, k); },
-                          row * p.k_row_stride + (int64_t)head * p.k_head_stride + gamma * GS, cb, t.g_max, 1 << t.bits[s], open, code);
+  float k[GS];
+  if ((open >> (threadIdx.x & 31)) & 1u) {
+    load_group<GS>(p.k_src, p.k_dtype, row * p.k_row_stride + (int64_t)head * p.k_head_stride + gamma * GS, k);
+  } else {
+#pragma unroll
+    for (int d = 0; d < GS; ++d) k[d] = 0.f;
+  }
+  if (__popc(open) > 4) {
+    const bool first = ((open >> (threadIdx.x & 31)) & 1u) && first_wins(k, cb);
+    if (first) code = kFirstWins;
+    open &= ~__ballot_sync(0xffffffffu, first);
+    if (open == 0) return code;
+  }
+  return exact_search(k, cb, t.g_max, 1 << t.bits[s], open, code);
 }
 
 constexpr int kCodeStages = 4;                                  // slices in flight
@@ -1224,8 +1241,8 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
       const bool have = row < a.rows;
       constexpr int kC0 = Fix::kFixed ? Fix::C0 : 16, kC1 = Fix::C1 ? Fix::C1 : 16, kC2 = Fix::C2 ? Fix::C2 : 16;
       float s0a[kC0 < 16 ? 16 : kC0], s0b[kC0 < 16 ? 16 : kC0], s1a[kC1 < 16 ? 16 : kC1], s1b[kC1 < 16 ? 16 : kC1], s2[kC2 < 16 ? 16 : kC2];
-      float2 far0, far1;
-      float far2;
+      float2 far0 = {}, far1 = {};
+      float far2 = 0.f;
       if constexpr (Fix::kFixed) {
         tmem_ld_row<kC0>(my_rows, s0a);
         tmem_ld_row<kC0>(my_rows + Fix::kHalf, s0b);
@@ -1253,10 +1270,10 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
           if (__any_sync(0xffffffffu, have && (lost || !(sa && sb)))) {
             const unsigned open_a = __ballot_sync(0xffffffffu, have && (lost || !sa)), open_b = __ballot_sync(0xffffffffu, have && (lost || !sb));
             if (two) {
-              if (open_a) ca = settle<16>(a, head, s, 2 * slice, row, open_a, ca);
-              if (open_b) cb = settle<16>(a, head, s, 2 * slice + 1, row, open_b, cb);
+              if (open_a) ca = settle<16>(a, head, s, 2 * slice, row, open_a, ca) & 255;
+              if (open_b) cb = settle<16>(a, head, s, 2 * slice + 1, row, open_b, cb) & 255;
             } else {
-              ca = settle<32>(a, head, s, slice, row, open_a, ca);
+              ca = settle<32>(a, head, s, slice, row, open_a, ca) & 255;
             }
           }
           if (have) {
@@ -1297,16 +1314,20 @@ __global__ void __launch_bounds__(kSearchThreads, 1) encode_codes_kernel(const _
         }
         if constexpr (Fix::C2 > 0) sure[4] = nearest_column<kC2>(s2, n0.ab, far2, c[4]);
         if (__any_sync(0xffffffffu, have && (lost || !(sure[0] && sure[1] && sure[2] && sure[3] && sure[4])))) {
+          const float far[5] = {far0.x, far0.y, far1.x, far1.y, far2};
+          int firsts = 0;
 #pragma unroll
           for (int i = 0; i < 5; ++i) {
             const int s = i == 4 ? Fix::kSlots - 1 : i >> 1;
             if ((i >= 2 && i < 4 && Fix::C1 == 0) || (i == 4 && Fix::C2 == 0)) continue;
-            const unsigned open = __ballot_sync(0xffffffffu, have && (lost || !sure[i]));
+            // what the first slot's searches found of zeros holds for the others, if their centroids are finite
+            const bool first = i >= 2 && far[i] > 0.f && (i == 4 ? firsts == 3 : (firsts >> (i & 1) & 1) != 0);
+            if (first) c[i] = 0;
+            const unsigned open = __ballot_sync(0xffffffffu, have && (lost || !sure[i]) && !first);
             if (open) {
-              if (i == 4)
-                c[i] = settle<32>(a, head, s, slice, row, open, c[i]);
-              else
-                c[i] = settle<16>(a, head, s, 2 * slice + (i & 1), row, open, c[i]);
+              const int found = i == 4 ? settle<32>(a, head, s, slice, row, open, c[i]) : settle<16>(a, head, s, 2 * slice + (i & 1), row, open, c[i]);
+              c[i] = found & 255;
+              if (i < 2) firsts |= (found >> 8 & 1) << i;
             }
           }
         }

@@ -188,6 +188,130 @@ __device__ __forceinline__ float lds_f1(uint32_t addr) {
   return v;
 }
 
+// The vote of search.cuh with the columns above t as bits, up to 24 to a float (exact sums): where there are more than one, it says
+// which the chains have to decide between.  1M points of 16 dims, K 64, all centroids for an open point before / now / the chains'
+// kernel: random 45 / 46 / 72 us, a tenth of the points' mean as spread 79 / 53 / 72, zeros 125 / 50 / 72, all centroids equal
+// 123 / 123 / 72.  (The code cache's kernel has no registers for these.)
+template <int C>
+struct Leaders {
+  static constexpr int kParts = (C + 23) / 24;
+  float part[kParts];  // bit c - 24 i of part i: column c is above t; part 0 is NaN where this cannot be said
+};
+template <int C>
+__device__ __forceinline__ void find_leaders(const float (&v)[C < 16 ? 16 : C], const Lead& l, Leaders<C>& who) {
+  constexpr int kSums = Leaders<C>::kParts > 1 ? 2 : 4;  // chains of a part
+  float sum[Leaders<C>::kParts][kSums] = {};
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    float& to = sum[c / 24][c & (kSums - 1)];
+    to = __fmaf_rn(__saturatef(__fmaf_rn(v[c], l.scale, l.shift)), (float)(1 << c % 24), to);
+  }
+#pragma unroll
+  for (int i = 0; i < Leaders<C>::kParts; ++i) {
+    if constexpr (kSums == 4)
+      who.part[i] = (sum[i][0] + sum[i][1]) + (sum[i][2] + sum[i][3]);
+    else
+      who.part[i] = sum[i][0] + sum[i][1];
+  }
+  if (!l.fit) who.part[0] = __int_as_float(0x7fc00000);
+}
+// one leader: one part that is not 0 (their sum is the largest of them: parts are whole and below 2^24), and it a power of two,
+// whose exponent is the leader's number
+template <int C>
+__device__ __forceinline__ bool one_leader(const Leaders<C>& who, int& code) {
+  float one = who.part[0];
+  bool single = true;
+  if constexpr (Leaders<C>::kParts == 2) {
+    single = who.part[0] + who.part[1] == fmaxf(who.part[0], who.part[1]);
+    one = __fmaf_rn(who.part[1], 16777216.f, one);
+  } else if constexpr (Leaders<C>::kParts == 3) {
+    single = (who.part[0] + who.part[1]) + who.part[2] == max3(who.part[0], who.part[1], who.part[2]);
+    one = __fmaf_rn(who.part[2], 281474976710656.f, __fmaf_rn(who.part[1], 16777216.f, one));
+  }
+  code = (__float_as_int(one) >> 23) - 127;
+  return single && (__float_as_int(one) & 0x7fffff) == 0;  // (the NaN's has bits there)
+}
+// those columns, or all where the sums do not say (`lost`: they are not there)
+template <int C>
+__device__ __forceinline__ uint64_t open_columns(const Leaders<C>& who, bool lost) {
+  if (lost || who.part[0] != who.part[0]) return ~0ull >> (64 - C);
+  uint64_t open = 0;
+#pragma unroll
+  for (int i = 0; i < Leaders<C>::kParts; ++i) open |= (uint64_t)(uint32_t)who.part[i] << (24 * i);
+  return open;
+}
+
+// The chains of N centroids side by side
+template <int N, int GS>
+__device__ __forceinline__ void chains(const float (&k)[GS], const float* __restrict__ cb, int pitch, const int (&c)[N], float (&sum)[N]) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) sum[j] = 0.f;
+#pragma unroll
+  for (int i = 0; i < GS / 4; ++i)
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float4 x = *reinterpret_cast<const float4*>(cb + c[j] * pitch + 4 * i);
+      sum[j] = __fmaf_rn(k[4 * i], x.x, sum[j]);
+      sum[j] = __fmaf_rn(k[4 * i + 1], x.y, sum[j]);
+      sum[j] = __fmaf_rn(k[4 * i + 2], x.z, sum[j]);
+      sum[j] = __fmaf_rn(k[4 * i + 3], x.w, sum[j]);
+    }
+}
+// the first maximum of all C (past the end the last one again, which is not larger than itself)
+template <int GS>
+__device__ __forceinline__ int walk_all(const float (&k)[GS], const float* __restrict__ cb, int pitch, int C) {
+  constexpr int N = GS < 32 ? 4 : 2;
+  float best = -INFINITY;
+  int code = 0;
+#pragma unroll 1
+  for (int c0 = 0; c0 < C; c0 += N) {
+    int c[N];
+    float sum[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) c[j] = min(c0 + j, C - 1);
+    chains(k, cb, pitch, c, sum);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (sum[j] > best) { best = sum[j]; code = c[j]; }
+  }
+  return code;
+}
+// the same among the columns c0 + (bits of `open`), two at a time (bits ascend: the first maximum stays the first)
+template <int GS, typename Bits>
+__device__ __forceinline__ void walk_open(const float (&k)[GS], const float* __restrict__ cb, int pitch, int c0, Bits open, float& best, int& code) {
+#pragma unroll 1
+  while (open) {
+    int c[2];
+    float sum[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int at = sizeof(Bits) == 8 ? __ffsll((long long)open) : __ffs((int)open);
+      c[j] = at > 0 ? c0 + at - 1 : c[0];
+      open &= open - 1;
+    }
+    chains(k, cb, pitch, c, sum);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (sum[j] > best) { best = sum[j]; code = c[j]; }
+  }
+}
+// a lane's point k, with the columns `open`
+template <int GS>
+__device__ __forceinline__ int settle_point(const float (&k)[GS], const float* __restrict__ cb, int pitch, int C, uint64_t open, int code) {
+  if (open && first_wins(k, cb)) {
+    code = 0;
+    open = 0;
+  }
+  if (__any_sync(0xffffffffu, __popcll(open) > 8)) {
+    if (open) code = walk_all(k, cb, pitch, C);
+  } else if (open) {
+    float best = -INFINITY;
+    code = 0;
+    walk_open(k, cb, pitch, 0, open, best, code);
+  }
+  return code;
+}
+
 // Bound: latency -- twelve warps an SM, each with a chain of tensor memory, shared-memory adds and a barrier per batch; DRAM at
 // 30 % of the copy rate.  4M points, d 16, K 64: 255 us with the chains, 170 here, 148 without bank conflicts on the winners.
 // A CTA has up to three search groups (four warps, thread = point = lane of tensor memory), each striding over batches
@@ -349,20 +473,36 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
     tc_fence_after();
     const int64_t idx = base + 32 * w + lane;
     const bool live = idx < a.N;
+    const uint32_t rows = points + stage * (32 * D * 4);
+    auto load = [&](float (&k)[D]) {
+#pragma unroll
+      for (int q = 0; q < kRowChunks; ++q) {
+        const float4 v = lds_f4(rows + lane * (D * 4) + ((q ^ turn(lane)) << 4));
+        k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+      }
+    };
     int code;
-    bool sure;
     auto whole = [&](auto n) {  // all sums of a point at once
       constexpr int C = decltype(n)::value;
       float v[C < 16 ? 16 : C];
+      Leaders<C> who;
       tmem_ld_row<C>(my_rows, v);
       tmem_wait_ld();
-      sure = nearest_column<C>(v, norm, most, code);
+      find_leaders<C>(v, lead_of(largest_of<C>(v), norm, most), who);
+      const bool unsure = live && !(one_leader<C>(who, code) && !waits.lost);
+      tc_fence_before();
+      if (more) products();  // runs while this batch is added up
+      if (__any_sync(0xffffffffu, unsure)) {
+        float k[D];
+        load(k);
+        code = settle_point(k, c_s, kPitch, K, unsure ? open_columns<C>(who, waits.lost) : 0, code);
+      }
     };
     if (K == 64) {
       whole(std::integral_constant<int, 64>());
-    } else if (K == 16) {
+    } else if (D == 32 && K == 16) {  // (points of fewer dims come with more centroids)
       whole(std::integral_constant<int, 16>());
-    } else if (K == 8) {
+    } else if (D == 32 && K == 8) {
       whole(std::integral_constant<int, 8>());
     } else {  // sixteen columns at a time, twice: the largest, then what comes near it
       float top = -INFINITY;
@@ -381,30 +521,45 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
         top = fmaxf(top, largest_of<16>(v));
       }
       const Lead l = lead_of(top, norm, most);
-      float all = 0.f;
+      Leaders<16> who = {{0.f}};
       int base_of = 0;
+      uint32_t blocks = 0;  // of sixteen columns, with some above t
       for (int c0 = 0; c0 < K; c0 += 16) {
         float v[16];
         columns(c0, v);
-        const float some = count_leaders<16>(v, l);
-        all += some;
-        if (some > 0.f) base_of = c0;
+        Leaders<16> some;
+        find_leaders<16>(v, l, some);
+        if (!(some.part[0] == 0.f)) { who = some; base_of = c0; blocks |= 1u << (c0 >> 4); }
       }
-      code = leader_of(all) + base_of;
-      sure = l.fit && one_leader(all);
-    }
-    tc_fence_before();
-    if (more) products();  // runs while this batch is added up
-    const unsigned open = __ballot_sync(0xffffffffu, live && (waits.lost || !sure));
-    const uint32_t rows = points + stage * (32 * D * 4);
-    if (open)
-      code = exact_search<D>([&](int64_t off, float (&k)[D]) {
-#pragma unroll
-        for (int q = 0; q < kRowChunks; ++q) {
-          const float4 v = *reinterpret_cast<const float4*>(a.U + off + 4 * q);
-          k[4 * q] = v.x; k[4 * q + 1] = v.y; k[4 * q + 2] = v.z; k[4 * q + 3] = v.w;
+      const bool one = one_leader<16>(who, code) && (blocks & (blocks - 1)) == 0;
+      code += base_of;
+      bool unsure = live && !(one && !waits.lost);
+      if (__any_sync(0xffffffffu, unsure)) {
+        float k[D];
+        load(k);
+        if (unsure && first_wins(k, c_s)) {
+          code = 0;
+          unsure = false;
         }
-      }, idx * D, c_s, kPitch, K, open, code);
+        bool walk = unsure && (waits.lost || !l.fit);
+        int n_open = 0;
+        float best = -INFINITY;
+        for (uint32_t todo = __reduce_or_sync(0xffffffffu, unsure ? blocks : 0u); todo && !__any_sync(0xffffffffu, walk); todo &= todo - 1) {
+          const int c0 = 16 * (__ffs((int)todo) - 1);
+          float v[16];
+          columns(c0, v);
+          Leaders<16> some;
+          find_leaders<16>(v, l, some);
+          const uint32_t above = unsure ? (uint32_t)some.part[0] : 0u;
+          n_open += __popc(above);
+          walk = n_open > 32;  // all are as fast one after the other
+          if (!__any_sync(0xffffffffu, walk)) walk_open(k, c_s, kPitch, c0, above, best, code);
+        }
+        if (__any_sync(0xffffffffu, walk) && unsure) code = walk_all(k, c_s, kPitch, K);
+      }
+      tc_fence_before();
+      if (more) products();
+    }
     if (!live) code = 0;
     if (live) {
       a.assigns[idx] = code;

@@ -163,55 +163,95 @@ __device__ __forceinline__ SliceNorms store_slice(const float (&k)[32], uint32_t
   return n;
 }
 
-// The chains themselves, for the lanes in `todo` (warp-uniform).  `k_off` = element offset of a lane's group vector,
-// `cb` = the group's centroids, `pitch` floats apart.  Few lanes: the warp spreads one lane's centroids; many (keys
-// of zeros, equal centroids): every lane walks its own.  Returns a lane's code, or `code` where it has nothing to do.
-template <int GS, typename Load>
-__device__ __forceinline__ int exact_search(Load load, int64_t k_off, const float* __restrict__ cb, int pitch, int C, unsigned todo,
-                                            int code) {
-  const int lane = threadIdx.x & 31;
-  float k[GS];
-  auto chain = [&](int c) {
-    const float4* row = reinterpret_cast<const float4*>(cb + (int64_t)c * pitch);
-    float s = 0.f;
+// Number 0 whatever the chains say: a vector with a NaN has NaN sums only, which never win, and one of zeros has sums of zero, or NaN
+// with centroids that are not finite (the first one is looked at).  Padding is such vectors, and whole warps of them.
+template <int GS>
+__device__ __forceinline__ bool first_wins(const float (&k)[GS], const float* __restrict__ cb) {
+  uint32_t largest = 0;
 #pragma unroll
-    for (int i = 0; i < GS / 4; ++i) {
-      const float4 x = row[i];
-      s = __fmaf_rn(k[4 * i], x.x, s);
-      s = __fmaf_rn(k[4 * i + 1], x.y, s);
-      s = __fmaf_rn(k[4 * i + 2], x.z, s);
-      s = __fmaf_rn(k[4 * i + 3], x.w, s);
-    }
-    return s;
-  };
-  if (__popc(todo) > 6) {
-    if ((todo >> lane) & 1u) {
-      load(k_off, k);
-      float best = -INFINITY;
-      code = 0;
-#pragma unroll 2
-      for (int c = 0; c < C; ++c) {
-        const float s = chain(c);
-        if (s > best) { best = s; code = c; }
+  for (int d = 0; d < GS; ++d) largest = max(largest, __float_as_uint(k[d]) & 0x7fffffffu);
+  float sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < GS / 4; ++i) {
+    const float4 x = reinterpret_cast<const float4*>(cb)[i];
+    sum = __fmaf_rn(0.f, x.x, __fmaf_rn(0.f, x.y, __fmaf_rn(0.f, x.z, __fmaf_rn(0.f, x.w, sum))));
+  }
+  return largest == 0 ? sum == 0.f : largest > 0x7f800000u;
+}
+
+// sums as integers of the same order; NaN, which never wins, as -inf
+__device__ __forceinline__ int ordered(float s) {
+  const int i = __float_as_int(s == s ? s + 0.f : -INFINITY);  // (-0 + 0 = 0)
+  return i ^ ((i >> 31) & 0x7fffffff);
+}
+// The chains themselves, for the lanes in `todo` (warp-uniform); k = a lane's group vector, `cb` = the group's centroids, `pitch`
+// floats apart.  Lane after lane: the warp's lanes hold centroids in registers and get the vectors by
+// shuffles.  More lanes than centroids: every lane walks the centroids for itself.  Returns a lane's code, or `code` where it
+// has nothing to do.
+template <int GS>
+__device__ __forceinline__ int exact_search(const float (&k)[GS], const float* __restrict__ cb, int pitch, int C, unsigned todo, int code) {
+  constexpr int kRows = GS >= 32 ? 1 : 2;  // centroids a lane holds
+  const int lane = threadIdx.x & 31;
+  const bool mine = (todo >> lane) & 1u;
+  int best = ordered(-INFINITY);
+  if (mine) code = 0;
+  if (__popc(todo) > C) {
+    if (mine) {
+#pragma unroll 1
+      for (int c0 = 0; c0 < C; c0 += 2) {
+        const int c1 = min(c0 + 1, C - 1);
+        const float4* row0 = reinterpret_cast<const float4*>(cb + c0 * pitch);
+        const float4* row1 = reinterpret_cast<const float4*>(cb + c1 * pitch);
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < GS / 4; ++i) {
+          const float4 x = row0[i], y = row1[i];
+          s0 = __fmaf_rn(k[4 * i], x.x, s0);
+          s1 = __fmaf_rn(k[4 * i], y.x, s1);
+          s0 = __fmaf_rn(k[4 * i + 1], x.y, s0);
+          s1 = __fmaf_rn(k[4 * i + 1], y.y, s1);
+          s0 = __fmaf_rn(k[4 * i + 2], x.z, s0);
+          s1 = __fmaf_rn(k[4 * i + 2], y.z, s1);
+          s0 = __fmaf_rn(k[4 * i + 3], x.w, s0);
+          s1 = __fmaf_rn(k[4 * i + 3], y.w, s1);
+        }
+        const int v0 = ordered(s0), v1 = ordered(s1);
+        if (v0 > best) { best = v0; code = c0; }
+        if (v1 > best) { best = v1; code = c1; }
       }
     }
     return code;
   }
-  while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    load(__shfl_sync(0xffffffffu, k_off, src), k);
-    float best = -INFINITY;
-    int at = 0x7fffffff;
-    for (int c = lane; c < C; c += 32) {  // ascending per lane; sums that are NaN never win
-      const float s = chain(c);
-      if (s > best) { best = s; at = c; }
-    }
-    float top = best;
+#pragma unroll 1
+  for (int c0 = 0; c0 < C; c0 += 32 * kRows) {
+    float x[kRows][GS];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    const int first = __reduce_min_sync(0xffffffffu, best == top ? at : 0x7fffffff);
-    if (lane == src) code = first == 0x7fffffff ? 0 : first;
+    for (int r = 0; r < kRows; ++r) {  // (past the end the last one again: the first lane of equal sums counts)
+      const float4* row = reinterpret_cast<const float4*>(cb + min(c0 + 32 * r + lane, C - 1) * pitch);
+#pragma unroll
+      for (int i = 0; i < GS / 4; ++i) {
+        const float4 v = row[i];
+        x[r][4 * i] = v.x; x[r][4 * i + 1] = v.y; x[r][4 * i + 2] = v.z; x[r][4 * i + 3] = v.w;
+      }
+    }
+#pragma unroll 1
+    for (unsigned left = todo; left; left &= left - 1) {
+      const int src = __ffs((int)left) - 1;
+      float s[kRows];
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) s[r] = 0.f;
+#pragma unroll
+      for (int d = 0; d < GS; ++d) {
+        const float q = __shfl_sync(0xffffffffu, k[d], src);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) s[r] = __fmaf_rn(q, x[r][d], s[r]);
+      }
+      const int v0 = ordered(s[0]), v1 = kRows > 1 ? ordered(s[kRows - 1]) : v0;
+      const int top = __reduce_max_sync(0xffffffffu, max(v0, v1));
+      const unsigned in0 = __ballot_sync(0xffffffffu, v0 == top), in1 = __ballot_sync(0xffffffffu, v1 == top);
+      const int at = c0 + (in0 ? __ffs((int)in0) - 1 : 31 + __ffs((int)in1));
+      if (lane == src && top > best) { best = top; code = at; }
+    }
   }
   return code;
 }

@@ -33,6 +33,10 @@ def keys(kind, rows, hkv, dh, cbs, g):
     elif kind == "worst mantissas":  # where a value is farthest from its bf16 pair; sums around 0, relative to the norms
         k = (1 + 2.0 ** -8 - 2.0 ** -16 + 2.0 ** -17) * torch.randint(0, 2, k.shape, generator=g, device=DEV).float().mul(2).sub(1)
         k *= 2.0 ** torch.randint(-2, 3, (rows, hkv, 1), generator=g, device=DEV).float()
+    elif kind == "cone":  # most lanes of a warp open, each with a few columns
+        k = 1 + 0.03 * k
+    elif kind == "padding":  # whole warps of zeros
+        k[rows // 3:] = 0
     elif kind == "zeros":
         k[::3] = 0
         k[1::3, :, ::2] = 0
@@ -45,7 +49,7 @@ def keys(kind, rows, hkv, dh, cbs, g):
     return k
 
 
-@pytest.mark.parametrize("kind", ["random", "near ties", "worst mantissas", "zeros", "scales", "not finite"])
+@pytest.mark.parametrize("kind", ["random", "near ties", "worst mantissas", "cone", "padding", "zeros", "scales", "not finite"])
 @pytest.mark.parametrize("tiers", SETS)
 @pytest.mark.parametrize("dh,rows,dtype", [(128, 129, torch.float32), (64, 300, torch.float32), (128, 127, torch.bfloat16),
                                            (64, 128, torch.float16)])
@@ -55,6 +59,8 @@ def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
     cbs = []
     for t in specs:
         c = torch.randn(hkv, dh // t.g, t.codebook_size, t.g, generator=g, device=DEV)
+        if kind == "cone":
+            c = 1 + 0.03 * c
         cbs.append(c / c.norm(dim=-1, keepdim=True))
     if kind == "worst mantissas":
         for c in cbs:
@@ -62,6 +68,8 @@ def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
             c[:, :, 1::2] = -c[:, :, ::2] * (1 + 2.0 ** -7 * torch.randint(0, 2, c[:, :, ::2].shape, generator=g, device=DEV))
     cbs[0][:, 0, -1] = cbs[0][:, 0, 0]  # two equal centroids, and one of zeros
     cbs[0][:, 1, 0] = 0
+    if kind == "padding":
+        cbs[-1][:, :, 0, 0] = float("inf")  # its sum with zeros is NaN: the next centroid is the first maximum
     ts = pkg.TierSet(dh, specs)
     cb = ts.pack_codebooks(cbs)
     K = keys(kind, rows, hkv, dh, cbs, g).to(dtype)
@@ -71,3 +79,23 @@ def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
         want = pkg.encode_pages(K, None, lists, cb, ts, use_scratch=False)
         got = pkg.pages_from_codes(codes, None, lists, cb)
         assert torch.equal(got.k_pages, want.k_pages)
+
+
+def test_padding_costs_no_more_than_keys():
+    """whole warps of undecided searches: 11 times the time of random keys when every lane walked all centroids"""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    ts = pkg.TierSet(128, REF)
+    cb = ts.pack_codebooks(pkg.synth.make_codebooks(8, 128, REF, seed=2)).to(DEV)
+    K = torch.randn(16384, 8, 128, generator=g, device=DEV)
+
+    def us(k):
+        events = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        times = []
+        for _ in range(8):
+            events[0].record()
+            pkg.encode_codes(k, cb, ts)
+            events[1].record()
+            events[1].synchronize()
+            times.append(events[0].elapsed_time(events[1]))
+        return min(times)
+    assert us(torch.zeros_like(K)) <= 4 * us(K)

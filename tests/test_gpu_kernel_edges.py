@@ -152,6 +152,39 @@ def test_kmeans_ties_and_special_points(d, K):
     assert torch.equal(counts.long(), torch.bincount(assigns.long(), minlength=K))
 
 
+def test_kmeans_kernels_agree_bit_for_bit():
+    """one point more, and the tensor-core search takes the call: ties, narrow cones, zeros and all, the chains' answers"""
+    g = torch.Generator(device=DEV).manual_seed(7)
+    U = torch.randn(200000, 32, generator=g, device=DEV)
+    U[1::4] = 1 + 0.02 * U[1::4]
+    C = U[torch.randint(200000, (128,), generator=g, device=DEV)].clone()
+    C[::9] = C[5]
+    U[2::4] = C[torch.randint(128, (50000,), generator=g, device=DEV)] + C[torch.randint(128, (50000,), generator=g, device=DEV)]
+    U[3::64] = 0
+    U[7::64, 3] = float("nan")
+    U[11::64, 30] = float("inf")
+    U[4096:4160] = 0
+    few, all_ = pkg.kmeans_assign(U[:199999], C), pkg.kmeans_assign(U, C)
+    assert torch.equal(few[0], all_[0][:199999])
+    assert torch.equal(few[1].view(torch.int32), all_[1][:199999].view(torch.int32))
+
+
+# the column loop (sixteen at a time) and the whole rows, with most points open and a few columns each
+@pytest.mark.parametrize("d,K", [(8, 48), (8, 200), (16, 64), (16, 100), (16, 256), (32, 8), (32, 16), (32, 64), (32, 72)])
+def test_kmeans_narrow_cones(d, K):
+    g = torch.Generator(device=DEV).manual_seed(d * K)
+    U = 1 + 0.02 * torch.randn(1500, d, generator=g, device=DEV)
+    C = 1 + 0.02 * torch.randn(K, d, generator=g, device=DEV)
+    C[K // 2] = C[1]
+    sims = torch.zeros(1500, K, dtype=torch.float64, device=DEV)
+    for i in range(d):  # an fma rounds the exact product and sum once
+        sims = (U[:, i:i + 1].double() * C[:, i].double() + sims).float().double()
+    assigns, best, _, _ = pkg.kmeans_assign(U, C)
+    # (a 64-bit product and sum rounds a second time, in one of 2^29 cases differently from the fma)
+    assert (assigns.long() == (sims == sims.max(1).values[:, None]).int().argmax(1)).sum() >= 1498
+    assert (best.double() == sims.max(1).values).sum() >= 1498
+
+
 # both kernels: the chains (few centroids; few points of the largest codebooks) and the tensor-core search
 @pytest.mark.parametrize("d,K", [(8, 47), (8, 64), (16, 16), (16, 64), (16, 200), (32, 8), (32, 64), (32, 128)])
 def test_kmeans_points_that_are_not_finite(d, K):
