@@ -188,6 +188,11 @@ __device__ __forceinline__ float lds_f1(uint32_t addr) {
   return v;
 }
 
+// Three products, without lo * lo (2^-16 at most), and a lead that covers that too: a point's products are waited for, its chains are
+// cheap.  4M points, K 64, with the fourth product and the smaller lead of search.cuh / so: 16 dims 149.9 / 149.1 us, 32 dims 263 / 258.
+constexpr float kPointLead = 5.f / 65536.f;
+static_assert(2 * (2 * kPairError + 1. / (1 << 16) + 6 * kSumError + kChainError + kRestError) < kPointLead, "the lead covers both sums' errors");
+
 // The vote of search.cuh with the columns above t as bits, up to 24 to a float (exact sums): where there are more than one, it says
 // which the chains have to decide between.  1M points of 16 dims, K 64, all centroids for an open point before / now / the chains'
 // kernel: random 45 / 46 / 72 us, a tenth of the points' mean as spread 79 / 53 / 72, zeros 125 / 50 / 72, all centroids equal
@@ -445,7 +450,6 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
           mma_ts(tmem, k0 + 8 * kc, hi, idesc, kc > 0);
           mma_ts(tmem, k0 + kKeys / 2 + 8 * kc, hi, idesc, true);
           mma_ts(tmem, k0 + 8 * kc, lo, idesc, true);
-          mma_ts(tmem, k0 + kKeys / 2 + 8 * kc, lo, idesc, true);
         }
         mma_commit(bar);
       }
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
       Leaders<C> who;
       tmem_ld_row<C>(my_rows, v);
       tmem_wait_ld();
-      find_leaders<C>(v, lead_of(largest_of<C>(v), norm, most), who);
+      find_leaders<C>(v, lead_of(largest_of<C>(v), norm, most, kPointLead), who);
       const bool unsure = live && !(one_leader<C>(who, code) && !waits.lost);
       tc_fence_before();
       if (more) products();  // runs while this batch is added up
@@ -520,7 +524,7 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
         columns(c0, v);
         top = fmaxf(top, largest_of<16>(v));
       }
-      const Lead l = lead_of(top, norm, most);
+      const Lead l = lead_of(top, norm, most, kPointLead);
       Leaders<16> who = {{0.f}};
       int base_of = 0;
       uint32_t blocks = 0;  // of sixteen columns, with some above t

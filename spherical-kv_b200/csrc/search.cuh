@@ -10,7 +10,8 @@
 //
 // Error of an approximate sum, relative to |k| |c| (Cauchy-Schwarz over the dims): a value less its two bf16 parts
 // (kPairError), for the key and for the centroid; the chains' own rounding (kChainError); and the tensor core's sums (kSumError).
-// Twice all of it is 0.98 kGap; without the product lo * lo, up to 2^-16, it would be 1.6 kGap.  The tensor core, measured on this part
+// Twice all of it is 0.98 kGap; without the product lo * lo, up to 2^-16, it would be 1.6 kGap (k-means leaves it out, with a lead
+// of its own).  The tensor core, measured on this part
 // (one term 1, fifteen of 2^-18 .. 2^-29): a product's addends are cut off below 2^-25 of the largest, the sum at
 // fp32, so a product of 16 addends and the accumulator lose at most 17 x 2^-25 + 2^-23 (seen on random vectors: 2^-21.2 in
 // all).  Norms outside 2^-30 .. 2^30 (underflow, overflow, infinities, NaN) are never decided here.
@@ -21,10 +22,10 @@ namespace sphkv {
 
 constexpr float kGap = 3.f / 65536.f;       // lead over the runner-up, relative to |k| max |c|, that settles a search
 constexpr double kPairError = 1. / (1 << 17);                                // half a place of lo, which is at most 2^-8
-constexpr double kSumError = 8 * (17. / (1 << 25) + 1. / (1 << 23));         // four products of two halves of 32 dims
+constexpr double kSumError = 17. / (1 << 25) + 1. / (1 << 23);               // of one product; four for each half of 32 dims
 constexpr double kChainError = 32. / (1 << 24);
 constexpr double kRestError = 1. / (1 << 23);                                // of norms, t and products of two remainders
-static_assert(2 * (2 * kPairError + kSumError + kChainError + kRestError) < kGap, "the lead covers both sums' errors");
+static_assert(2 * (2 * kPairError + 8 * kSumError + kChainError + kRestError) < kGap, "the lead covers both sums' errors");
 constexpr int kSearchWarps = 4;             // warps of a search group: the 128 lanes (token rows) of tensor memory
 constexpr int kSearchGroups = 2;            // search groups of a CTA
 constexpr int kSearchThreads = kSearchGroups * kSearchWarps * 32;
@@ -111,9 +112,9 @@ struct Lead {
   float gap, t, scale, shift;
   bool fit;  // norms and t in the range where the sums below are exact
 };
-__device__ __forceinline__ Lead lead_of(float top, float norm, float most) {
+__device__ __forceinline__ Lead lead_of(float top, float norm, float most, float lead = kGap) {
   Lead l;
-  l.gap = kGap * norm * most;
+  l.gap = lead * norm * most;
   l.t = top - l.gap;
   // 2^36 / 2^exponent(gap): t at least 2^-10 gap away from 0 differs from any other float by 2^-35 gap or more
   l.scale = __uint_as_float((290u - (__float_as_uint(l.gap) >> 23)) << 23);

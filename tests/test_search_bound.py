@@ -31,8 +31,8 @@ def test_the_lead_covers_the_pairs(tmp_path):
     off = ((x.double() - hi.double() - lo.double()).abs() / x.double()).max().item()
     assert 0.9 * pair < off <= pair
     assert (lo.abs() / x).max().item() <= 2.0 ** -8  # lo * lo is a product of its own: 2^-16 is more than a third of the lead
-    assert sums >= 8 * (17 * 2.0 ** -25 + 2.0 ** -23) and chains >= 32 * 2.0 ** -24
-    assert 2 * (2 * pair + sums + chains) < gap
+    assert sums >= 17 * 2.0 ** -25 + 2.0 ** -23 and chains >= 32 * 2.0 ** -24
+    assert 2 * (2 * pair + 8 * sums + chains) < gap
 
 
 SRC = r"""
