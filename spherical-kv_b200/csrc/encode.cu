@@ -780,7 +780,7 @@ __device__ __forceinline__ void search_slice(const float (&k)[kCodeTok][32], con
 #endif
 constexpr int kChainThreads = SPHKV_CODE_WARPS * 32;  // a multiple of four warps: dh / 32 warps share a token set
 
-// Few centroids (see the rule at the launch): the chains on the fp32 pipe.  A thread holds four tokens' 32-dim slice; the two
+// Few centroids, short inputs (see the rule at the launch): the chains on the fp32 pipe.  A thread holds four tokens' 32-dim slice; the two
 // 16-dim halves serve the g = 16 tiers, the whole slice the g = 32 tiers, and the squared norm of the 32-dim group
 // continues the fma chain of its first half, so every value equals what the per-tier encoder computes.
 // Persistent: the (head, row block) units are dealt out in contiguous runs, one run per resident
@@ -1589,20 +1589,32 @@ extern "C" int sphkv_encode_codes(const void* k_src, int32_t k_dtype, int64_t k_
     }
   }
   SPHKV_REQUIRE(wanted != 0, SPHKV_E_ARG, "encode_codes: no output requested");
-  // The chains cost 1.2 instructions per centroid and dim, the tensor-core kernel a fixed 45 us for 32768 tokens x 8 heads whatever
-  // it searches: centroids per dim 8 (one 32-dim slot) 32 us against 45, 16 49 / 50, 24 64 / 64, 32 74 / 55, 64 124 / 67,
-  // 88 (the three reference tiers) 170 / 75; of 500 tokens 4 / 8, 5 / 9, 7 / 10, 7 / 10, 11 / 12, 14 / 14.
+  // rows staged through shared memory when every 32-element slice starts on a 16-byte boundary (and, below, where they fit beside
+  // the centroids: not with four 64-centroid slots)
+  const int esz = k_dtype == SPHKV_F32 ? 4 : 2;
+  const bool aligned = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 && (k_head_stride * esz) % 16 == 0;
+  // The chains cost 1.2 instructions per centroid and dim; the tensor-core kernel has 5 us of set-up and 45 us for 32768 tokens x 8 heads
+  // whatever it searches.  Chains / tensor cores in us at dh 128 by the centroids (of a 32-dim slot, with fewer compares to
+  // a dim, 15 of 16 count), 8 heads of 1000, 2048, 4096 and 32768 fp32 tokens:
+  //   16: 5 / 9, 6 / 9, 9 / 12, 48 / 50        24: 6 / 11, 8 / 11, 11 / 14, 64 / 64        32: 7.0 / 9.9, 8.8 / 10.3, 12.6 / 13.3, 73 / 55
+  //   48: 9.3 / 12.0, 11.8 / 12.2, 17.2 / 16.4, 104 / 71      64: 10.8 / 12.3, 13.7 / 12.3, 20.2 / 16.1, 123 / 66
+  //   80: 13.1 / 12.8, 16.8 / 13.4, 24.9 / 16.9, 154 / 64
+  // so the lines lie where the chains need more than one round of blocks with four, two or one tokens per thread.  Keys off a 16-byte
+  // boundary, 88 centroids: 18.5 / 26.1, 26.2 / 25.6, 43 / 40, 274 / 207.  At dh 64 (half the centroids to lay out) 64 centroids
+  // take 9.5 / 8.1 from 64 tokens on, with such keys 13.7 / 12.3.
   int centroids = 0;
-  for (int s = 0; s < tiers->n_slots; ++s) centroids += (wanted >> s) & 1u ? 1 << tiers->bits[s] : 0;
-  if (centroids < 48) return launch_codes_chains(a, Hkv, reinterpret_cast<cudaStream_t>(stream));
+  for (int s = 0; s < tiers->n_slots; ++s) centroids += (wanted >> s) & 1u ? (1 << tiers->bits[s]) * (tiers->g[s] == 32 ? 15 : 16) : 0;
+  centroids /= 16;
+  const auto one_round = [&](int tok) { return (rows + 64 * tok - 1) / (64 * tok) * Hkv <= sm_count_current_device(); };
+  const bool chains = dh == 64 ? centroids < 45
+                               : centroids < 30 || (centroids < 45 && one_round(4)) || (centroids < 64 && one_round(2)) ||
+                                     ((centroids < 80 || !aligned) && one_round(1));
+  if (chains) return launch_codes_chains(a, Hkv, reinterpret_cast<cudaStream_t>(stream));
   a.wide = (ends & 15) == 0;
   a.plan = plan_search(*tiers, dh, wanted);
   a.kbuf_off = a.plan.bytes + kCodeTail;
-  // rows staged through shared memory when every 32-element slice starts on a 16-byte boundary and they fit beside
-  // the centroids (not with four 64-centroid slots)
-  const int esz = k_dtype == SPHKV_F32 ? 4 : 2, staged_bytes = kSearchThreads / 32 * kCodeStages * kSliceBlock;
-  const bool staged = (reinterpret_cast<uintptr_t>(k_src) & 15) == 0 && (k_row_stride * esz) % 16 == 0 &&
-                      (k_head_stride * esz) % 16 == 0 && a.kbuf_off + staged_bytes <= 227 * 1024;
+  const int staged_bytes = kSearchThreads / 32 * kCodeStages * kSliceBlock;
+  const bool staged = aligned && a.kbuf_off + staged_bytes <= 227 * 1024;
   const int smem_bytes = a.kbuf_off + (staged ? staged_bytes : 0);
   // The reference's tiers (its first two, or all three) have a kernel of their own: 172 us with the chains, 89 us with branches
   // and loops over the slots, 79 us with their sums in registers at once (32768 fp32 tokens x 8 heads, three tiers).

@@ -19,7 +19,7 @@ namespace sphkv {
 // points per thread: 4 (2 for 32-dim points) keeps the kernel at two CTAs per SM
 __host__ __device__ constexpr int pts_for(int d) { return d >= 32 ? 2 : 4; }
 
-// Few centroids (see the rule at the launch): the chains on the fp32 pipe.  A CTA takes passes of 32 * pts_for(D) points per
+// Few centroids, and some numbers of points (see the rule at the launch): the chains on the fp32 pipe.  A CTA takes passes of 32 * pts_for(D) points per
 // warp; its warps walk them without meeting; a warp's rows are turned through a 32-row tile for the adds.  Bound: fp32 FMA
 // issue, then the shared-memory adds.
 template <int D, int WARPS>
@@ -676,11 +676,20 @@ extern "C" int sphkv_kmeans_assign(const float* U, int64_t N, int32_t d, const f
     return (int)e;
   }
   if (N == 0) return SPHKV_OK;
-  // The chains cost K fmas per value, the tensor cores hardly anything, but that kernel has fewer warps to hide the sums behind:
-  // 4M points (2M of 32 dims), chains / tensor cores: d 8: K 32 97 / 114 us, 48 126 / 125, 64 156 / 116; d 16: K 16 120 / 140,
-  // 32 163 / 165, 48 210 / 180, 64 255 / 171, 256 917 / 627; d 32: K 8 130 / 123, 64 289 / 182.
-  // Of 32 dims and 128 centroids on, one search group is all that fits a CTA: 60000 points 31 / 37 us, 500000 148 / 109.
-  if ((d < 32 && K < 48) || (d == 32 && K >= 128 && N < 200000)) {
+  // The chains cost K fmas per value, the tensor cores hardly anything, but that kernel has fewer warps to hide the sums behind.
+  // Chains / tensor cores in us, without similarities:
+  //   d 8   4M points K 32 96 / 103, 48 125 / 115, 64 156 / 101, 256 540 / 512; 30000 points K 32 11.1 / 10.3, 48 12.4 / 10.8
+  //   d 16  4M K 16 121 / 114 (36.9 / 36.2 of 1M; with similarities slower), 24 142 / 139, 32 162 / 128, 64 254 / 125;
+  //         30000 K 32 14.4 / 11.8
+  //   d 32  4M K 2 219 / 173, 8 249 / 146, 64 557 / 211, 179 1519 / 628; 4096 points K 2 12.1 / 10.4, 128 29.1 / 22.7
+  // In between, where the chains are done in one round of blocks and this kernel begins its second or third, or has only one
+  // search group (more than 224 centroids of 8 dims): d 8 150000 points K 48 13.1 / 14.4, 256 30.9 / 37.3 (500000: 89.6 / 82.1);
+  // d 16 150000 K 32 14.6 / 16.2 (100000: 14.4 / 12.4); d 32 65536 K 4 12.3 / 14.4.
+  const auto between = [&](int lo, int hi) { return N > (int64_t)sms * lo && N <= (int64_t)sms * hi; };
+  const bool chains = d == 8    ? K < 48 || (K < 64 && between(768, 2048)) || (K > 224 && between(512, 2048))
+                      : d == 16 ? K < 32 || (K < 48 && between(768, 1024))
+                                : K <= 8 && between(384, 512);
+  if (chains) {
     return d == 8    ? launch_chains<8>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
            : d == 16 ? launch_chains<16>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st)
                      : launch_chains<32>(U, N, centers, K, assigns, best_sim, sums, counts, sms, st);

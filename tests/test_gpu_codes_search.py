@@ -18,6 +18,10 @@ SETS = {
     "small and odd": (T(1, 16, 1), T(2, 32, 2), T(3, 16, 5), T(4, 32, 6)),
     "two passes": (T(1, 16, 6), T(2, 16, 5), T(3, 32, 6)),
     "four passes, rows not staged": (T(1, 16, 6), T(2, 16, 6), T(3, 16, 6), T(4, 16, 6)),
+    "16 centroids": (T(1, 16, 4),),
+    "40 centroids": (T(1, 16, 5), T(2, 32, 3)),
+    "48 centroids": (T(1, 16, 5), T(2, 16, 4)),
+    "64 centroids": (T(1, 16, 6),),
 }
 
 
@@ -79,6 +83,46 @@ def test_codes_equal_the_chains(kind, tiers, dh, rows, dtype):
         want = pkg.encode_pages(K, None, lists, cb, ts, use_scratch=False)
         got = pkg.pages_from_codes(codes, None, lists, cb)
         assert torch.equal(got.k_pages, want.k_pages)
+
+
+def compare_with_chains(tiers, K, dh, hkv, seed):
+    """every code of K against the fused encoder's pages, every radius against the fma chain's root"""
+    specs = SETS[tiers]
+    ts = pkg.TierSet(dh, specs)
+    cb = ts.pack_codebooks(pkg.synth.make_codebooks(hkv, dh, specs, seed=seed)).to(DEV)
+    codes = pkg.encode_codes(K, cb, ts)
+    rows = K.shape[0]
+    for s, t in enumerate(specs):
+        lists = pkg.build_page_lists(torch.full((1, hkv, rows), t.tier_id, dtype=torch.uint8, device=DEV), ts, 64)
+        want = pkg.encode_pages(K, None, lists, cb, ts, use_scratch=False)
+        assert torch.equal(pkg.pages_from_codes(codes, None, lists, cb).k_pages, want.k_pages)
+        k = K.double().reshape(rows, hkv, dh // t.g, t.g).transpose(0, 1)
+        n = torch.zeros(k.shape[:3], dtype=torch.float64, device=DEV)
+        for d in range(t.g):  # an fma rounds the exact product and sum once
+            n = (k[..., d] * k[..., d] + n).float().double()
+        # (a 64-bit product and sum rounds a second time, in one of 2^29 cases differently from the fma)
+        assert (codes.r[s].view(torch.int32) != n.float().sqrt().view(torch.int32)).sum() <= 2
+
+
+# more than 148 blocks of 128 rows: blocks in a row, blocks of two heads in one CTA, a last block that is not full
+@pytest.mark.parametrize("tiers", SETS)
+@pytest.mark.parametrize("dh,dtype,shift", [(128, torch.float32, 0), (64, torch.bfloat16, 0), (128, torch.float16, 1), (64, torch.float32, 1)])
+def test_long_inputs_cross_blocks_and_heads(tiers, dh, dtype, shift):
+    rows, hkv = 9001, 8
+    g = torch.Generator(device=DEV).manual_seed(dh + shift)
+    flat = torch.randn(rows * hkv * dh + 8, generator=g, device=DEV).to(dtype)
+    compare_with_chains(tiers, flat[shift:shift + rows * hkv * dh].view(rows, hkv, dh), dh, hkv, seed=rows)
+
+
+# both sides of the lines of the dispatch (148 blocks): one round of the chains with one, two, four tokens per thread
+@pytest.mark.parametrize("tiers,edge", [("64 centroids", 18 * 64), ("48 centroids", 18 * 128), ("40 centroids", 18 * 256), ("reference", 18 * 64)])
+@pytest.mark.parametrize("past", [0, 1])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_lines_of_the_dispatch(tiers, edge, past, shift):
+    rows, hkv, dh = edge + past, 8, 128
+    g = torch.Generator(device=DEV).manual_seed(edge)
+    flat = torch.randn(rows * hkv * dh + 8, generator=g, device=DEV)
+    compare_with_chains(tiers, flat[shift:shift + rows * hkv * dh].view(rows, hkv, dh), dh, hkv, seed=edge)
 
 
 def test_padding_costs_no_more_than_keys():

@@ -68,19 +68,22 @@ def test_decode_honours_the_header_count(page):
     assert torch.equal(pkg.decode_paged(Q.to(DEV), cache, rope), want)
 
 
-# one, two and four tokens per thread; staged and direct loads
+# the chains' kernel with one, two and four tokens per thread, staged and direct loads (16 centroids always take it, 40 up to 4700
+# rows of 8 heads), and the tensor-core kernel (80 centroids)
+@pytest.mark.parametrize("bits", [(4,), (5, 3), (6, 4)])
 @pytest.mark.parametrize("T,Hkv,dh", [(2047, 8, 128), (4097, 8, 128), (9001, 8, 128), (6001, 8, 64)])
 @pytest.mark.parametrize("dtype,shift", [(torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)])
-def test_codes_do_not_depend_on_tokens_per_thread(T, Hkv, dh, dtype, shift):
-    """large inputs equal the codes of 64-row slices of them (one token per thread, checked against the oracle)"""
-    tiers = pkg.TierSet(dh)
-    cb = tiers.pack_codebooks(synth.make_codebooks(Hkv, dh, pkg.REFERENCE_TIERS[:2], seed=T)).to(DEV)
+def test_codes_do_not_depend_on_tokens_per_thread(bits, T, Hkv, dh, dtype, shift):
+    """large inputs equal the codes of 64-row slices of them (one token per thread)"""
+    specs = tuple(pkg.pages.TierSpec(i + 1, 32 if b == 3 else 16, b) for i, b in enumerate(bits))
+    tiers = pkg.TierSet(dh, specs)
+    cb = tiers.pack_codebooks(synth.make_codebooks(Hkv, dh, specs, seed=T)).to(DEV)
     flat = torch.randn(T * Hkv * dh + 8, generator=torch.Generator(device=DEV).manual_seed(T), device=DEV).to(dtype)
     K = flat[shift:shift + T * Hkv * dh].view(T, Hkv, dh)
     got = pkg.encode_codes(K, cb, tiers)
     for t0 in (0, 64 * (T // 128), T - 64):
         part = pkg.encode_codes(K[t0:t0 + 64], cb, tiers)
-        for s in range(2):
+        for s in range(len(specs)):
             assert torch.equal(got.r[s][:, t0:t0 + 64].view(torch.int32), part.r[s].view(torch.int32))
             assert torch.equal(got.theta[s][:, t0:t0 + 64], part.theta[s])
 
@@ -123,9 +126,10 @@ def test_kmeans_sums_and_counts(N, d, K):
     assert ((sums.double() - want).abs() <= bound).all()
 
 
-# both sides of the rules that choose the tensor-core search: centroids, and points of the largest codebooks; batches of 128
-@pytest.mark.parametrize("N,d,K", [(129, 8, 47), (129, 8, 48), (385, 16, 47), (385, 16, 48), (199999, 32, 128), (200000, 32, 128),
-                                   (50000, 16, 256), (3000, 32, 17)])
+# both sides of the rules that choose the tensor-core search (148 SMs): centroids, rounds of the chains' blocks; batches of 128
+@pytest.mark.parametrize("N,d,K", [(129, 8, 47), (129, 8, 48), (113664, 8, 48), (113665, 8, 48), (75777, 8, 225), (75777, 8, 224),
+                                   (385, 16, 31), (385, 16, 32), (113665, 16, 32), (151553, 16, 32), (50000, 16, 256),
+                                   (56832, 32, 8), (56833, 32, 8), (75777, 32, 8), (60000, 32, 9), (3000, 32, 17), (3000, 32, 128)])
 def test_kmeans_search_rules(N, d, K):
     test_kmeans_sums_and_counts(N, d, K)
 
@@ -152,21 +156,23 @@ def test_kmeans_ties_and_special_points(d, K):
     assert torch.equal(counts.long(), torch.bincount(assigns.long(), minlength=K))
 
 
-def test_kmeans_kernels_agree_bit_for_bit():
-    """one point more, and the tensor-core search takes the call: ties, narrow cones, zeros and all, the chains' answers"""
-    g = torch.Generator(device=DEV).manual_seed(7)
-    U = torch.randn(200000, 32, generator=g, device=DEV)
+@pytest.mark.parametrize("d,K,N", [(32, 8, 70000), (16, 40, 140000), (8, 60, 200000), (8, 256, 200000)])
+def test_kmeans_kernels_agree_bit_for_bit(d, K, N):
+    """the chains take these numbers of points, the tensor-core search their first 30000: ties, narrow cones, zeros and all"""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    U = torch.randn(N, d, generator=g, device=DEV)
     U[1::4] = 1 + 0.02 * U[1::4]
-    C = U[torch.randint(200000, (128,), generator=g, device=DEV)].clone()
+    C = U[torch.randint(N, (K,), generator=g, device=DEV)].clone()
     C[::9] = C[5]
-    U[2::4] = C[torch.randint(128, (50000,), generator=g, device=DEV)] + C[torch.randint(128, (50000,), generator=g, device=DEV)]
+    n = U[2::4].shape[0]
+    U[2::4] = C[torch.randint(K, (n,), generator=g, device=DEV)] + C[torch.randint(K, (n,), generator=g, device=DEV)]
     U[3::64] = 0
     U[7::64, 3] = float("nan")
-    U[11::64, 30] = float("inf")
+    U[11::64, d - 1] = float("inf")
     U[4096:4160] = 0
-    few, all_ = pkg.kmeans_assign(U[:199999], C), pkg.kmeans_assign(U, C)
-    assert torch.equal(few[0], all_[0][:199999])
-    assert torch.equal(few[1].view(torch.int32), all_[1][:199999].view(torch.int32))
+    few, all_ = pkg.kmeans_assign(U[:30000], C), pkg.kmeans_assign(U, C)
+    assert torch.equal(few[0], all_[0][:30000])
+    assert torch.equal(few[1].view(torch.int32), all_[1][:30000].view(torch.int32))
 
 
 # the column loop (sixteen at a time) and the whole rows, with most points open and a few columns each
@@ -185,7 +191,7 @@ def test_kmeans_narrow_cones(d, K):
     assert (best.double() == sims.max(1).values).sum() >= 1498
 
 
-# both kernels: the chains (few centroids; few points of the largest codebooks) and the tensor-core search
+# both kernels: the chains (few centroids) and the tensor-core search
 @pytest.mark.parametrize("d,K", [(8, 47), (8, 64), (16, 16), (16, 64), (16, 200), (32, 8), (32, 64), (32, 128)])
 def test_kmeans_points_that_are_not_finite(d, K):
     """sums that are NaN never win; a point that has no other gets cluster 0 and a similarity of -inf"""

@@ -23,9 +23,9 @@ def dev_lists(lists):
                                                 (128, 450, torch.float32, 1), (128, 450, torch.bfloat16, 3)])
 def test_code_cache_equals_per_tier_encode(dh, T, k_dtype, shift):
     """codes of all three reference tiers from one kernel == oracle.encode per tier, bit for bit
-    (radii as f32 bit patterns, centroid indices as bytes).  The long cases make a CTA walk several
-    row blocks and cross from one head to the next; shift > 0 puts the keys `shift` elements off a
-    16-byte boundary, which takes the kernel's direct-load route instead of the staged one."""
+    (radii as f32 bit patterns, centroid indices as bytes); shift > 0 puts the keys `shift` elements off a
+    16-byte boundary, which takes the direct-load route instead of the staged one.  (Inputs that make a CTA walk
+    several row blocks and cross heads: test_gpu_codes_search.py.)"""
     Hkv, specs = 3, pkg.REFERENCE_TIERS
     tiers = pkg.TierSet(dh, specs)
     K, _, _, _ = synth.make_kvq(1, Hkv, Hkv, dh, T, seed=dh + T, outlier_frac=0.02)
