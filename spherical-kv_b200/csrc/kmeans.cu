@@ -200,7 +200,7 @@ static_assert(2 * (2 * kPairError + 1. / (1 << 16) + 6 * kSumError + kChainError
 template <int C>
 struct Leaders {
   static constexpr int kParts = (C + 23) / 24;
-  float part[kParts];  // bit c - 24 i of part i: column c is above t; part 0 is NaN where this cannot be said
+  float part[kParts];  // bit c - 24 i of part i: column c is above t, if t fits
 };
 template <int C>
 __device__ __forceinline__ void find_leaders(const float (&v)[C < 16 ? 16 : C], const Lead& l, Leaders<C>& who) {
@@ -218,7 +218,6 @@ __device__ __forceinline__ void find_leaders(const float (&v)[C < 16 ? 16 : C], 
     else
       who.part[i] = sum[i][0] + sum[i][1];
   }
-  if (!l.fit) who.part[0] = __int_as_float(0x7fc00000);
 }
 // one leader: one part that is not 0 (their sum is the largest of them: parts are whole and below 2^24), and it a power of two,
 // whose exponent is the leader's number
@@ -234,12 +233,12 @@ __device__ __forceinline__ bool one_leader(const Leaders<C>& who, int& code) {
     one = __fmaf_rn(who.part[2], 281474976710656.f, __fmaf_rn(who.part[1], 16777216.f, one));
   }
   code = (__float_as_int(one) >> 23) - 127;
-  return single && (__float_as_int(one) & 0x7fffff) == 0;  // (the NaN's has bits there)
+  return single && (__float_as_int(one) & 0x7fffff) == 0;
 }
-// those columns, or all where the sums do not say (`lost`: they are not there)
+// those columns, or all where the sums do not say
 template <int C>
-__device__ __forceinline__ uint64_t open_columns(const Leaders<C>& who, bool lost) {
-  if (lost || who.part[0] != who.part[0]) return ~0ull >> (64 - C);
+__device__ __forceinline__ uint64_t open_columns(const Leaders<C>& who, bool all) {
+  if (all) return ~0ull >> (64 - C);
   uint64_t open = 0;
 #pragma unroll
   for (int i = 0; i < Leaders<C>::kParts; ++i) open |= (uint64_t)(uint32_t)who.part[i] << (24 * i);
@@ -492,14 +491,15 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
       Leaders<C> who;
       tmem_ld_row<C>(my_rows, v);
       tmem_wait_ld();
-      find_leaders<C>(v, lead_of(largest_of<C>(v), norm, most, kPointLead), who);
-      const bool unsure = live && !(one_leader<C>(who, code) && !waits.lost);
+      const Lead l = lead_of(largest_of<C>(v), norm, most, kPointLead);
+      find_leaders<C>(v, l, who);
+      const bool unsure = live && !(one_leader<C>(who, code) && l.fit && !waits.lost);
       tc_fence_before();
       if (more) products();  // runs while this batch is added up
       if (__any_sync(0xffffffffu, unsure)) {
         float k[D];
         load(k);
-        code = settle_point(k, c_s, kPitch, K, unsure ? open_columns<C>(who, waits.lost) : 0, code);
+        code = settle_point(k, c_s, kPitch, K, unsure ? open_columns<C>(who, waits.lost || !l.fit) : 0, code);
       }
     };
     if (K == 64) {
@@ -528,14 +528,14 @@ __global__ void __launch_bounds__(kKmeansGroups * 128, 1) kmeans_search_kernel(c
       Leaders<16> who = {{0.f}};
       int base_of = 0;
       uint32_t blocks = 0;  // of sixteen columns, with some above t
-      for (int c0 = 0; c0 < K; c0 += 16) {
+      for (int c0 = 0, bit = 1; c0 < K; c0 += 16, bit <<= 1) {
         float v[16];
         columns(c0, v);
         Leaders<16> some;
         find_leaders<16>(v, l, some);
-        if (!(some.part[0] == 0.f)) { who = some; base_of = c0; blocks |= 1u << (c0 >> 4); }
+        if (some.part[0] != 0.f) { who = some; base_of = c0; blocks |= bit; }
       }
-      const bool one = one_leader<16>(who, code) && (blocks & (blocks - 1)) == 0;
+      const bool one = one_leader<16>(who, code) && l.fit && (blocks & (blocks - 1)) == 0;
       code += base_of;
       bool unsure = live && !(one && !waits.lost);
       if (__any_sync(0xffffffffu, unsure)) {
