@@ -316,8 +316,9 @@ __device__ __forceinline__ int settle_point(const float (&k)[GS], const float* _
   return code;
 }
 
-// Bound: latency -- twelve warps an SM, each with a chain of tensor memory, shared-memory adds and a barrier per batch; DRAM at
-// 30 % of the copy rate.  4M points, d 16, K 64: 255 us with the chains, 170 here, 148 without bank conflicts on the winners.
+// Bound: latency -- twelve warps an SM, each with a chain of tensor memory, shared-memory adds and a barrier per batch (58 % of
+// issue slots, L1 and shared memory 56 %, DRAM 22 %).  4M points, d 16, K 64: 254 us with the chains, 170 here, 148 without bank
+// conflicts on the winners.
 // A CTA has up to three search groups (four warps, thread = point = lane of tensor memory), each striding over batches
 // of 128 points; a warp stages, splits, searches and adds its 32 points by itself and meets the group's other warps
 // once per batch, before the products.
