@@ -58,17 +58,21 @@ struct DecodeArgs {
   float* rows;  // [(n_ctas + n_units)][8][dh + 2]
 };
 
-// shared-memory carve-up, shared by host and device: V tiles and weights of the teams in use, K stages,
-// metadata, query operand, barriers; then codebooks and the block prefix
-__host__ __device__ constexpr int smem_v_bytes(int dh) { return kMacroTiles * 16 * dh * 2; }  // per team
-constexpr int kSmemP = kMacroTiles * 512;                                                      // per team
-constexpr int kSmemK = 3 * kMacroTiles * 384;                                                  // per team (f16 radii: 2 x 512)
-constexpr int kSmemMeta = kMetaRing * 16;                                                      // per team
-constexpr int kSmemBars = 1792;
+// shared-memory carve-up, shared by host and device: query operand; per team barriers, votes and statistics, two words of the
+// CTA; per team in use V tiles, weights, K stages, metadata; then codebooks and the block prefix.  Everything a team
+// touches per tile lies at a constant offset from two bases: addresses that depended on the number of teams
+// were made again at every use, 110 of 750 instructions a tile.
+constexpr int kSmemQ = 128 / 16 * 512;
+constexpr int kBarStride = 128, kSmemTeamBars = kBarStride + 32 + 128 + 256 + 32;
+constexpr int kSmemHead = (kSmemQ + kTeams * kSmemTeamBars + 16 + 1023) / 1024 * 1024;
 __host__ __device__ constexpr int smem_q_bytes(int dh) { return dh / 16 * 512; }
-__host__ __device__ constexpr int smem_fixed_bytes(int dh, int teams) {
-  return teams * (smem_v_bytes(dh) + kSmemP + kSmemK + kSmemMeta) + smem_q_bytes(dh) + kSmemBars;
-}
+__host__ __device__ constexpr int smem_v_bytes(int dh) { return kMacroTiles * 16 * dh * 2; }
+constexpr int kSmemP = kMacroTiles * 512;
+constexpr int kSmemK = 3 * kMacroTiles * 384;  // (f16 radii: 2 x 512)
+constexpr int kSmemMeta = kMetaRing * 16;
+__host__ __device__ constexpr int smem_team_bytes(int dh) { return smem_v_bytes(dh) + kSmemP + kSmemK + kSmemMeta; }
+static_assert(smem_team_bytes(64) % 1024 == 0 && smem_team_bytes(128) % 1024 == 0, "V tiles start on 1024 bytes");
+__host__ __device__ constexpr int smem_fixed_bytes(int dh, int teams) { return kSmemHead + teams * smem_team_bytes(dh); }
 // room for the group shifts of a slot's codebook (see stage_codebooks)
 constexpr int kCbShift = 128;
 
@@ -207,8 +211,7 @@ static_assert(kKTh + 112 <= kKRd && kKRd + 128 + 16 <= 384 - 64 && kKRd + 256 + 
 
 // barriers of a team (8 bytes each, kBarStride per team)
 enum { kBarKFull = 0, kBarKeys = kKStages, kBarKeys2, kBarLogits, kBarWeights, kBarV, kBarOut, kBarVote, kBarDrain, kBarCount };
-constexpr int kBarStride = 128;
-static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 256 + 32) + 64 <= kSmemBars, "barrier block");
+static_assert(kBarCount * 8 <= kBarStride, "barrier block");
 
 // A team of four warps rebuilds 128 keys (eight 16-token tiles) into tensor memory, its driver warp --
 // which also fetches everything -- issues the two contractions:
@@ -220,8 +223,8 @@ static_assert(kBarCount * 8 <= kBarStride && kTeams * (kBarStride + 32 + 128 + 2
 // keys in flight and nothing else, twelve team warps fit an SM (the mma.sync version it replaced: eight, at
 // 244 registers, and shuffles, ldmatrix and accumulator moves around both products).
 // Bound: instruction issue and the waits between the roles, not HBM.  A 96-bit, 32768-token, batch-8 layer
-// step, merge included: 223 -> 178 us in a long loop under the power cap, 153 us in a burst (2.4 -> 3.0 and
-// 3.5 TB/s of the bytes it has to read).
+// step, merge included, in a short loop: 159 -> 147 us (3.4 -> 3.7 TB/s of the bytes it has to read) with 666
+// instructions a tile instead of 755, since team addresses lie at constant offsets and stay in registers.
 // Lane map of the rebuild (lane = 4 r + j): rows r and r + 8 of a tile are the lane's two tokens; in each
 // rotary half the lane owns the contiguous block of W = dh / 8 dimensions  W j .. W j + W - 1, and in the
 // other half the same block shifted by dh / 2: the RoPE partner of every value a lane holds is in the same
@@ -246,26 +249,27 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
 
   extern __shared__ __align__(1024) uint8_t smem[];
   const sphkv_decode_params& p = a.p;
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  // What the loops use most of the thread's place comes out of shuffles, whose results stay in registers: short of those,
+  // the compiler reads the special register again, and waits for it, or makes an address again at every use.  Of four such
+  // addresses these two fit (barriers or the base of shared memory as well: spills, 8 x 32768 147 -> 159 us).
+  auto keep = [](auto x) { return __shfl_sync(0xffffffffu, x, 0); };
+  const int warp = keep((int)(threadIdx.x >> 5)), lane = __shfl_sync(0xffffffffu, (int)(threadIdx.x & 31), (int)(threadIdx.x & 31));
   const bool driver = warp >= 4 * kTeams;
   const int team = driver ? warp - 4 * kTeams : warp >> 2;
-  const bool in_use = team < a.teams;  // (the fourth driver warp never is)
-  const int tix = in_use ? team : 0;   // idle warps form valid addresses and do no work
+  const bool in_use = team < a.teams;  // (the fourth driver warp never is; idle warps do not use their addresses)
 
   const uint32_t smem0 = smem_u32(smem);
-  const uint32_t v_buf = smem0 + tix * smem_v_bytes(DH);
-  const uint32_t p_all = smem0 + a.teams * smem_v_bytes(DH), p_buf = p_all + tix * kSmemP;
-  const uint32_t k_all = p_all + a.teams * kSmemP, k_ring = k_all + tix * kSmemK;
-  const uint32_t m_all = k_all + a.teams * kSmemK, meta = m_all + tix * kSmemMeta;
-  const uint32_t q_u32 = m_all + a.teams * kSmemMeta;
-  const uint32_t bar_all = q_u32 + smem_q_bytes(DH), bar = bar_all + tix * kBarStride;
-  const uint32_t votes = bar_all + kTeams * kBarStride + tix * 32;           // [2][4 warps]
-  const uint32_t wmax = bar_all + kTeams * (kBarStride + 32) + tix * 128;    // [4 warps][8 heads]
-  // per team: [4 warps][8 heads] (sum, true maximum), [8 heads] reference maximum
-  float* stats_all = reinterpret_cast<float*>(smem + (bar_all - smem0) + kTeams * (kBarStride + 32 + 128));
-  float* mref_all = stats_all + kTeams * 64;
-  volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + (bar_all - smem0) + kSmemBars - 16);
-  const uint32_t cb_u32 = bar_all + kSmemBars;
+  const uint32_t q_u32 = smem0;
+  const uint32_t bar = smem0 + kSmemQ + team * kSmemTeamBars;
+  const uint32_t votes = bar + kBarStride;   // [2][4 warps]
+  const uint32_t wmax = votes + 32;          // [4 warps][8 heads]
+  // of a team: [4 warps][8 heads] (sum, true maximum), [8 heads] reference maximum
+  auto stats_of = [&](int t) { return reinterpret_cast<float*>(smem + kSmemQ + t * kSmemTeamBars + kBarStride + 32 + 128); };
+  auto mref_of = [&](int t) { return stats_of(t) + 64; };
+  volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + kSmemQ + kTeams * kSmemTeamBars);
+  const uint32_t v_buf = keep(smem0 + kSmemHead + team * smem_team_bytes(DH));
+  const uint32_t p_buf = v_buf + smem_v_bytes(DH), k_ring = p_buf + kSmemP, meta = k_ring + kSmemK;
+  const uint32_t cb_off = kSmemHead + a.teams * smem_team_bytes(DH);
 
   // ---- set-up: barriers, tensor memory, the zero columns of the weights and of the query operand ----
   if (driver && in_use && lane == 0) {
@@ -293,7 +297,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, shared_words[0], 0);
-  const uint32_t tmem = tmem_base + tix * kTeamCols;
+  const uint32_t tmem = keep(tmem_base + team * kTeamCols);
   // everything above touched shared and tensor memory only: this grid's launch overlaps the tail of the
   // kernel before it in the stream (the previous step's merge kernel, which lets it in early)
   griddep_wait();
@@ -303,7 +307,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   //      when there are many units ----
   const int32_t* pfx = a.pfx;
   if (a.plan_in_kernel) {
-    int32_t* pfx_s = reinterpret_cast<int32_t*>(smem + (cb_u32 - smem0) + a.cb_smem_bytes);
+    int32_t* pfx_s = reinterpret_cast<int32_t*>(smem + cb_off + a.cb_smem_bytes);
     if (warp == 0) {
       int carry = 0;
       for (int base = 0; base < a.n_units; base += 128) {
@@ -541,8 +545,15 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         const uint32_t bits = tw & 0xFF, G = (uint32_t)DH >> ((tw >> 8) & 0xF);
         const uint32_t poff = (uint32_t)m.poff;
         const int sub = meta_sub(m);
-        if (TPP == 1) {
-          piece(kb, poff, poff - meta_hdr(m) + meta_radius(m) + (uint32_t)meta_tokens(m) * G * rb);
+        const uint32_t stop = poff - meta_hdr(m) + meta_radius(m) + (uint32_t)meta_tokens(m) * G * rb;
+        if (FAST && a.wide) {  // at most 20 chunks, then the last words
+          const uint32_t s0 = poff & ~15u, full = stop & ~15u;
+#pragma unroll
+          for (int e = 0; e < 20; e += 4)
+            if (s0 + 16 * (q + e) < full) cp_async_16(kb + 16 * (q + e), p.k_pages + s0 + 16 * (q + e));
+          if (full + 4 * q < stop) cp_async_4(kb + (full - s0) + 4 * q, p.k_pages + full + 4 * q);
+        } else if (TPP == 1) {
+          piece(kb, poff, stop);
         } else {
           const uint32_t t0 = 16u * sub, t1 = t0 + (uint32_t)meta_tokens(m);
           const uint32_t toff = poff + (((m.rad >> 9) & 0x7F) | (((m.where >> 25) & 0x7) << 7)), roff = toff + (m.rad >> 16);
@@ -657,7 +668,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       const int g = tg.g[s], bits = tg.bits[s], G = DH / g, cpr = g >> 2;
       const int dup = a.cb_dup[s];
       const float* src = p.codebooks + ((int64_t)(hkv * tg.n_slots + s) * tg.G_max) * tg.C_max * tg.g_max;
-      const uint32_t dst = cb_u32 + a.cb_smem_off[s];
+      const uint32_t dst = smem0 + cb_off + a.cb_smem_off[s];
       const int lc = g == 32 ? 3 : 2;  // log2 of the chunks per row
       const int chunks = (G << bits) << lc;
       // asynchronous 16-byte copies: every chunk of the codebook is in flight at once instead
@@ -704,7 +715,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       const float x = q_val[l] * qscale;
       const float hi = __uint_as_float(__float_as_uint(x) & 0xFFFF0000u);
       auto put = [&](int n, float v) {
-        reinterpret_cast<__nv_bfloat16*>(smem + (q_u32 - smem0) + (half * NCH + chunk) * 512 + (n >> 3) * 256 +
+        reinterpret_cast<__nv_bfloat16*>(smem + (half * NCH + chunk) * 512 + (n >> 3) * 256 +
                                          (k >> 3) * 128)[(n & 7) * 8 + (k & 7)] = __float2bfloat16_rn(v);
       };
       put(head, hi);  // exact
@@ -755,7 +766,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         c_bits = tw & 0xFF;
         c_mask = (1u << c_bits) - 1u;
         c_rowb = 4u << (lg + dup);  // bytes from one centroid row to the next
-        const uint32_t base = cb_u32 + (tw >> 13) + sub_off * 4 + (dup ? (r & 1) * 64 : 0);
+        const uint32_t base = smem0 + cb_off + (tw >> 13) + sub_off * 4 + (dup ? (r & 1) * 64 : 0);
         c_cb_lo = base + ((uint32_t)glo << c_bits) * c_rowb + 16 * glo;
         c_cb_hi = base + ((uint32_t)ghi << c_bits) * c_rowb + 16 * glo + 64;
         // 16-token pages: the theta stream starts 8 + 4 G bytes into the page (pagebuilder.py:8-33;
@@ -1087,7 +1098,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     // ---- merge the teams of this CTA and write one partial row.  The accumulators [HEADS][DH] go where the
     //      weights were (the first eight columns of a packed tile: the zero columns stay) ----
     auto acc_at = [&](int t, int e) -> float* {
-      return reinterpret_cast<float*>(smem + (p_all - smem0) + t * kSmemP + (PACK ? (e >> 6) * 512 + (e & 63) * 4 : e * 4));
+      return reinterpret_cast<float*>(smem + kSmemHead + t * smem_team_bytes(DH) + smem_v_bytes(DH) + (PACK ? (e >> 6) * 512 + (e & 63) * 4 : e * 4));
     };
     if (in_use) {
       const int w = warp & 3;
@@ -1109,9 +1120,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
           m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, q));
         }
         if (lane == 0) {
-          stats_all[((team * 4 + w) * 8 + h) * 2] = l;
-          stats_all[((team * 4 + w) * 8 + h) * 2 + 1] = dead ? -INFINITY : m;
-          if (w == 0) mref_all[team * 8 + h] = dead ? -INFINITY : m_ref[h];
+          stats_of(team)[(w * 8 + h) * 2] = l;
+          stats_of(team)[(w * 8 + h) * 2 + 1] = dead ? -INFINITY : m;
+          if (w == 0) mref_of(team)[h] = dead ? -INFINITY : m_ref[h];
         }
         if (32 * w + lane < DH) *acc_at(team, h * DH + 32 * w + lane) = o[h] + o[h + HEADS];
       }
@@ -1125,19 +1136,19 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
         float M = -INFINITY, L = 0.f, o = 0.f;
 #pragma unroll
         for (int tw = 0; tw < 4 * kTeams; ++tw)
-          if (tw < 4 * a.teams) M = fmaxf(M, stats_all[(tw * 8 + n) * 2 + 1]);
+          if (tw < 4 * a.teams) M = fmaxf(M, stats_of(tw >> 2)[((tw & 3) * 8 + n) * 2 + 1]);
         if (M != -INFINITY) {
 #pragma unroll
           for (int t = 0; t < kTeams; ++t) {
             if (t >= a.teams) break;
-            const float mw = mref_all[t * 8 + n];
+            const float mw = mref_of(t)[n];
             if (mw == -INFINITY) continue;
             const float sc = fast_exp2(mw - M);
             o += *acc_at(t, i) * sc;
             if (d == 0) {
               float l = 0.f;
 #pragma unroll
-              for (int w = 0; w < 4; ++w) l += stats_all[((t * 4 + w) * 8 + n) * 2];
+              for (int w = 0; w < 4; ++w) l += stats_of(t)[(w * 8 + n) * 2];
               L += l * sc;
             }
           }
