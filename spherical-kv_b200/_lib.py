@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsphkv_b200.so")
@@ -40,6 +41,18 @@ class EncodeParams(C.Structure):
         ("k_dtype", C.c_int32), ("v_src_dtype", C.c_int32), ("v_pool_dtype", C.c_int32),
         ("radius_fmt", C.c_int32), ("tiers", Tiers),
     ]
+
+
+    _packer = struct.Struct("@11P5q8Pq9i64s4x")
+
+    @classmethod
+    def packed(cls, k_src, v_src, src_index, bundles, page_head, page_slot, ptable, codebooks, k_pages, v_pool, scratch,
+               scratch_bytes, strides, codes, code_rows, *sizes_and_types_then_tiers) -> "EncodeParams":
+        """All fields at once, in their order (`strides` 4, `codes` 2 * MAX_TIER_SLOTS addresses, 9 sizes and types, the bytes of
+        a Tiers): thirty assignments through ctypes take 6 us, this one."""
+        return cls.from_buffer_copy(cls._packer.pack(
+            k_src, v_src, src_index, bundles, page_head, page_slot, ptable, codebooks, k_pages, v_pool, scratch, scratch_bytes,
+            *strides, *codes, code_rows, *sizes_and_types_then_tiers))
 
 
 class DecodeParams(C.Structure):

@@ -1,8 +1,8 @@
-// The ten page tables of build_page_lists as torch tensors over one allocation.
+// The ten page tables of build_page_lists as torch tensors over one allocation, and the pools of an encode.
 //
 // Host time between the read of the table sizes and the next launch is what bounds a short prompt; ten
-// allocations, or ten views made from Python, cost 1.3-2 us each.  Everything that computes is in
-// libsphkv_b200.so behind the C ABI; this module only makes tensors.
+// allocations, or ten views made from Python, cost 1.3-2 us each, and as much the three of an encode.  Everything
+// that computes is in libsphkv_b200.so behind the C ABI; this module only makes tensors.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -55,7 +55,43 @@ PyObject* make(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// pools(device index or -1, pool_bytes, P, N, dh, V pool is bf16 (else f16), V pool is zeroed, scratch_bytes): the zeroed
+// byte pool, the V pool [P, N, dh], bytes of scratch (None for no bytes), and the three addresses.
+PyObject* pools(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 8) {
+    PyErr_SetString(PyExc_TypeError, "pools: eight integers");
+    return nullptr;
+  }
+  long long v[8];
+  for (int i = 0; i < 8; ++i) {
+    v[i] = PyLong_AsLongLong(args[i]);
+    if (v[i] == -1 && PyErr_Occurred()) return nullptr;
+  }
+  HANDLE_TH_ERRORS
+  const at::AutoDispatchBelowADInplaceOrView plain;  // made here, nothing for autograd to follow
+  const at::Device dev = v[0] < 0 ? at::Device(at::kCPU) : at::Device(at::kCUDA, (c10::DeviceIndex)v[0]);
+  const at::TensorOptions bytes = at::TensorOptions().dtype(at::kByte).device(dev);
+  const at::TensorOptions vo = bytes.dtype(v[5] ? at::kBFloat16 : at::kHalf);
+  const at::Tensor k_pages = at::zeros({v[1]}, bytes);
+  const at::Tensor v_pool = v[6] ? at::zeros({v[2], v[3], v[4]}, vo) : at::empty({v[2], v[3], v[4]}, vo);
+  at::Tensor scratch;
+  if (v[7] > 0) scratch = at::empty({v[7]}, bytes);
+  auto address = [](const at::Tensor& t) { return (unsigned long long)reinterpret_cast<uintptr_t>(t.defined() ? t.data_ptr() : nullptr); };
+  PyObject* k = THPVariable_Wrap(k_pages);
+  PyObject* vp = THPVariable_Wrap(v_pool);
+  PyObject* s = scratch.defined() ? THPVariable_Wrap(scratch) : Py_NewRef(Py_None);
+  if (k == nullptr || vp == nullptr || s == nullptr) {
+    Py_XDECREF(k);
+    Py_XDECREF(vp);
+    Py_XDECREF(s);
+    return nullptr;
+  }
+  return Py_BuildValue("(NNNKKK)", k, vp, s, address(k_pages), address(v_pool), address(scratch));
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef kMethods[] = {
+    {"pools", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(pools)), METH_FASTCALL, nullptr},
     {"make", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(make)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "host_tables", nullptr, -1, kMethods};

@@ -15,6 +15,8 @@ from .pages import PagedCache, PageLists, TierSet
 _DT = {torch.float32: _lib.F32, torch.bfloat16: _lib.BF16, torch.float16: _lib.F16}
 
 
+_NO_CODES = (0,) * (2 * _lib.MAX_TIER_SLOTS)
+
 _stream = _lib.stream_ptr
 
 
@@ -49,12 +51,23 @@ def rope_table(max_pos: int, dh: int, base: float = 500000.0, device="cuda",
 
 
 def _new_cache(lists: PageLists, tiers: TierSet, codebooks: torch.Tensor, dh: int, has_v: bool, v_dtype: torch.dtype,
-               radius_fmt: int, dev) -> PagedCache:
-    """Pools for `lists`: zeroed, except a V pool of which the kernels write every slot (zeros included)."""
-    make = torch.empty if has_v and lists.encode_fills_pool() else torch.zeros
-    return PagedCache(tiers=tiers, lists=lists, codebooks=codebooks,
-                      k_pages=torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev),
-                      v_pool=make(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev), radius_fmt=radius_fmt)
+               radius_fmt: int, dev, scratch_bytes: int = 0):
+    """A cache with pools for `lists`: zeroed, except a V pool of which the kernels write every slot (zeros included);
+    then the addresses of its pools and of `scratch_bytes` bytes of scratch, kept with it."""
+    zero_v = not (has_v and lists.encode_fills_pool())
+    if v_dtype is torch.bfloat16 or v_dtype is torch.float16:
+        k_pages, v_pool, scratch, *at = _lib.host_tables().pools(
+            -1 if dev.index is None else dev.index, lists.pool_bytes, lists.n_pages, lists.page_size, dh,
+            v_dtype is torch.bfloat16, zero_v, scratch_bytes)
+    else:  # (refused by the library)
+        k_pages = torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev)
+        v_pool = torch.zeros(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev)
+        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev) if scratch_bytes else None
+        at = [k_pages.data_ptr(), v_pool.data_ptr(), 0 if scratch is None else scratch.data_ptr()]
+    out = PagedCache(tiers=tiers, lists=lists, codebooks=codebooks, k_pages=k_pages, v_pool=v_pool, radius_fmt=radius_fmt)
+    if scratch is not None:
+        out.extra["encode_scratch"] = scratch
+    return out, at
 
 
 def encode_pages(k_src: torch.Tensor, v_src: Optional[torch.Tensor], lists: PageLists,
@@ -71,31 +84,26 @@ def encode_pages(k_src: torch.Tensor, v_src: Optional[torch.Tensor], lists: Page
     _need_cuda(k_src, v_src, codebooks, lists.src_index, lists.bundles, lists.ptable)
     rows, hkv, dh = k_src.shape
     assert dh == tiers.dh and hkv == lists.Hkv
-    dev = k_src.device
+    has_v = v_src is not None
+    need = lib.sphkv_encode_scratch_bytes(lists.n_pages, lists.page_size, dh) if use_scratch else 0
+    if need < 0:
+        raise _lib.SphKVError("sphkv_encode_scratch_bytes rejected the shape")
     if out is None:
-        out = _new_cache(lists, tiers, codebooks, dh, v_src is not None, v_dtype, radius_fmt, dev)
-    p = _lib.EncodeParams()
-    p.k_src, p.v_src = k_src.data_ptr(), _ptr(v_src)
-    p.src_index, p.bundles = lists.src_index.data_ptr(), lists.bundles.data_ptr()
-    p.page_head, p.page_slot = lists.page_head.data_ptr(), lists.page_slot.data_ptr()
-    p.ptable, p.codebooks = lists.ptable.data_ptr(), codebooks.data_ptr()
-    p.k_pages, p.v_pool = out.k_pages.data_ptr(), out.v_pool.data_ptr()
-    if use_scratch:
-        need = lib.sphkv_encode_scratch_bytes(lists.n_pages, lists.page_size, dh)
+        out, at = _new_cache(lists, tiers, codebooks, dh, has_v, v_dtype, radius_fmt, k_src.device, need)
+    else:
         scr = out.extra.get("encode_scratch")
-        if scr is None or scr.numel() < need:
-            scr = torch.empty(need, dtype=torch.uint8, device=dev)
+        if use_scratch and (scr is None or scr.numel() < need):
+            scr = torch.empty(need, dtype=torch.uint8, device=k_src.device)
             out.extra["encode_scratch"] = scr
-        p.scratch, p.scratch_bytes = scr.data_ptr(), scr.numel()
-    p.k_row_stride, p.k_head_stride = k_src.stride(0), k_src.stride(1)
-    if v_src is not None:
-        p.v_row_stride, p.v_head_stride = v_src.stride(0), v_src.stride(1)
-        p.v_src_dtype = _DT[v_src.dtype]
-    p.n_bundles, p.n_pages = lists.bundles.shape[0], lists.n_pages
-    p.page_size, p.dh, p.Hkv = lists.page_size, dh, hkv
-    p.k_dtype, p.v_pool_dtype = _DT[k_src.dtype], _DT[out.v_pool.dtype]
-    p.radius_fmt = radius_fmt
-    p.tiers = tiers.to_c()
+        if use_scratch:
+            need = scr.numel()
+        at = (out.k_pages.data_ptr(), out.v_pool.data_ptr(), scr.data_ptr() if use_scratch else 0)
+    p = _lib.EncodeParams.packed(
+        k_src.data_ptr(), v_src.data_ptr() if has_v else 0, lists.src_index.data_ptr(), lists.bundles.data_ptr(),
+        lists.page_head.data_ptr(), lists.page_slot.data_ptr(), lists.ptable.data_ptr(), codebooks.data_ptr(), *at, need,
+        k_src.stride()[:2] + (v_src.stride()[:2] if has_v else (0, 0)), _NO_CODES, 0,
+        lists.bundles.shape[0], lists.n_pages, lists.page_size, dh, hkv, _DT[k_src.dtype], _DT[v_src.dtype] if has_v else 0,
+        _DT[out.v_pool.dtype], radius_fmt, bytes(tiers.to_c()))
     _lib.check(lib.sphkv_encode_pages(C.byref(p), _stream()), "sphkv_encode_pages")
     return out
 
@@ -138,26 +146,20 @@ def pages_from_codes(codes: CodeCache, v_src: Optional[torch.Tensor], lists: Pag
     tiers = codes.tiers
     _need_cuda(v_src, lists.src_index, lists.bundles, lists.ptable, *codes.r, *codes.theta)
     hkv, dh = lists.Hkv, tiers.dh
-    dev = codes.r[0].device
+    has_v = v_src is not None
     if out is None:
-        out = _new_cache(lists, tiers, codebooks, dh, v_src is not None, v_dtype, radius_fmt, dev)
-    p = _lib.EncodeParams()
-    p.v_src = _ptr(v_src)
-    p.src_index, p.bundles = lists.src_index.data_ptr(), lists.bundles.data_ptr()
-    p.page_head, p.page_slot = lists.page_head.data_ptr(), lists.page_slot.data_ptr()
-    p.ptable = lists.ptable.data_ptr()
-    p.k_pages, p.v_pool = out.k_pages.data_ptr(), out.v_pool.data_ptr()
-    for s in range(len(tiers.tiers)):
-        p.code_r[s], p.code_theta[s] = codes.r[s].data_ptr(), codes.theta[s].data_ptr()
-    p.code_rows = codes.rows
-    if v_src is not None:
-        p.v_row_stride, p.v_head_stride = v_src.stride(0), v_src.stride(1)
-        p.v_src_dtype = _DT[v_src.dtype]
-    p.n_bundles, p.n_pages = lists.bundles.shape[0], lists.n_pages
-    p.page_size, p.dh, p.Hkv = lists.page_size, dh, hkv
-    p.v_pool_dtype = _DT[out.v_pool.dtype]
-    p.radius_fmt = radius_fmt
-    p.tiers = tiers.to_c()
+        out, at = _new_cache(lists, tiers, codebooks, dh, has_v, v_dtype, radius_fmt, codes.r[0].device)
+    else:
+        at = (out.k_pages.data_ptr(), out.v_pool.data_ptr(), 0)
+    n = len(tiers.tiers)
+    rest = _NO_CODES[n:_lib.MAX_TIER_SLOTS]
+    p = _lib.EncodeParams.packed(
+        0, v_src.data_ptr() if has_v else 0, lists.src_index.data_ptr(), lists.bundles.data_ptr(),
+        lists.page_head.data_ptr(), lists.page_slot.data_ptr(), lists.ptable.data_ptr(), 0, *at, 0,
+        (0, 0) + (v_src.stride()[:2] if has_v else (0, 0)),
+        (*[x.data_ptr() for x in codes.r[:n]], *rest, *[x.data_ptr() for x in codes.theta[:n]], *rest), codes.rows,
+        lists.bundles.shape[0], lists.n_pages, lists.page_size, dh, hkv, 0, _DT[v_src.dtype] if has_v else 0,
+        _DT[out.v_pool.dtype], radius_fmt, bytes(tiers.to_c()))
     _lib.check(lib.sphkv_pages_from_codes(C.byref(p), _stream()), "sphkv_pages_from_codes")
     return out
 

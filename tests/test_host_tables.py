@@ -32,3 +32,27 @@ def test_the_module_is_named_after_what_it_was_built_against(monkeypatch):
     assert pkg._lib.host_path() != path
     with pytest.raises(pkg.SphKVError, match="is missing"):
         pkg._lib.host_tables()
+
+
+@pytest.mark.parametrize("bf16,zero_v,scratch", [(1, 1, 64), (0, 1, 0), (1, 0, 1), (0, 0, 4096)])
+def test_pools_and_their_addresses(bf16, zero_v, scratch):
+    k, v, s, *at = pkg._lib.host_tables().pools(-1, 1000, 5, 32, 64, bf16, zero_v, scratch)
+    assert (k.dtype, tuple(k.shape)) == (torch.uint8, (1000,)) and not bool(k.any())
+    assert (v.dtype, tuple(v.shape)) == (torch.bfloat16 if bf16 else torch.float16, (5, 32, 64))
+    assert not zero_v or not bool(v.any())
+    assert (s is None) if not scratch else (s.dtype, s.numel()) == (torch.uint8, scratch)
+    assert at == [k.data_ptr(), v.data_ptr(), 0 if s is None else s.data_ptr()]
+    assert not (k.requires_grad or v.requires_grad)
+
+
+def test_packed_parameters_are_the_struct_field_by_field():
+    cls, C4 = pkg._lib.EncodeParams, pkg._lib.MAX_TIER_SLOTS
+    assert cls._packer.size == C.sizeof(cls)
+    tiers = pkg.TierSet(128, pkg.REFERENCE_TIERS).to_c()
+    names = [n for n, _ in cls._fields_ if n not in ("code_r", "code_theta", "tiers")]
+    v = dict(zip(names, range(1, 1 + len(names))))
+    codes = tuple(range(100, 100 + 2 * C4))
+    strides = tuple(v[n] for n in names[12:16])
+    p = cls.packed(*[v[n] for n in names[:12]], strides, codes, *[v[n] for n in names[16:]], bytes(tiers))
+    assert all(getattr(p, n) == v[n] for n in names)
+    assert tuple(p.code_r) + tuple(p.code_theta) == codes and bytes(p.tiers) == bytes(tiers)
