@@ -251,11 +251,15 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   const sphkv_decode_params& p = a.p;
   // What the loops use most of the thread's place comes out of shuffles, whose results stay in registers: short of those,
   // the compiler reads the special register again, and waits for it, or makes an address again at every use.  Of four such
-  // addresses these two fit (barriers or the base of shared memory as well: spills, 8 x 32768 147 -> 159 us).
-  auto keep = [](auto x) { return __shfl_sync(0xffffffffu, x, 0); };
-  const int warp = keep((int)(threadIdx.x >> 5)), lane = __shfl_sync(0xffffffffu, (int)(threadIdx.x & 31), (int)(threadIdx.x & 31));
+  // addresses two fit beside the code for 16-token int8 pages, or beside dh 64 (barriers or the base of shared memory as
+  // well: spills, 8 x 32768 147 -> 159 us); elsewhere the team alone (2 x 30614 tokens, 32-token pages: 55.6 us with
+  // none, 57.0 with the two, 54.8).
+  constexpr bool kKeepBases = FAST || DH == 64;
+  auto keep = [](bool yes, auto x) { return yes ? __shfl_sync(0xffffffffu, x, 0) : x; };
+  const int warp = keep(true, (int)(threadIdx.x >> 5));
+  const int lane = __shfl_sync(0xffffffffu, (int)(threadIdx.x & 31), (int)(threadIdx.x & 31));
   const bool driver = warp >= 4 * kTeams;
-  const int team = driver ? warp - 4 * kTeams : warp >> 2;
+  const int team = keep(!kKeepBases, driver ? warp - 4 * kTeams : warp >> 2);
   const bool in_use = team < a.teams;  // (the fourth driver warp never is; idle warps do not use their addresses)
 
   const uint32_t smem0 = smem_u32(smem);
@@ -267,7 +271,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   auto stats_of = [&](int t) { return reinterpret_cast<float*>(smem + kSmemQ + t * kSmemTeamBars + kBarStride + 32 + 128); };
   auto mref_of = [&](int t) { return stats_of(t) + 64; };
   volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + kSmemQ + kTeams * kSmemTeamBars);
-  const uint32_t v_buf = keep(smem0 + kSmemHead + team * smem_team_bytes(DH));
+  const uint32_t v_buf = keep(kKeepBases, smem0 + kSmemHead + team * smem_team_bytes(DH));
   const uint32_t p_buf = v_buf + smem_v_bytes(DH), k_ring = p_buf + kSmemP, meta = k_ring + kSmemK;
   const uint32_t cb_off = kSmemHead + a.teams * smem_team_bytes(DH);
 
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, shared_words[0], 0);
-  const uint32_t tmem = keep(tmem_base + team * kTeamCols);
+  const uint32_t tmem = keep(kKeepBases, tmem_base + team * kTeamCols);
   // everything above touched shared and tensor memory only: this grid's launch overlaps the tail of the
   // kernel before it in the stream (the previous step's merge kernel, which lets it in early)
   griddep_wait();
