@@ -20,6 +20,10 @@ constexpr int kListThreads = 256;
 constexpr int kListPer = 8;                           // tokens per thread
 constexpr int kListChunk = kListThreads * kListPer;   // tokens per CTA
 constexpr int kScanThreads = 1024;
+constexpr int kScanRuns = 1024;                       // runs whose token counts the scan keeps in shared memory
+// The four totals go to the host as words that carry the number of the call in their upper 16 bits, so that each
+// says by itself that it has arrived.
+constexpr int kTotalBits = 48;
 
 struct ListArgs {
   const void* assign;  // [U][T] tier ids
@@ -28,7 +32,7 @@ struct ListArgs {
   int U, Hkv, S, n_chunks, N, n_shift, rb, align;
   int tier_id[SPHKV_MAX_TIER_SLOTS], G[SPHKV_MAX_TIER_SLOTS], bits[SPHKV_MAX_TIER_SLOTS];
   // scratch; run r = slot * U + unit
-  int64_t* totals;     // pinned host memory: pages, most blocks of a unit, bundles, pool bytes, call number
+  int64_t* totals;     // pinned host memory: pages, most blocks of a unit, bundles, pool bytes (see kTotalBits)
   int64_t call;
   int64_t* byte_base;  // [S*U] pool offset of the run's first page
   int32_t* cnt;        // [S*U] tokens
@@ -127,6 +131,7 @@ __device__ __forceinline__ T block_exclusive(T v, T* s_part, T& total) {
 __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs a) {
   __shared__ int64_t s_part[kScanThreads / 32];
   __shared__ int s_max[kScanThreads / 32];
+  __shared__ int s_n[kScanRuns];
   griddep_wait();
   const int n_runs = a.S * a.U, ppb = 128 >> a.n_shift;
   int64_t c_pages = 0, c_bundles = 0, c_bytes = 0;
@@ -155,6 +160,7 @@ __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs 
     const int64_t x_pb = block_exclusive<int64_t>(((int64_t)pages << 32) | (int64_t)((pages + ppb - 1) / ppb), s_part, t_pb);
     const int64_t x_bytes = block_exclusive<int64_t>(bytes, s_part, t_bytes);
     if (r < n_runs) {
+      if (n_runs <= kScanRuns) s_n[r] = n;
       a.cnt[r] = n;
       a.run_base[r] = (int32_t)(c_pages + (x_pb >> 32));
       a.bun_base[r] = (int32_t)(c_bundles + (x_pb & 0xFFFFFFFFLL));
@@ -165,47 +171,53 @@ __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs 
     c_bytes += t_bytes;
   }
   __syncthreads();
+  const int* counts = n_runs <= kScanRuns ? s_n : a.cnt;
   int most = 0;
   for (int u = threadIdx.x; u < a.U; u += blockDim.x) {
     int col = 0;
     for (int s = 0; s < a.S; ++s) {
       a.col_base[s * a.U + u] = col;
-      col += (a.cnt[s * a.U + u] + a.N - 1) >> a.n_shift;
+      col += (counts[s * a.U + u] + a.N - 1) >> a.n_shift;
     }
     most = max(most, col);
   }
   most = __reduce_max_sync(0xffffffffu, most);
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = most;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) most = max(most, s_max[w]);
-    a.totals[0] = c_pages;
-    a.totals[1] = most;
-    a.totals[2] = c_bundles;
-    a.totals[3] = c_bytes + 16;
-    __threadfence_system();
-    *reinterpret_cast<volatile int64_t*>(a.totals + 4) = a.call;  // the host polls this word
+  if (threadIdx.x < 4) {  // the host polls these words
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) most = max(most, s_max[w]);
+    const int64_t v = threadIdx.x == 0 ? c_pages : threadIdx.x == 1 ? most : threadIdx.x == 2 ? c_bundles : c_bytes + 16;
+    *reinterpret_cast<volatile int64_t*>(a.totals + threadIdx.x) = v | (int64_t)((uint64_t)a.call << kTotalBits);
   }
 }
-
 // grid (chunk, unit): the chunk's tokens are compacted per tier slot in shared memory (order kept) and
 // written out in rank order, so neighbouring threads write neighbouring page slots; the unit's page
 // records are dealt out over its chunks' threads.
 __global__ void __launch_bounds__(kListThreads) list_fill_kernel(const ListArgs a, const ListOut o) {
   __shared__ uint16_t s_tok[kListChunk];
   __shared__ int s_part[kListThreads / 32];
+  __shared__ int s_run[SPHKV_MAX_TIER_SLOTS][5];  // tokens, first page, bundle and column, tokens before this chunk
+  __shared__ int64_t s_byte[SPHKV_MAX_TIER_SLOTS];
   const int chunk = blockIdx.x, u = blockIdx.y, tid = threadIdx.x;
   const int N = a.N, ppb = 128 >> a.n_shift;
   griddep_launch();
+  // what the loop over the slots reads of the scan: one latency instead of one per slot and use
+  if (tid < 32 * SPHKV_MAX_TIER_SLOTS && (tid >> 5) < a.S) {
+    const int s = tid >> 5, r = s * a.U + u, e = tid & 31;
+    const int32_t* from = e == 0 ? a.cnt : e == 1 ? a.run_base : e == 2 ? a.bun_base : a.col_base;
+    if (e < 4) s_run[s][e] = from[r];
+    if (e == 4) s_run[s][4] = a.chunk_cnt[(int64_t)r * a.n_chunks + chunk];
+    if (e == 5) s_byte[s] = a.byte_base[r];
+  }
   const int64_t t_first = (int64_t)chunk * kListChunk;
   const int64_t row_first = (int64_t)(u / a.Hkv) * a.T;
   int64_t v[kListPer];
   load_tiers(a, u, t_first + tid * kListPer, v);
+  __syncthreads();
   auto phys = [&](int64_t lp) -> int64_t { return o.perm != nullptr ? o.perm[lp] : lp; };
   int nb = 0;
   for (int s = 0; s < a.S; ++s) {
-    const int r = s * a.U + u;
-    const int n = a.cnt[r], pages = (n + N - 1) >> a.n_shift, base = a.run_base[r];
+    const int n = s_run[s][0], pages = (n + N - 1) >> a.n_shift, base = s_run[s][1];
     uint32_t m = slot_mask(a, s, v);
     int mine;
     int at = block_exclusive<int>(__popc(m), s_part, mine);  // its barriers also order s_tok between slots
@@ -214,7 +226,7 @@ __global__ void __launch_bounds__(kListThreads) list_fill_kernel(const ListArgs 
       m &= m - 1;
     }
     __syncthreads();
-    const int rank0 = a.chunk_cnt[(int64_t)r * a.n_chunks + chunk];
+    const int rank0 = s_run[s][4];
     for (int i = tid; i < mine; i += kListThreads) {
       const int rank = rank0 + i;
       const int64_t t = t_first + s_tok[i];
@@ -238,15 +250,15 @@ __global__ void __launch_bounds__(kListThreads) list_fill_kernel(const ListArgs 
       if (o.perm != nullptr) {
         o.ptable[3 * ph] = (int32_t)page_bytes(a, s, count);  // list_offsets_kernel turns sizes into offsets
       } else {
-        const int64_t off = a.byte_base[r] + p * full, th = off + 8 + 4 * a.G[s];
+        const int64_t off = s_byte[s] + p * full, th = off + 8 + 4 * a.G[s];
         o.ptable[3 * ph] = (int32_t)off;
         o.ptable[3 * ph + 1] = (int32_t)th;
         o.ptable[3 * ph + 2] = (int32_t)(th + (((int64_t)count * a.G[s] * a.bits[s] + 7) >> 3));
       }
-      const int64_t cell = (int64_t)u * o.max_blocks + a.col_base[r] + p;
+      const int64_t cell = (int64_t)u * o.max_blocks + s_run[s][3] + p;
       o.block_table[cell] = (int32_t)ph;
       o.bits_table[cell] = s;
-      int32_t* bun = o.bundles + 8 * ((int64_t)a.bun_base[r] + p / ppb);
+      int32_t* bun = o.bundles + 8 * ((int64_t)s_run[s][2] + p / ppb);
       bun[p % ppb] = (int32_t)ph;
       if (p == pages - 1 || p % ppb == ppb - 1)  // the record's last page clears what follows it
         for (int e = p % ppb + 1; e < 8; ++e) bun[e] = -1;
@@ -298,10 +310,10 @@ struct PinnedTotals {
   int64_t calls = 0;
   int64_t* get() {
     if (p == nullptr) {
-      if (cudaHostAlloc(reinterpret_cast<void**>(&p), 5 * sizeof(int64_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+      if (cudaHostAlloc(reinterpret_cast<void**>(&p), 4 * sizeof(int64_t), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
         p = nullptr;
       else
-        p[4] = 0;
+        p[0] = p[1] = p[2] = p[3] = 0;
     }
     return p;
   }
@@ -368,21 +380,26 @@ extern "C" int sphkv_page_lists_count(const sphkv_page_lists_params* p, int64_t*
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   a.totals = host;
   a.call = ++pinned.calls;
-  list_count_kernel<<<dim3(a.n_chunks, a.U), kListThreads, 0, st>>>(a);
   // as many warps as there are runs for (the prefix over the warps is serial)
   const int scan_threads = std::min(kScanThreads, (a.S * a.U + 31) / 32 * 32);
+  list_count_kernel<<<dim3(a.n_chunks, a.U), kListThreads, 0, st>>>(a);
   (void)launch_overlapped(list_scan_kernel, dim3(1), dim3(scan_threads), 0, st, a);
   if (int rc = check_launch("page_lists_count")) return rc;
-  // The host needs nothing but the totals, so it waits for the word behind them, not for the stream.  An
-  // error, or a stream that has ended without it, ends the wait.
-  for (int64_t spins = 1; __atomic_load_n(host + 4, __ATOMIC_ACQUIRE) != a.call; ++spins) {
+  // The host needs nothing but the totals, so it waits for these words, not for the stream.  An error, or a stream
+  // that has ended without them, ends the wait.
+  const auto arrived = [&]() {
+    for (int i = 0; i < 4; ++i)
+      if ((uint64_t)__atomic_load_n(host + i, __ATOMIC_ACQUIRE) >> kTotalBits != ((uint64_t)a.call & 0xFFFF)) return false;
+    return true;
+  };
+  for (int64_t spins = 1; !arrived(); ++spins) {
     if (spins % 16384 != 0) continue;
     const cudaError_t e = cudaStreamQuery(st);
-    if (e == cudaErrorNotReady || __atomic_load_n(host + 4, __ATOMIC_ACQUIRE) == a.call) continue;
+    if (e == cudaErrorNotReady || arrived()) continue;
     set_error("page_lists_count: %s", e == cudaSuccess ? "the totals did not arrive" : cudaGetErrorString(e));
     return e == cudaSuccess ? (int)cudaErrorUnknown : (int)e;
   }
-  for (int i = 0; i < 4; ++i) totals[i] = host[i];
+  for (int i = 0; i < 4; ++i) totals[i] = host[i] & ((INT64_C(1) << kTotalBits) - 1);
   return 0;
 }
 

@@ -30,6 +30,22 @@ def test_page_lists_on_device_equal_host_construction(B, Hkv, T, page_size, radi
         assert torch.equal(getattr(got, name).cpu(), getattr(want, name)), name
 
 
+# runs (heads x tiers) that one warp, several, all of a block take, and more than it keeps counts of in shared memory
+@pytest.mark.parametrize("Hkv,T", [(5, 100), (11, 2049), (341, 64), (342, 64), (700, 40)])
+def test_totals_of_each_call_and_tables_equal_host_construction(Hkv, T):
+    tiers = pkg.TierSet(128, pkg.REFERENCE_TIERS)
+    assign = pkg.synth.make_tier_assign(1, Hkv, T, {1: 0.3, 2: 0.4, 3: 0.1}, seed=T, per_head=True)
+    assign[0, Hkv // 2] = 0
+    want = pkg.build_page_lists(assign, tiers, 32)
+    for _ in range(3):  # the totals of one call are not taken for the next one's
+        got = pkg.build_page_lists(assign.to("cuda:0"), tiers, 32)
+        assert (got.n_pages, got.max_blocks, got.pool_bytes) == (want.n_pages, want.max_blocks, want.pool_bytes)
+        for name in TABLES:
+            assert torch.equal(getattr(got, name).cpu(), getattr(want, name)), name
+        assign[0, 0, : T // 2] = 0
+        want = pkg.build_page_lists(assign, tiers, 32)
+
+
 def test_page_lists_reject_empty_assignment():
     with pytest.raises(ValueError, match="no retained tokens"):
         pkg.build_page_lists(torch.zeros(1, 2, 50, dtype=torch.uint8, device="cuda:0"), pkg.TierSet(128), 16)
