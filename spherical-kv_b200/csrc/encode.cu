@@ -100,30 +100,32 @@ __device__ __forceinline__ uint4 load_v_chunk(const sphkv_encode_params& p, bool
 
 constexpr int kMaxBundlesPerCta = 8;  // consecutive bundles one CTA walks (they mostly share a codebook)
 
-// Squared norm and nearest centroid of four tokens' GS-dim group vectors: the fixed fma chains that
+// Squared norm and nearest centroid of TOK tokens' GS-dim group vectors: the fixed fma chains that
 // define the encoder bit for bit (d = 0 .. GS-1 from 0; first maximum wins).  Every centroid row
-// read from shared memory (`cbg`, [C][GS]) feeds four dot products.
-template <int GS>
-__device__ __forceinline__ void search_four_tokens(const float (&k)[4][GS], const float* __restrict__ cbg, int C,
-                                                   float (&nsq)[4], int (&code)[4]) {
+// read from shared memory (`cbg`, [C][GS]) feeds TOK dot products.
+template <int GS, int TOK>
+__device__ __forceinline__ void search_tokens(const float (&k)[TOK][GS], const float* __restrict__ cbg, int C, float (&nsq)[TOK],
+                                              int (&code)[TOK]) {
 #pragma unroll
-  for (int h = 0; h < 4; ++h) nsq[h] = 0.f;
+  for (int h = 0; h < TOK; ++h) nsq[h] = 0.f;
 #pragma unroll
   for (int d = 0; d < GS; ++d)
 #pragma unroll
-    for (int h = 0; h < 4; ++h) nsq[h] = __fmaf_rn(k[h][d], k[h][d], nsq[h]);
-  float best[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    for (int h = 0; h < TOK; ++h) nsq[h] = __fmaf_rn(k[h][d], k[h][d], nsq[h]);
+  float best[TOK];
 #pragma unroll
-  for (int h = 0; h < 4; ++h) code[h] = 0;
+  for (int h = 0; h < TOK; ++h) { best[h] = -INFINITY; code[h] = 0; }
   SPHKV_UNROLL_SEARCH
   for (int c = 0; c < C; ++c) {
     const float4* row = reinterpret_cast<const float4*>(cbg + c * GS);
-    float sacc[4] = {0.f, 0.f, 0.f, 0.f};
+    float sacc[TOK];
+#pragma unroll
+    for (int h = 0; h < TOK; ++h) sacc[h] = 0.f;
 #pragma unroll
     for (int i = 0; i < GS / 4; ++i) {
       const float4 v = row[i];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
+      for (int h = 0; h < TOK; ++h) {
         sacc[h] = __fmaf_rn(k[h][4 * i], v.x, sacc[h]);
         sacc[h] = __fmaf_rn(k[h][4 * i + 1], v.y, sacc[h]);
         sacc[h] = __fmaf_rn(k[h][4 * i + 2], v.z, sacc[h]);
@@ -131,7 +133,7 @@ __device__ __forceinline__ void search_four_tokens(const float (&k)[4][GS], cons
       }
     }
 #pragma unroll
-    for (int h = 0; h < 4; ++h)
+    for (int h = 0; h < TOK; ++h)
       if (sacc[h] > best[h]) { best[h] = sacc[h]; code[h] = c; }
   }
 }
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
       }
       float nsq[4];
       int code[4];
-      search_four_tokens<GS>(k, cbg, C, nsq, code);
+      search_tokens<GS>(k, cbg, C, nsq, code);
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
         const int ts = lane + 32 * h;
@@ -416,7 +418,9 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
 // load fetched 32 sectors and used half of each (GS 16: 106 -> 86 us for a 32768-token prompt).  Chunk c
 // of row s is stored at chunk c ^ turn(s), so neither the copies nor the row-per-lane reads meet in a bank.
 // Not STAGED: slices off a 16-byte boundary.
-template <int GS, bool STAGED>
+// TOK token slots per lane: 4 are a bundle; of few bundles a CTA takes a half or a quarter (blockIdx.y), so that all SMs
+// search (see the rule at the launch).
+template <int GS, bool STAGED, int TOK>
 __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
   griddep_wait();
@@ -428,30 +432,30 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int G = dh / GS, GST = dh >> 4;
   const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
-  const int chunk_len = a.search_chunk;
+  const int chunk_len = a.search_chunk, slot0 = 32 * TOK * blockIdx.y;
   float* scr_r = reinterpret_cast<float*>(p.scratch);
   uint8_t* scr_t = reinterpret_cast<uint8_t*>(p.scratch) + (int64_t)p.n_pages * N * GST * 4;
-  // page and source row of this lane's four token slots of bundle bi
-  auto lookup = [&](int64_t bi, int (&pg)[4], int (&row)[4]) {
+  // page and source row of this lane's token slots of bundle bi
+  auto lookup = [&](int64_t bi, int (&pg)[TOK], int (&row)[TOK]) {
     const int32_t* bundle = p.bundles + 8 * bi;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const int ts = lane + 32 * h;
+    for (int h = 0; h < TOK; ++h) {
+      const int ts = slot0 + lane + 32 * h;
       pg[h] = bundle[ts >> n_shift];
       row[h] = pg[h] >= 0 ? p.src_index[(int64_t)pg[h] * N + (ts & (N - 1))] : -1;
     }
   };
   // 16-byte chunks of a row slice: GS / 4 (fp32) or GS / 8
   const int ch_shift = (GS == 32 ? 3 : 2) - (esize == 2 ? 1 : 0), ch = 1 << ch_shift;
-  const uint32_t kbuf = smem_u32(smem + a.search_kbuf) + warp * (128 * GS * 4);
+  const uint32_t kbuf = smem_u32(smem + a.search_kbuf) + warp * (32 * TOK * GS * 4);
   auto turn = [&](int s) { return (s >> (3 - ch_shift)) & (ch - 1); };
-  auto issue_rows = [&](const int (&row)[4], int head) {
+  auto issue_rows = [&](const int (&row)[TOK], int head) {
     const int s_l = lane >> ch_shift, c = lane & (ch - 1), rows_per = 32 >> ch_shift;
     const char* base = reinterpret_cast<const char*>(p.k_src) + ((int64_t)head * p.k_head_stride + warp * GS) * esize + c * 16;
     const int64_t row_bytes = p.k_row_stride * esize;
 #pragma unroll
-    for (int h = 0; h < 4; ++h)
-      for (int i = 0; i < ch; ++i) {  // 32 rows of quarter h, rows_per at a time
+    for (int h = 0; h < TOK; ++h)
+      for (int i = 0; i < ch; ++i) {  // 32 rows, rows_per at a time
         const int s = i * rows_per + s_l;
         const int r = __shfl_sync(0xffffffffu, row[h], s);
         cp_async_16_zfill(kbuf + (((32 * h + s) << ch_shift) + (c ^ turn(s))) * 16, r >= 0 ? base + r * row_bytes : reinterpret_cast<const char*>(p.k_src),
@@ -478,7 +482,7 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
       }
     }
     unsigned todo = __ballot_sync(0xffffffffu, my_head >= 0 && p.tiers.g[my_slot] == GS);  // same in every warp
-    int pg_n[4], row_n[4];
+    int pg_n[TOK], row_n[TOK];
     if (todo) {
       lookup(chunk * chunk_len + (__ffs(todo) - 1), pg_n, row_n);
       if (STAGED && warp < G) issue_rows(row_n, __shfl_sync(0xffffffffu, my_head, __ffs(todo) - 1));
@@ -487,9 +491,9 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
       const int q = __ffs(todo) - 1;
       todo &= todo - 1;
       const int head = __shfl_sync(0xffffffffu, my_head, q), slot = __shfl_sync(0xffffffffu, my_slot, q);
-      int pg[4], row[4];
+      int pg[TOK], row[TOK];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) { pg[h] = pg_n[h]; row[h] = row_n[h]; }
+      for (int h = 0; h < TOK; ++h) { pg[h] = pg_n[h]; row[h] = row_n[h]; }
       int head_n = -1;
       if (todo) {  // the next bundle of the chunk: its rows load while this one is searched
         const int qn = __ffs(todo) - 1;
@@ -504,12 +508,12 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
       }
       if (warp >= G) continue;
       const int bits = p.tiers.bits[slot];
-      float k[4][GS];
+      float k[TOK][GS];
       if (STAGED) {
         cp_async_wait<0>();
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
+        for (int h = 0; h < TOK; ++h) {
           const uint32_t src = kbuf + (((32 * h + lane) << ch_shift) * 16);
           if (esize == 4) {
 #pragma unroll
@@ -532,14 +536,14 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
       } else {
         if (head_n >= 0) {
 #pragma unroll
-          for (int h = 0; h < 4; ++h)
+          for (int h = 0; h < TOK; ++h)
             if (row_n[h] >= 0)
               asm volatile("prefetch.global.L2 [%0];" ::"l"(
                   reinterpret_cast<const char*>(p.k_src) +
                   ((int64_t)row_n[h] * p.k_row_stride + (int64_t)head_n * p.k_head_stride + warp * GS) * esize));
         }
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
+        for (int h = 0; h < TOK; ++h) {
           if (row[h] >= 0) {
             load_group<GS>(p.k_src, p.k_dtype,
                            (int64_t)row[h] * p.k_row_stride + (int64_t)head * p.k_head_stride + warp * GS, k[h]);
@@ -549,13 +553,13 @@ __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_
           }
         }
       }
-      float nsq[4];
-      int code[4];
-      search_four_tokens<GS>(k, cb_s + (warp << bits) * GS, 1 << bits, nsq, code);
+      float nsq[TOK];
+      int code[TOK];
+      search_tokens<GS>(k, cb_s + (warp << bits) * GS, 1 << bits, nsq, code);
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
+      for (int h = 0; h < TOK; ++h) {
         if (pg[h] < 0) continue;
-        const int64_t si = ((int64_t)pg[h] * N + ((lane + 32 * h) & (N - 1))) * GST + warp;
+        const int64_t si = ((int64_t)pg[h] * N + ((slot0 + lane + 32 * h) & (N - 1))) * GST + warp;
         scr_r[si] = row[h] >= 0 ? __fsqrt_rn(nsq[h]) : 0.f;
         scr_t[si] = (uint8_t)code[h];
       }
@@ -1375,27 +1379,37 @@ int validate_tiers(const sphkv_tiers& t, int dh);
 
 using namespace sphkv;
 
+template <int GS, int TOK>
+static int launch_search_parts(const EncodeArgs& a, int resident, cudaStream_t st) {
+  static SmemOptIn opt_in[2];
+  const sphkv_encode_params& p = a.p;
+  const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
+  const int cb_bytes = p.dh * p.tiers.C_max * 4, row_bytes = p.dh / GS * 32 * TOK * GS * 4;
+  // staged rows need aligned slices, and room beside a codebook tensor of any C_max (dh 128, four slots a lane: up to 326)
+  const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
+                      (p.k_head_stride * esize) % 16 == 0 && cb_bytes + row_bytes <= 227 * 1024;
+  const int smem = cb_bytes + (staged ? row_bytes : 0);
+  auto kern = staged ? search_bundles_kernel<GS, true, TOK> : search_bundles_kernel<GS, false, TOK>;
+  if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem, "encode search")) return rc;
+  EncodeArgs b = a;
+  b.search_kbuf = cb_bytes;
+  b.search_chunk = std::max(1, std::min(8, p.n_bundles / (resident * 4)));  // >= 4 chunks per CTA, <= 8 bundles each
+  const int grid = std::max(1, std::min((p.n_bundles + b.search_chunk - 1) / b.search_chunk, resident));
+  (void)launch_overlapped(kern, dim3(grid, 4 / TOK), dim3(kEncThreads), smem, st, b);
+  return check_launch("search_bundles_kernel");
+}
+
 template <int GS>
 static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaStream_t st) {
   if (split) {
-    // persistent: as many CTAs as are resident at once, each striding over chunks of bundles
-    static SmemOptIn opt_in[2];
-    const sphkv_encode_params& p = a.p;
-    const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
-    const int cb_bytes = p.dh * p.tiers.C_max * 4, row_bytes = p.dh / GS * 128 * GS * 4;
-    // staged rows need aligned slices, and room beside a codebook tensor of any C_max (dh 128: up to 326)
-    const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
-                        (p.k_head_stride * esize) % 16 == 0 && cb_bytes + row_bytes <= 227 * 1024;
-    const int smem = cb_bytes + (staged ? row_bytes : 0);
-    auto kern = staged ? search_bundles_kernel<GS, true> : search_bundles_kernel<GS, false>;
-    if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem, "encode search")) return rc;
+    // Persistent: as many CTAs as are resident at once, each striding over chunks of bundles.  A CTA takes all 128 slots
+    // of a bundle, or a half or a quarter while that still leaves every CTA resident: few bundles leave SMs idle, and the
+    // search of one alone is half of the launch.  Lists and pages of 777 tokens x 8 heads (45 bundles, quarters): 59.4 -> 57.4 us.
     const int resident = sm_count_current_device() * (GS == 16 ? 2 : 1);
-    EncodeArgs b = a;
-    b.search_kbuf = cb_bytes;
-    b.search_chunk = std::max(1, std::min(8, a.p.n_bundles / (resident * 4)));  // >= 4 chunks per CTA, <= 8 bundles each
-    const int grid = std::max(1, std::min((a.p.n_bundles + b.search_chunk - 1) / b.search_chunk, resident));
-    (void)launch_overlapped(kern, dim3(grid), dim3(kEncThreads), smem, st, b);
-    return check_launch("search_bundles_kernel");
+    const int parts = 4 * a.p.n_bundles <= resident ? 4 : 2 * a.p.n_bundles <= resident ? 2 : 1;
+    return parts == 4   ? launch_search_parts<GS, 1>(a, resident, st)
+           : parts == 2 ? launch_search_parts<GS, 2>(a, resident, st)
+                        : launch_search_parts<GS, 4>(a, resident, st);
   }
   const int grid = (a.p.n_bundles + a.bundles_per_cta - 1) / a.bundles_per_cta;
   encode_bundle_kernel<GS><<<grid, kEncThreads, smem_bytes, st>>>(a);

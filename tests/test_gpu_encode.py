@@ -190,3 +190,20 @@ def test_encode_ties_and_near_ties_pick_the_chain_argmax(use_scratch):
     got = cache.k_pages.cpu().numpy()
     bad = np.nonzero(got != want)[0]
     assert bad.size == 0, f"{bad.size} byte(s) differ, first at {bad[:8]}"
+
+
+# bundles (of 128 slots) at the lines between quarters, halves and whole ones per CTA, on 148 SMs, for groups of 16 and of
+# 32 dims; keys off a 16-byte boundary take the kernel without staged rows
+@pytest.mark.parametrize("tier,bundles", [(1, 1), (1, 74), (1, 75), (2, 148), (2, 149), (3, 37), (3, 38), (3, 74), (3, 75)])
+@pytest.mark.parametrize("dtype,offset", [(torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)])
+def test_parts_of_bundles_give_the_fused_encoders_pages(tier, bundles, dtype, offset):
+    dh, T = 128, 128 * bundles - 3
+    tiers = pkg.TierSet(dh, pkg.REFERENCE_TIERS)
+    g = torch.Generator(device="cuda:0").manual_seed(bundles)
+    K = torch.randn(T * dh + offset, generator=g, device="cuda:0").to(dtype)[offset:].view(T, 1, dh)
+    cb = tiers.pack_codebooks([torch.randn(1, dh // t.g, 1 << t.b_theta, t.g, generator=g, device="cuda:0") for t in pkg.REFERENCE_TIERS])
+    lists = pkg.build_page_lists(torch.full((1, 1, T), tier, dtype=torch.uint8, device="cuda:0"), tiers, 64)
+    assert lists.bundles.shape[0] == bundles
+    split = pkg.encode_pages(K, K, lists, cb, tiers)
+    fused = pkg.encode_pages(K, K, lists, cb, tiers, use_scratch=False)
+    assert torch.equal(split.k_pages, fused.k_pages) and torch.equal(split.v_pool, fused.v_pool)
