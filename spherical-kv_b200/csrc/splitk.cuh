@@ -223,8 +223,9 @@ static_assert(kBarCount * 8 <= kBarStride, "barrier block");
 // keys in flight and nothing else, twelve team warps fit an SM (the mma.sync version it replaced: eight, at
 // 244 registers, and shuffles, ldmatrix and accumulator moves around both products).
 // Bound: instruction issue and the waits between the roles, not HBM.  A 96-bit, 32768-token, batch-8 layer
-// step, merge included, in a short loop: 159 -> 147 us (3.4 -> 3.7 TB/s of the bytes it has to read) with 666
-// instructions a tile instead of 755, since team addresses lie at constant offsets and stay in registers.
+// step, merge included, in a short loop: 159 -> 141 us (3.4 -> 3.8 TB/s of the bytes it has to read): 666
+// instructions a tile instead of 755, since team addresses lie at constant offsets and stay in registers (147), then
+// cos/sin past L1.
 // Lane map of the rebuild (lane = 4 r + j): rows r and r + 8 of a tile are the lane's two tokens; in each
 // rotary half the lane owns the contiguous block of W = dh / 8 dimensions  W j .. W j + W - 1, and in the
 // other half the same block shifted by dh / 2: the RoPE partner of every value a lane holds is in the same
@@ -790,7 +791,9 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       auto clamp_pos = [&](int pos) -> uint32_t { return (uint32_t)pos < (uint32_t)p.max_pos ? (uint32_t)pos : 0u; };
       // cos/sin of this lane's two key positions: one 256-bit load per (token, chunk) brings the
       // chunk's {cos x 4, sin x 4} (the table is L2 resident), issued for the next pass once this one
-      // has used its own
+      // has used its own.  A row's lines are used whole by one load and not again: past the 30 KB of L1 that the
+      // shared memory leaves (1 x 131072 88.5 -> 83.7 us, 8 x 32768 146.9 -> 141.0; the read-only path, without L1,
+      // 84.4 and 143.8).  Pages that are staged in pieces gain nothing (one of 424 tokens: 14.25 us, past L1 14.39)
       float4 cs[2][NCH][2];
       const float4* cs_src[2] = {nullptr, nullptr};  // this lane's pieces of the two table rows
       auto cs_rows = [&](uint32_t st) {              // positions of K stage `st`
@@ -804,11 +807,17 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       auto issue_cs_chunk = [&](int i) {
         if constexpr (ROT) {
 #pragma unroll
-          for (int tk = 0; tk < 2; ++tk)
-            asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                         : "=f"(cs[tk][i][0].x), "=f"(cs[tk][i][0].y), "=f"(cs[tk][i][0].z), "=f"(cs[tk][i][0].w),
-                           "=f"(cs[tk][i][1].x), "=f"(cs[tk][i][1].y), "=f"(cs[tk][i][1].z), "=f"(cs[tk][i][1].w)
-                         : "l"(cs_src[tk] + i * 8));
+          for (int tk = 0; tk < 2; ++tk) {
+            float4 &c = cs[tk][i][0], &n = cs[tk][i][1];
+            if (FAST)
+              asm volatile("ld.global.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                           : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w), "=f"(n.x), "=f"(n.y), "=f"(n.z), "=f"(n.w)
+                           : "l"(cs_src[tk] + i * 8));
+            else
+              asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                           : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w), "=f"(n.x), "=f"(n.y), "=f"(n.z), "=f"(n.w)
+                           : "l"(cs_src[tk] + i * 8));
+          }
         }
       };
       // K stage of tile x in ring slot `slot`; parities of the slots are bits of par_k
