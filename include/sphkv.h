@@ -247,6 +247,10 @@ typedef struct sphkv_decode_params {
 #define SPHKV_ST_INTERNAL 16    /* the kernel found its shared memory misaligned      */
 
 int64_t sphkv_decode_scratch_bytes(int32_t B, int32_t Hkv, int32_t dh, int32_t n_ctas);
+/* What a decode of n_units = B * Hkv units has in a block's shared memory: the teams of warps that
+ * work side by side (0: the codebooks do not fit) and, per tier slot, the copies of its codebook
+ * (two spread the centroid reads over the banks).  Host only.  Returns the bytes, or an error < 0. */
+int sphkv_decode_smem(const sphkv_tiers* tiers, int32_t dh, int32_t n_units, int32_t* teams, int32_t* copies);
 /* Two launches on `stream`: the split-K decode kernel and the merge kernel.  The decode kernel is
  * launched with programmatic stream serialization: its CTAs may become resident while the kernel
  * before it in the stream is still running, but it reads and writes no global memory before that

@@ -103,6 +103,7 @@ SIGNATURES = {
                                      C.c_void_p]),
     "sphkv_encode_scratch_bytes": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32]),
     "sphkv_decode_scratch_bytes": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "sphkv_decode_smem": (C.c_int, [C.POINTER(Tiers), C.c_int32, C.c_int32, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]),
     "sphkv_decode_paged": (C.c_int, [C.POINTER(DecodeParams), C.c_void_p]),
     "sphkv_decode_paged_static": (C.c_int, [C.POINTER(DecodeParams), C.c_void_p]),
     "sphkv_merge_partials": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,

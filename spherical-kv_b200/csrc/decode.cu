@@ -377,6 +377,24 @@ static int smem_cb_layout(const sphkv_tiers& t, int dh, int budget_bytes, int* o
   return off;
 }
 
+// all that a block can have: the decode kernel's 512 threads launch with every register of an SM, so its blocks never
+// share one with the merge blocks of the step before, and overlap with them on the SMs that have none
+constexpr int kSmemMax = 227 * 1024;
+
+// Shared memory of a decode: as many teams as fit beside every codebook and the block prefix (0: not one), then the copies of
+// codebooks that still do.  Returns the bytes.
+static int plan_smem(const sphkv_tiers& t, int dh, int n_units, int& teams, int* offs, int* dup, int& cb_bytes) {
+  const int pfx_bytes = n_units <= kMaxUnitsInKernelPlan ? (n_units + 1) * 4 : 0;
+  int bytes = 0;
+  for (teams = kTeams; teams >= 1; --teams) {
+    const int fixed_bytes = smem_fixed_bytes(dh, teams) + pfx_bytes;
+    cb_bytes = smem_cb_layout(t, dh, kSmemMax - fixed_bytes, offs, dup);
+    bytes = fixed_bytes + cb_bytes;
+    if (bytes <= kSmemMax) break;
+  }
+  return bytes;
+}
+
 int validate_tiers(const sphkv_tiers& t, int dh) {
   SPHKV_REQUIRE(t.n_slots >= 1 && t.n_slots <= SPHKV_MAX_TIER_SLOTS, SPHKV_E_ARG,
                 "tiers.n_slots=%d outside 1..%d", t.n_slots, SPHKV_MAX_TIER_SLOTS);
@@ -495,6 +513,17 @@ extern "C" int64_t sphkv_decode_scratch_bytes(int32_t B, int32_t Hkv, int32_t dh
   return prefix_bytes(n_units) + (int64_t)(n_ctas + n_units) * 8 * (dh + 2) * 4;
 }
 
+extern "C" int sphkv_decode_smem(const sphkv_tiers* tiers, int32_t dh, int32_t n_units, int32_t* teams, int32_t* copies) {
+  SPHKV_REQUIRE(tiers && teams && copies, SPHKV_E_ARG, "decode_smem: NULL pointer");
+  SPHKV_REQUIRE((dh == 64 || dh == 128) && n_units > 0, SPHKV_E_ARG, "decode_smem: dh=%d units=%d", dh, n_units);
+  if (int rc = validate_tiers(*tiers, dh)) return rc;
+  int offs[SPHKV_MAX_TIER_SLOTS], dup[SPHKV_MAX_TIER_SLOTS], cb_bytes = 0, n = 0;
+  const int bytes = plan_smem(*tiers, dh, n_units, n, offs, dup, cb_bytes);
+  *teams = n;
+  for (int s = 0; s < tiers->n_slots; ++s) copies[s] = 1 + dup[s];
+  return bytes;
+}
+
 extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
   SPHKV_REQUIRE(pp != nullptr, SPHKV_E_ARG, "decode: params is NULL");
   const sphkv_decode_params& p = *pp;
@@ -556,17 +585,7 @@ extern "C" int sphkv_decode_paged(const sphkv_decode_params* pp, void* stream) {
   a.n_ctas = min(a.n_ctas, 0xFFFF);  // a span packs two CTA counts into a word
   a.wide = ((reinterpret_cast<uintptr_t>(p.k_pages) | reinterpret_cast<uintptr_t>(p.positions)) & 15) == 0;
   a.plan_in_kernel = a.n_units <= kMaxUnitsInKernelPlan ? 1 : 0;
-  const int pfx_bytes = a.plan_in_kernel ? (a.n_units + 1) * 4 : 0;
-  // all that a block can have: this kernel's 512 threads launch with every register of an SM, so its blocks never
-  // share one with the merge blocks of the step before, and overlap with them on the SMs that have none
-  constexpr int kSmemMax = 227 * 1024;
-  int smem_bytes = 0;
-  for (a.teams = kTeams; a.teams >= 1; --a.teams) {
-    const int fixed_bytes = smem_fixed_bytes(p.dh, a.teams) + pfx_bytes;
-    a.cb_smem_bytes = smem_cb_layout(p.tiers, p.dh, kSmemMax - fixed_bytes, a.cb_smem_off, a.cb_dup);
-    smem_bytes = fixed_bytes + a.cb_smem_bytes;
-    if (smem_bytes <= kSmemMax) break;
-  }
+  const int smem_bytes = plan_smem(p.tiers, p.dh, a.n_units, a.teams, a.cb_smem_off, a.cb_dup, a.cb_smem_bytes);
   SPHKV_REQUIRE(a.teams >= 1, SPHKV_E_LIMIT,
                 "decode: codebooks need %d B of shared memory (limit %d)", smem_bytes, kSmemMax);
   if (int rc = make_v_map(&a.v_map, p)) return rc;

@@ -58,21 +58,24 @@ struct DecodeArgs {
   float* rows;  // [(n_ctas + n_units)][8][dh + 2]
 };
 
-// shared-memory carve-up, shared by host and device: query operand; per team barriers, votes and statistics, two words of the
-// CTA; per team in use V tiles, weights, K stages, metadata; then codebooks and the block prefix.  Everything a team
-// touches per tile lies at a constant offset from two bases: addresses that depended on the number of teams
-// were made again at every use, 110 of 750 instructions a tile.
-constexpr int kSmemQ = 128 / 16 * 512;
-constexpr int kBarStride = 128, kSmemTeamBars = kBarStride + 32 + 128 + 256 + 32;
-constexpr int kSmemHead = (kSmemQ + kTeams * kSmemTeamBars + 16 + 1023) / 1024 * 1024;
+// shared-memory carve-up, shared by host and device: query operand; per team barriers, votes and reference maxima, two words of
+// the CTA; per team in use V tiles, weights, K stages, metadata; per team in use statistics; then codebooks and the block
+// prefix.  Everything a team touches per tile lies at a constant offset from two bases: addresses that depended on the number
+// of teams were made again at every use, 110 of 755 instructions a tile.  The statistics are read at a merge only, and
+// behind the teams they leave the rest of the head 1024 bytes: a byte more here is a byte less for teams and codebook copies.
+constexpr int kBarStride = 96, kSmemTeamBars = kBarStride + 32 + 128 + 32;
+constexpr int kSmemStats = 256;  // per team
 __host__ __device__ constexpr int smem_q_bytes(int dh) { return dh / 16 * 512; }
+__host__ __device__ constexpr int smem_head_bytes(int dh) { return smem_q_bytes(dh) + 1024; }
+static_assert(kTeams * kSmemTeamBars + 16 <= 1024, "barrier block");
 __host__ __device__ constexpr int smem_v_bytes(int dh) { return kMacroTiles * 16 * dh * 2; }
 constexpr int kSmemP = kMacroTiles * 512;
 constexpr int kSmemK = 3 * kMacroTiles * 384;  // (f16 radii: 2 x 512)
 constexpr int kSmemMeta = kMetaRing * 16;
 __host__ __device__ constexpr int smem_team_bytes(int dh) { return smem_v_bytes(dh) + kSmemP + kSmemK + kSmemMeta; }
-static_assert(smem_team_bytes(64) % 1024 == 0 && smem_team_bytes(128) % 1024 == 0, "V tiles start on 1024 bytes");
-__host__ __device__ constexpr int smem_fixed_bytes(int dh, int teams) { return kSmemHead + teams * smem_team_bytes(dh); }
+static_assert(smem_team_bytes(64) % 1024 == 0 && smem_team_bytes(128) % 1024 == 0 && smem_head_bytes(64) % 1024 == 0 &&
+                  smem_head_bytes(128) % 1024 == 0, "V tiles start on 1024 bytes");
+__host__ __device__ constexpr int smem_fixed_bytes(int dh, int teams) { return smem_head_bytes(dh) + teams * (smem_team_bytes(dh) + kSmemStats); }
 // room for the group shifts of a slot's codebook (see stage_codebooks)
 constexpr int kCbShift = 128;
 
@@ -265,16 +268,16 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
 
   const uint32_t smem0 = smem_u32(smem);
   const uint32_t q_u32 = smem0;
-  const uint32_t bar = smem0 + kSmemQ + team * kSmemTeamBars;
+  const uint32_t bar = smem0 + smem_q_bytes(DH) + team * kSmemTeamBars;
   const uint32_t votes = bar + kBarStride;   // [2][4 warps]
   const uint32_t wmax = votes + 32;          // [4 warps][8 heads]
   // of a team: [4 warps][8 heads] (sum, true maximum), [8 heads] reference maximum
-  auto stats_of = [&](int t) { return reinterpret_cast<float*>(smem + kSmemQ + t * kSmemTeamBars + kBarStride + 32 + 128); };
-  auto mref_of = [&](int t) { return stats_of(t) + 64; };
-  volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + kSmemQ + kTeams * kSmemTeamBars);
-  const uint32_t v_buf = keep(kKeepBases, smem0 + kSmemHead + team * smem_team_bytes(DH));
+  auto stats_of = [&](int t) { return reinterpret_cast<float*>(smem + smem_head_bytes(DH) + a.teams * smem_team_bytes(DH) + t * kSmemStats); };
+  auto mref_of = [&](int t) { return reinterpret_cast<float*>(smem + smem_q_bytes(DH) + t * kSmemTeamBars + kBarStride + 32 + 128); };
+  volatile uint32_t* shared_words = reinterpret_cast<volatile uint32_t*>(smem + smem_q_bytes(DH) + kTeams * kSmemTeamBars);
+  const uint32_t v_buf = keep(kKeepBases, smem0 + smem_head_bytes(DH) + team * smem_team_bytes(DH));
   const uint32_t p_buf = v_buf + smem_v_bytes(DH), k_ring = p_buf + kSmemP, meta = k_ring + kSmemK;
-  const uint32_t cb_off = kSmemHead + a.teams * smem_team_bytes(DH);
+  const uint32_t cb_off = smem_fixed_bytes(DH, a.teams);
 
   // ---- set-up: barriers, tensor memory, the zero columns of the weights and of the query operand ----
   if (driver && in_use && lane == 0) {
@@ -1111,7 +1114,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
     // ---- merge the teams of this CTA and write one partial row.  The accumulators [HEADS][DH] go where the
     //      weights were (the first eight columns of a packed tile: the zero columns stay) ----
     auto acc_at = [&](int t, int e) -> float* {
-      return reinterpret_cast<float*>(smem + kSmemHead + t * smem_team_bytes(DH) + smem_v_bytes(DH) + (PACK ? (e >> 6) * 512 + (e & 63) * 4 : e * 4));
+      return reinterpret_cast<float*>(smem + smem_head_bytes(DH) + t * smem_team_bytes(DH) + smem_v_bytes(DH) + (PACK ? (e >> 6) * 512 + (e & 63) * 4 : e * 4));
     };
     if (in_use) {
       const int w = warp & 3;

@@ -28,6 +28,16 @@ def test_decode_segment_shapes(B, Hkv, dh, ctx, page, specs, fr, radius_fmt):
     check_against_oracle(cache, cbs, Q, ctx, dh)
 
 
+# batch x KV heads and tier sets at which one, two or three teams and one or two copies of a codebook just fit shared memory
+@pytest.mark.parametrize("B,Hkv,dh,ctx,bits", [
+    (16, 8, 128, 150, (6, 6, 6, 6)), (16, 8, 128, 100, (6, 6, 6)), (75, 2, 128, 100, (6, 6, 5, 2)), (80, 8, 128, 40, (6, 4)),
+    (24, 8, 128, 90, (6, 6, 6, 6)), (64, 8, 64, 70, (6, 6, 6, 6))])
+def test_decode_where_teams_and_copies_just_fit(B, Hkv, dh, ctx, bits):
+    specs = [pkg.TierSpec(i + 1, 16, b) for i, b in enumerate(bits)]
+    cache, cbs, K, V, Q, _ = build(B, 2 * Hkv, Hkv, dh, ctx, 16, specs, {t.tier_id: 0.9 / len(bits) for t in specs}, seed=ctx)
+    check_against_oracle(cache, cbs, Q, ctx, dh)
+
+
 def test_decode_many_partial_rows_and_idle_ctas():
     """more than 32 partial rows per unit (the merge's general path), and CTAs without a block"""
     cache, cbs, K, V, Q, _ = build(1, 4, 1, 128, 2300, 16, (T1, T2), {1: 0.3, 2: 0.6}, seed=3)
