@@ -22,8 +22,10 @@ constexpr int kListChunk = kListThreads * kListPer;   // tokens per CTA
 constexpr int kScanThreads = 1024;
 constexpr int kScanRuns = 1024;                       // runs whose token counts the scan keeps in shared memory
 // The four totals go to the host as words that carry the number of the call in their upper 16 bits, so that each
-// says by itself that it has arrived.
+// says by itself that it has arrived.  The byte total can need more than the other 48 (a large page_align): it stays at
+// their largest value then, which is refused like any pool past 32-bit offsets.
 constexpr int kTotalBits = 48;
+constexpr int64_t kTotalMax = (INT64_C(1) << kTotalBits) - 1;
 
 struct ListArgs {
   const void* assign;  // [U][T] tier ids
@@ -187,9 +189,10 @@ __global__ void __launch_bounds__(kScanThreads) list_scan_kernel(const ListArgs 
   if (threadIdx.x < 4) {  // the host polls these words
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) most = max(most, s_max[w]);
     const int64_t v = threadIdx.x == 0 ? c_pages : threadIdx.x == 1 ? most : threadIdx.x == 2 ? c_bundles : c_bytes + 16;
-    *reinterpret_cast<volatile int64_t*>(a.totals + threadIdx.x) = v | (int64_t)((uint64_t)a.call << kTotalBits);
+    *reinterpret_cast<volatile int64_t*>(a.totals + threadIdx.x) = min(v, kTotalMax) | (int64_t)((uint64_t)a.call << kTotalBits);
   }
 }
+
 // grid (chunk, unit): the chunk's tokens are compacted per tier slot in shared memory (order kept) and
 // written out in rank order, so neighbouring threads write neighbouring page slots; the unit's page
 // records are dealt out over its chunks' threads.
@@ -303,8 +306,8 @@ __global__ void __launch_bounds__(kScanThreads) list_offsets_kernel(const ListAr
   }
 }
 
-// The scan writes the four totals and a call number straight into pinned host memory: one small buffer per
-// calling thread, freed with it.
+// The scan writes the four totals straight into pinned host memory: one small buffer per calling thread, freed
+// with it.
 struct PinnedTotals {
   int64_t* p = nullptr;
   int64_t calls = 0;
@@ -399,7 +402,7 @@ extern "C" int sphkv_page_lists_count(const sphkv_page_lists_params* p, int64_t*
     set_error("page_lists_count: %s", e == cudaSuccess ? "the totals did not arrive" : cudaGetErrorString(e));
     return e == cudaSuccess ? (int)cudaErrorUnknown : (int)e;
   }
-  for (int i = 0; i < 4; ++i) totals[i] = host[i] & ((INT64_C(1) << kTotalBits) - 1);
+  for (int i = 0; i < 4; ++i) totals[i] = host[i] & kTotalMax;
   return 0;
 }
 

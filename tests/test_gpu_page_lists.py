@@ -46,6 +46,20 @@ def test_totals_of_each_call_and_tables_equal_host_construction(Hkv, T):
         want = pkg.build_page_lists(assign, tiers, 32)
 
 
+# 2^18 pages of 2^30 bytes and of the largest alignment, one page too many for 32-bit offsets, one that just fits
+@pytest.mark.parametrize("pages,align,fits", [(1 << 18, 1 << 30, False), (1 << 18, (1 << 31) - 4, False), (2, 1 << 30, False),
+                                              (1, (1 << 31) - 64, True)])
+def test_pools_past_32_bit_offsets_are_refused(pages, align, fits):
+    tiers = pkg.TierSet(128, pkg.REFERENCE_TIERS[:1])
+    assign = torch.ones(1, 1, 16 * pages, dtype=torch.uint8, device="cuda:0")
+    for _ in range(2):  # the totals' words carry an odd and an even call number
+        if fits:
+            assert pkg.build_page_lists(assign, tiers, 16, page_align=align).pool_bytes == align + 16
+        else:
+            with pytest.raises(ValueError, match="pointer-table offsets"):
+                pkg.build_page_lists(assign, tiers, 16, page_align=align)
+
+
 def test_page_lists_reject_empty_assignment():
     with pytest.raises(ValueError, match="no retained tokens"):
         pkg.build_page_lists(torch.zeros(1, 2, 50, dtype=torch.uint8, device="cuda:0"), pkg.TierSet(128), 16)
