@@ -168,8 +168,13 @@ def host_path() -> str:
     return os.path.join(HERE, "host_tables.%s.torch-%s.so" % (sys.implementation.cache_tag, torch.__version__))
 
 
+def host_built() -> bool:
+    """Whether the host module is there, for the callers that can do without."""
+    return _host is not None or os.path.exists(host_path())
+
+
 def host_tables():
-    """The module of csrc/host_tables.cpp; raises if it is missing (no fallback exists)."""
+    """The module of csrc/host_tables.cpp; raises if it is missing (the page tables have no other maker)."""
     global _host
     if _host is None:
         import importlib.util

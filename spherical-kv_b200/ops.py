@@ -55,13 +55,13 @@ def _new_cache(lists: PageLists, tiers: TierSet, codebooks: torch.Tensor, dh: in
     """A cache with pools for `lists`: zeroed, except a V pool of which the kernels write every slot (zeros included);
     then the addresses of its pools and of `scratch_bytes` bytes of scratch, kept with it."""
     zero_v = not (has_v and lists.encode_fills_pool())
-    if v_dtype is torch.bfloat16 or v_dtype is torch.float16:
+    if (v_dtype is torch.bfloat16 or v_dtype is torch.float16) and _lib.host_built():
         k_pages, v_pool, scratch, *at = _lib.host_tables().pools(
             -1 if dev.index is None else dev.index, lists.pool_bytes, lists.n_pages, lists.page_size, dh,
             v_dtype is torch.bfloat16, zero_v, scratch_bytes)
-    else:  # (refused by the library)
+    else:  # lists that were built on the host need no host module; other types are refused by the library
         k_pages = torch.zeros(lists.pool_bytes, dtype=torch.uint8, device=dev)
-        v_pool = torch.zeros(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev)
+        v_pool = (torch.zeros if zero_v else torch.empty)(lists.n_pages, lists.page_size, dh, dtype=v_dtype, device=dev)
         scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev) if scratch_bytes else None
         at = [k_pages.data_ptr(), v_pool.data_ptr(), 0 if scratch is None else scratch.data_ptr()]
     out = PagedCache(tiers=tiers, lists=lists, codebooks=codebooks, k_pages=k_pages, v_pool=v_pool, radius_fmt=radius_fmt)

@@ -45,6 +45,24 @@ def test_pools_and_their_addresses(bf16, zero_v, scratch):
     assert not (k.requires_grad or v.requires_grad)
 
 
+# with the module and without it
+@pytest.mark.parametrize("built", [True, False])
+@pytest.mark.parametrize("v_dtype,scratch", [(torch.bfloat16, 64), (torch.float16, 0)])
+def test_pools_of_host_built_lists_do_without_the_module(monkeypatch, built, v_dtype, scratch):
+    tiers = pkg.TierSet(128)
+    lists = pkg.build_page_lists(torch.ones(1, 2, 40, dtype=torch.uint8), tiers, 16)
+    if not built:
+        monkeypatch.setattr(torch, "__version__", "0.0.1")
+        monkeypatch.setattr(pkg._lib, "_host", None)
+    new_cache = pkg.encode_pages.__globals__["_new_cache"]
+    cache, at = new_cache(lists, tiers, torch.zeros(1), 128, False, v_dtype, 0, torch.device("cpu"), scratch)
+    assert cache.k_pages.numel() == lists.pool_bytes and not bool(cache.k_pages.any())
+    assert (cache.v_pool.dtype, tuple(cache.v_pool.shape)) == (v_dtype, (lists.n_pages, 16, 128)) and not bool(cache.v_pool.any())
+    s = cache.extra.get("encode_scratch")
+    assert (s is None) if not scratch else s.numel() == scratch
+    assert list(at) == [cache.k_pages.data_ptr(), cache.v_pool.data_ptr(), 0 if s is None else s.data_ptr()]
+
+
 def test_packed_parameters_are_the_struct_field_by_field():
     cls, C4 = pkg._lib.EncodeParams, pkg._lib.MAX_TIER_SLOTS
     assert cls._packer.size == C.sizeof(cls)
