@@ -9,6 +9,7 @@
 #include <ATen/ATen.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
 
 namespace {
 
@@ -36,7 +37,11 @@ PyObject* make(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   const at::AutoDispatchBelowADInplaceOrView plain;  // integer tables: nothing for autograd to follow
   const at::Device dev = v[1] < 0 ? at::Device(at::kCPU) : at::Device(at::kCUDA, (c10::DeviceIndex)v[1]);
-  const at::Tensor buf = at::empty({at[kTables]}, at::TensorOptions().dtype(at::kInt).device(dev));
+  at::Tensor buf;
+  {
+    const pybind11::gil_scoped_release no_gil;  // an allocation can wait for the device, and other threads go on
+    buf = at::empty({at[kTables]}, at::TensorOptions().dtype(at::kInt).device(dev));
+  }
   int32_t* base = buf.data_ptr<int32_t>();
   void** out = reinterpret_cast<void**>(static_cast<intptr_t>(v[0]));
   PyObject* tables = PyTuple_New(kTables);
@@ -72,10 +77,13 @@ PyObject* pools(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const at::Device dev = v[0] < 0 ? at::Device(at::kCPU) : at::Device(at::kCUDA, (c10::DeviceIndex)v[0]);
   const at::TensorOptions bytes = at::TensorOptions().dtype(at::kByte).device(dev);
   const at::TensorOptions vo = bytes.dtype(v[5] ? at::kBFloat16 : at::kHalf);
-  const at::Tensor k_pages = at::zeros({v[1]}, bytes);
-  const at::Tensor v_pool = v[6] ? at::zeros({v[2], v[3], v[4]}, vo) : at::empty({v[2], v[3], v[4]}, vo);
-  at::Tensor scratch;
-  if (v[7] > 0) scratch = at::empty({v[7]}, bytes);
+  at::Tensor k_pages, v_pool, scratch;
+  {
+    const pybind11::gil_scoped_release no_gil;  // as in make(); the zeroing is a launch, which waits where the queue is full
+    k_pages = at::zeros({v[1]}, bytes);
+    v_pool = v[6] ? at::zeros({v[2], v[3], v[4]}, vo) : at::empty({v[2], v[3], v[4]}, vo);
+    if (v[7] > 0) scratch = at::empty({v[7]}, bytes);
+  }
   auto address = [](const at::Tensor& t) { return (unsigned long long)reinterpret_cast<uintptr_t>(t.defined() ? t.data_ptr() : nullptr); };
   PyObject* k = THPVariable_Wrap(k_pages);
   PyObject* vp = THPVariable_Wrap(v_pool);

@@ -63,6 +63,30 @@ def test_pools_of_host_built_lists_do_without_the_module(monkeypatch, built, v_d
     assert list(at) == [cache.k_pages.data_ptr(), cache.v_pool.data_ptr(), 0 if s is None else s.data_ptr()]
 
 
+# A zeroed pool takes its time, at an allocation or a full launch queue more of it: other threads go on meanwhile.
+def test_other_threads_run_while_pools_are_made():
+    import threading
+    import time
+    pools = pkg._lib.host_tables().pools
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.wait(0.001):
+            ticks.append(time.monotonic())
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        begin = time.monotonic()
+        made = pools(-1, 1 << 30, 1, 16, 64, 1, 1, 0)
+        end = time.monotonic()
+    finally:
+        stop.set()
+        thread.join()
+    margin = (end - begin) / 8
+    assert any(begin + margin < t < end - margin for t in ticks), (end - begin, len(ticks), made[0].shape)
+
+
 def test_packed_parameters_are_the_struct_field_by_field():
     cls, C4 = pkg._lib.EncodeParams, pkg._lib.MAX_TIER_SLOTS
     assert cls._packer.size == C.sizeof(cls)
