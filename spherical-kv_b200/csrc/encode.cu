@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_bundle_kernel(const Encode
 // of row s is stored at chunk c ^ turn(s), so neither the copies nor the row-per-lane reads meet in a bank.
 // Not STAGED: slices off a 16-byte boundary.
 // TOK token slots per lane: 4 are a bundle; of few bundles a CTA takes a half or a quarter (blockIdx.y), so that all SMs
-// search (see the rule at the launch).
+// search (see search_parts).
 template <int GS, bool STAGED, int TOK>
 __global__ void __launch_bounds__(kEncThreads, GS == 16 ? 2 : 1) search_bundles_kernel(const EncodeArgs a) {
   const sphkv_encode_params& p = a.p;
@@ -1379,34 +1379,57 @@ int validate_tiers(const sphkv_tiers& t, int dh);
 
 using namespace sphkv;
 
+struct SearchSmem {
+  int codebook_bytes, bytes;
+  bool staged;
+};
+// Staged rows need aligned slices, and room beside a codebook tensor of any C_max (dh 128, four slots a lane: up to 326).
+static SearchSmem search_smem(const sphkv_encode_params& p, int tok) {
+  const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
+  const int cb_bytes = p.dh * p.tiers.C_max * 4, row_bytes = 32 * tok * p.dh * 4;
+  const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
+                      (p.k_head_stride * esize) % 16 == 0 && cb_bytes + row_bytes <= 227 * 1024;
+  return {cb_bytes, cb_bytes + (staged ? row_bytes : 0), staged};
+}
+
 template <int GS, int TOK>
 static int launch_search_parts(const EncodeArgs& a, int resident, cudaStream_t st) {
   static SmemOptIn opt_in[2];
   const sphkv_encode_params& p = a.p;
-  const int esize = p.k_dtype == SPHKV_F32 ? 4 : 2;
-  const int cb_bytes = p.dh * p.tiers.C_max * 4, row_bytes = p.dh / GS * 32 * TOK * GS * 4;
-  // staged rows need aligned slices, and room beside a codebook tensor of any C_max (dh 128, four slots a lane: up to 326)
-  const bool staged = (reinterpret_cast<uintptr_t>(p.k_src) & 15) == 0 && (p.k_row_stride * esize) % 16 == 0 &&
-                      (p.k_head_stride * esize) % 16 == 0 && cb_bytes + row_bytes <= 227 * 1024;
-  const int smem = cb_bytes + (staged ? row_bytes : 0);
-  auto kern = staged ? search_bundles_kernel<GS, true, TOK> : search_bundles_kernel<GS, false, TOK>;
-  if (int rc = ensure_dynamic_smem(opt_in[staged], (const void*)kern, smem, "encode search")) return rc;
+  const SearchSmem m = search_smem(p, TOK);
+  auto kern = m.staged ? search_bundles_kernel<GS, true, TOK> : search_bundles_kernel<GS, false, TOK>;
+  if (int rc = ensure_dynamic_smem(opt_in[m.staged], (const void*)kern, m.bytes, "encode search")) return rc;
   EncodeArgs b = a;
-  b.search_kbuf = cb_bytes;
+  b.search_kbuf = m.codebook_bytes;
   b.search_chunk = std::max(1, std::min(8, p.n_bundles / (resident * 4)));  // >= 4 chunks per CTA, <= 8 bundles each
   const int grid = std::max(1, std::min((p.n_bundles + b.search_chunk - 1) / b.search_chunk, resident));
-  (void)launch_overlapped(kern, dim3(grid, 4 / TOK), dim3(kEncThreads), smem, st, b);
+  (void)launch_overlapped(kern, dim3(grid, 4 / TOK), dim3(kEncThreads), m.bytes, st, b);
   return check_launch("search_bundles_kernel");
+}
+
+// Parts that a bundle is cut into while there are few: the search of one alone is half of the launch.  Cut, the CTAs may fill
+// four fifths of the chip: blocks of the assembly launch come in early, and where more CTAs leave a few SMs free they pile up
+// there (6 and 4 bits, 132 bundles in halves 28.1, without the early launch 22.1).  Quarters of 16-dim groups, two CTAs to
+// an SM while the codebooks leave the room, gain up to a full chip.  Encode, dh 128, 148 SMs, us whole / halves / quarters:
+//   16 dims, 6 bits      45 bundles 20.1 / 17.0 / 16.9, 73: 20.3 / 18.9 / 17.6, 86: 21.1 / 21.3 / 22.4, 118: 22.7 / 22.1 / 28.0, 130: 22.6 / 28.4 / 30
+//   6 and 4 bits         64 bundles 20.2 / 18.8 / 17.7, 96: 20.8 / 18.2 / 19.9, 109: 22.0 / 21.8 / 21.4, 132: 22.2 / 28.1 / 24.4
+//   6 bits, one CTA an SM (C_max 196)   32 bundles 20.3 / 16.9 / 15.4, 35: 20.2 / 16.7 / 20.1, 58: 20.3 / 17.7 / 20.5, 68: 20.2 / 24.1 / 22.6
+//   32 dims, 3 bits      31 bundles 13.6 / 12.0 / 12.0, 35: 13.4 / 11.9 / 13.2, 58: 13.6 / 12.7 / 11.8, 68: 13.9 / 17.7 / 13.9
+static int search_parts(const sphkv_encode_params& p, int gs, int sms) {
+  for (int parts = 4; parts >= 2; parts /= 2) {
+    const bool two = gs == 16 && 2 * (search_smem(p, 4 / parts).bytes + 1024) <= 228 * 1024;
+    const int64_t slots = sms * (two ? 2 : 1), ctas = (int64_t)parts * p.n_bundles;
+    if (parts == 4 && two ? ctas <= slots : 5 * ctas <= 4 * slots) return parts;
+  }
+  return 1;
 }
 
 template <int GS>
 static int launch_encode(const EncodeArgs& a, bool split, int smem_bytes, cudaStream_t st) {
   if (split) {
-    // Persistent: as many CTAs as are resident at once, each striding over chunks of bundles.  A CTA takes all 128 slots
-    // of a bundle, or a half or a quarter while that still leaves every CTA resident: few bundles leave SMs idle, and the
-    // search of one alone is half of the launch.  Lists and pages of 777 tokens x 8 heads (45 bundles, quarters): 59.4 -> 57.4 us.
-    const int resident = sm_count_current_device() * (GS == 16 ? 2 : 1);
-    const int parts = 4 * a.p.n_bundles <= resident ? 4 : 2 * a.p.n_bundles <= resident ? 2 : 1;
+    // persistent: as many CTAs as are resident at once, each striding over chunks of bundles
+    const int sms = sm_count_current_device(), resident = sms * (GS == 16 ? 2 : 1);
+    const int parts = search_parts(a.p, GS, sms);
     return parts == 4   ? launch_search_parts<GS, 1>(a, resident, st)
            : parts == 2 ? launch_search_parts<GS, 2>(a, resident, st)
                         : launch_search_parts<GS, 4>(a, resident, st);

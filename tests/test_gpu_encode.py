@@ -194,7 +194,7 @@ def test_encode_ties_and_near_ties_pick_the_chain_argmax(use_scratch):
 
 # bundles (of 128 slots) at the lines between quarters, halves and whole ones per CTA, on 148 SMs, for groups of 16 and of
 # 32 dims; keys off a 16-byte boundary take the kernel without staged rows
-@pytest.mark.parametrize("tier,bundles", [(1, 1), (1, 74), (1, 75), (2, 148), (2, 149), (3, 37), (3, 38), (3, 74), (3, 75)])
+@pytest.mark.parametrize("tier,bundles", [(1, 1), (1, 74), (1, 75), (2, 118), (2, 119), (2, 149), (3, 29), (3, 30), (3, 59), (3, 60), (3, 75)])
 @pytest.mark.parametrize("dtype,offset", [(torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)])
 def test_parts_of_bundles_give_the_fused_encoders_pages(tier, bundles, dtype, offset):
     dh, T = 128, 128 * bundles - 3
@@ -207,3 +207,44 @@ def test_parts_of_bundles_give_the_fused_encoders_pages(tier, bundles, dtype, of
     split = pkg.encode_pages(K, K, lists, cb, tiers)
     fused = pkg.encode_pages(K, K, lists, cb, tiers, use_scratch=False)
     assert torch.equal(split.k_pages, fused.k_pages) and torch.equal(split.v_pool, fused.v_pool)
+
+
+def replay_us(fn, calls=20):
+    stream, times = torch.cuda.Stream(), []
+    with torch.cuda.stream(stream):
+        for _ in range(3):
+            fn()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(calls):
+                fn()
+        for _ in range(9):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            graph.replay()
+            b.record(stream)
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3 / calls)
+    return min(times)
+
+
+# token counts (hundredths of 128 per SM) at which bundles in halves or quarters would leave a few SMs idle, and larger ones that
+# stay whole: fewer bundles take no longer (a fifth longer where every cut is taken whose CTAs are all resident)
+@pytest.mark.parametrize("tiers,heads,fewer,more", [((1, 2), 8, 85, 102), ((3,), 1, 47, 55), ((3,), 1, 49, 55)])
+def test_fewer_bundles_are_not_slower(tiers, heads, fewer, more):
+    dh, dev = 128, "cuda:0"
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    specs = [t for t in pkg.REFERENCE_TIERS if t.tier_id in tiers]
+    ts = pkg.TierSet(dh, specs)
+    g = torch.Generator(device=dev).manual_seed(2)
+    cb = ts.pack_codebooks([torch.randn(heads, dh // t.g, 1 << t.b_theta, t.g, generator=g, device=dev) for t in specs])
+    took = []
+    for share in (fewer, more):
+        T = 128 * (sms * share // 100) // heads
+        ids = torch.randint(len(tiers), (1, heads, T), generator=g, device=dev)
+        K = torch.randn(T, heads, dh, generator=g, device=dev)
+        lists = pkg.build_page_lists(torch.tensor(tiers, dtype=torch.uint8, device=dev)[ids], ts, 16)
+        cache = pkg.encode_pages(K, K, lists, cb, ts)
+        took.append(replay_us(lambda: (cache.k_pages.zero_(), pkg.encode_pages(K, K, lists, cb, ts, out=cache))))  # as without `out`
+    assert took[0] <= 1.1 * took[1], took
