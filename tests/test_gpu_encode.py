@@ -209,6 +209,31 @@ def test_parts_of_bundles_give_the_fused_encoders_pages(tier, bundles, dtype, of
     assert torch.equal(split.k_pages, fused.k_pages) and torch.equal(split.v_pool, fused.v_pool)
 
 
+# Bundles per SM at which 16- and 32-dim groups are searched in quarters both, in quarters and halves, in halves and whole, whole
+# both; three tiers of five heads in one list, heads of different lengths, bundles with missing pages
+@pytest.mark.parametrize("share,low,high", [(0.1, 0.0, 0.2), (0.3, 0.2, 0.4), (0.6, 0.5, 0.8), (1.1, 0.8, 1.5)])
+@pytest.mark.parametrize("dh,page,dtype,offset,c_max", [
+    (128, 16, torch.float32, 0, 64), (128, 32, torch.float16, 0, 80), (128, 128, torch.bfloat16, 1, 64),
+    (64, 16, torch.float16, 1, 64), (64, 32, torch.float32, 0, 64), (64, 128, torch.bfloat16, 0, 100)])
+def test_cut_and_whole_bundles_of_mixed_tiers_give_the_fused_encoders_pages(share, low, high, dh, page, dtype, offset, c_max):
+    Hkv, dev = 5, "cuda:0"
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    T = int(128 * (share * sms - 7.5) / (0.78 * Hkv))
+    tiers = pkg.TierSet(dh, pkg.REFERENCE_TIERS)
+    tiers.C_max = c_max
+    g = torch.Generator(device=dev).manual_seed(T + dh)
+    K = torch.randn(T * Hkv * dh + offset, generator=g, device=dev).to(dtype)[offset:].view(T, Hkv, dh)
+    cb = tiers.pack_codebooks([torch.randn(Hkv, dh // t.g, 1 << t.b_theta, t.g, generator=g, device=dev) for t in pkg.REFERENCE_TIERS])
+    assign = torch.tensor([0, 1, 1, 1, 2, 2, 2, 2, 3, 3], dtype=torch.uint8, device=dev)[torch.randint(10, (1, Hkv, T), generator=g, device=dev)]
+    assign[0, 3, T // 3:] = 0
+    lists = pkg.build_page_lists(assign, tiers, page)
+    assert low < lists.bundles.shape[0] / sms <= high
+    assert page == 128 or bool((lists.bundles[:, :128 // page] < 0).any())
+    split = pkg.encode_pages(K, K, lists, cb, tiers)
+    fused = pkg.encode_pages(K, K, lists, cb, tiers, use_scratch=False)
+    assert torch.equal(split.k_pages, fused.k_pages) and torch.equal(split.v_pool, fused.v_pool)
+
+
 def replay_us(fn, calls=20):
     stream, times = torch.cuda.Stream(), []
     with torch.cuda.stream(stream):

@@ -256,19 +256,28 @@ def test_importance_update_with_statistics_off_an_8_byte_boundary(page):
     pkg.check_status(cache)
 
 
-def test_encode_with_a_wide_codebook_tensor():
-    """codebook tensors of any C_max that the encoder takes: rows are staged beside the codebook while they fit"""
-    Hkv, T, dh = 2, 700, 128
+# Rows are staged beside the codebook tensor while they fit: up to C_max 422, 390 and 326 for bundles in quarters, in halves and
+# whole.  With such tensors an SM takes one CTA, and bundles are cut up to 0.2 and 0.4 of them per SM (`share`).
+@pytest.mark.parametrize("share,sizes", [(0.1, (64, 326, 327, 422, 423, 430)), (0.3, (64, 390, 391)), (0.6, (64, 326, 327))])
+def test_encode_with_a_wide_codebook_tensor(share, sizes):
+    """codebook tensors of any C_max that the encoder takes"""
+    Hkv, dh = 2, 128
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    T = int(128 * (share * sms - 2) / (0.8 * Hkv))
     K = torch.randn(T, Hkv, dh, generator=torch.Generator(device=DEV).manual_seed(4), device=DEV)
     assign = synth.make_tier_assign(1, Hkv, T, {1: 0.5, 2: 0.3}, seed=1, per_head=True).to(DEV)
     cbs = synth.make_codebooks(Hkv, dh, (T1, T2), seed=2)
     got = []
-    for c_max in (64, 326, 327, 430):
+    for c_max in sizes:
         tiers = pkg.TierSet(dh, (T1, T2))
         tiers.C_max = c_max
-        got.append(pkg.encode_pages(K, K, pkg.build_page_lists(assign, tiers, 16), tiers.pack_codebooks(cbs).to(DEV), tiers))
+        lists = pkg.build_page_lists(assign, tiers, 16)
+        assert share - 0.1 < lists.bundles.shape[0] / sms < share + 0.1
+        got.append(pkg.encode_pages(K, K, lists, tiers.pack_codebooks(cbs).to(DEV), tiers))
     for other in got[1:]:
         assert torch.equal(other.k_pages, got[0].k_pages) and torch.equal(other.v_pool, got[0].v_pool)
+    fused = pkg.encode_pages(K, K, lists, got[0].codebooks, got[0].tiers, use_scratch=False)
+    assert torch.equal(fused.k_pages, got[0].k_pages)
 
 
 def test_a_refused_size_does_not_fail_the_next_call():
