@@ -226,7 +226,7 @@ static_assert(kBarCount * 8 <= kBarStride, "barrier block");
 // keys in flight and nothing else, twelve team warps fit an SM (the mma.sync version it replaced: eight, at
 // 244 registers, and shuffles, ldmatrix and accumulator moves around both products).
 // Bound: instruction issue and the waits between the roles, not HBM.  A 96-bit, 32768-token, batch-8 layer
-// step, merge included, in a short loop: 159 -> 141 us (3.4 -> 3.8 TB/s of the bytes it has to read): 666
+// step, merge included, in a short loop: 159 -> 141 us (3.4 -> 3.8 TB/s of the bytes it has to read): 670
 // instructions a tile instead of 755, since team addresses lie at constant offsets and stay in registers (147), then
 // cos/sin past L1.
 // Lane map of the rebuild (lane = 4 r + j): rows r and r + 8 of a tile are the lane's two tokens; in each
@@ -796,7 +796,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 1) decode_splitk_kernel(const 
       // chunk's {cos x 4, sin x 4} (the table is L2 resident), issued for the next pass once this one
       // has used its own.  A row's lines are used whole by one load and not again: past the 30 KB of L1 that the
       // shared memory leaves (1 x 131072 88.5 -> 83.7 us, 8 x 32768 146.9 -> 141.0; the read-only path, without L1,
-      // 84.4 and 143.8).  Pages that are staged in pieces gain nothing (one of 424 tokens: 14.25 us, past L1 14.39)
+      // 84.4 and 143.8).  The other page formats still take the read-only path.  At 128 dims it costs them up to 4 %
+      // of a long context (read-only / past L1, 1 x 131072: 16-token f16 radii 115.1 / 111.1, 32-token pages 112.7 / 110.6,
+      // 128-token 110.5 / 107.7, with f16 radii 125.2 / 120.0; 8 x 32768: 162.6 / 160.1, 190.1 / 189.2, 187.2 / 186.5,
+      // 194.0 / 193.8), nothing at 64 dims (within 0.3 %) nor of a short one (424 tokens: 14.25 / 14.39)
       float4 cs[2][NCH][2];
       const float4* cs_src[2] = {nullptr, nullptr};  // this lane's pieces of the two table rows
       auto cs_rows = [&](uint32_t st) {              // positions of K stage `st`

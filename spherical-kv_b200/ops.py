@@ -20,10 +20,6 @@ _NO_CODES = (0,) * (2 * _lib.MAX_TIER_SLOTS)
 _stream = _lib.stream_ptr
 
 
-def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
-    return None if t is None else t.data_ptr()
-
-
 def _need_cuda(*ts: torch.Tensor) -> None:
     for t in ts:
         if t is not None and not (t.is_cuda and t.is_contiguous()):
